@@ -216,6 +216,7 @@ static void free_tables(Tables* t) {
     cudaFree(t->tw_S);
     cudaFree(t->tw_D);
     free_split(t);
+    dg_put(t->dg);
     delete[] t->h_off;
     delete t;
 }
@@ -311,6 +312,7 @@ static int do_fst(double* rdata, double* idata, double* rcoeffs, double* icoeffs
     TabRef tref_{base};
     Tables view = *base;
     view.split = nullptr;
+    view.dg = nullptr;  // the caller's own tables
     if (table) S2G_TRY(upload_table(base, table, 0, &view.fwd));  // null: the device's own table (on the fly)
     const size_t S = 2 * (size_t)bw, ng = S * S, nc = (size_t)bw * bw;
     const size_t need = 2 * rnd(ng) + 2 * rnd(nc) + rnd(4 * (size_t)bw) + f64_work_bytes(bw, 1, fmt) + 256;
@@ -344,6 +346,7 @@ static int do_inv_fst(double* rcoeffs, double* icoeffs, double* rdata, double* i
     TabRef tref_{base};
     Tables view = *base;
     view.split = nullptr;
+    view.dg = nullptr;  // the caller's own tables
     if (ttable) S2G_TRY(upload_table(base, ttable, 1, &view.inv));  // null: the device's own table
     const size_t S = 2 * (size_t)bw, ng = S * S, nc = (size_t)bw * bw;
     const size_t need = 2 * rnd(ng) + 2 * rnd(nc) + f64_work_bytes(bw, 1, fmt) + 256;
@@ -372,6 +375,7 @@ static int do_fzt(double* rdata, double* idata, double* rres, double* ires, int 
     TabRef tref_{base};
     Tables view = *base;
     view.split = nullptr;
+    view.dg = nullptr;  // the caller's own tables
     const size_t S = 2 * (size_t)bw, ng = S * S, nt = (size_t)table_size(0, bw);
     const size_t need = 2 * rnd(ng) + 2 * rnd(S) + rnd(nt) + rnd(4 * (size_t)bw) + f64_work_bytes(bw, 1, REAL) + 256;
     S2G_TRY(g_dscratch.s.ensure(need));
@@ -403,12 +407,13 @@ static int do_fzt(double* rdata, double* idata, double* rres, double* ires, int 
 }
 
 // t without Legendre tables (cutoff 0): the on-the-fly kernels.
-static int conv_device(const Tables* t, const double* dr, const double* di, const double* fr, const double* fi,
+static int conv_device(Tables* t, const double* dr, const double* di, const double* fr, const double* fi,
                        double* rr, double* ri, int batch, Scratch& scr, cudaStream_t st) {
     const bool fly = (t->cutoff == 0);
     const int bw = t->bw;
     const size_t nc = (size_t)bw * bw;
-    const size_t work = f64_work_bytes(bw, batch, REAL);
+    const size_t work = fly ? f64_work_bytes(bw, batch, REAL) : f64_plan_bytes(bw, batch, REAL, di || ri);
+    if (!fly) S2G_TRY(dg_prepare(t, st));
     const size_t need = 4 * rnd(nc * batch) + 2 * rnd(2 * (size_t)bw * batch) + work + 256;
     S2G_TRY(scr.ensure(need));
     Carve c{(char*)scr.ptr};
@@ -1040,7 +1045,7 @@ int s2g_plan_destroy(s2g_plan p) {
 
 size_t s2g_plan_workspace_size(s2g_plan p, int batch, int precision) {
     if (!p || batch < 1) return 0;
-    if (precision == S2G_PREC_FP64) return f64_work_bytes(p->bw, batch, COMPLEX) + 256;
+    if (precision == S2G_PREC_FP64) return f64_plan_bytes(p->bw, batch, COMPLEX, true) + 256;
     return split_work_bytes(p->bw, batch);
 }
 
@@ -1064,7 +1069,9 @@ int s2g_fst(s2g_plan p, const double* rdata, const double* idata, double* rcoeff
             DataFormat fmt, void* stream) {
     S2G_TRY(plan_check(p, batch, false, true));
     if (!rdata || !rcoeffs || !icoeffs || (fmt == COMPLEX && !idata)) return fail(S2G_ERR_ARG, "NULL argument");
-    S2G_TRY(p->work.ensure(f64_work_bytes(p->bw, batch, fmt)));
+    S2G_TRY(p->work.ensure(p->fly ? f64_work_bytes(p->bw, batch, fmt)
+                                  : f64_plan_bytes(p->bw, batch, fmt, idata != nullptr)));
+    if (!p->fly) S2G_TRY(dg_prepare(p->t, (cudaStream_t)stream));
     if (p->fly) return fst_f64_fly(p->t, rdata, idata, rcoeffs, icoeffs, batch, fmt, p->work.ptr, (cudaStream_t)stream);
     return fst_f64(p->t, rdata, idata, rcoeffs, icoeffs, batch, fmt, p->cutoff, p->work.ptr, (cudaStream_t)stream);
 }
@@ -1073,7 +1080,9 @@ int s2g_inv_fst(s2g_plan p, const double* rcoeffs, const double* icoeffs, double
                 DataFormat fmt, void* stream) {
     S2G_TRY(plan_check(p, batch, false, true));
     if (!rdata || !rcoeffs || !icoeffs || (fmt == COMPLEX && !idata)) return fail(S2G_ERR_ARG, "NULL argument");
-    S2G_TRY(p->work.ensure(f64_work_bytes(p->bw, batch, fmt)));
+    S2G_TRY(p->work.ensure(p->fly ? f64_work_bytes(p->bw, batch, fmt)
+                                  : f64_plan_bytes(p->bw, batch, fmt, idata != nullptr)));
+    if (!p->fly) S2G_TRY(dg_prepare(p->t, (cudaStream_t)stream));
     if (p->fly)
         return inv_fst_f64_fly(p->t, rcoeffs, icoeffs, rdata, idata, batch, fmt, p->work.ptr, (cudaStream_t)stream);
     return inv_fst_f64(p->t, rcoeffs, icoeffs, rdata, idata, batch, fmt, p->cutoff, p->work.ptr,
@@ -1167,7 +1176,8 @@ int s2g_plan_sync_status(s2g_plan p) {
     S2G_CUDA(cudaSetDevice(p->device));
     S2G_TRY(drain_host(p));
     S2G_CUDA(cudaDeviceSynchronize());
-    return split_device_status(p->t, 1);
+    const int r = split_device_status(p->t, 1), d = dg_status(p->t, 1);
+    return r != S2G_OK ? r : d;
 }
 
 // Host-buffer variants: chunks of the batch flow H2D (stream 0) -> compute (stream 1) -> D2H

@@ -1,0 +1,1530 @@
+// digit_gemm.cu -- FP64 transforms on the tensor cores.
+//
+// GB300 gives FP64 about 1.2 TFLOP/s and its FP16 tensor cores about 1900, so the FP64 path's two
+// contractions per direction (the row DFT and the Legendre transform) run as exact integer products:
+// every operand is a 55-bit fixed-point number relative to its row's (table) or column's (data)
+// largest value, written as seven balanced base-256 digits d in [-128, 127]; digits are exact in
+// FP16, their products and the FP32 sums of up to 2^24 / 2^14 of them are exact, and the digit
+// products of equal weight share one accumulator:
+//     sum_k T_k x_k = sum_g 256^-g sum_{a+b=g} sum_k d_a(T_k) d_b(x_k),   g <= 6
+// (products of weight 256^-7 and below are under 2^-54 of the operands' scale and are left out; the
+// scheme is Ozaki, Ogita, Oishi and Rump's error-free matrix product, Numer. Algorithms 59 (2012)).
+// Leading digits may take up to 256 (FP16 holds them): a data value, folds included, has 56 bits up to
+// K = 256 and 54 beyond, a table value 54 to 56, as many as keep the leading group's bound K d_0 d'_0 at
+// 2^22 (dg_table_bits).  A group's sum is exact while at most 2^24: by these bounds group 0 and 1 always
+// are; the others pass 2^24 only where the low digits of table and data agree in sign over almost the
+// whole K range.
+//
+// One MMA covers all data digits of a table digit: the data digits b = 0..6-a lie one after another
+// along N, so A = table digit a times B = [x_0 | ... | x_(6-a)] adds to the accumulator groups
+// a..6, which lie one after another along TMEM columns.  28 digit products take 7 MMAs per 16-deep
+// K step with N = 7 NT, 6 NT, ... NT columns.
+//
+// Four stages share one kernel (k_dg); D[row, column] with the table on the M side:
+//   F1  rows forward    row = order m        K = folded longitude    column = (field, latitude part)
+//   F2  Legendre fwd    row = degree l       K = latitude            column = (field, re / im)
+//   I1  Legendre inv    row = latitude j     K = degree              column = (field, re / im)
+//   I2  rows inverse    row = longitude      K = order               column = (field, latitude part)
+// F2 and I1 are the naive transform (naive.c:34-96) in every order: on the tensor cores its extra
+// multiply-adds cost less than the DCTs of the seminaive form would, and it is the better
+// conditioned of the two.  k_dg_fold turns samples into fixed point and takes the even and odd
+// parts in latitude (P(m,l) has one parity) and, for even B, twice in longitude (cos and sin, m even
+// and odd), so that each of F1's four tables is a quarter of the DFT matrix; k_dg_unfold undoes the
+// same after I2.  Between the stages the forward keeps integers (one scale per function).  COMPLEX
+// data are two real fields g + i h, combined per coefficient in F2's epilogue and split before I1.
+//
+#include <math.h>
+
+#include <map>
+#include <mutex>
+#include <vector>
+
+#include "s2g_common.cuh"
+#include "s2g_internal.h"
+#include "tc_sm103.cuh"
+
+namespace s2g {
+
+constexpr int kDigits = 7;
+constexpr int kDgThreads = 896;          // warp 0 tables, 1 MMA, 4-19 epilogue, 20-27 data digits
+constexpr int kDgProdWarps = 8;
+constexpr int kDgStagesA = 4;            // table ring: 16-deep K steps of 7 x 128 x 16 FP16
+constexpr uint32_t kDgABytes = kDigits * 128 * 32;
+constexpr uint32_t kDgBRing = 100352;    // data ring: as many K steps as fit
+constexpr int kDgMaxStagesB = 16;
+enum { kF1 = 0, kF2 = 1, kI1 = 2, kI2 = 3 };
+// REAL without imaginary arrays / REAL with them / COMPLEX
+enum { kReal = 0, kReal2 = 1, kCplx = 2 };
+
+// One M tile of a table: up to 128 rows.  Blobs hold, per 16-deep K step, the seven digits' r8 x 16
+// tiles in core-matrix order.
+struct DgTile {
+    int64_t off;      // byte offset of the first K step's blob
+    int ks;           // K steps
+    int row0, nrows;  // rows row0 .. row0 + nrows of the panel
+    int r8;           // rows stored (nrows rounded up to 8)
+    int qoff;         // row scales at q[qoff + row]
+    int m, t;         // F1, I2: first order, part (cos / sin); F2, I1: order, parity
+    int kind;         // F1, I2: fold (0..3 two longitude folds, 4, 5 one)
+    int zoff;         // F1, I2: the panel's place in a column of Z
+    int vb;           // bits of a data value
+    int tb;           // bits of a table value
+};
+
+struct DgArgs {
+    const DgTile* tiles;
+    const uint8_t* tab;
+    const short* q;            // table value = digits * 2^-q
+    int ntiles, ncolblk, col_major;
+    int B, S, N, ncols, mode;  // N functions as the caller counts them
+    int BP, RL;                // latitudes of a half row of X (B, made even); values of a column of Z
+    int vbz;                   // bits of Z's samples before folds
+    int tbz;                   // F2: bits of F1's table
+    const double* in_r;        // I1: coefficients
+    const double* in_i;
+    double* out_r;             // F2: coefficients
+    double* out_i;
+    void* X;                   // [field, part][m][t][BP]: integers (F1 -> F2) or doubles (I1 -> I2)
+    long long* Z;              // [field][t][j][RL]: folded samples (F1) or parts of samples (I2)
+    const uint32_t* ein;       // F1: exponents of the latitude pairs; I1: of the orders; I2: of the fields
+    const uint32_t* efield;    // F1, F2: exponents of the fields
+    uint32_t* emax;            // F1 writes, F2 reads: bits of X's rows; I1 writes: exponents of the fields
+    int* err;
+};
+
+__device__ __forceinline__ uint32_t dexp(double x) { return ((uint32_t)__double2hiint(x) >> 20) & 0x7ffu; }
+
+// x as an integer of unit 2^(em - 1022 - vb) (|x| < 2^(em - 1022)), rounded to nearest
+__device__ __forceinline__ long long dg_fix(double x, int em, int vb) {
+    const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+    int e = (hi >> 20) & 0x7ff;
+    uint32_t mh = hi & 0xfffffu;
+    if (e) mh |= 0x100000u;
+    else e = 1;
+    const unsigned long long mant = (((unsigned long long)mh << 32) | lo) << 3;
+    const int rs = min(em - e + 55 - vb, 63);
+    const long long v = (long long)(((mant >> rs) + 1) >> 1);
+    return (int)hi < 0 ? -v : v;
+}
+
+// Digit b (0 most significant) of the biased values u0, u1 as two FP16 numbers.
+template <int b>
+__device__ __forceinline__ uint32_t dg_digit2(unsigned long long u0, unsigned long long u1) {
+    if (b == 0) {  // the leading digit has 10 bits, biased by 512
+        const uint32_t t = (__byte_perm((uint32_t)(u0 >> 32), (uint32_t)(u1 >> 32), 0x7632) & 0x03ff03ffu) | 0x64006400u;
+        const __half2 d = __hsub2(*reinterpret_cast<const __half2*>(&t), __half2half2(__ushort_as_half(0x6600)));
+        return *reinterpret_cast<const uint32_t*>(&d);
+    }
+    constexpr int i = 6 - b;  // byte
+    const uint32_t w0 = i < 4 ? (uint32_t)u0 : (uint32_t)(u0 >> 32), w1 = i < 4 ? (uint32_t)u1 : (uint32_t)(u1 >> 32);
+    const uint32_t t = (__byte_perm(w0, w1, (i & 3) | ((4 + (i & 3)) << 8)) & 0x00ff00ffu) | 0x64006400u;  // 1024 + byte
+    const __half2 d = __hsub2(*reinterpret_cast<const __half2*>(&t), __half2half2(__ushort_as_half(0x6480)));  // - 1152
+    return *reinterpret_cast<const uint32_t*>(&d);
+}
+
+// Stores the seven digits of the pair (v0, v1) (columns k, k + 1 of row n of every digit's tile).
+template <int NT>
+__device__ __forceinline__ void dg_store2(uint8_t* dst, long long v0, long long v1) {
+    constexpr unsigned long long bias = 0x0200808080808080ull;
+    const unsigned long long u0 = (unsigned long long)v0 + bias, u1 = (unsigned long long)v1 + bias;
+    constexpr int step = NT * 32;  // bytes between digits
+    *(uint32_t*)(dst) = dg_digit2<0>(u0, u1);
+    *(uint32_t*)(dst + step) = dg_digit2<1>(u0, u1);
+    *(uint32_t*)(dst + 2 * step) = dg_digit2<2>(u0, u1);
+    *(uint32_t*)(dst + 3 * step) = dg_digit2<3>(u0, u1);
+    *(uint32_t*)(dst + 4 * step) = dg_digit2<4>(u0, u1);
+    *(uint32_t*)(dst + 5 * step) = dg_digit2<5>(u0, u1);
+    *(uint32_t*)(dst + 6 * step) = dg_digit2<6>(u0, u1);
+}
+
+// Accumulator groups (exact integers) -> their sum in units of group 5.  Adding 1.5 2^23 leaves an
+// integer below 2^22 in a float's low bits (full-rate adds; the conversion instruction runs at an eighth
+// of their rate and set the epilogue's pace); the biases are taken off once, modulo 2^64.
+__device__ __forceinline__ long long dg_sum(const uint32_t* a, int stride, uint32_t& odd) {
+    constexpr float M = 12582912.0f;
+    constexpr long long b = 0x4B400000ll;
+    int i[kDigits];
+#pragma unroll
+    for (int g = 0; g < 6; ++g) i[g] = __float_as_int(__uint_as_float(a[g * stride]) + M);
+    i[6] = __float_as_int(fmaf(__uint_as_float(a[6 * stride]), 0.00390625f, M));
+    uint32_t x = 0;
+#pragma unroll
+    for (int g = 0; g < kDigits; ++g) x |= (uint32_t)i[g] ^ 0x4b000000u;
+    odd |= x;
+    const long long lo = (long long)i[2] * (1 << 24) + (long long)i[3] * 65536 + (long long)i[4] * 256 + (long long)i[5] + i[6];
+    constexpr unsigned long long bias = ((unsigned long long)(b * 257) << 32) + (unsigned long long)(b * ((1 << 24) + 65536 + 256 + 2));
+    const unsigned long long hi = (unsigned long long)(uint32_t)(i[0] * 256 + i[1]) << 32;
+    return (long long)(hi + (unsigned long long)lo - bias);
+}
+// The same for groups of any size; dg_sum sets bits 23.. of `odd` where one is outside its range.
+__device__ __noinline__ long long dg_sum_big(float a0, float a1, float a2, float a3, float a4, float a5, float a6) {
+    const float a[kDigits] = {a0, a1, a2, a3, a4, a5, a6};
+    long long i[kDigits];
+#pragma unroll
+    for (int g = 0; g < kDigits; ++g) i[g] = __float2int_rn(a[g]);
+    return ((i[0] * 256 + i[1]) << 32) + i[2] * (1 << 24) + i[3] * 65536 + i[4] * 256 + i[5] + (i[6] >> 8);
+}
+
+// T 2^(eb - 1086) as a double, rounded to nearest; kDgNan in eb stands for a column that held an
+// infinity or a NaN.  dg_fast is free of branches, so that several run interleaved; where it sets
+// `bad` (NaN, overflow, subnormal results) dg_slow gives the value.
+constexpr int kDgNan = 1 << 20;
+__device__ __forceinline__ double dg_fast(long long T, int eb, bool& bad) {
+    const unsigned long long m0 = T < 0 ? (unsigned long long)-T : (unsigned long long)T;
+    const uint32_t mh = (uint32_t)(m0 >> 32), mw = mh ? mh : (uint32_t)m0;
+    const int lz = __clz((int)mw) + (mh ? 0 : 32), e = eb - lz;
+    const unsigned long long m = m0 << (lz & 63);
+    bad |= (m0 != 0 && (uint32_t)(e - 1) >= 2046u) || eb >= kDgNan / 2;
+    unsigned long long bits = ((unsigned long long)(uint32_t)((e - 1) << 20) << 32) + (m >> 11) + ((m >> 10) & 1);
+    bits = m0 ? bits : 0;
+    return __longlong_as_double((long long)(bits | ((unsigned long long)T & 0x8000000000000000ull)));
+}
+__device__ __noinline__ double dg_slow(long long T, int eb) {
+    if (eb >= kDgNan / 2) return __longlong_as_double(0x7ff8000000000000ll);
+    return T ? ldexp((double)T, eb - 1086) : 0.0;
+}
+// dg_fast's exponent of a column whose largest value has exponent field em
+__device__ __forceinline__ int dg_eb(uint32_t em, int base) { return em == 0x7ffu ? kDgNan : base + max((int)em, 1); }
+
+__device__ __forceinline__ void tm_ld8(uint32_t ta, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(ta));
+}
+__device__ __forceinline__ void tm_ld4(uint32_t ta, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(ta));
+}
+// Shared-memory descriptors of the digit tiles: LBO 128 B (K), SBO 256 B (rows), no swizzle; the high
+// word is the same for all.
+constexpr uint32_t kDescHi = (256u >> 4) | (1u << 14);
+__device__ __forceinline__ uint32_t dg_desc(const void* s) { return (tc::smem_u32(s) >> 4) | ((128u >> 4) << 16); }
+__device__ __forceinline__ void dg_mma(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "mov.b64 da, {%1, %5};\n\t"
+        "mov.b64 db, {%2, %5};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}\n" ::"r"(d),
+        "r"(a), "r"(b), "r"(idesc), "r"(acc), "n"(kDescHi)
+        : "memory");
+}
+__device__ __forceinline__ void tm_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// Eight of I2's sums are added: each gives up its last bits.
+constexpr int kDgOutShift = 2;
+
+// Waits for a phase, for about half a second at most; another role's failure ends the wait at once.
+__device__ __forceinline__ bool dg_wait(uint64_t* bar, uint32_t parity, volatile int* failed) {
+    if (tc::mbar_try_wait(bar, parity)) return true;
+    const long long t0 = clock64();
+    while (!tc::mbar_try_wait(bar, parity)) {
+        if (*failed) return false;
+        if (clock64() - t0 > 1000000000LL) {
+            *failed = 1;
+            return false;
+        }
+    }
+    return true;
+}
+
+// The same for a whole warp: every lane gets the same answer.
+__device__ __forceinline__ bool dg_wait_warp(uint64_t* bar, uint32_t parity, volatile int* failed) {
+    return __all_sync(0xffffffffu, dg_wait(bar, parity, failed));
+}
+
+// F2's columns keep the two fields of COMPLEX data together: column -> (field, part).
+__device__ __forceinline__ int dg_f2_field(const DgArgs& p, int col) {
+    if (p.mode == kReal) return col;
+    const int f = col >> 2, gh = (col >> 1) & 1;
+    return ((gh * p.N + f) << 1) | (col & 1);
+}
+
+// What one lane of a data warp needs of an item: its two columns (8 apart).
+template <int STAGE>
+struct DgLane {
+    const char* src[2];  // null: no such column
+    int par[2];          // F2: right shift; I1, I2: exponent
+    int n;               // K entries there are
+    int vb;
+};
+
+template <int STAGE>
+__device__ __forceinline__ void dg_lane(const DgArgs& p, const DgTile& tl, int col0, DgLane<STAGE>& L) {
+    L.vb = tl.vb;
+    const int B = p.B;
+    if constexpr (STAGE == kF1) L.n = tl.ks * 16;
+    if constexpr (STAGE == kF2) L.n = B;
+    if constexpr (STAGE == kI1) L.n = (B - tl.m - tl.t + 1) / 2;
+    if constexpr (STAGE == kI2) L.n = tl.kind < 4 ? (B + 1 - tl.m) / 2 : B;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        const int col = col0 + 8 * c;
+        L.src[c] = nullptr;
+        L.par[c] = 0;
+        if (col >= p.ncols) continue;
+        if constexpr (STAGE == kF1) {
+            L.src[c] = (const char*)(p.Z + (size_t)col * p.RL + tl.zoff);
+        } else if constexpr (STAGE == kF2) {
+            const size_t row = (size_t)dg_f2_field(p, col) * B + tl.m;
+            L.src[c] = (const char*)((const long long*)p.X + row * 2 * p.BP + tl.t * p.BP);
+            L.par[c] = max((int)p.emax[row] - tl.vb, 0);
+        } else if constexpr (STAGE == kI1) {
+            const double* x = (col & 1) ? p.in_i : p.in_r;
+            if (tl.m || !(col & 1))  // a real field's Im f(l, 0) is ignored
+                L.src[c] = (const char*)(x + (size_t)(col >> 1) * B * B + index_of_harmonic_coeff(tl.m, tl.m + tl.t, B));
+            L.par[c] = max((int)p.ein[(size_t)col * B + tl.m], 1);
+        } else {
+            const int f = col / p.S, rem = col - f * p.S, t = rem >= B, j = rem - t * B;
+            L.src[c] = (const char*)((const double*)p.X + ((size_t)(f * 2 + tl.t) * B + tl.m) * 2 * p.BP + t * p.BP + j);
+            L.par[c] = max((int)p.ein[f], 1);
+        }
+    }
+}
+
+// Loads entries k, k + 1 of column c.
+template <int STAGE>
+__device__ __forceinline__ longlong2 dg_load(const DgArgs& p, const DgTile& tl, const DgLane<STAGE>& L, int c, int k) {
+    longlong2 v = make_longlong2(0, 0);
+    if (!L.src[c] || k >= L.n) return v;
+    if constexpr (STAGE == kF1) {
+        v = *((const longlong2*)L.src[c] + (k >> 1));
+    } else if constexpr (STAGE == kF2) {
+        v = *((const longlong2*)L.src[c] + (k >> 1));  // rows have an even length
+        if (k + 1 >= L.n) v.y = 0;
+    } else {
+        const size_t step = STAGE == kI1 ? 2 : (size_t)(tl.kind < 4 ? 2 : 1) * 2 * p.BP;
+        const long long* x = (const long long*)L.src[c];
+        v.x = __ldg(x + step * k);
+        if (k + 1 < L.n) v.y = __ldg(x + step * (k + 1));
+    }
+    return v;
+}
+
+// Raw entry -> integer of at most vb bits.
+template <int STAGE>
+__device__ __forceinline__ long long dg_conv(const DgLane<STAGE>& L, int c, long long v) {
+    if constexpr (STAGE == kF1) return v;
+    if constexpr (STAGE == kF2) return L.par[c] ? ((v >> (L.par[c] - 1)) + 1) >> 1 : v;
+    return dg_fix(__longlong_as_double(v), L.par[c], L.vb);
+}
+
+template <int STAGE, int NT>
+__global__ void __launch_bounds__(kDgThreads, 1) k_dg(DgArgs p) {
+    extern __shared__ __align__(1024) uint8_t dsm[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)dsm + 1023) & ~(uintptr_t)1023);
+    __shared__ uint64_t fullA[kDgStagesA], emptyA[kDgStagesA], fullB[kDgMaxStagesB], emptyB[kDgMaxStagesB];
+    __shared__ uint64_t accFull[2], accEmpty[2], drained;
+    __shared__ uint32_t tmem_slot;
+    __shared__ volatile int failed;
+    constexpr uint32_t accCols = kDigits * NT;        // TMEM columns of one accumulator
+    constexpr int kSlots = NT == 64 ? 1 : 2;          // accumulators
+    constexpr int kEpi = 4 / kSlots, kCols = NT / kEpi;  // epilogue groups of an accumulator, columns of each
+    constexpr uint32_t stageB = kDigits * NT * 32;    // bytes of one K step's data digits
+    constexpr int nsb = kDgBRing / stageB < kDgMaxStagesB ? kDgBRing / stageB : kDgMaxStagesB;
+    constexpr int W = NT / 16;                        // data warps per K step
+    constexpr int groups = kDgProdWarps / W;
+    uint8_t* ringA = smem;
+    uint8_t* ringB = smem + kDgStagesA * kDgABytes;
+    const uint32_t sdA0 = dg_desc(ringA), sdB0 = dg_desc(ringB);
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        failed = 0;
+        for (int i = 0; i < kDgStagesA; ++i) tc::mbar_init(&fullA[i], 1), tc::mbar_init(&emptyA[i], 1);
+        for (int i = 0; i < nsb; ++i) tc::mbar_init(&fullB[i], W), tc::mbar_init(&emptyB[i], 1);
+        for (int i = 0; i < 2; ++i) tc::mbar_init(&accFull[i], 1), tc::mbar_init(&accEmpty[i], kEpi * 4);
+        tc::mbar_init(&drained, 1);
+        tc::fence_mbar_init();
+    }
+    if (warp == 0) tc::tmem_alloc(&tmem_slot, 512);
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    const int nitems = p.ntiles * p.ncolblk;
+    auto decode = [&](int it, int& tile, int& cb) {
+        if (p.col_major) cb = it / p.ntiles, tile = it - cb * p.ntiles;
+        else tile = it / p.ncolblk, cb = it - tile * p.ncolblk;
+    };
+
+    if (warp == 0) {
+        if (lane == 0) {  // table digits
+            uint32_t c = 0;
+            bool ok = true;
+            for (int it = blockIdx.x; it < nitems && ok; it += gridDim.x) {
+                int tile, cb;
+                decode(it, tile, cb);
+                const DgTile* tl = p.tiles + tile;
+                const uint32_t bytes = kDigits * (uint32_t)tl->r8 * 32;
+                const uint8_t* src = p.tab + tl->off;
+                const int n = tl->ks;
+                for (int k = 0; k < n; ++k, ++c) {
+                    const uint32_t slot = c % kDgStagesA;
+                    if (!dg_wait(&emptyA[slot], ((c / kDgStagesA) & 1) ^ 1, &failed)) {
+                        ok = false;
+                        break;
+                    }
+                    tc::mbar_arrive_expect_tx(&fullA[slot], bytes);
+                    tc::bulk_g2s(ringA + slot * kDgABytes, src + (size_t)k * bytes, bytes, &fullA[slot]);
+                }
+            }
+            if (!ok)  // own copies still in flight land before the block ends
+                for (uint32_t b = c >= kDgStagesA ? c - kDgStagesA : 0; b < c; ++b)
+                    tc::mbar_wait(&fullA[b % kDgStagesA], (b / kDgStagesA) & 1);
+        }
+    } else if (warp == 1) {
+        // MMAs: the whole warp runs the loop (its values stay warp-uniform), one elected lane issues
+        const bool leader = tc::elect_one();
+        uint32_t sa = 0, pa = 0, sb = 0, pb = 0, use[2] = {0, 0}, nit = 0;
+        bool ok = true;
+        for (int it = blockIdx.x; it < nitems && ok; it += gridDim.x, ++nit) {
+            int tile, cb;
+            decode(it, tile, cb);
+            const DgTile* tl = p.tiles + tile;
+            const uint32_t stepA = (uint32_t)__shfl_sync(0xffffffffu, tl->r8, 0) * 2;  // descriptor units of 16 B
+            const int n = __shfl_sync(0xffffffffu, tl->ks, 0);
+            const int s0 = kSlots == 1 ? 0 : (int)(nit & 1);
+            ok = dg_wait_warp(&accEmpty[s0], (use[s0]++ & 1) ^ 1, &failed);
+            tc::tc_fence_after();
+            const uint32_t d0 = tmem + s0 * accCols;
+            for (int k = 0; k < n && ok; ++k) {
+                ok = dg_wait_warp(&fullA[sa], pa, &failed) && dg_wait_warp(&fullB[sb], pb, &failed);
+                if (!ok) break;
+                tc::tc_fence_after();
+                if (leader) {
+                    const uint32_t da = sdA0 + sa * (kDgABytes >> 4), db = sdB0 + sb * (stageB >> 4);
+#pragma unroll
+                    for (int a = 0; a < kDigits; ++a) {
+                        // groups a .. 6; an MMA takes at most 256 columns
+                        constexpr uint32_t one = 1;
+                        const uint32_t acc = a > 0 ? one : (uint32_t)(k > 0);
+                        const int n1 = (kDigits - a) * NT, parts = n1 > 256 ? 2 : 1, np = n1 / parts;
+                        const uint32_t idesc = tc::idesc_f16_f32(128, np);
+#pragma unroll
+                        for (int h = 0; h < parts; ++h)
+                            dg_mma(d0 + a * NT + h * np, da + a * stepA, db + h * np * 2, idesc, acc);
+                    }
+                    tc::mma_commit(&emptyA[sa]);
+                    tc::mma_commit(&emptyB[sb]);
+                }
+                if (++sa == kDgStagesA) sa = 0, pa ^= 1;
+                if (++sb == nsb) sb = 0, pb ^= 1;
+            }
+            if (ok && leader) tc::mma_commit(&accFull[s0]);
+        }
+        if (!ok && leader) {  // MMAs already issued end before the block gives up its memory
+            tc::mma_commit(&drained);
+            tc::mbar_wait(&drained, 0);
+        }
+    } else if (warp >= 20) {  // data digits
+        const int pw = warp - 20, g = pw / W, wi = pw - g * W;
+        // this group's K steps: every groups-th of the block's; the next one's values are loaded
+        // before the current one is turned into digits
+        struct Step {
+            DgLane<STAGE> L;
+            longlong2 v[4];
+        };
+        int it = blockIdx.x, ks = 0, tile, cb;
+        uint32_t c = 0;
+        DgTile tl{};
+        DgLane<STAGE> L{};
+        auto enter = [&]() {  // per-item state
+            decode(it, tile, cb);
+            tl = p.tiles[tile];
+            dg_lane<STAGE>(p, tl, cb * NT + wi * 16 + (lane >> 2), L);
+        };
+        auto skip = [&](int n) {  // n K steps on; false past the last item
+            ks += n;
+            c += n;
+            bool moved = false;
+            while (it < nitems && ks >= tl.ks) {
+                ks -= tl.ks;
+                it += gridDim.x;
+                moved = true;
+                if (it < nitems) {
+                    int t2, c2;
+                    decode(it, t2, c2);
+                    tl.ks = p.tiles[t2].ks;
+                }
+            }
+            if (it >= nitems) return false;
+            if (moved) enter();
+            return true;
+        };
+        auto fetch = [&](Step& st) {
+            st.L = L;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                st.v[q] = dg_load<STAGE>(p, tl, L, q >> 1, ks * 16 + ((q & 1) ^ (lane >> 4)) * 8 + (lane & 3) * 2);
+        };
+        bool more = it < nitems;
+        if (more) {
+            enter();
+            more = skip(g);
+        }
+        Step cur{};
+        if (more) fetch(cur);
+        while (more) {
+            const uint32_t cc = c;
+            more = skip(groups);
+            Step nxt{};
+            if (more) fetch(nxt);
+            const uint32_t slot = cc % nsb;
+            if (!dg_wait_warp(&emptyB[slot], ((cc / nsb) & 1) ^ 1, &failed)) break;
+            uint8_t* dst = ringB + slot * stageB;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int r = wi * 16 + (q >> 1) * 8 + (lane >> 2);  // column of the item
+                dg_store2<NT>(dst + (r >> 3) * 256 + ((q & 1) ^ (lane >> 4)) * 128 + (r & 7) * 16 + (lane & 3) * 4,
+                              dg_conv<STAGE>(cur.L, q >> 1, cur.v[q].x), dg_conv<STAGE>(cur.L, q >> 1, cur.v[q].y));
+            }
+            tc::fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&fullB[slot]);
+            cur = nxt;
+        }
+    } else if (warp >= 4) {  // epilogue
+        const int slot = kSlots == 1 ? 0 : (warp - 4) >> 3, grp = ((warp - 4) >> 2) % kEpi, ew = warp & 3;
+        const uint32_t lane_off = (uint32_t)(ew * 32) << 16;
+        const int B = p.B, S = p.S;
+        uint32_t nit = 0, use = 0;
+        for (int it = blockIdx.x; it < nitems; it += gridDim.x, ++nit) {
+            if (kSlots == 2 && (int)(nit & 1) != slot) continue;
+            int tile, cb;
+            decode(it, tile, cb);
+            const DgTile tl = p.tiles[tile];
+            const int r = ew * 32 + lane;
+            const bool live = r < tl.nrows;
+            const int row = tl.row0 + r;
+            const int qrow = live ? p.q[tl.qoff + row] : 0;
+            const int colb = cb * NT + grp * kCols;
+            const int ncol = min(kCols, p.ncols - colb);  // may be negative
+            // lane c holds what the rows need to know of column c: field, place in X, exponent or shift
+            int cfield = 0, cpar = 0;
+            uint32_t coff = 0;
+            if (lane < ncol) {
+                const int col = colb + lane;
+                if constexpr (STAGE == kF1) {
+                    cfield = col / S;
+                    const int rem = col - cfield * S, t = rem >= B, j = rem - t * B;
+                    cpar = min(max((int)p.efield[cfield], 1) - max((int)p.ein[cfield * B + j], 1), 63);
+                    coff = (uint32_t)(cfield * 2 + tl.t) * B * 2 * p.BP + t * p.BP + j;
+                } else if constexpr (STAGE == kF2) {
+                    const int fp = dg_f2_field(p, col);
+                    cpar = dg_eb(p.efield[fp >> 1], 176 - p.tbz - p.vbz + max((int)p.emax[(size_t)fp * B + tl.m] - tl.vb, 0));
+                } else if constexpr (STAGE == kI1) {
+                    cpar = dg_eb(p.ein[(size_t)col * B + tl.m], 120 - tl.vb);
+                }
+            }
+            if (!dg_wait_warp(&accFull[slot], use & 1, &failed)) break;
+            ++use;
+            tc::tc_fence_after();
+            const uint32_t tb = tmem + lane_off + slot * accCols + grp * kCols;
+            constexpr int CH = 4;  // columns at a time
+            uint32_t mx = 0;
+#pragma unroll 1
+            for (int c0 = 0; c0 < ncol; c0 += CH) {
+                uint32_t a[kDigits * CH];
+#pragma unroll
+                for (int d = 0; d < kDigits; ++d) tm_ld4(tb + d * NT + c0, &a[d * CH]);
+                tm_wait();
+                long long T[CH];
+                uint32_t odd = 0;
+#pragma unroll
+                for (int c = 0; c < CH; ++c) T[c] = dg_sum(&a[c], CH, odd);
+                if (odd & 0xff800000u) {
+#pragma unroll
+                    for (int c = 0; c < CH; ++c)
+                        T[c] = dg_sum_big(__uint_as_float(a[c]), __uint_as_float(a[CH + c]), __uint_as_float(a[2 * CH + c]),
+                                          __uint_as_float(a[3 * CH + c]), __uint_as_float(a[4 * CH + c]),
+                                          __uint_as_float(a[5 * CH + c]), __uint_as_float(a[6 * CH + c]));
+                }
+                double v[CH];
+                if constexpr (STAGE == kF2 || STAGE == kI1) {
+                    bool bad = false;
+                    int eb[CH];
+#pragma unroll
+                    for (int c = 0; c < CH; ++c) {
+                        eb[c] = __shfl_sync(0xffffffffu, cpar, (c0 + c) & 31) - qrow;
+                        v[c] = dg_fast(T[c], eb[c], bad);
+                    }
+                    if (bad)
+#pragma unroll
+                        for (int c = 0; c < CH; ++c) v[c] = dg_slow(T[c], eb[c]);
+                }
+                const int col0 = colb + c0, nc = ncol - c0;  // columns of this chunk: min(CH, nc)
+                if constexpr (STAGE == kF1) {
+                    // integers in the scale of the function
+                    const size_t xm = (size_t)((tl.kind < 4 ? 2 : 1) * row + tl.m) * 2 * p.BP;
+                    long long* X = (long long*)p.X + xm;
+#pragma unroll
+                    for (int c = 0; c < CH; ++c) T[c] >>= __shfl_sync(0xffffffffu, cpar, (c0 + c) & 31);
+                    const int fa = __shfl_sync(0xffffffffu, cfield, c0 & 31);
+                    const int fb = __shfl_sync(0xffffffffu, cfield, (c0 + min(CH - 1, nc - 1)) & 31);
+                    if ((B & 1) == 0) {
+#pragma unroll
+                        for (int c = 0; c < CH; c += 2) {
+                            const uint32_t o = __shfl_sync(0xffffffffu, coff, (c0 + c) & 31);
+                            if (live && c < nc) *(longlong2*)(X + o) = make_longlong2(T[c], T[c + 1]);
+                        }
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < CH; ++c) {
+                            const uint32_t o = __shfl_sync(0xffffffffu, coff, (c0 + c) & 31);
+                            if (live && c < nc) X[o] = T[c];
+                        }
+                    }
+                    // bits of the row's largest value, per field
+                    const int m = (tl.kind < 4 ? 2 : 1) * row + tl.m;
+                    if (fa == fb) {
+                        uint32_t x = 0;
+#pragma unroll
+                        for (int c = 0; c < CH; ++c) x = max(x, c < nc ? 64u - (uint32_t)__clzll(T[c] < 0 ? -T[c] : T[c]) : 0u);
+                        mx = max(mx, x);
+                        const int fn = c0 + CH < ncol ? __shfl_sync(0xffffffffu, cfield, (c0 + CH) & 31) : -1;
+                        if (fn != fa) {
+                            if (live) atomicMax(p.emax + (size_t)(fa * 2 + tl.t) * B + m, mx);
+                            mx = 0;
+                        }
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < CH; ++c) {
+                            const int f = __shfl_sync(0xffffffffu, cfield, (c0 + c) & 31);
+                            mx = max(mx, 64u - (uint32_t)__clzll(T[c] < 0 ? -T[c] : T[c]));
+                            if (live && c < nc) atomicMax(p.emax + (size_t)(f * 2 + tl.t) * B + m, mx);
+                            const int fn = __shfl_sync(0xffffffffu, cfield, (c0 + c + 1) & 31);
+                            if (fn != f) mx = 0;
+                        }
+                    }
+                } else if constexpr (STAGE == kF2) {
+                    const int m = tl.m, l = m + tl.t + 2 * row;
+                    const bool modd = (m & 1) != 0;
+                    const int i0 = index_of_harmonic_coeff(m, l, B), i1 = index_of_harmonic_coeff(-m, l, B);
+                    if (p.mode == kReal) {
+                        double* qr = p.out_r + (size_t)(col0 >> 1) * B * B;
+                        double* qi = p.out_i + (size_t)(col0 >> 1) * B * B;
+#pragma unroll
+                        for (int c = 0; c < CH; c += 2) {
+                            if (live && c < nc) {
+                                qr[i0] = v[c];
+                                qi[i0] = v[c + 1];
+                                if (m) {
+                                    qr[i1] = modd ? -v[c] : v[c];
+                                    qi[i1] = modd ? v[c + 1] : -v[c + 1];
+                                }
+                            }
+                            qr += B * B;
+                            qi += B * B;
+                        }
+                    } else {
+                        double* qr = p.out_r + (size_t)(col0 >> 2) * B * B;
+                        double* qi = p.out_i + (size_t)(col0 >> 2) * B * B;
+#pragma unroll
+                        for (int c = 0; c < CH; c += 4) {
+                            const double gr = v[c], gi = v[c + 1], hr = v[c + 2], hi = v[c + 3];
+                            if (live && c < nc) {
+                                const double vr = gr - hi, vi = gi + hr;
+                                qr[i0] = vr;
+                                qi[i0] = vi;
+                                if (m) {
+                                    const double nr = p.mode == kCplx ? gr + hi : vr;
+                                    const double ni = p.mode == kCplx ? hr - gi : -vi;
+                                    qr[i1] = modd ? -nr : nr;
+                                    qi[i1] = modd ? -ni : ni;
+                                }
+                            }
+                            qr += B * B;
+                            qi += B * B;
+                        }
+                    }
+                } else if constexpr (STAGE == kI1) {
+                    double* X = (double*)p.X + ((size_t)col0 * B + tl.m) * 2 * p.BP + tl.t * p.BP + row;
+                    const size_t step = (size_t)B * 2 * p.BP;
+                    uint32_t x[CH];
+#pragma unroll
+                    for (int c = 0; c < CH; ++c) {
+                        if (live && c < nc) X[c * step] = v[c];
+                        x[c] = live ? dexp(v[c]) : 0;
+                    }
+                    // exponent of the field: lane c / 2 ends with that of columns c, c + 1
+#pragma unroll
+                    for (int c = 0; c < CH; c += 2) {
+                        const uint32_t y = __reduce_max_sync(0xffffffffu, max(x[c], x[c + 1]));
+                        if (lane == c / 2) mx = y;
+                    }
+                    if (lane < CH / 2 && 2 * lane < nc) atomicMax(p.emax + (col0 >> 1) + lane, mx);
+                } else {
+                    long long* Z = p.Z + (size_t)col0 * p.RL + tl.zoff + row;
+#pragma unroll
+                    for (int c = 0; c < CH; ++c)
+                        if (live && c < nc) Z[(size_t)c * p.RL] = (T[c] + 2) >> kDgOutShift;
+                }
+            }
+            tc::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&accEmpty[slot]);
+        }
+    }
+    __syncwarp();
+    tc::tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tc::tc_fence_after();
+        tc::tmem_dealloc(tmem, 512);
+        if (lane == 0 && failed) atomicExch(p.err, S2G_ERR_TIMEOUT);
+    }
+}
+
+// ------------------------------------------------------------------------------------
+// Folded longitudes: where value k of fold kd lies in a column, and the column's length.
+struct DgFold {
+    int n[6], off[6], len;  // entries, place and total (padded to the K steps)
+};
+static DgFold dg_fold_layout(int B, bool inv) {
+    DgFold f{};
+    const int h = B / 2;
+    auto put = [&](int kd, int n) {
+        f.n[kd] = n;
+        f.off[kd] = f.len;
+        f.len += (n + 15) & ~15;
+    };
+    if (B % 2 == 0) {
+        // inverse: the cosines of even orders at longitude index B/2 come from k_dg_mid
+        put(0, inv ? h : h + 1);
+        for (int kd = 1; kd < 4; ++kd) put(kd, h);
+    } else {
+        put(4, B + 1);
+        put(5, B - 1);
+    }
+    return f;
+}
+
+// Latitudes j and 2B-1-j of one field -> fixed point (|x| < 2^vb, scale in e[field][j]) -> even and odd
+// latitude parts of the folded rows, Z[field][t][j][..].  One block per (j, field).
+__global__ void __launch_bounds__(128) k_dg_fold(const double* __restrict__ r, const double* __restrict__ im, int B,
+                                                 int N, int vb, DgFold fl, long long* Z, uint32_t* e, uint32_t* ef) {
+    extern __shared__ long long rows[];  // [2][S]
+    __shared__ uint32_t red[4];
+    const int S = 2 * B, j = blockIdx.x, ff = blockIdx.y;
+    const double* g = ff < N ? r + (size_t)ff * S * S : im + (size_t)(ff - N) * S * S;
+    const double* x[2] = {g + (size_t)j * S, g + (size_t)(S - 1 - j) * S};
+    uint32_t mx = 0;
+    for (int i = threadIdx.x; i < 2 * S; i += blockDim.x) {
+        const double v = i < S ? x[0][i] : x[1][i - S];
+        rows[i] = __double_as_longlong(v);
+        mx = max(mx, dexp(v));
+    }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    mx = max(max(red[0], red[1]), max(red[2], red[3]));
+    if (threadIdx.x == 0) {
+        e[ff * B + j] = mx;
+        atomicMax(ef + ff, mx);
+    }
+    const int em = max((int)mx, 1);
+    for (int i = threadIdx.x; i < 2 * S; i += blockDim.x) rows[i] = dg_fix(__longlong_as_double(rows[i]), em, vb);
+    __syncthreads();
+    long long* z0 = Z + ((size_t)ff * S + j) * fl.len;
+    long long* z1 = z0 + (size_t)B * fl.len;
+    const long long* a = rows;
+    const long long* b = rows + S;
+    auto both = [&](int at, long long u, long long w) {
+        z0[at] = u + w;
+        z1[at] = u - w;
+    };
+    if (B % 2 == 0) {
+        const int h = B / 2, pad = ((h + 1 + 15) & ~15);
+        for (int k = threadIdx.x; k < pad; k += blockDim.x) {
+            long long c[2][4] = {};
+            if (k <= h) {
+                const int ks = k ? S - k : 0;
+                const long long* row[2] = {a, b};
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const long long p0 = row[q][k], p1 = row[q][ks], p2 = row[q][B - k], p3 = row[q][B + k];
+                    c[q][0] = (p0 + p1) + (p2 + p3);
+                    c[q][1] = (p0 + p1) - (p2 + p3);
+                    c[q][2] = (p0 - p1) - (p2 - p3);
+                    c[q][3] = (p0 - p1) + (p2 - p3);
+                }
+            }
+            const int hp = (h + 15) & ~15;
+            both(fl.off[0] + k, c[0][0], c[1][0]);
+            if (k < hp) {
+                const bool in = k < h;
+                both(fl.off[1] + k, in ? c[0][1] : 0, in ? c[1][1] : 0);
+                both(fl.off[2] + k, in ? c[0][2] : 0, in ? c[1][2] : 0);
+            }
+            // the sines of odd orders run over k = 1 .. h; their padding follows
+            if (k >= 1 && k <= h) both(fl.off[3] + k - 1, c[0][3], c[1][3]);
+            if (k >= h && k < hp) both(fl.off[3] + k, 0, 0);
+        }
+    } else {
+        const int pad = ((B + 1 + 15) & ~15), sp = ((B - 1 + 15) & ~15);
+        for (int k = threadIdx.x; k < pad; k += blockDim.x) {
+            long long u0 = 0, u1 = 0, w0 = 0, w1 = 0;
+            if (k <= B) {
+                const int ks = k ? S - k : 0;
+                u0 = a[k] + a[ks];
+                w0 = b[k] + b[ks];
+                u1 = a[k] - a[ks];
+                w1 = b[k] - b[ks];
+            }
+            both(fl.off[4] + k, u0, w0);
+            if (k >= 1 && k < B) both(fl.off[5] + k - 1, u1, w1);
+            if (k >= B - 1 && k < sp) both(fl.off[5] + k, 0, 0);
+        }
+    }
+}
+
+// Inverse, even B: sum over the even orders of c_m (-1)^(m/2) Re F_m, the cosine part at longitude index
+// B/2, for every column of I2.
+__global__ void __launch_bounds__(256) k_dg_mid(const double* __restrict__ X, int B, int ncols, double* mid) {
+    __shared__ double part[8][33];
+    const int col = blockIdx.x * 32 + threadIdx.x, S = 2 * B;  // 32 columns, eight runs of orders
+    const int nb = (B + 3) / 4, per = (nb + 7) / 8;
+    double s = 0.0;
+    if (col < ncols) {
+        const int f = col / S, rem = col - f * S;
+        const double* x = X + (size_t)(f * 2) * B * S + rem;  // even B: rows of X have 2B values
+        const int b1 = min(nb, (int)(threadIdx.y + 1) * per);
+#pragma unroll 4
+        for (int b = threadIdx.y * per; b < b1; ++b) {
+            const int m = 4 * b;
+            s += x[(size_t)m * S] - (m + 2 < B ? x[(size_t)(m + 2) * S] : 0.0);
+        }
+    }
+    part[threadIdx.y][threadIdx.x] = s;
+    __syncthreads();
+    if (threadIdx.y == 0 && col < ncols) {
+        for (int q = 1; q < 8; ++q) s += part[q][threadIdx.x];
+        const int f = col / S;
+        mid[col] = (2.0 * s - X[(size_t)(f * 2) * B * S + (col - f * S)]) * 0.39894228040143267794;
+    }
+}
+
+// Parts of I2 -> samples of latitudes j and 2B-1-j.  One block per (j, field).
+__global__ void __launch_bounds__(128) k_dg_unfold(const long long* __restrict__ Z, const double* __restrict__ mid,
+                                                   const uint32_t* __restrict__ ef, int B, int N, int qv, DgFold fl,
+                                                   double* r, double* im) {
+    const int S = 2 * B, j = blockIdx.x, ff = blockIdx.y;
+    double* g = ff < N ? r + (size_t)ff * S * S : im + (size_t)(ff - N) * S * S;
+    double* out[2] = {g + (size_t)j * S, g + (size_t)(S - 1 - j) * S};
+    const long long* z0 = Z + ((size_t)ff * S + j) * fl.len;
+    const long long* z1 = z0 + (size_t)B * fl.len;
+    const uint32_t em = ef[ff];
+    const int eb = dg_eb(em, 120 + kDgOutShift - qv);  // qv: bits of table and data values
+    auto value = [&](long long T) {
+        bool bad = false;
+        const double v = dg_fast(T, eb, bad);
+        return bad ? dg_slow(T, eb) : v;
+    };
+    auto put = [&](int k, long long u, long long w) {  // even and odd latitude parts
+        out[0][k] = value(u + w);
+        out[1][k] = value(u - w);
+    };
+    if (B % 2 == 0) {
+        const int h = B / 2;
+        for (int k = threadIdx.x; k < h; k += blockDim.x) {
+            long long c[2], d[2], s[2], q[2];
+            const long long* z[2] = {z0, z1};
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                const long long ce = z[t][fl.off[0] + k], co = z[t][fl.off[1] + k];
+                const long long se = k ? z[t][fl.off[2] + k] : 0, so = k ? z[t][fl.off[3] + k - 1] : 0;
+                c[t] = ce + co;
+                d[t] = ce - co;
+                s[t] = se + so;
+                q[t] = so - se;
+            }
+            put(k, c[0] + s[0], c[1] + s[1]);
+            put(B + k, d[0] - q[0], d[1] - q[1]);
+            if (k) {
+                put(S - k, c[0] - s[0], c[1] - s[1]);
+                put(B - k, d[0] + q[0], d[1] + q[1]);
+            }
+        }
+        if (threadIdx.x < 2) {  // k = B/2 and 3B/2
+            const double sg = threadIdx.x ? -1.0 : 1.0;
+            const double m0 = mid[(size_t)ff * S + j], m1 = mid[(size_t)ff * S + B + j];
+            const double s0 = value(z0[fl.off[3] + h - 1]), s1 = value(z1[fl.off[3] + h - 1]);
+            const int k = threadIdx.x ? B + h : h;
+            out[0][k] = (m0 + m1) + sg * (s0 + s1);
+            out[1][k] = (m0 - m1) + sg * (s0 - s1);
+        }
+    } else {
+        for (int k = threadIdx.x; k <= B; k += blockDim.x) {
+            const long long c0 = z0[fl.off[4] + k], c1 = z1[fl.off[4] + k];
+            const bool in = k >= 1 && k < B;
+            const long long s0 = in ? z0[fl.off[5] + k - 1] : 0, s1 = in ? z1[fl.off[5] + k - 1] : 0;
+            put(k, c0 + s0, c1 + s1);
+            if (in) put(S - k, c0 - s0, c1 - s1);
+        }
+    }
+}
+
+// Largest exponent of every order's coefficients (I1), e[field, part][m]; COMPLEX data, and REAL data with an
+// imaginary output, are first split into two real fields' coefficients (cr, ci, orders m >= 0):
+//   g = (a + s conj b) / 2, h = (a - s conj b) / 2i with a = f(l,m), b = f(l,-m), s = (-1)^m.
+// One warp per (function, order).
+__global__ void k_dg_coefmax(const double* __restrict__ rc, const double* __restrict__ ic, int B, int N, int mode,
+                             double* cr, double* ci, uint32_t* e) {
+    const int id = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (id >= N * B) return;
+    const int f = id / B, m = id - f * B;
+    const size_t cb = (size_t)f * B * B, hb = (size_t)(N + f) * B * B;
+    uint32_t mx[4] = {0, 0, 0, 0};
+    for (int l = m + lane; l < B; l += 32) {
+        const int i = index_of_harmonic_coeff(m, l, B);
+        const double ar = rc[cb + i], ai = ic[cb + i];
+        if (mode == kReal) {
+            mx[0] = max(mx[0], dexp(ar));
+            if (m) mx[1] = max(mx[1], dexp(ai));
+            continue;
+        }
+        double v[4] = {ar, m ? ai : 0.0, m ? 0.0 : ai, 0.0};  // Im f(l, 0) is the second field's
+        if (mode == kCplx && m) {
+            const int k = index_of_harmonic_coeff(-m, l, B);
+            const double s = (m & 1) ? -1.0 : 1.0, br = s * rc[cb + k], bi = s * ic[cb + k];
+            v[0] = 0.5 * ar + 0.5 * br;
+            v[1] = 0.5 * ai - 0.5 * bi;
+            v[2] = 0.5 * ai + 0.5 * bi;
+            v[3] = 0.5 * br - 0.5 * ar;
+        }
+        cr[cb + i] = v[0];
+        ci[cb + i] = v[1];
+        cr[hb + i] = v[2];
+        ci[hb + i] = v[3];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) mx[q] = max(mx[q], dexp(v[q]));
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) mx[q] = __reduce_max_sync(0xffffffffu, mx[q]);
+    if (lane) return;
+    e[(size_t)(2 * f) * B + m] = mx[0];
+    e[(size_t)(2 * f + 1) * B + m] = mx[1];
+    if (mode != kReal) {
+        e[(size_t)(2 * (N + f)) * B + m] = mx[2];
+        e[(size_t)(2 * (N + f) + 1) * B + m] = mx[3];
+    }
+}
+
+// ------------------------------------------------------------------------------------
+// Tables.  P(m,l)(x_j) by the three-term recurrence in double-double arithmetic, rounded to
+// double once, so that the digits carry the table to its last place.
+struct dd {
+    double h, l;
+};
+__device__ __forceinline__ dd dd_mul(dd a, dd b) {
+    const double p = a.h * b.h;
+    const double e = fma(a.h, b.h, -p) + (a.h * b.l + a.l * b.h);
+    const double s = p + e;
+    return {s, e - (s - p)};
+}
+__device__ __forceinline__ dd dd_add(dd a, dd b) {
+    const double s = a.h + b.h, t = s - a.h;
+    const double e = (a.h - (s - t)) + (b.h - t) + (a.l + b.l);
+    const double r = s + e;
+    return {r, e - (r - s)};
+}
+// sqrt(n / d) for integers n, d held exactly
+__device__ __forceinline__ dd dd_sqrt_ratio(double n, double d) {
+    if (n == 0.0) return {0.0, 0.0};
+    const double q = n / d, q1 = fma(-q, d, n) / d;
+    const double s = sqrt(q), e = (fma(-s, s, q) + q1) / (2.0 * s);
+    const double r = s + e;
+    return {r, e - (r - s)};
+}
+
+// One block per order m0 + blockIdx.x: rows l - m of P at the B northern nodes into tmp + off[blockIdx.x].
+__global__ void k_dg_legendre(int B, int m0, const double2* __restrict__ cosn, const double2* __restrict__ sinn,
+                              const double2* __restrict__ seed, double* tmp, const int64_t* __restrict__ off) {
+    extern __shared__ double2 ac[];  // [B] a, [B] c
+    const int m = m0 + blockIdx.x;
+    for (int l = m + threadIdx.x; l < B; l += blockDim.x) {
+        const double d = (l + 1.0 - m) * (l + 1.0 + m);
+        const dd a = dd_sqrt_ratio((2.0 * l + 3.0) * (2.0 * l + 1.0), d);
+        dd c{0.0, 0.0};
+        if (l > m) c = dd_sqrt_ratio((2.0 * l + 3.0) * (double)(l - m) * (l + m), (2.0 * l - 1.0) * d);
+        ac[l] = make_double2(a.h, a.l);
+        ac[B + l] = make_double2(-c.h, -c.l);
+    }
+    __syncthreads();
+    double* out = tmp + off[blockIdx.x];
+    for (int j = threadIdx.x; j < B; j += blockDim.x) {
+        const dd x{cosn[j].x, cosn[j].y};
+        dd cur{seed[m].x, seed[m].y}, prev{0.0, 0.0}, b{sinn[j].x, sinn[j].y};
+        for (int e = m; e; e >>= 1) {  // sin^m
+            if (e & 1) cur = dd_mul(cur, b);
+            b = dd_mul(b, b);
+        }
+        for (int l = m; l < B; ++l) {
+            out[(size_t)(l - m) * B + j] = cur.h;
+            const dd a{ac[l].x, ac[l].y}, c{ac[B + l].x, ac[B + l].y};
+            const dd nx = dd_add(dd_mul(a, dd_mul(x, cur)), dd_mul(c, prev));
+            prev = cur;
+            cur = nx;
+        }
+    }
+}
+
+// Rows of an odd order m as the forward seminaive transform applies them (seminaive.c:170-197): the
+// order's cosine series (cospml.c:161-242), evaluated at the nodes and times sin.  One block per degree.
+__global__ void k_dg_seminaive(int B, int m, const double* __restrict__ T, const double2* __restrict__ tw4S,
+                               double* out) {
+    const int S = 2 * B, l = m + blockIdx.x, t = (l - m) & 1, n = row_size(m, l);
+    const double* row = T + table_offset(m, l);
+    const double nrm = 2.0 / sqrt(2.0 * S);
+    for (int j = threadIdx.x; j < B; j += blockDim.x) {
+        dd acc{0.0, 0.0};
+        int r = (int)((long long)t * (2 * j + 1) % (4 * S));  // angle k (2j + 1) pi / 2S, k = t, t + 2, ..
+        const int step = (4 * j + 2) % (4 * S);
+        for (int i = 0; i < n; ++i) {
+            const double a = row[i] * ((2 * i + t) ? nrm : nrm * 0.70710678118654752440), c = tw4S[r].x;
+            const double q = a * c;
+            acc = dd_add(acc, {q, fma(a, c, -q)});
+            r += step;
+            if (r >= 4 * S) r -= 4 * S;
+        }
+        out[(size_t)(l - m) * B + j] = acc.h * sinpi((2.0 * j + 1.0) / (2.0 * S));
+    }
+}
+
+// Scale of a row whose largest value is mx: 2^(tb-1) <= mx 2^q < 2^tb.
+__device__ __forceinline__ int dg_scale(double mx, int tb) {
+    if (!(mx > 0.0)) return 0;
+    int e;
+    frexp(mx, &e);
+    return tb - e;
+}
+
+// Digits of one 8-row group; 128 threads = 8 rows x 16 K entries per step.  val(row, k): the table value.
+template <class Val>
+__device__ __forceinline__ void dg_pack_rows(Val val, int q, uint8_t* blob, int r8, int ks, int rg) {
+    const int r = threadIdx.x >> 4, kk = threadIdx.x & 15;
+    const uint32_t bytes = kDigits * (uint32_t)r8 * 32;
+    for (int s = 0; s < ks; ++s) {
+        const double x = val(r, s * 16 + kk);
+        const long long v = __double2ll_rn(scalbn(x, q));
+        const unsigned long long u = (unsigned long long)v + 0x0200808080808080ull;
+        uint8_t* d = blob + (size_t)s * bytes + rg * 256 + (kk >> 3) * 128 + r * 16 + (kk & 7) * 2;
+#pragma unroll
+        for (int a = 0; a < kDigits; ++a)
+            *(__half*)(d + (size_t)a * r8 * 32) =
+                __int2half_rn(a ? (int)((u >> (8 * (6 - a))) & 255) - 128 : (int)(u >> 48) - 512);
+    }
+}
+
+// Legendre tables of the orders m0 ..: one block per (tile, 8-row group); tiles of kind F2 (rows degrees,
+// weighted) or I1 (rows nodes).
+__global__ void __launch_bounds__(128) k_dg_pack_leg(int B, int fwd, const DgTile* __restrict__ tiles, int m0,
+                                                     const double* __restrict__ tmp, const int64_t* __restrict__ off,
+                                                     const double* __restrict__ w, double wscale, uint8_t* tab,
+                                                     short* qs) {
+    __shared__ double red[8][17];
+    const DgTile tl = tiles[blockIdx.x];
+    const int rg = blockIdx.y;
+    if (rg * 8 >= tl.r8) return;
+    const double* P = tmp + off[tl.m - m0];
+    const int nl = (B - tl.m - tl.t + 1) / 2;  // degrees of this parity
+    auto val = [&](int r, int k) -> double {
+        const int row = tl.row0 + rg * 8 + r;
+        if (rg * 8 + r >= tl.nrows) return 0.0;
+        if (fwd) return k < B ? P[(size_t)(tl.t + 2 * row) * B + k] * (w[k] * wscale) : 0.0;
+        return k < nl ? P[(size_t)(tl.t + 2 * k) * B + row] : 0.0;
+    };
+    const int r = threadIdx.x >> 4, kk = threadIdx.x & 15;
+    double mx = 0.0;
+    for (int s = 0; s < tl.ks; ++s) mx = fmax(mx, fabs(val(r, s * 16 + kk)));
+    red[r][kk] = mx;
+    __syncthreads();
+    for (int q = 0; q < 16; ++q) mx = fmax(mx, red[r][q]);
+    const int q = dg_scale(mx, tl.tb);
+    if (kk == 0 && rg * 8 + r < tl.nrows) qs[tl.qoff + tl.row0 + rg * 8 + r] = (short)q;
+    dg_pack_rows(val, q, tab + tl.off, tl.r8, tl.ks, rg);
+}
+
+// DFT tables: F1 (rows orders, K longitudes) and I2 (rows longitudes, K orders), folds as k_dg_fold.
+__global__ void __launch_bounds__(128) k_dg_pack_dft(int B, int inv, const DgTile* __restrict__ tiles, uint8_t* tab,
+                                                     short* qs) {
+    const DgTile tl = tiles[blockIdx.x];
+    const int rg = blockIdx.y, S = 2 * B;
+    if (rg * 8 >= tl.r8) return;
+    const int kd = tl.kind, k0 = (kd == 3 || kd == 5) ? 1 : 0, mstep = kd < 4 ? 2 : 1;
+    const int nlon = kd < 4 ? B / 2 + (kd == 0 ? 1 : 0) : (kd == 5 ? B - 1 : B + 1);
+    auto val = [&](int r, int k) -> double {
+        const int row = tl.row0 + rg * 8 + r;
+        if (rg * 8 + r >= tl.nrows) return 0.0;
+        const int m = (inv ? k : row) * mstep + tl.m, lon = (inv ? row : k) + k0;
+        if (m >= B || (!inv && k >= nlon)) return 0.0;
+        // forward: the folds count the samples at their fixed points twice; inverse: orders m and -m,
+        // 1/sqrt(2 pi) (FST_semi_memo.c:344-348)
+        double f = (lon == 0 || (kd < 4 ? 2 * lon == B : lon == B)) ? 0.5 : 1.0;
+        if (inv) f = (m ? 2.0 : 1.0) * 0.39894228040143267794;
+        const double a = 2.0 * (double)((long long)m * lon % S) / (double)S;  // angle / pi
+        return tl.t ? -f * sinpi(a) : f * cospi(a);
+    };
+    dg_pack_rows(val, tl.tb, tab + tl.off, tl.r8, tl.ks, rg);
+    const int r = threadIdx.x >> 4;
+    if ((threadIdx.x & 15) == 0 && rg * 8 + r < tl.nrows) qs[tl.qoff + tl.row0 + rg * 8 + r] = (short)tl.tb;
+}
+
+// ------------------------------------------------------------------------------------
+struct DgTable {
+    std::vector<DgTile> h;
+    DgTile* tiles = nullptr;
+    uint8_t* tab = nullptr;
+    short* q = nullptr;
+    int64_t bytes = 0;
+    int rows = 0;
+    void release() {
+        cudaFree(tiles);
+        cudaFree(tab);
+        cudaFree(q);
+        tiles = nullptr;
+        tab = nullptr;
+        q = nullptr;
+    }
+};
+
+struct DgTabs {
+    int device = -1, bw = 0, refs = 0;
+    DgTable t[4];
+    int* err = nullptr;
+};
+
+static std::mutex g_dg_mu;
+static std::map<std::pair<int, int>, DgTabs*> g_dg;
+
+static void dg_free(DgTabs* d) {
+    for (auto& t : d->t) t.release();
+    cudaFree(d->err);
+    delete d;
+}
+
+void dg_put(void* h) {
+    DgTabs* d = (DgTabs*)h;
+    if (!d) return;
+    std::lock_guard<std::mutex> lk(g_dg_mu);
+    if (--d->refs == 0) {
+        g_dg.erase({d->device, d->bw});
+        dg_free(d);
+    }
+}
+
+static int dg_vbz(int bw) {  // bits of a sample: eight (odd bw: four) of them add up to a data value
+    return (bw % 2 ? 52 : 51) + (dg_fold_layout(bw, false).n[bw % 2 ? 4 : 0] <= 272 ? 2 : 0);
+}
+
+// Bits of a table value: the leading group, at most K 2^(vb - 48) 2^(tb - 48), stays near 2^22, so that the
+// sum in units of 2^8 of the last group's has 63 bits.  I2 (values up to 2/sqrt(2 pi), eight sums of
+// which each gives up kDgOutShift bits) keeps strictly below 2^22.
+static int dg_table_bits(int K, int vb, bool inv_rows) {
+    int kb = 0;
+    while ((inv_rows ? 2 : 3) << kb < 2 * K) ++kb;
+    return 48 + std::min(8, 22 - kb - (vb - 48));
+}
+
+static void dg_tiles(DgTable& t, int stage, int B) {
+    auto add = [&](int rows, int k, int m, int par, int kind, int zoff) {
+        const int q0 = t.rows;
+        for (int r0 = 0; r0 < rows; r0 += 128) {
+            DgTile tl{};
+            tl.row0 = r0;
+            tl.nrows = std::min(128, rows - r0);
+            tl.r8 = (tl.nrows + 7) & ~7;
+            tl.qoff = q0;
+            tl.m = m;
+            tl.t = par;
+            tl.kind = kind;
+            tl.zoff = zoff;
+            tl.ks = std::max(1, (k + 15) / 16);  // no degree of a parity: one zero step
+            // F1's data have vbz bits and folds; I2's sums of eight parts stay below 2^63
+            tl.vb = stage == kI2 ? (k <= 128 ? 55 : k <= 256 ? 54 : 53) : (stage == kI1 ? (k <= 256 ? 55 : 54) : (k <= 256 ? 56 : 54));
+            tl.tb = dg_table_bits(k, stage == kF1 ? (dg_vbz(B) >= 53 ? 56 : 54) : tl.vb, stage == kI2);
+            tl.off = t.bytes;
+            t.bytes += (int64_t)tl.ks * kDigits * tl.r8 * 32;
+            t.h.push_back(tl);
+        }
+        t.rows += rows;
+    };
+    if (stage == kF1 || stage == kI2) {
+        const DgFold f = dg_fold_layout(B, stage == kI2);
+        for (int kd = B % 2 ? 4 : 0; kd < (B % 2 ? 6 : 4); ++kd) {
+            const int m0 = kd < 4 ? kd & 1 : 0, part = kd < 4 ? kd >> 1 : kd - 4, nm = kd < 4 ? B / 2 : B;
+            if (stage == kF1) add(nm, f.n[kd], m0, part, kd, f.off[kd]);
+            else add(f.n[kd], nm, m0, part, kd, f.off[kd]);
+        }
+        return;
+    }
+    for (int m = 0; m < B; ++m)
+        for (int par = 0; par < 2; ++par) {
+            const int nl = (B - m - par + 1) / 2;
+            if (stage == kI1) add(B, nl, m, par, 0, 0);
+            else if (nl > 0) add(nl, B, m, par, 0, 0);
+        }
+}
+
+static int dg_upload(DgTable& t, int stage, int B, cudaStream_t st) {
+    dg_tiles(t, stage, B);
+    S2G_CUDA(cudaMalloc(&t.tiles, sizeof(DgTile) * t.h.size()));
+    S2G_CUDA(cudaMalloc(&t.tab, (size_t)t.bytes + 4096));
+    S2G_CUDA(cudaMalloc(&t.q, sizeof(short) * t.rows));
+    S2G_CUDA(cudaMemcpyAsync(t.tiles, t.h.data(), sizeof(DgTile) * t.h.size(), cudaMemcpyHostToDevice, st));
+    return S2G_OK;
+}
+
+// Above this bandwidth the forward's orders 1, 3 and 5 take their rows from the cosine series.  The
+// series of G = P / sin have large coefficients there, and their FP64 rounding is part of the reference's
+// results: on samples that are not band-limited, at bw 1024, the exact transform is 3.2e-11 away from
+// them at order 1 (8e-12 at order 3), more than the 1e-11 that the FP64 path keeps to the reference.
+constexpr int kDgNaiveBw = 512;
+static int dg_low_orders(int B, double* tmp, const std::vector<int64_t>& off, int m1, cudaStream_t st) {
+    const int S = 2 * B;
+    struct Buf {
+        void* p[3] = {nullptr, nullptr, nullptr};
+        ~Buf() {
+            for (void* q : p) cudaFree(q);
+        }
+    } b;
+    int64_t most = 0;
+    for (int m = 1; m <= 5 && m < m1; m += 2) most = std::max(most, table_size(m, B));
+    const std::vector<int64_t> zero(8, 0);  // each order's table alone, at the buffer's start
+    S2G_CUDA(cudaMalloc(&b.p[0], sizeof(double) * (size_t)most));
+    S2G_CUDA(cudaMalloc(&b.p[1], sizeof(double2) * 4 * S));
+    S2G_CUDA(cudaMalloc(&b.p[2], sizeof(int64_t) * zero.size()));
+    S2G_CUDA(cudaMemcpyAsync(b.p[2], zero.data(), sizeof(int64_t) * zero.size(), cudaMemcpyHostToDevice, st));
+    S2G_TRY(twiddles_device(4 * S, (double2*)b.p[1], nullptr, st));
+    for (int m = 1; m <= 5 && m < m1; m += 2) {
+        S2G_TRY(generate_cos_pml_device(B, m, m + 1, (double*)b.p[0], (const int64_t*)b.p[2], st));
+        ProfScope ps_("dg_seminaive", st);
+        k_dg_seminaive<<<B - m, 256, 0, st>>>(B, m, (const double*)b.p[0], (const double2*)b.p[1], tmp + off[m]);
+        S2G_CUDA(cudaGetLastError());
+    }
+    S2G_CUDA(cudaStreamSynchronize(st));
+    return S2G_OK;
+}
+
+static int dg_build(DgTabs* d, const double* weights, cudaStream_t st) {
+    const int B = d->bw, S = 2 * B;
+    S2G_CUDA(cudaMalloc(&d->err, sizeof(int)));
+    S2G_CUDA(cudaMemsetAsync(d->err, 0, sizeof(int), st));
+    for (int s = 0; s < 4; ++s) S2G_TRY(dg_upload(d->t[s], s, B, st));
+    for (int s = kF1; s <= kI2; s += kI2 - kF1) {
+        const DgTable& t = d->t[s];
+        ProfScope ps_("dg_pack_dft", st);
+        k_dg_pack_dft<<<dim3((unsigned)t.h.size(), 16), 128, 0, st>>>(B, s == kI2, t.tiles, t.tab, t.q);
+        S2G_CUDA(cudaGetLastError());
+    }
+    // nodes, seeds P(m,m) = seed_m sin^m: long double, split in two doubles
+    std::vector<double2> h(3 * (size_t)B);
+    auto put = [](long double v) {
+        const double a = (double)v;
+        return make_double2(a, (double)(v - (long double)a));
+    };
+    const long double pi = 3.141592653589793238462643383279502884L;
+    long double c = sqrtl(0.5L);
+    for (int j = 0; j < B; ++j) {
+        const long double a = pi * (2 * j + 1) / (2 * (long double)S);
+        h[j] = put(cosl(a));
+        h[B + j] = put(sinl(a));
+        if (j) c *= -sqrtl((2 * j + 1) / (2 * (long double)j));
+        h[2 * (size_t)B + j] = put(c);
+    }
+    struct Tmp {
+        void* p[3] = {nullptr, nullptr, nullptr};
+        ~Tmp() {
+            for (void* q : p) cudaFree(q);
+        }
+    } tmp;
+    S2G_CUDA(cudaMalloc(&tmp.p[0], sizeof(double2) * h.size()));
+    S2G_CUDA(cudaMemcpyAsync(tmp.p[0], h.data(), sizeof(double2) * h.size(), cudaMemcpyHostToDevice, st));
+    // orders in chunks of at most 1 GiB of table values; off[m]: doubles before order m in its chunk
+    const int64_t most = std::max<int64_t>((int64_t)B * B, (int64_t)1 << 27);
+    std::vector<int64_t> off(B);
+    int64_t at = 0, need = 0;
+    for (int m = 0; m < B; ++m) {
+        const int64_t n = (int64_t)(B - m) * B;
+        if (at + n > most) at = 0;
+        off[m] = at;
+        at += n;
+        need = std::max(need, at);
+    }
+    S2G_CUDA(cudaMalloc(&tmp.p[1], sizeof(double) * (size_t)need));
+    S2G_CUDA(cudaMalloc(&tmp.p[2], sizeof(int64_t) * B));
+    S2G_CUDA(cudaMemcpyAsync(tmp.p[2], off.data(), sizeof(int64_t) * B, cudaMemcpyHostToDevice, st));
+    const double2* nodes = (const double2*)tmp.p[0];
+    const size_t smem = sizeof(double2) * 2 * (size_t)B;
+    S2G_CUDA(cudaFuncSetAttribute((const void*)k_dg_legendre, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    for (int m0 = 0; m0 < B;) {
+        int m1 = m0 + 1;
+        while (m1 < B && off[m1] != 0) ++m1;
+        {
+            ProfScope ps_("dg_legendre", st);
+            k_dg_legendre<<<m1 - m0, std::min(1024, (B + 31) & ~31), smem, st>>>(
+                B, m0, nodes, nodes + B, nodes + 2 * (size_t)B, (double*)tmp.p[1], (const int64_t*)tmp.p[2] + m0);
+        }
+        S2G_CUDA(cudaGetLastError());
+        for (int s = kI1; s >= kF2; --s) {
+            if (s == kF2 && B > kDgNaiveBw && m0 <= 1) S2G_TRY(dg_low_orders(B, (double*)tmp.p[1], off, m1, st));
+            const DgTable& t = d->t[s];
+            size_t a = 0, b = t.h.size();
+            while (a < b && t.h[a].m < m0) ++a;
+            while (b > a && t.h[b - 1].m >= m1) --b;
+            ProfScope ps_("dg_pack_leg", st);
+            k_dg_pack_leg<<<dim3((unsigned)(b - a), 16), 128, 0, st>>>(
+                B, s == kF2, t.tiles + a, m0, (const double*)tmp.p[1], (const int64_t*)tmp.p[2] + m0, weights,
+                sqrt(2.0 * 3.14159265358979323846) / S, t.tab, t.q);
+            S2G_CUDA(cudaGetLastError());
+        }
+        m0 = m1;
+    }
+    S2G_CUDA(cudaStreamSynchronize(st));
+    return S2G_OK;
+}
+
+// Digit tables of bandwidth bw on the current device, shared by every plan; the caller holds a reference.
+static int dg_get(int bw, const double* weights, DgTabs** out) {
+    int dev = 0;
+    S2G_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(g_dg_mu);
+    auto it = g_dg.find({dev, bw});
+    if (it != g_dg.end()) {
+        ++it->second->refs;
+        *out = it->second;
+        return S2G_OK;
+    }
+    DgTabs* d = new DgTabs();
+    d->device = dev;
+    d->bw = bw;
+    cudaStream_t st;
+    S2G_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+    const int r = dg_build(d, weights, st);
+    cudaStreamDestroy(st);
+    if (r != S2G_OK) {
+        dg_free(d);
+        return r;
+    }
+    d->refs = 1;
+    g_dg[{dev, bw}] = d;
+    *out = d;
+    return S2G_OK;
+}
+
+template <int STAGE, int NT>
+static int launch_dg_nt(const DgArgs& p, cudaStream_t st) {
+    static const char* names[4] = {"dg_rows_fwd", "dg_leg_fwd", "dg_leg_inv", "dg_rows_inv"};
+    const size_t smem = 1024 + kDgStagesA * kDgABytes + kDgBRing;
+    S2G_CUDA(cudaFuncSetAttribute((const void*)k_dg<STAGE, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int dev = 0, sms = 0;
+    S2G_CUDA(cudaGetDevice(&dev));
+    S2G_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int64_t items = (int64_t)p.ntiles * p.ncolblk;
+    {
+        ProfScope ps_(names[STAGE], st);
+        k_dg<STAGE, NT><<<(unsigned)std::min<int64_t>(items, sms), kDgThreads, smem, st>>>(p);
+    }
+    S2G_CUDA(cudaGetLastError());
+    return S2G_OK;
+}
+
+// 64 columns per item: an accumulator of 7 x 64 TMEM columns, each table digit read once per 64 columns;
+// fewer columns in all take 32 or 16 (two accumulators, so that the epilogue of one item runs beside the
+// MMAs of the next).  Items of F1 and I2 go column by column (their four tables, 1 MB at bw 256, stay in
+// L2), those of F2 and I1 table by table (117 MB each at bw 256).
+// At bw 256, 64 functions: F1 160 us, F2 130, I1 135, I2 127, k_dg_fold 68, k_dg_unfold 54, k_dg_mid 17;
+// forward and inverse together 0.69 ms against 4.59 ms on the FP64 units (DFMA-bound there).  The tensor
+// pipe alone would take 47 us for each of the four; MMA issue and the part of the epilogue that the next
+// item's MMAs wait for (dg_sum, the stores) make up the rest.
+template <int STAGE>
+static int launch_dg(const DgTabs* d, DgArgs p, cudaStream_t st) {
+    const DgTable& t = d->t[STAGE];
+    p.tiles = t.tiles;
+    p.tab = t.tab;
+    p.q = t.q;
+    p.ntiles = (int)t.h.size();
+    p.col_major = STAGE == kF1 || STAGE == kI2;
+    p.err = d->err;
+    const int per = p.ncols <= 16 ? 16 : (p.ncols <= 32 ? 32 : 64);
+    p.ncolblk = (p.ncols + per - 1) / per;
+    if (per == 16) return launch_dg_nt<STAGE, 16>(p, st);
+    if (per == 32) return launch_dg_nt<STAGE, 32>(p, st);
+    return launch_dg_nt<STAGE, 64>(p, st);
+}
+
+static int dg_fields(int mode) { return mode == kReal ? 1 : 2; }
+static int dg_mode(const void* imag, int fmt) { return fmt == COMPLEX ? kCplx : (imag ? kReal2 : kReal); }
+
+// Functions transformed at a time.
+static int dg_chunk(int bw, int batch) {
+    const int64_t per = 2 * 8 * 4 * (int64_t)bw * bw;
+    return (int)std::min<int64_t>(batch, std::min<int64_t>(16384, std::max<int64_t>(64, ((int64_t)256 << 20) / per)));
+}
+
+struct DgWork {
+    void* X;
+    long long* Z;
+    uint32_t *ej, *ef, *ex;
+    double *mid, *cr, *ci;
+    size_t bytes;
+};
+static DgWork dg_work(char* w, int bw, int n, bool two) {
+    const size_t ff = (size_t)n * (two ? 2 : 1), S = 2 * (size_t)bw, BP = bw + (bw & 1);
+    const size_t len = std::max(dg_fold_layout(bw, false).len, dg_fold_layout(bw, true).len);
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        char* q = w + at;
+        at += (bytes + 255) & ~(size_t)255;
+        return (void*)q;
+    };
+    DgWork k{};
+    k.X = take(ff * 2 * bw * 2 * BP * 8);
+    k.Z = (long long*)take(ff * S * len * 8);
+    k.ej = (uint32_t*)take(ff * bw * 4);
+    k.ef = (uint32_t*)take(ff * 4);
+    k.ex = (uint32_t*)take(ff * 2 * bw * 4);
+    k.mid = (double*)take(ff * S * 8);
+    k.cr = (double*)take(two ? ff * bw * bw * 8 : 0);
+    k.ci = (double*)take(two ? ff * bw * bw * 8 : 0);
+    k.bytes = at;
+    return k;
+}
+
+size_t dg_work_bytes(int bw, int batch, bool two) { return dg_work(nullptr, bw, dg_chunk(bw, batch), two).bytes; }
+
+// Bandwidths of the digit path: up to 1024 (its Legendre tables take 14 bw^3 bytes: 15 GB there).  Below 32
+// its five or six launches cost more than the FP64 kernels' two where those have a radix-2 FFT (one
+// function at bw 16: 24 and 33 us against 24 and 25), but not where they take Bluestein's (bw 12: 25 and
+// 34 us against 87 and 87).
+bool dg_takes(int bw) { return bw <= 1024 && (bw >= 32 || (bw > 8 && (bw & (bw - 1)))); }
+
+// Builds (or finds) the digit tables of t's bandwidth.  Where the stream is being captured, or they do
+// not fit in device memory, t stays without them and the FP64 kernels run.
+int dg_prepare(Tables* t, cudaStream_t st) {
+    if (!dg_takes(t->bw) || __atomic_load_n(&t->dg, __ATOMIC_ACQUIRE) || t->dg_off) return S2G_OK;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return S2G_OK;
+    }
+    DgTabs* d;
+    const int r = dg_get(t->bw, t->weights, &d);
+    if (r == S2G_ERR_NOMEM) {
+        cudaGetLastError();
+        t->dg_off = true;
+        return S2G_OK;
+    }
+    if (r != S2G_OK) return r;
+    void* none = nullptr;
+    if (!__atomic_compare_exchange_n(&t->dg, &none, (void*)d, false, __ATOMIC_ACQ_REL, __ATOMIC_ACQUIRE)) dg_put(d);
+    return S2G_OK;
+}
+
+static int set_dyn_smem(const void* fn, size_t bytes) {
+    S2G_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    return S2G_OK;
+}
+
+int fst_f64_dg(const Tables* t, const double* rdata, const double* idata, double* rc, double* ic, int batch, int fmt,
+               void* work, cudaStream_t st) {
+    const DgTabs* d = (const DgTabs*)t->dg;
+    const int B = t->bw, S = 2 * B, mode = dg_mode(idata, fmt), chunk = dg_chunk(B, batch);
+    const DgFold fl = dg_fold_layout(B, false);
+    const DgWork w = dg_work((char*)work, B, chunk, mode != kReal);
+    S2G_TRY(set_dyn_smem((const void*)k_dg_fold, 2 * (size_t)S * 8));
+    for (int f0 = 0; f0 < batch; f0 += chunk) {
+        const int n = std::min(chunk, batch - f0), ff = n * dg_fields(mode);
+        const size_t g0 = (size_t)f0 * S * S, c0 = (size_t)f0 * B * B;
+        S2G_CUDA(cudaMemsetAsync(w.ef, 0, (size_t)((char*)(w.ex + (size_t)ff * 2 * B) - (char*)w.ef), st));
+        DgArgs p{};
+        p.B = B;
+        p.S = S;
+        p.N = n;
+        p.mode = mode;
+        p.BP = B + (B & 1);
+        p.RL = fl.len;
+        p.vbz = dg_vbz(B);
+        p.tbz = d->t[kF1].h[0].tb;
+        p.X = w.X;
+        p.Z = w.Z;
+        {
+            ProfScope ps_("dg_fold", st);
+            k_dg_fold<<<dim3(B, ff), 128, 2 * (size_t)S * 8, st>>>(rdata + g0, idata ? idata + g0 : nullptr, B, n, p.vbz, fl,
+                                                                 w.Z, w.ej, w.ef);
+        }
+        S2G_CUDA(cudaGetLastError());
+        p.ncols = ff * S;
+        p.ein = w.ej;
+        p.efield = w.ef;
+        p.emax = w.ex;
+        S2G_TRY(launch_dg<kF1>(d, p, st));
+        p.ncols = ff * 2;
+        p.out_r = rc + c0;
+        p.out_i = ic + c0;
+        S2G_TRY(launch_dg<kF2>(d, p, st));
+    }
+    return S2G_OK;
+}
+
+int inv_fst_f64_dg(const Tables* t, const double* rc, const double* ic, double* rdata, double* idata, int batch,
+                   int fmt, void* work, cudaStream_t st) {
+    const DgTabs* d = (const DgTabs*)t->dg;
+    const int B = t->bw, S = 2 * B, mode = dg_mode(idata, fmt), chunk = dg_chunk(B, batch);
+    const DgFold fl = dg_fold_layout(B, true);
+    const DgWork w = dg_work((char*)work, B, chunk, mode != kReal);
+    for (int f0 = 0; f0 < batch; f0 += chunk) {
+        const int n = std::min(chunk, batch - f0), ff = n * dg_fields(mode);
+        const size_t g0 = (size_t)f0 * S * S, c0 = (size_t)f0 * B * B;
+        S2G_CUDA(cudaMemsetAsync(w.ef, 0, (size_t)ff * 4, st));
+        {
+            ProfScope ps_("dg_coefmax", st);
+            k_dg_coefmax<<<(n * B + 7) / 8, 256, 0, st>>>(rc + c0, ic + c0, B, n, mode, w.cr, w.ci, w.ex);
+        }
+        S2G_CUDA(cudaGetLastError());
+        DgArgs p{};
+        p.B = B;
+        p.S = S;
+        p.N = n;
+        p.mode = mode;
+        p.BP = B + (B & 1);
+        p.RL = fl.len;
+        p.X = w.X;
+        p.Z = w.Z;
+        p.ncols = ff * 2;
+        p.in_r = mode == kReal ? rc + c0 : w.cr;
+        p.in_i = mode == kReal ? ic + c0 : w.ci;
+        p.ein = w.ex;
+        p.emax = w.ef;
+        S2G_TRY(launch_dg<kI1>(d, p, st));
+        p.ncols = ff * S;
+        p.ein = w.ef;
+        S2G_TRY(launch_dg<kI2>(d, p, st));
+        if (B % 2 == 0) {
+            ProfScope ps_("dg_mid", st);
+            k_dg_mid<<<(ff * S + 31) / 32, dim3(32, 8), 0, st>>>((const double*)w.X, B, ff * S, w.mid);
+            S2G_CUDA(cudaGetLastError());
+        }
+        {
+            ProfScope ps_("dg_unfold", st);
+            k_dg_unfold<<<dim3(B, ff), 128, 0, st>>>(w.Z, w.mid, w.ef, B, n, d->t[kI2].h[0].vb + d->t[kI2].h[0].tb, fl,
+                                                    rdata + g0,
+                                                    idata ? idata + g0 : nullptr);
+        }
+        S2G_CUDA(cudaGetLastError());
+    }
+    return S2G_OK;
+}
+
+int dg_status(const Tables* t, int clear) {
+    const DgTabs* d = (const DgTabs*)t->dg;
+    if (!d) return S2G_OK;
+    int v = 0;
+    S2G_CUDA(cudaMemcpy(&v, d->err, sizeof(int), cudaMemcpyDeviceToHost));
+    if (clear && v) S2G_CUDA(cudaMemset(d->err, 0, sizeof(int)));
+    if (v) return fail(v, "a bounded wait in the digit-product kernel expired");
+    return S2G_OK;
+}
+
+}  // namespace s2g

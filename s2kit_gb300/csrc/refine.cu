@@ -57,13 +57,14 @@ size_t refine_io_bytes(int bw, int batch) {
 }
 
 size_t refine_work_bytes(int bw, int batch) {
-    return std::max(split_work_bytes(bw, batch), f64_work_bytes(bw, batch, REAL) + 256);
+    return std::max(split_work_bytes(bw, batch), f64_plan_bytes(bw, batch, REAL, false) + 256);
 }
 
 int fst_refined(Tables* t, const double* grid, double* rc, double* ic, int batch, int precision, void* io,
                 void* work, cudaStream_t st) {
     const int B = t->bw;
     const size_t ng = 4 * (size_t)B * B * batch, nc = (size_t)B * B * batch;
+    S2G_TRY(dg_prepare(t, st));
     char* p = (char*)io;
     float* g32 = (float*)p;
     p += rnd(4 * ng);
@@ -91,6 +92,7 @@ int inv_fst_refined(Tables* t, const double* rc, const double* ic, double* grid,
                     void* work, cudaStream_t st) {
     const int B = t->bw;
     const size_t ng = 4 * (size_t)B * B * batch, nc = (size_t)B * B * batch;
+    S2G_TRY(dg_prepare(t, st));
     char* p = (char*)io;
     float* g32 = (float*)p;
     p += rnd(4 * ng);

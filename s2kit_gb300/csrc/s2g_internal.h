@@ -59,6 +59,9 @@ struct Tables {
     double2* tw_D = nullptr;    // exp(i pi k / (2 * 2bw)), k < 2bw (DCT pre/post twiddle)
     // split-precision (tensor core) operands, built on first use
     void* split = nullptr;
+    // digit tables of the tensor-core FP64 path (digit_gemm.cu), built on first use
+    void* dg = nullptr;
+    bool dg_off = false;        // they did not fit in device memory
     int refs = 0;               // references (cache, plans, groups, calls in flight); under the cache lock
 };
 
@@ -107,6 +110,18 @@ struct F64Work {
     int rows;    // rows per function in X (bw for REAL, 2bw for COMPLEX)
 };
 size_t f64_work_bytes(int bw, int batch, int data_format);
+// The same for calls that may take the digit path (dg_prepare); two: the data have imaginary parts.
+size_t f64_plan_bytes(int bw, int batch, int data_format, bool two);
+// ---- FP64 transforms as exact digit products on the tensor cores (digit_gemm.cu) ----
+bool dg_takes(int bw);
+size_t dg_work_bytes(int bw, int batch, bool two);
+int dg_prepare(Tables* t, cudaStream_t st);
+void dg_put(void* dg);
+int dg_status(const Tables* t, int clear);
+int fst_f64_dg(const Tables* t, const double* rdata, const double* idata, double* rc, double* ic, int batch,
+               int data_format, void* work, cudaStream_t st);
+int inv_fst_f64_dg(const Tables* t, const double* rc, const double* ic, double* rdata, double* idata, int batch,
+                   int data_format, void* work, cudaStream_t st);
 int fst_f64(const Tables* t, const double* rdata, const double* idata, double* rc, double* ic, int batch,
             int data_format, int cutoff, void* work, cudaStream_t st);
 // fst_f64 with the DFT geometry of length 2bw (Bluestein tables included when 2bw is not a

@@ -17,6 +17,7 @@
 // The real-field fast path (no imaginary samples) packs two latitudes into one complex DFT.
 #include <math.h>
 
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <vector>
@@ -599,8 +600,14 @@ size_t f64_work_bytes(int bw, int batch, int data_format) {
     return 2 * (size_t)batch * rows * S * sizeof(double);
 }
 
+size_t f64_plan_bytes(int bw, int batch, int data_format, bool two) {
+    const size_t plain = f64_work_bytes(bw, batch, data_format);
+    return dg_takes(bw) ? std::max(plain, dg_work_bytes(bw, batch, two || data_format == COMPLEX)) : plain;
+}
+
 int fst_f64(const Tables* t, const double* rdata, const double* idata, double* rc, double* ic, int batch,
             int data_format, int cutoff, void* work, cudaStream_t st) {
+    if (t->dg) return fst_f64_dg(t, rdata, idata, rc, ic, batch, data_format, work, st);
     return fst_f64_len(t, nullptr, rdata, idata, rc, ic, batch, data_format, cutoff, work, st);
 }
 
@@ -635,6 +642,7 @@ int fst_f64_len(const Tables* t, const Len* len_S, const double* rdata, const do
 
 int inv_fst_f64(const Tables* t, const double* rc, const double* ic, double* rdata, double* idata, int batch,
                 int data_format, int cutoff, void* work, cudaStream_t st) {
+    if (t->dg) return inv_fst_f64_dg(t, rc, ic, rdata, idata, batch, data_format, work, st);
     const int B = t->bw, S = 2 * B;
     const int rows = (data_format == COMPLEX) ? S : B;
     double* Fr = (double*)work;

@@ -85,6 +85,17 @@ __device__ __forceinline__ bool named_bar_and(int id, int n, bool v) {
     return r != 0;
 }
 
+// One lane of a converged warp (the same one each time).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(r));
+    return r != 0;
+}
+
 // Bounded wait for the phase with the given parity to complete.  Returns false after
 // `budget` SM clock cycles (about half a second at the default budget).
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long long budget = 1000000000LL) {

@@ -1,0 +1,121 @@
+"""The FP64 plan transforms on the tensor cores (exact digit products, csrc/digit_gemm.cu) against the
+oracle, at the sizes where tiles, folds and column blocks have remainders.
+
+Tolerance: the digit path rounds operands to 53 bits and more of their row's largest value, a few
+1e-15 normwise; the oracle's recurrence adds up to 1e-13 at these bandwidths, so 1e-12 holds for both.
+"""
+import numpy as np
+import pytest
+
+from s2kit_gb300 import api
+from tests._util import degree_of_index, real_field_coeffs, rel_err_norm
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-12
+
+
+def _run(bw, nb, mode, cutoff, rc, ic, gr, gi, shift=0):
+    """Inverse of (rc, ic) and forward of (gr, gi); device buffers start `shift` doubles into an allocation."""
+    import torch
+
+    def dev(x):
+        t = torch.full((x.size + shift,), 7.0, dtype=torch.float64, device="cuda")
+        t[shift:] = torch.from_numpy(np.ascontiguousarray(x)).cuda().reshape(-1)
+        return t[shift:]
+
+    fmt = api.COMPLEX if mode == "complex" else api.REAL
+    two = mode != "real"
+    plan = api.Plan(bw, cutoff)
+    n, c = 4 * bw * bw, bw * bw
+    og, oc = [dev(np.full((nb, n), 7.0)) for _ in range(2)], [dev(np.full((nb, c), 7.0)) for _ in range(2)]
+    plan.inv_fst(dev(rc), dev(ic), og[0], og[1] if two else None, nb, fmt)
+    plan.fst(dev(gr), dev(gi) if two else None, oc[0], oc[1], nb, fmt)
+    torch.cuda.synchronize()
+    plan.sync_status()
+    og, oc = [g.cpu().numpy().reshape(nb, n) for g in og], [x.cpu().numpy().reshape(nb, c) for x in oc]
+    if not two:
+        assert (og[1] == 7.0).all()
+        og[1] = np.zeros_like(og[0])
+    return og, oc
+
+
+def _data(bw, nb, mode):
+    rng = np.random.default_rng(bw * 1000 + nb)
+    rc, ic = real_field_coeffs(rng, bw, 1.0, nb)
+    if mode == "complex":
+        rc, ic = rng.standard_normal(rc.shape), rng.standard_normal(rc.shape)
+    elif mode == "imag":  # REAL with imaginary arrays: Im f(l, 0) counts
+        ic += (degree_of_index(bw)[1] == 0) * rng.standard_normal(ic.shape)
+    gr = rng.standard_normal((nb, 4 * bw * bw))
+    gi = rng.standard_normal(gr.shape) if mode != "real" else np.zeros_like(gr)
+    return rc, ic, gr, gi
+
+
+@pytest.mark.parametrize("bw,nb,mode,cutoff", [
+    (9, 1, "complex", 9), (12, 9, "real", 5), (15, 70, "real", 15), (31, 3, "complex", 31), (32, 8, "real", 32),
+    (33, 17, "imag", 20), (34, 16, "complex", 34), (64, 33, "real", 64), (100, 5, "imag", 100), (127, 2, "real", 64),
+    (130, 9, "complex", 130), (255, 1, "real", 255), (256, 1, "imag", 256), (256, 40, "real", 256),
+    (257, 2, "real", 257), (258, 1, "complex", 200), (511, 1, "real", 511), (512, 1, "real", 512)])
+def test_digit_path_matches_oracle(oracle, bw, nb, mode, cutoff):
+    rc, ic, gr, gi = _data(bw, nb, mode)
+    og, oc = _run(bw, nb, mode, cutoff, rc, ic, gr, gi)
+    fmt = api.COMPLEX if mode == "complex" else api.REAL
+    for f in {0, nb // 2, nb - 1}:
+        er, ei = oracle.inv_fst(rc[f], ic[f], bw, fmt, cutoff)
+        assert rel_err_norm(og[0][f], og[1][f], er, ei if mode != "real" else 0.0) <= TOL
+        # the samples are noise: the oracle's naive form (cutoff 1), since the seminaive form's tables are
+        # themselves up to 3e-12 off at order 1 on samples that are not band-limited
+        er, ei = oracle.fst(gr[f], gi[f], bw, fmt, 1)
+        assert rel_err_norm(oc[0][f], oc[1][f], er, ei) <= TOL
+
+
+def test_digit_path_unaligned_buffers():
+    """8-byte aligned device pointers give the same bits as 16-byte aligned ones."""
+    for mode in ("real", "imag", "complex"):
+        d = _data(40, 3, mode)
+        a, b = _run(40, 3, mode, 40, *d), _run(40, 3, mode, 40, *d, shift=1)
+        for x, y in zip(a[0] + a[1], b[0] + b[1]):
+            assert (x == y).all()
+
+
+@pytest.mark.parametrize("bw", [33, 64])
+def test_digit_path_special_values(oracle, bw):
+    """A NaN or an infinity stays within its function; zeros, tiny and huge scales keep their precision."""
+    rc, ic, gr, gi = _data(bw, 5, "real")
+    gr[1, 7] = np.nan
+    gr[2, bw] = np.inf
+    rc[1, 3], ic[2, bw + 2] = np.nan, -np.inf
+    gr[3], rc[3], ic[3] = 0.0, 0.0, 0.0
+    rc[4], ic[4], gr[4] = rc[4] * 1e-290, ic[4] * 1e-290, gr[4] * 1e290
+    og, oc = _run(bw, 5, "real", bw, rc, ic, gr, gi)
+    for f in (1, 2):
+        assert np.isnan(og[0][f]).all() and np.isnan(oc[0][f]).all()
+    assert (og[0][3] == 0).all() and (oc[0][3] == 0).all() and (oc[1][3] == 0).all()
+    for f in (0, 4):
+        er, _ = oracle.inv_fst(rc[f], ic[f], bw, api.REAL, bw)
+        assert rel_err_norm(og[0][f], 0 * er, er, 0 * er) <= TOL
+        s = 1e-290 if f == 4 else 1.0  # the metric squares its arguments
+        er, ei = oracle.fst(gr[f], gi[f], bw, api.REAL, bw)
+        assert rel_err_norm(oc[0][f] * s, oc[1][f] * s, er * s, ei * s) <= TOL
+
+
+def test_digit_path_under_capture():
+    """A captured call on a warm plan replays with new inputs; a capture before the first call still works."""
+    import torch
+    bw, nb = 48, 4
+    d = _data(bw, nb, "real")
+    gr = torch.from_numpy(d[2]).cuda()
+    rc, ic = (torch.empty(nb, bw * bw, dtype=torch.float64, device="cuda") for _ in range(2))
+    plan = api.Plan(bw, bw)
+    plan.fst(gr, None, rc, ic, nb, api.REAL)
+    want = [rc.clone(), ic.clone()]
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=s):
+        plan.fst(gr, None, rc, ic, nb, api.REAL, stream=s)
+    gr.mul_(2.0)
+    graph.replay()
+    torch.cuda.synchronize()
+    plan.sync_status()
+    assert (rc == 2 * want[0]).all() and (ic == 2 * want[1]).all()
