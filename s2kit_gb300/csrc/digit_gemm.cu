@@ -1143,7 +1143,9 @@ static void dg_tiles(DgTable& t, int stage, int B) {
             tl.ks = std::max(1, (k + 15) / 16);  // no degree of a parity: one zero step
             // F1's data have vbz bits and folds; I2's sums of eight parts stay below 2^63
             tl.vb = stage == kI2 ? (k <= 128 ? 55 : k <= 256 ? 54 : 53) : (stage == kI1 ? (k <= 256 ? 55 : 54) : (k <= 256 ? 56 : 54));
-            tl.tb = dg_table_bits(k, stage == kF1 ? (dg_vbz(B) >= 53 ? 56 : 54) : tl.vb, stage == kI2);
+            // the panels of F1 share one scale
+            if (stage == kF1) tl.tb = dg_table_bits(B % 2 ? B + 1 : B / 2 + 1, dg_vbz(B) >= 53 ? 56 : 54, false);
+            else tl.tb = dg_table_bits(k, tl.vb, stage == kI2);
             tl.off = t.bytes;
             t.bytes += (int64_t)tl.ks * kDigits * tl.r8 * 32;
             t.h.push_back(tl);

@@ -53,7 +53,7 @@ def _data(bw, nb, mode):
 
 @pytest.mark.parametrize("bw,nb,mode,cutoff", [
     (9, 1, "complex", 9), (12, 9, "real", 5), (15, 70, "real", 15), (31, 3, "complex", 31), (32, 8, "real", 32),
-    (33, 17, "imag", 20), (34, 16, "complex", 34), (64, 33, "real", 64), (100, 5, "imag", 100), (127, 2, "real", 64),
+    (33, 17, "imag", 20), (34, 16, "complex", 34), (48, 9, "real", 48), (96, 2, "imag", 96), (64, 33, "real", 64), (100, 5, "imag", 100), (127, 2, "real", 64),
     (130, 9, "complex", 130), (255, 1, "real", 255), (256, 1, "imag", 256), (256, 40, "real", 256),
     (257, 2, "real", 257), (258, 1, "complex", 200), (511, 1, "real", 511), (512, 1, "real", 512)])
 def test_digit_path_matches_oracle(oracle, bw, nb, mode, cutoff):
