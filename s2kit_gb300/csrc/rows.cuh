@@ -19,13 +19,18 @@ namespace s2g {
 template <typename T, typename T2>
 __global__ void k_rows_fwd(const T* __restrict__ rdata, const T* __restrict__ idata,
                            T* __restrict__ Xr, T* __restrict__ Xi, int S, const Len L, int rows_out, int R,
-                           T scale, const T2* __restrict__ tw) {
+                           T scale, const T2* tw) {
     extern __shared__ __align__(16) unsigned char sm_raw[];
     T* sm = reinterpret_cast<T*>(sm_raw);
     const int SP = S + 1;
     T* re = sm;
     T* im = re + (size_t)R * SP;
     T* tmp = im + (size_t)R * SP;
+    if (L.pow2()) {  // one latency for all stages' twiddles (the DFT needs no tmp)
+        T2* t = reinterpret_cast<T2*>(tmp + ((size_t)(2 * R * SP) & 1));
+        for (int k = threadIdx.x; k < S / 2; k += blockDim.x) t[k] = tw[k];
+        tw = t;
+    }
     const int f = blockIdx.y;
     const bool real_mode = (idata == nullptr);
     const int lat_per_cta = real_mode ? 2 * R : R;
@@ -84,7 +89,7 @@ __global__ void k_rows_fwd(const T* __restrict__ rdata, const T* __restrict__ id
 template <typename T, typename T2>
 __global__ void k_rows_inv(const T* __restrict__ Fr, const T* __restrict__ Fi, int frows, int fmt_complex,
                            T* __restrict__ rdata, T* __restrict__ idata, int S, const Len L, int R,
-                           const T2* __restrict__ tw) {
+                           const T2* tw) {
     extern __shared__ __align__(16) unsigned char sm_raw[];
     T* sm = reinterpret_cast<T*>(sm_raw);
     const int B = S / 2;
@@ -92,6 +97,11 @@ __global__ void k_rows_inv(const T* __restrict__ Fr, const T* __restrict__ Fi, i
     T* re = sm;
     T* im = re + (size_t)R * SP;
     T* tmp = im + (size_t)R * SP;
+    if (L.pow2()) {  // one latency for all stages' twiddles (the DFT needs no tmp)
+        T2* t = reinterpret_cast<T2*>(tmp + ((size_t)(2 * R * SP) & 1));
+        for (int k = threadIdx.x; k < S / 2; k += blockDim.x) t[k] = tw[k];
+        tw = t;
+    }
     const int f = blockIdx.y;
     const bool real_out = (idata == nullptr);
     const int lat_per_cta = real_out ? 2 * R : R;

@@ -85,7 +85,7 @@ __global__ void k_fwd_dlt(FwdDlt p) {
     extern __shared__ double sm[];
     const int B = p.B, S = p.S;
     const Len L = p.L;
-    const int Ge = (p.G + 1) & ~1;
+    const int Ge = p.G == 1 ? 1 : (p.G + 1) & ~1;
     int row, m;
     bool neg = false;
     if (p.one_d) {
@@ -108,6 +108,12 @@ __global__ void k_fwd_dlt(FwdDlt p) {
     const int clen = semi ? B : S;  // per function per part
     double* cre = cbuf;                          // [Ge][clen]
     double* cim = cbuf + (size_t)Ge * clen;      // [Ge][clen]
+    const double2* twS = p.twS;
+    if (p.G == 1 && semi && L.pow2()) {  // one latency for all stages' twiddles
+        double2* t = (double2*)(cim + clen);
+        for (int k = threadIdx.x; k < S / 2; k += blockDim.x) t[k] = p.twS[k];
+        twS = t;
+    }
     const double* w = p.w + ((semi && (m & 1)) ? S : 0);
     const int xrow = p.one_d ? 0 : row;
 
@@ -137,7 +143,7 @@ __global__ void k_fwd_dlt(FwdDlt p) {
             zi[L.pos(d)] = xi ? xi[q] * w[q] : 0.0;
         }
         __syncthreads();
-        block_dft<double, double2>(zr, zi, L, 1, S, p.twS, -1.0, tmp);
+        block_dft<double, double2>(zr, zi, L, 1, S, twS, -1.0, tmp);
         // REDFT10 of both parts, c[0] *= sqrt(1/2), c *= 1/sqrt(2S)   (seminaive.c:170-176)
         const double nrm = 1.0 / sqrt(2.0 * S);
         for (int k = threadIdx.x; k < B; k += blockDim.x) {
@@ -158,6 +164,48 @@ __global__ void k_fwd_dlt(FwdDlt p) {
     const int nch = Ge / 2;
     const int64_t tab0 = p.off ? p.off[m] : 0;
     const double* tab = p.tab + tab0;
+    auto store = [&](int li, int f, double vr, double vi) {
+        const int l = m + li;
+        double* rc = p.rc + (size_t)f * p.c_stride;
+        double* ic = p.ic ? p.ic + (size_t)f * p.c_stride : nullptr;
+        const int idx = p.one_d ? li : index_of_harmonic_coeff(neg ? -m : m, l, B);
+        rc[idx] = vr;
+        if (ic) ic[idx] = vi;
+        if (p.real_mirror && m > 0) {
+            const int i2 = index_of_harmonic_coeff(-m, l, B);
+            const double s = (m & 1) ? -1.0 : 1.0;
+            rc[i2] = s * vr;
+            if (ic) ic[i2] = -s * vi;
+        }
+    };
+    if (p.G == 1) {
+        // one function: eight lanes per degree along the table row, gridDim.z blocks sharing the degrees (a
+        // thread per degree leaves the row's loads uncoalesced and one after another: bw 64 21.6 us, now 11.8;
+        // one order at bw 256 154 us, now 20)
+        const int sub = threadIdx.x & 7, per = blockDim.x >> 3;
+        for (int l0 = blockIdx.z * per; l0 < nrows; l0 += gridDim.z * per) {
+            const int li = l0 + (threadIdx.x >> 3);
+            double a0 = 0.0, a1 = 0.0;
+            if (li < nrows) {
+                const int n = semi ? row_size(m, m + li) : S, st = semi ? 2 : 1;
+                const double* trow = semi ? tab + table_offset(m, m + li) : tab + (size_t)li * S;
+                const double* c0 = cre + (semi ? (li & 1) : 0);
+                const double* c1 = cim + (semi ? (li & 1) : 0);
+#pragma unroll 4
+                for (int j = sub; j < n; j += 8) {
+                    const double v = trow[j];
+                    a0 = fma(v, c0[st * j], a0);
+                    a1 = fma(v, c1[st * j], a1);
+                }
+            }
+            for (int o = 4; o; o >>= 1) {
+                a0 += __shfl_xor_sync(0xffffffffu, a0, o);
+                a1 += __shfl_xor_sync(0xffffffffu, a1, o);
+            }
+            if (li < nrows && sub == 0) store(li, f0, sgn * a0, sgn * a1);
+        }
+        return;
+    }
     for (int task = threadIdx.x; task < nrows * nch; task += blockDim.x) {
         const int li = task % nrows, ch = task / nrows;
         const int l = m + li;
@@ -196,18 +244,7 @@ __global__ void k_fwd_dlt(FwdDlt p) {
             const int g = g0 + h;
             const int f = f0 + g;
             if (g >= p.G || f >= p.nfunc) continue;
-            const double vr = sgn * (h ? a2 : a0), vi = sgn * (h ? a3 : a1);
-            double* rc = p.rc + (size_t)f * p.c_stride;
-            double* ic = p.ic ? p.ic + (size_t)f * p.c_stride : nullptr;
-            const int idx = p.one_d ? li : index_of_harmonic_coeff(neg ? -m : m, l, B);
-            rc[idx] = vr;
-            if (ic) ic[idx] = vi;
-            if (p.real_mirror && m > 0) {
-                const int i2 = index_of_harmonic_coeff(-m, l, B);
-                const double s = (m & 1) ? -1.0 : 1.0;
-                rc[i2] = s * vr;
-                if (ic) ic[i2] = -s * vi;
-            }
+            store(li, f, sgn * (h ? a2 : a0), sgn * (h ? a3 : a1));
         }
     }
 }
@@ -236,7 +273,7 @@ __global__ void k_inv_dlt(InvDlt p) {
     extern __shared__ double sm[];
     const int B = p.B, S = p.S;
     const Len L = p.L;
-    const int Ge = (p.G + 1) & ~1;
+    const int Ge = p.G == 1 ? 1 : (p.G + 1) & ~1;
     int row, m;
     bool neg = false;
     if (p.one_d) {
@@ -262,6 +299,12 @@ __global__ void k_inv_dlt(InvDlt p) {
     double* fim = fre + (size_t)Ge * B;
     int* toff = (int*)(fim + (size_t)Ge * B);     // B + 1 ints
     int* wtot = toff + B + 1;                     // 32 ints
+    const double2* twS = p.twS;
+    if (p.G == 1 && semi && L.pow2()) {  // one latency for all stages' twiddles
+        double2* t = (double2*)(((uintptr_t)(wtot + 32) + 15) & ~(uintptr_t)15);
+        for (int k = threadIdx.x; k < S / 2; k += blockDim.x) t[k] = p.twS[k];
+        twS = t;
+    }
 
     for (int t = threadIdx.x; t < Ge * nl; t += blockDim.x) {
         const int g = t / nl, li = t - g * nl;
@@ -279,6 +322,21 @@ __global__ void k_inv_dlt(InvDlt p) {
     const double* tab = p.tab + tab0;
     const int nch = Ge / 2;
 
+    if (!semi && Ge == 1) {
+        __syncthreads();
+        for (int q = threadIdx.x; q < S; q += blockDim.x) {
+            double a0 = 0.0, a1 = 0.0;
+            for (int li = 0; li < nl; ++li) {
+                const double v = tab[(size_t)li * S + q];
+                a0 = fma(are[li], v, a0);
+                a1 = fma(aim[li], v, a1);
+            }
+            const size_t o = ((size_t)f0 * p.frows + (p.one_d ? 0 : row)) * S + q;
+            p.Fr[o] = sgn * a0;
+            if (p.Fi) p.Fi[o] = sgn * a1;
+        }
+        return;
+    }
     if (!semi) {
         __syncthreads();
         // naive synthesis: F[q] = sum_l a[l-m] P(m,l)(x_q)
@@ -311,7 +369,34 @@ __global__ void k_inv_dlt(InvDlt p) {
 
     const double scale = 0.5 / sqrt((double)B);
     const double scale0 = 1.0 / sqrt((double)S);
-    for (int task = threadIdx.x; task < B * nch; task += blockDim.x) {
+    if (Ge == 1) {  // as in k_fwd_dlt: eight lanes per frequency along the transposed table's row
+        const int sub = threadIdx.x & 7;
+        for (int i0 = 0; i0 < B; i0 += blockDim.x >> 3) {
+            const int i = i0 + (threadIdx.x >> 3);
+            const int rs = i < B ? transpose_row_size(i, m, B) : 0;
+            double a0 = 0.0, a1 = 0.0;
+            if (rs > 0) {
+                const int base = trans_first_l(i, m) - m;
+                const double* trow = tab + toff[i];
+#pragma unroll 4
+                for (int j = sub; j < rs; j += 8) {
+                    const double v = trow[j];
+                    a0 = fma(are[base + 2 * j], v, a0);
+                    a1 = fma(aim[base + 2 * j], v, a1);
+                }
+            }
+            for (int o = 4; o; o >>= 1) {
+                a0 += __shfl_xor_sync(0xffffffffu, a0, o);
+                a1 += __shfl_xor_sync(0xffffffffu, a1, o);
+            }
+            if (i < B && sub == 0) {
+                const double s = (i == 0) ? scale0 : scale;
+                fre[i] = a0 * s;
+                fim[i] = a1 * s;
+            }
+        }
+    }
+    for (int task = threadIdx.x; Ge > 1 && task < B * nch; task += blockDim.x) {
         const int i = task % B, ch = task / B;
         const int g0 = 2 * ch;
         const int rs = transpose_row_size(i, m, B);
@@ -355,7 +440,7 @@ __global__ void k_inv_dlt(InvDlt p) {
             zi[L.pos(k)] = wr * s + wi * c;
         }
         __syncthreads();
-        block_dft<double, double2>(zr, zi, L, 1, S, p.twS, 1.0, tmp);
+        block_dft<double, double2>(zr, zi, L, 1, S, twS, 1.0, tmp);
         const size_t ob = ((size_t)f * p.frows + (p.one_d ? 0 : row)) * S;
         for (int q = threadIdx.x; q < S; q += blockDim.x) {
             const int src = (q & 1) ? S - 1 - (q >> 1) : (q >> 1);
@@ -417,11 +502,31 @@ __global__ void k_transmult(const double* __restrict__ rd, const double* __restr
 // ------------------------------------------------------------------------------------
 // Host-side launchers.
 
-static int rows_per_cta(int S) {
+static int sm_count() {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 152;
+    return n;
+}
+
+// Sequences of length S per block, of nseq in all: up to 4096 values, but no more than leave two blocks
+// for each SM (one function at bw 64 in blocks of 32 rows took 2 to 4 SMs and 48 us).
+static int rows_per_cta(int S, int64_t nseq) {
     int R = 4096 / S;
     if (R < 1) R = 1;
     if (R > 32) R = 32;
+    const int want = 2 * sm_count();
+    while (R > 1 && nseq / R < want) R >>= 1;
     return R;
+}
+
+// Functions per block of the DLT kernels, at most G: fewer where the blocks would not fill the GPU (8 for
+// one function spent 7/8 of the contraction on zeros).  1, or even.
+static int fill_group(int G, int nrows, int nfunc) {
+    if (nfunc == 1) return 1;
+    const int want = 2 * sm_count();
+    while (G > 2 && (int64_t)nrows * ((nfunc + G - 1) / G) < want) G -= 2;
+    return std::min(G, (nfunc + 1) & ~1);
 }
 
 // DFT length n with, when n is not a power of two, Bluestein tables on the current device
@@ -492,7 +597,8 @@ static int dft_len(int n, Len* out) {
 }
 
 static size_t rows_smem(const Len& L, int R) {
-    return ((size_t)2 * R * (L.n + 1) + L.tmp_len()) * sizeof(double);
+    // sequences, Bluestein scratch or the twiddles of all stages (k_rows_*)
+    return ((size_t)2 * R * (L.n + 1) + L.tmp_len() + (L.pow2() ? L.n + 2 : 0)) * sizeof(double);
 }
 
 // `given`: the geometry of length 2B (with its Bluestein tables) built by the caller; null looks
@@ -505,7 +611,7 @@ static int launch_rows_fwd(const double* rdata, const double* idata, double* Xr,
         L = *given;
     else
         S2G_TRY(dft_len(S, &L));
-    const int R = rows_per_cta(S);
+    const int R = rows_per_cta(S, (int64_t)batch * (idata ? S : S / 2));
     const int lat_per = idata ? R : 2 * R;
     const size_t smem = rows_smem(L, R);
     S2G_TRY(set_smem((const void*)k_rows_fwd<double, double2>, smem));
@@ -518,13 +624,14 @@ static int launch_rows_fwd(const double* rdata, const double* idata, double* Xr,
     return S2G_OK;
 }
 
-static int pick_group(int B, int S, bool naive, int tmp_len, size_t* smem_out, size_t per_g_extra = 0) {
+static int pick_group(int B, int S, bool naive, int tmp_len, int nrows, int nfunc, size_t* smem_out) {
     const size_t fixed = ((size_t)2 * S + tmp_len) * sizeof(double);
-    const size_t per_g = (size_t)2 * (naive ? S : B) * sizeof(double) + per_g_extra;
+    const size_t per_g = (size_t)2 * (naive ? S : B) * sizeof(double);
     const size_t budget = 160 * 1024;
     int G = 8;
     while (G > 2 && fixed + (size_t)G * per_g > budget) G -= 2;
     if (fixed + (size_t)G * per_g > 220 * 1024) return 0;
+    G = fill_group(G, nrows, nfunc);
     *smem_out = fixed + (size_t)G * per_g;
     return G;
 }
@@ -537,12 +644,15 @@ static int launch_fwd_dlt(FwdDlt p, int nrows_grid, cudaStream_t st, const Len* 
         S2G_TRY(dft_len(p.S, &L));
     size_t smem = 0;
     const bool any_naive = p.one_d ? (p.m1d >= p.cutoff) : (p.cutoff < p.B);
-    const int G = pick_group(p.B, p.S, any_naive, L.tmp_len(), &smem);
+    const int G = pick_group(p.B, p.S, any_naive, L.tmp_len(), nrows_grid, p.nfunc, &smem);
     if (!G) return fail(S2G_ERR_UNSUPPORTED, "bandwidth %d too large for the FP64 DLT kernel", p.B);
     p.G = G;
     p.L = L;
+    if (G == 1 && L.pow2()) smem += (size_t)p.S * sizeof(double);
     S2G_TRY(set_smem((const void*)k_fwd_dlt, smem));
-    dim3 grid(nrows_grid, (p.nfunc + G - 1) / G);
+    // one order (FZT, DLTSemi) or few: blocks that each repeat the DCT and share the degrees
+    const int split = G == 1 ? std::max(1, std::min({8, sm_count() / nrows_grid, (p.B + 31) / 32})) : 1;
+    dim3 grid(nrows_grid, (p.nfunc + G - 1) / G, split);
     {
         ProfScope ps_("fwd_dlt_f64", st);
         k_fwd_dlt<<<grid, 256, smem, st>>>(p);
@@ -560,8 +670,10 @@ static int launch_inv_dlt(InvDlt p, int nrows_grid, cudaStream_t st) {
     const size_t per_g = (size_t)4 * p.B * sizeof(double);
     int G = 8;
     while (G > 2 && fixed + (size_t)G * per_g > 160 * 1024) G -= 2;
-    const size_t smem = fixed + (size_t)G * per_g;
-    if (smem > 220 * 1024) return fail(S2G_ERR_UNSUPPORTED, "bandwidth %d too large for the FP64 DLT kernel", p.B);
+    if (fixed + (size_t)G * per_g > 220 * 1024)
+        return fail(S2G_ERR_UNSUPPORTED, "bandwidth %d too large for the FP64 DLT kernel", p.B);
+    G = fill_group(G, nrows_grid, p.nfunc);
+    const size_t smem = fixed + (size_t)G * per_g + (G == 1 && L.pow2() ? (size_t)p.S * sizeof(double) + 16 : 0);
     p.G = G;
     p.L = L;
     S2G_TRY(set_smem((const void*)k_inv_dlt, smem));
@@ -580,7 +692,7 @@ static int launch_rows_inv(const double* Fr, const double* Fi, int rows, int dat
     const int S = 2 * B;
     Len L;
     S2G_TRY(dft_len(S, &L));
-    const int R = rows_per_cta(S);
+    const int R = rows_per_cta(S, (int64_t)batch * (idata ? S : S / 2));
     const int lat_per = idata ? R : 2 * R;
     const size_t smem = rows_smem(L, R);
     S2G_TRY(set_smem((const void*)k_rows_inv<double, double2>, smem));
