@@ -297,6 +297,41 @@ static void report(const char* fn, int r) {
     if (r != S2G_OK) fprintf(stderr, "s2kit_gb300: %s failed (%d): %s\n", fn, r, g_last_error.c_str());
 }
 
+// True where kernels can address any host memory through the host's page tables (Grace hosts): the
+// drop-ins' kernels then read the caller's samples and coefficients, and write the results, over the
+// host link, instead of a copy call for each array (8 to 10 us a call up to 256 KB; the kernels' own
+// accesses reach the same 200 GB/s).  Elsewhere the arrays are copied.
+static bool host_direct() {
+    static std::atomic<int> known[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return false;
+    int k = known[dev].load(std::memory_order_relaxed);
+    if (!k) {
+        int a = 0, b = 0;
+        cudaDeviceGetAttribute(&a, cudaDevAttrPageableMemoryAccess, dev);
+        cudaDeviceGetAttribute(&b, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev);
+        k = a && b ? 2 : 1;
+        known[dev].store(k, std::memory_order_relaxed);
+    }
+    return k == 2;
+}
+
+// Results computed in device scratch (scattered writes) -> the caller's arrays.
+__global__ void k_to_host(const double* __restrict__ a, const double* __restrict__ b, double* ha, double* hb, size_t n) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        ha[i] = a[i];
+        hb[i] = b[i];
+    }
+}
+static int to_host(const double* a, const double* b, double* ha, double* hb, size_t n) {
+    {
+        ProfScope ps_("to_host", 0);
+        k_to_host<<<(unsigned)std::min<size_t>((n + 255) / 256, 608), 256>>>(a, b, ha, hb, n);
+    }
+    S2G_CUDA(cudaGetLastError());
+    return S2G_OK;
+}
+
 // ---------------------------------------------------------------------------------
 // Drop-in implementations (return a status; the exported void wrappers print it).
 
@@ -320,16 +355,27 @@ static int do_fst(double* rdata, double* idata, double* rcoeffs, double* icoeffs
     Carve c{(char*)g_dscratch.s.ptr};
     double *dr = c.take(ng), *di = c.take(ng), *cr = c.take(nc), *ci = c.take(nc), *dw = c.take(4 * bw);
     void* work = c.take(f64_work_bytes(bw, 1, fmt) / sizeof(double));
-    S2G_CUDA(cudaMemcpy(dr, rdata, ng * 8, cudaMemcpyHostToDevice));
-    S2G_CUDA(cudaMemcpy(di, idata, ng * 8, cudaMemcpyHostToDevice));
+    const bool direct = host_direct();
+    if (direct) {
+        dr = rdata;
+        di = idata;
+    } else {
+        S2G_CUDA(cudaMemcpy(dr, rdata, ng * 8, cudaMemcpyHostToDevice));
+        S2G_CUDA(cudaMemcpy(di, idata, ng * 8, cudaMemcpyHostToDevice));
+    }
     if (weights) {
-        S2G_CUDA(cudaMemcpy(dw, weights, 4 * (size_t)bw * 8, cudaMemcpyHostToDevice));
+        S2G_CUDA(cudaMemcpyAsync(dw, weights, 4 * (size_t)bw * 8, cudaMemcpyHostToDevice, 0));
         view.weights = dw;
     }
     if (fly)
         S2G_TRY(fst_f64_fly(&view, dr, di, cr, ci, 1, fmt, work, 0));
     else
         S2G_TRY(fst_f64(&view, dr, di, cr, ci, 1, fmt, cutoff, work, 0));
+    if (direct) {
+        S2G_TRY(to_host(cr, ci, rcoeffs, icoeffs, nc));
+        S2G_CUDA(cudaStreamSynchronize(0));
+        return S2G_OK;
+    }
     S2G_CUDA(cudaMemcpy(rcoeffs, cr, nc * 8, cudaMemcpyDeviceToHost));
     S2G_CUDA(cudaMemcpy(icoeffs, ci, nc * 8, cudaMemcpyDeviceToHost));
     return S2G_OK;
@@ -354,12 +400,24 @@ static int do_inv_fst(double* rcoeffs, double* icoeffs, double* rdata, double* i
     Carve c{(char*)g_dscratch.s.ptr};
     double *dr = c.take(ng), *di = c.take(ng), *cr = c.take(nc), *ci = c.take(nc);
     void* work = c.take(f64_work_bytes(bw, 1, fmt) / sizeof(double));
-    S2G_CUDA(cudaMemcpy(cr, rcoeffs, nc * 8, cudaMemcpyHostToDevice));
-    S2G_CUDA(cudaMemcpy(ci, icoeffs, nc * 8, cudaMemcpyHostToDevice));
+    const bool direct = host_direct();
+    if (direct) {
+        cr = rcoeffs;
+        ci = icoeffs;
+        dr = rdata;
+        di = idata;
+    } else {
+        S2G_CUDA(cudaMemcpy(cr, rcoeffs, nc * 8, cudaMemcpyHostToDevice));
+        S2G_CUDA(cudaMemcpy(ci, icoeffs, nc * 8, cudaMemcpyHostToDevice));
+    }
     if (fly)
         S2G_TRY(inv_fst_f64_fly(&view, cr, ci, dr, di, 1, fmt, work, 0));
     else
         S2G_TRY(inv_fst_f64(&view, cr, ci, dr, di, 1, fmt, cutoff, work, 0));
+    if (direct) {
+        S2G_CUDA(cudaStreamSynchronize(0));
+        return S2G_OK;
+    }
     S2G_CUDA(cudaMemcpy(rdata, dr, ng * 8, cudaMemcpyDeviceToHost));
     S2G_CUDA(cudaMemcpy(idata, di, ng * 8, cudaMemcpyDeviceToHost));
     return S2G_OK;
@@ -449,6 +507,11 @@ static int do_conv(double* rdata, double* idata, double* rfilter, double* ifilte
     Carve c{(char*)io.s.ptr};
     double *dr = c.take(ng), *di = c.take(ng), *fr = c.take(ng), *fi = c.take(ng), *orr = c.take(ng),
            *oi = c.take(ng);
+    if (host_direct()) {
+        S2G_TRY(conv_device(t, rdata, idata, rfilter, ifilter, rres, ires, 1, g_dscratch.s, 0));
+        S2G_CUDA(cudaStreamSynchronize(0));
+        return S2G_OK;
+    }
     S2G_CUDA(cudaMemcpy(dr, rdata, ng * 8, cudaMemcpyHostToDevice));
     S2G_CUDA(cudaMemcpy(di, idata, ng * 8, cudaMemcpyHostToDevice));
     S2G_CUDA(cudaMemcpy(fr, rfilter, ng * 8, cudaMemcpyHostToDevice));
