@@ -178,8 +178,11 @@ typedef struct s2g_plan_s* s2g_plan;
 int s2g_plan_create(s2g_plan* plan, int bw, int cutoff);
 int s2g_plan_destroy(s2g_plan plan);
 /* A plan for the on-the-fly family (src/FST_semi_fly.c, as the Fly drop-ins above): it holds no
- * Legendre table, only weights and twiddles.  s2g_fst, s2g_inv_fst, s2g_fzt and s2g_conv on it
- * run the on-the-fly kernels; the split-precision entry points reject it (S2G_ERR_ARG). */
+ * Legendre table, only weights, twiddles, DFT tables and per (order, node) values.  s2g_fst,
+ * s2g_inv_fst, s2g_fzt and s2g_conv on it run without one: single functions through kernels that
+ * run the recurrence themselves, batches through tables generated a few orders at a time in the
+ * plan's scratch (64 to 384 MiB by bandwidth); the split-precision entry points reject it
+ * (S2G_ERR_ARG). */
 int s2g_plan_create_fly(s2g_plan* plan, int bw);
 /* Device bytes of scratch a call with this batch needs (the plan grows its own scratch
  * on demand when the caller passes none). */

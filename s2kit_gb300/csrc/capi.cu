@@ -1128,14 +1128,27 @@ static int plan_check(s2g_plan p, int batch, bool host = false, bool fly_ok = fa
     return S2G_OK;
 }
 
+// Scratch of an FP64 transform, and whether it takes the digit path (whose tables it readies).
+static int f64_scratch(s2g_plan p, int batch, DataFormat fmt, bool imag, cudaStream_t st, bool* digits) {
+    const bool two = imag || fmt == COMPLEX;
+    if (!p->fly) {
+        S2G_TRY(dg_prepare(p->t, st));
+        *digits = p->t->dg != nullptr;
+        return p->work.ensure(f64_plan_bytes(p->bw, batch, fmt, two));
+    }
+    if (dg_fly_takes(p->bw, two ? 2 * batch : batch)) S2G_TRY(dg_prepare(p->t, st));
+    *digits = p->t->dg && dg_fly_takes(p->bw, two ? 2 * batch : batch);
+    return p->work.ensure(*digits ? dg_fly_bytes(p->t, batch, two) : f64_work_bytes(p->bw, batch, fmt));
+}
+
 int s2g_fst(s2g_plan p, const double* rdata, const double* idata, double* rcoeffs, double* icoeffs, int batch,
             DataFormat fmt, void* stream) {
     S2G_TRY(plan_check(p, batch, false, true));
     if (!rdata || !rcoeffs || !icoeffs || (fmt == COMPLEX && !idata)) return fail(S2G_ERR_ARG, "NULL argument");
-    S2G_TRY(p->work.ensure(p->fly ? f64_work_bytes(p->bw, batch, fmt)
-                                  : f64_plan_bytes(p->bw, batch, fmt, idata != nullptr)));
-    if (!p->fly) S2G_TRY(dg_prepare(p->t, (cudaStream_t)stream));
-    if (p->fly) return fst_f64_fly(p->t, rdata, idata, rcoeffs, icoeffs, batch, fmt, p->work.ptr, (cudaStream_t)stream);
+    bool digits = false;
+    S2G_TRY(f64_scratch(p, batch, fmt, idata != nullptr, (cudaStream_t)stream, &digits));
+    if (p->fly && !digits)
+        return fst_f64_fly(p->t, rdata, idata, rcoeffs, icoeffs, batch, fmt, p->work.ptr, (cudaStream_t)stream);
     return fst_f64(p->t, rdata, idata, rcoeffs, icoeffs, batch, fmt, p->cutoff, p->work.ptr, (cudaStream_t)stream);
 }
 
@@ -1143,10 +1156,9 @@ int s2g_inv_fst(s2g_plan p, const double* rcoeffs, const double* icoeffs, double
                 DataFormat fmt, void* stream) {
     S2G_TRY(plan_check(p, batch, false, true));
     if (!rdata || !rcoeffs || !icoeffs || (fmt == COMPLEX && !idata)) return fail(S2G_ERR_ARG, "NULL argument");
-    S2G_TRY(p->work.ensure(p->fly ? f64_work_bytes(p->bw, batch, fmt)
-                                  : f64_plan_bytes(p->bw, batch, fmt, idata != nullptr)));
-    if (!p->fly) S2G_TRY(dg_prepare(p->t, (cudaStream_t)stream));
-    if (p->fly)
+    bool digits = false;
+    S2G_TRY(f64_scratch(p, batch, fmt, idata != nullptr, (cudaStream_t)stream, &digits));
+    if (p->fly && !digits)
         return inv_fst_f64_fly(p->t, rcoeffs, icoeffs, rdata, idata, batch, fmt, p->work.ptr, (cudaStream_t)stream);
     return inv_fst_f64(p->t, rcoeffs, icoeffs, rdata, idata, batch, fmt, p->cutoff, p->work.ptr,
                        (cudaStream_t)stream);

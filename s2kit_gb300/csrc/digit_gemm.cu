@@ -37,6 +37,7 @@
 
 #include <map>
 #include <mutex>
+#include <tuple>
 #include <vector>
 
 #include "s2g_common.cuh"
@@ -94,15 +95,15 @@ struct DgArgs {
 
 __device__ __forceinline__ uint32_t dexp(double x) { return ((uint32_t)__double2hiint(x) >> 20) & 0x7ffu; }
 
-// x as an integer of unit 2^(em - 1022 - vb) (|x| < 2^(em - 1022)), rounded to nearest
+// x as an integer of unit 2^(em - 1022 - vb) (|x| < 2^(em - 1022), vb at most 56), rounded to nearest
 __device__ __forceinline__ long long dg_fix(double x, int em, int vb) {
     const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
     int e = (hi >> 20) & 0x7ff;
     uint32_t mh = hi & 0xfffffu;
     if (e) mh |= 0x100000u;
     else e = 1;
-    const unsigned long long mant = (((unsigned long long)mh << 32) | lo) << 3;
-    const int rs = min(em - e + 55 - vb, 63);
+    const unsigned long long mant = (((unsigned long long)mh << 32) | lo) << 4;
+    const int rs = min(em - e + 56 - vb, 63);
     const long long v = (long long)(((mant >> rs) + 1) >> 1);
     return (int)hi < 0 ? -v : v;
 }
@@ -1046,6 +1047,101 @@ __global__ void __launch_bounds__(128) k_dg_pack_leg(int B, int fwd, const DgTil
     dg_pack_rows(val, q, tab + tl.off, tl.r8, tl.ks, rg);
 }
 
+// On-the-fly family: the same tables, a chunk of orders at a time in scratch, from what a plan keeps per
+// (order, degree) and (order, node): the recurrence's coefficients ac and the first row P(m,m).
+__global__ void k_dg_fly_init(int B, const double2* __restrict__ sinn, const double2* __restrict__ seed, double2* ac,
+                              double* first) {
+    const int m = blockIdx.x;
+    for (int l = threadIdx.x; l < B; l += blockDim.x) {
+        ac[(size_t)m * B + l] = l < m ? make_double2(0.0, 0.0) : make_double2(l2_an(m, l), l2_cn(m, l));
+        first[(size_t)m * B + l] = seed[m].x * pow(sinn[l].x, (double)m);
+    }
+}
+
+// Rows l - m of P (times the weight of the node where w is given) by the FP64 recurrence: one thread per
+// node, an x off the chain, so that a degree costs one dependent multiply-add.  Near the pole the rounding
+// of x would be the largest error (d theta = dx / sin theta), so the warps there add its low part.
+// FP64-bound, three or four operations a value; one-warp blocks keep the SMs evenly loaded (bw 256: 56 us a
+// chunk of 64 MB with four-warp blocks).
+__global__ void __launch_bounds__(32) k_dg_legendre64(int B, int m0, const double2* __restrict__ cosn,
+                                                      const double2* __restrict__ ac, const double* __restrict__ first,
+                                                      const double* __restrict__ w, double wscale, double* tmp,
+                                                      const int64_t* __restrict__ off) {
+    const int m = m0 + blockIdx.x, j = min(blockIdx.y * 32 + threadIdx.x, (unsigned)B - 1);
+    const double x = cosn[j].x, xl = cosn[j].y;
+    double pc = first[(size_t)m * B + j], pp = 0.0;
+    if (w) pc *= w[j] * wscale;  // the recurrence is linear: once
+    const double2* c = ac + (size_t)m * B;
+    double* out = tmp + off[m] + j;
+    if (__any_sync(0xffffffffu, x > 0.8)) {
+#pragma unroll 4
+        for (int l = m; l < B; ++l, out += B) {
+            *out = pc;
+            const double2 k = c[l];
+            const double nx = fma(fma(k.x, x, k.x * xl), pc, k.y * pp);
+            pp = pc;
+            pc = nx;
+        }
+    } else {
+#pragma unroll 4
+        for (int l = m; l < B; ++l, out += B) {
+            *out = pc;
+            const double2 k = c[l];
+            const double nx = fma(k.x * x, pc, k.y * pp);
+            pp = pc;
+            pc = nx;
+        }
+    }
+}
+
+// Digits of those rows (degrees, or nodes for the inverse).  One block per (tile, 8-row group): eight rows
+// by sixteen runs of eight K entries.
+__global__ void __launch_bounds__(128) k_dg_pack_fly(int B, int fwd, const DgTile* __restrict__ tiles,
+                                                     const double* __restrict__ tmp, const int64_t* __restrict__ off,
+                                                     uint8_t* tab, short* qs) {
+    __shared__ uint32_t red[8][17];
+    const DgTile tl = tiles[blockIdx.x];
+    const int rg = blockIdx.y;
+    if (rg * 8 >= tl.r8) return;
+    const int r = threadIdx.x & 7, kc = threadIdx.x >> 3;
+    const bool live = rg * 8 + r < tl.nrows;
+    const int row = tl.row0 + rg * 8 + r, nl = (B - tl.m - tl.t + 1) / 2;
+    const int n = live ? (fwd ? B : nl) : 0;
+    const double* src = tmp + off[tl.m] + (fwd ? (size_t)(tl.t + 2 * row) * B : (size_t)tl.t * B + row);
+    const size_t step = fwd ? 1 : 2 * (size_t)B;
+    uint32_t mx = 0;
+    for (int k = kc * 8; k < n; k += 128)
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (k + i < n) mx = max(mx, dexp(src[step * (k + i)]));
+    red[r][kc] = mx;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) mx = max(mx, red[r][i]);
+    const int em = max((int)mx, 1);
+    if (kc == 0 && live) qs[tl.qoff + row] = (short)(tl.tb + 1022 - em);
+    const uint32_t bytes = kDigits * (uint32_t)tl.r8 * 32;
+    for (int k = kc * 8; k < tl.ks * 16; k += 128) {
+        unsigned long long u[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            u[i] = (unsigned long long)(k + i < n ? dg_fix(src[step * (k + i)], em, tl.tb) : 0) + 0x0200808080808080ull;
+        uint8_t* d = tab + tl.off + (size_t)(k >> 4) * bytes + rg * 256 + ((k >> 3) & 1) * 128 + r * 16;
+        const size_t ds = (size_t)tl.r8 * 32;
+#define S2G_DG_PUT(a)                                                                                       \
+    *(uint4*)(d + a * ds) = make_uint4(dg_digit2<a>(u[0], u[1]), dg_digit2<a>(u[2], u[3]), dg_digit2<a>(u[4], u[5]), \
+                                       dg_digit2<a>(u[6], u[7]))
+        S2G_DG_PUT(0);
+        S2G_DG_PUT(1);
+        S2G_DG_PUT(2);
+        S2G_DG_PUT(3);
+        S2G_DG_PUT(4);
+        S2G_DG_PUT(5);
+        S2G_DG_PUT(6);
+#undef S2G_DG_PUT
+    }
+}
+
 // DFT tables: F1 (rows orders, K longitudes) and I2 (rows longitudes, K orders), folds as k_dg_fold.
 __global__ void __launch_bounds__(128) k_dg_pack_dft(int B, int inv, const DgTile* __restrict__ tiles, uint8_t* tab,
                                                      short* qs) {
@@ -1089,17 +1185,32 @@ struct DgTable {
     }
 };
 
+// A run of orders whose tables lie in scratch together (on-the-fly family).
+struct DgChunk {
+    int m0, m1;
+    size_t t0, t1;  // tiles
+};
+
 struct DgTabs {
     int device = -1, bw = 0, refs = 0;
+    bool fly = false;  // no Legendre tables: chunks, nodes and offsets instead
     DgTable t[4];
     int* err = nullptr;
+    std::vector<DgChunk> chunks[4];
+    size_t tmp_bytes[4] = {0, 0, 0, 0}, tab_bytes[4] = {0, 0, 0, 0};
+    double2* nodes = nullptr;          // cos, sin, seeds: B each; recurrence coefficients: B x B
+    double* first = nullptr;           // P(m,m) at the nodes: B x B
+    int64_t* off[4] = {nullptr, nullptr, nullptr, nullptr};
 };
 
 static std::mutex g_dg_mu;
-static std::map<std::pair<int, int>, DgTabs*> g_dg;
+static std::map<std::tuple<int, int, bool>, DgTabs*> g_dg;
 
 static void dg_free(DgTabs* d) {
     for (auto& t : d->t) t.release();
+    for (auto* o : d->off) cudaFree(o);
+    cudaFree(d->nodes);
+    cudaFree(d->first);
     cudaFree(d->err);
     delete d;
 }
@@ -1109,7 +1220,7 @@ void dg_put(void* h) {
     if (!d) return;
     std::lock_guard<std::mutex> lk(g_dg_mu);
     if (--d->refs == 0) {
-        g_dg.erase({d->device, d->bw});
+        g_dg.erase(std::make_tuple(d->device, d->bw, d->fly));
         dg_free(d);
     }
 }
@@ -1209,11 +1320,53 @@ static int dg_low_orders(int B, double* tmp, const std::vector<int64_t>& off, in
     return S2G_OK;
 }
 
+// Digits in scratch at a time, on-the-fly family: enough orders to fill the GPU.
+static int64_t dg_fly_budget(int bw) { return (int64_t)(bw <= 256 ? 64 : bw <= 512 ? 128 : 384) << 20; }
+
+// Tiles of F2 and I1 in chunks of orders, their offsets counted from the chunk's start.
+static int dg_fly_chunks(DgTabs* d, cudaStream_t st) {
+    const int B = d->bw;
+    for (int s = kF2; s <= kI1; ++s) {
+        DgTable& t = d->t[s];
+        dg_tiles(t, s, B);
+        std::vector<int64_t> off(B);
+        int64_t base = 0, at = 0;
+        size_t k = 0;
+        DgChunk c{0, 0, 0, 0};
+        for (int m = 0; m < B; ++m) {
+            size_t e = k;
+            while (e < t.h.size() && t.h[e].m == m) ++e;
+            const int64_t end = e < t.h.size() ? t.h[e].off : t.bytes;
+            if (m > c.m0 && end - base > dg_fly_budget(B)) {
+                d->chunks[s].push_back(c);
+                c = DgChunk{m, m, k, k};
+                base = t.h[k].off;
+                at = 0;
+            }
+            for (; k < e; ++k) t.h[k].off -= base;
+            c.m1 = m + 1;
+            c.t1 = e;
+            off[m] = at;
+            at += (int64_t)(B - m) * B;
+            d->tab_bytes[s] = std::max(d->tab_bytes[s], (size_t)(end - base));
+            d->tmp_bytes[s] = std::max(d->tmp_bytes[s], (size_t)at * sizeof(double));
+        }
+        d->chunks[s].push_back(c);
+        S2G_CUDA(cudaMalloc(&t.tiles, sizeof(DgTile) * t.h.size()));
+        S2G_CUDA(cudaMemcpyAsync(t.tiles, t.h.data(), sizeof(DgTile) * t.h.size(), cudaMemcpyHostToDevice, st));
+        S2G_CUDA(cudaMalloc(&d->off[s], sizeof(int64_t) * B));
+        S2G_CUDA(cudaMemcpyAsync(d->off[s], off.data(), sizeof(int64_t) * B, cudaMemcpyHostToDevice, st));
+        S2G_CUDA(cudaStreamSynchronize(st));  // off is a local
+    }
+    return S2G_OK;
+}
+
 static int dg_build(DgTabs* d, const double* weights, cudaStream_t st) {
     const int B = d->bw, S = 2 * B;
     S2G_CUDA(cudaMalloc(&d->err, sizeof(int)));
     S2G_CUDA(cudaMemsetAsync(d->err, 0, sizeof(int), st));
-    for (int s = 0; s < 4; ++s) S2G_TRY(dg_upload(d->t[s], s, B, st));
+    for (int s = 0; s < 4; ++s)
+        if (!d->fly || s == kF1 || s == kI2) S2G_TRY(dg_upload(d->t[s], s, B, st));
     for (int s = kF1; s <= kI2; s += kI2 - kF1) {
         const DgTable& t = d->t[s];
         ProfScope ps_("dg_pack_dft", st);
@@ -1234,6 +1387,17 @@ static int dg_build(DgTabs* d, const double* weights, cudaStream_t st) {
         h[B + j] = put(sinl(a));
         if (j) c *= -sqrtl((2 * j + 1) / (2 * (long double)j));
         h[2 * (size_t)B + j] = put(c);
+    }
+    if (d->fly) {
+        S2G_CUDA(cudaMalloc(&d->nodes, sizeof(double2) * (h.size() + (size_t)B * B)));
+        S2G_CUDA(cudaMalloc(&d->first, sizeof(double) * (size_t)B * B));
+        S2G_CUDA(cudaMemcpyAsync(d->nodes, h.data(), sizeof(double2) * h.size(), cudaMemcpyHostToDevice, st));
+        {
+            ProfScope ps_("dg_fly_init", st);
+            k_dg_fly_init<<<B, 128, 0, st>>>(B, d->nodes + B, d->nodes + 2 * (size_t)B, d->nodes + h.size(), d->first);
+        }
+        S2G_CUDA(cudaGetLastError());
+        return dg_fly_chunks(d, st);
     }
     struct Tmp {
         void* p[3] = {nullptr, nullptr, nullptr};
@@ -1288,11 +1452,11 @@ static int dg_build(DgTabs* d, const double* weights, cudaStream_t st) {
 }
 
 // Digit tables of bandwidth bw on the current device, shared by every plan; the caller holds a reference.
-static int dg_get(int bw, const double* weights, DgTabs** out) {
+static int dg_get(int bw, bool fly, const double* weights, DgTabs** out) {
     int dev = 0;
     S2G_CUDA(cudaGetDevice(&dev));
     std::lock_guard<std::mutex> lk(g_dg_mu);
-    auto it = g_dg.find({dev, bw});
+    auto it = g_dg.find(std::make_tuple(dev, bw, fly));
     if (it != g_dg.end()) {
         ++it->second->refs;
         *out = it->second;
@@ -1301,6 +1465,7 @@ static int dg_get(int bw, const double* weights, DgTabs** out) {
     DgTabs* d = new DgTabs();
     d->device = dev;
     d->bw = bw;
+    d->fly = fly;
     cudaStream_t st;
     S2G_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     const int r = dg_build(d, weights, st);
@@ -1310,7 +1475,7 @@ static int dg_get(int bw, const double* weights, DgTabs** out) {
         return r;
     }
     d->refs = 1;
-    g_dg[{dev, bw}] = d;
+    g_dg[std::make_tuple(dev, bw, fly)] = d;
     *out = d;
     return S2G_OK;
 }
@@ -1341,12 +1506,7 @@ static int launch_dg_nt(const DgArgs& p, cudaStream_t st) {
 // pipe alone would take 47 us for each of the four; MMA issue and the part of the epilogue that the next
 // item's MMAs wait for (dg_sum, the stores) make up the rest.
 template <int STAGE>
-static int launch_dg(const DgTabs* d, DgArgs p, cudaStream_t st) {
-    const DgTable& t = d->t[STAGE];
-    p.tiles = t.tiles;
-    p.tab = t.tab;
-    p.q = t.q;
-    p.ntiles = (int)t.h.size();
+static int launch_dg_tiles(const DgTabs* d, DgArgs p, cudaStream_t st) {
     p.col_major = STAGE == kF1 || STAGE == kI2;
     p.err = d->err;
     const int per = p.ncols <= 16 ? 16 : (p.ncols <= 32 ? 32 : 64);
@@ -1354,6 +1514,41 @@ static int launch_dg(const DgTabs* d, DgArgs p, cudaStream_t st) {
     if (per == 16) return launch_dg_nt<STAGE, 16>(p, st);
     if (per == 32) return launch_dg_nt<STAGE, 32>(p, st);
     return launch_dg_nt<STAGE, 64>(p, st);
+}
+
+// A stage over its whole table; on the fly, F2 and I1 generate theirs chunk by chunk in `scratch`.
+template <int STAGE>
+static int launch_dg(const DgTabs* d, DgArgs p, const double* weights, char* scratch, cudaStream_t st) {
+    const DgTable& t = d->t[STAGE];
+    p.tiles = t.tiles;
+    p.tab = t.tab;
+    p.q = t.q;
+    p.ntiles = (int)t.h.size();
+    if (!d->fly || STAGE == kF1 || STAGE == kI2) return launch_dg_tiles<STAGE>(d, p, st);
+    const int B = d->bw;
+    double* tmp = (double*)scratch;
+    uint8_t* tab = (uint8_t*)scratch + ((d->tmp_bytes[STAGE] + 255) & ~(size_t)255);
+    short* q = (short*)(tab + ((d->tab_bytes[STAGE] + 4096 + 255) & ~(size_t)255));
+    for (const DgChunk& c : d->chunks[STAGE]) {
+        {
+            ProfScope ps_("dg_fly_legendre", st);
+            k_dg_legendre64<<<dim3(c.m1 - c.m0, (B + 31) / 32), 32, 0, st>>>(
+                B, c.m0, d->nodes, d->nodes + 3 * (size_t)B, d->first, STAGE == kF2 ? weights : nullptr, sqrt(2.0 * 3.14159265358979323846) / (2 * B), tmp, d->off[STAGE]);
+        }
+        S2G_CUDA(cudaGetLastError());
+        {
+            ProfScope ps_("dg_fly_pack", st);
+            k_dg_pack_fly<<<dim3((unsigned)(c.t1 - c.t0), 16), 128, 0, st>>>(B, STAGE == kF2, t.tiles + c.t0, tmp, d->off[STAGE],
+                                                                            tab, q);
+        }
+        S2G_CUDA(cudaGetLastError());
+        p.tiles = t.tiles + c.t0;
+        p.ntiles = (int)(c.t1 - c.t0);
+        p.tab = tab;
+        p.q = q;
+        S2G_TRY(launch_dg_tiles<STAGE>(d, p, st));
+    }
+    return S2G_OK;
 }
 
 static int dg_fields(int mode) { return mode == kReal ? 1 : 2; }
@@ -1394,6 +1589,14 @@ static DgWork dg_work(char* w, int bw, int n, bool two) {
     return k;
 }
 
+size_t dg_fly_bytes(const Tables* t, int batch, bool two) {
+    const DgTabs* d = (const DgTabs*)t->dg;
+    size_t need = 0;
+    for (int s = kF2; s <= kI1; ++s)
+        need = std::max(need, d->tmp_bytes[s] + d->tab_bytes[s] + 2 * (size_t)d->t[s].rows + 4096 + 1024);
+    return dg_work(nullptr, t->bw, dg_chunk(t->bw, batch), two).bytes + need;
+}
+
 size_t dg_work_bytes(int bw, int batch, bool two) { return dg_work(nullptr, bw, dg_chunk(bw, batch), two).bytes; }
 
 // Bandwidths of the digit path: up to 1024 (its Legendre tables take 14 bw^3 bytes: 15 GB there).  Below 32
@@ -1404,6 +1607,8 @@ bool dg_takes(int bw) { return bw <= 1024 && (bw >= 32 || (bw > 8 && (bw & (bw -
 
 // Builds (or finds) the digit tables of t's bandwidth.  Where the stream is being captured, or they do
 // not fit in device memory, t stays without them and the FP64 kernels run.
+bool dg_fly_takes(int bw, int fields) { return dg_takes(bw) && bw >= 64 && fields >= (bw > 512 ? 4 : 2); }
+
 int dg_prepare(Tables* t, cudaStream_t st) {
     if (!dg_takes(t->bw) || __atomic_load_n(&t->dg, __ATOMIC_ACQUIRE) || t->dg_off) return S2G_OK;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -1412,7 +1617,7 @@ int dg_prepare(Tables* t, cudaStream_t st) {
         return S2G_OK;
     }
     DgTabs* d;
-    const int r = dg_get(t->bw, t->weights, &d);
+    const int r = dg_get(t->bw, t->cutoff == 0, t->weights, &d);
     if (r == S2G_ERR_NOMEM) {
         cudaGetLastError();
         t->dg_off = true;
@@ -1435,6 +1640,7 @@ int fst_f64_dg(const Tables* t, const double* rdata, const double* idata, double
     const int B = t->bw, S = 2 * B, mode = dg_mode(idata, fmt), chunk = dg_chunk(B, batch);
     const DgFold fl = dg_fold_layout(B, false);
     const DgWork w = dg_work((char*)work, B, chunk, mode != kReal);
+    char* scratch = (char*)work + w.bytes;  // on the fly: tables
     S2G_TRY(set_dyn_smem((const void*)k_dg_fold, 2 * (size_t)S * 8));
     for (int f0 = 0; f0 < batch; f0 += chunk) {
         const int n = std::min(chunk, batch - f0), ff = n * dg_fields(mode);
@@ -1461,11 +1667,11 @@ int fst_f64_dg(const Tables* t, const double* rdata, const double* idata, double
         p.ein = w.ej;
         p.efield = w.ef;
         p.emax = w.ex;
-        S2G_TRY(launch_dg<kF1>(d, p, st));
+        S2G_TRY(launch_dg<kF1>(d, p, t->weights, scratch, st));
         p.ncols = ff * 2;
         p.out_r = rc + c0;
         p.out_i = ic + c0;
-        S2G_TRY(launch_dg<kF2>(d, p, st));
+        S2G_TRY(launch_dg<kF2>(d, p, t->weights, scratch, st));
     }
     return S2G_OK;
 }
@@ -1476,6 +1682,7 @@ int inv_fst_f64_dg(const Tables* t, const double* rc, const double* ic, double* 
     const int B = t->bw, S = 2 * B, mode = dg_mode(idata, fmt), chunk = dg_chunk(B, batch);
     const DgFold fl = dg_fold_layout(B, true);
     const DgWork w = dg_work((char*)work, B, chunk, mode != kReal);
+    char* scratch = (char*)work + w.bytes;  // on the fly: tables
     for (int f0 = 0; f0 < batch; f0 += chunk) {
         const int n = std::min(chunk, batch - f0), ff = n * dg_fields(mode);
         const size_t g0 = (size_t)f0 * S * S, c0 = (size_t)f0 * B * B;
@@ -1499,10 +1706,10 @@ int inv_fst_f64_dg(const Tables* t, const double* rc, const double* ic, double* 
         p.in_i = mode == kReal ? ic + c0 : w.ci;
         p.ein = w.ex;
         p.emax = w.ef;
-        S2G_TRY(launch_dg<kI1>(d, p, st));
+        S2G_TRY(launch_dg<kI1>(d, p, t->weights, scratch, st));
         p.ncols = ff * S;
         p.ein = w.ef;
-        S2G_TRY(launch_dg<kI2>(d, p, st));
+        S2G_TRY(launch_dg<kI2>(d, p, t->weights, scratch, st));
         if (B % 2 == 0) {
             ProfScope ps_("dg_mid", st);
             k_dg_mid<<<(ff * S + 31) / 32, dim3(32, 8), 0, st>>>((const double*)w.X, B, ff * S, w.mid);

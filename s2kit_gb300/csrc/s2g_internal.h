@@ -115,6 +115,9 @@ size_t f64_plan_bytes(int bw, int batch, int data_format, bool two);
 // ---- FP64 transforms as exact digit products on the tensor cores (digit_gemm.cu) ----
 bool dg_takes(int bw);
 size_t dg_work_bytes(int bw, int batch, bool two);
+// On-the-fly family (tables of cutoff 0): real fields for which it pays, and the scratch once prepared.
+bool dg_fly_takes(int bw, int fields);
+size_t dg_fly_bytes(const Tables* t, int batch, bool two);
 int dg_prepare(Tables* t, cudaStream_t st);
 void dg_put(void* dg);
 int dg_status(const Tables* t, int clear);

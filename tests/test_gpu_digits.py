@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 TOL = 1e-12
 
 
-def _run(bw, nb, mode, cutoff, rc, ic, gr, gi, shift=0):
+def _run(bw, nb, mode, cutoff, rc, ic, gr, gi, shift=0, fly=False):
     """Inverse of (rc, ic) and forward of (gr, gi); device buffers start `shift` doubles into an allocation."""
     import torch
 
@@ -25,7 +25,7 @@ def _run(bw, nb, mode, cutoff, rc, ic, gr, gi, shift=0):
 
     fmt = api.COMPLEX if mode == "complex" else api.REAL
     two = mode != "real"
-    plan = api.Plan(bw, cutoff)
+    plan = api.Plan(bw, cutoff, fly=fly)
     n, c = 4 * bw * bw, bw * bw
     og, oc = [dev(np.full((nb, n), 7.0)) for _ in range(2)], [dev(np.full((nb, c), 7.0)) for _ in range(2)]
     plan.inv_fst(dev(rc), dev(ic), og[0], og[1] if two else None, nb, fmt)
@@ -67,6 +67,19 @@ def test_digit_path_matches_oracle(oracle, bw, nb, mode, cutoff):
         # themselves up to 3e-12 off at order 1 on samples that are not band-limited
         er, ei = oracle.fst(gr[f], gi[f], bw, fmt, 1)
         assert rel_err_norm(oc[0][f], oc[1][f], er, ei) <= TOL
+
+
+@pytest.mark.parametrize("bw,nb,mode", [(64, 2, "real"), (65, 9, "complex"), (100, 33, "real"), (127, 1, "imag"),
+                                        (255, 3, "complex"), (256, 17, "real"), (300, 2, "real"), (512, 2, "real")])
+def test_digit_path_without_tables_matches_oracle(oracle, bw, nb, mode):
+    """On-the-fly plans: the digit tables generated chunk by chunk in scratch (one chunk up to several)."""
+    rc, ic, gr, gi = _data(bw, nb, mode)
+    og, oc = _run(bw, nb, mode, bw, rc, ic, gr, gi, fly=True)
+    fmt = api.COMPLEX if mode == "complex" else api.REAL
+    for f in {0, nb - 1}:
+        er, ei = oracle.inv_fst(rc[f], ic[f], bw, fmt, bw)
+        assert rel_err_norm(og[0][f], og[1][f], er, ei if mode != "real" else 0.0) <= TOL
+        assert rel_err_norm(oc[0][f], oc[1][f], *oracle.fst(gr[f], gi[f], bw, fmt, 1)) <= TOL
 
 
 def test_digit_path_unaligned_buffers():
