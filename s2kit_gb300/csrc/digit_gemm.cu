@@ -62,6 +62,8 @@ enum { kReal = 0, kReal2 = 1, kCplx = 2 };
 struct DgTile {
     int64_t off;      // byte offset of the first K step's blob
     int ks;           // K steps
+    int k0;           // the first one with a digit that is not zero (Legendre tables: near the pole high
+                      // orders vanish below the last digit, a third of all entries)
     int row0, nrows;  // rows row0 .. row0 + nrows of the panel
     int r8;           // rows stored (nrows rounded up to 8)
     int qoff;         // row scales at q[qoff + row]
@@ -70,6 +72,7 @@ struct DgTile {
     int zoff;         // F1, I2: the panel's place in a column of Z
     int vb;           // bits of a data value
     int tb;           // bits of a table value
+    int pad_;
 };
 
 struct DgArgs {
@@ -360,7 +363,7 @@ __global__ void __launch_bounds__(kDgThreads, 1) k_dg(DgArgs p) {
                 const uint32_t bytes = kDigits * (uint32_t)tl->r8 * 32;
                 const uint8_t* src = p.tab + tl->off;
                 const int n = tl->ks;
-                for (int k = 0; k < n; ++k, ++c) {
+                for (int k = tl->k0; k < n; ++k, ++c) {
                     const uint32_t slot = c % kDgStagesA;
                     if (!dg_wait(&emptyA[slot], ((c / kDgStagesA) & 1) ^ 1, &failed)) {
                         ok = false;
@@ -384,7 +387,7 @@ __global__ void __launch_bounds__(kDgThreads, 1) k_dg(DgArgs p) {
             decode(it, tile, cb);
             const DgTile* tl = p.tiles + tile;
             const uint32_t stepA = (uint32_t)__shfl_sync(0xffffffffu, tl->r8, 0) * 2;  // descriptor units of 16 B
-            const int n = __shfl_sync(0xffffffffu, tl->ks, 0);
+            const int n = __shfl_sync(0xffffffffu, tl->ks - tl->k0, 0);
             const int s0 = kSlots == 1 ? 0 : (int)(nit & 1);
             ok = dg_wait_warp(&accEmpty[s0], (use[s0]++ & 1) ^ 1, &failed);
             tc::tc_fence_after();
@@ -440,13 +443,14 @@ __global__ void __launch_bounds__(kDgThreads, 1) k_dg(DgArgs p) {
             c += n;
             bool moved = false;
             while (it < nitems && ks >= tl.ks) {
-                ks -= tl.ks;
+                const int over = ks - tl.ks;
                 it += gridDim.x;
                 moved = true;
                 if (it < nitems) {
                     int t2, c2;
                     decode(it, t2, c2);
                     tl.ks = p.tiles[t2].ks;
+                    ks = p.tiles[t2].k0 + over;
                 }
             }
             if (it >= nitems) return false;
@@ -462,6 +466,7 @@ __global__ void __launch_bounds__(kDgThreads, 1) k_dg(DgArgs p) {
         bool more = it < nitems;
         if (more) {
             enter();
+            ks = tl.k0;
             more = skip(g);
         }
         Step cur{};
@@ -1003,12 +1008,14 @@ __device__ __forceinline__ int dg_scale(double mx, int tb) {
 
 // Digits of one 8-row group; 128 threads = 8 rows x 16 K entries per step.  val(row, k): the table value.
 template <class Val>
-__device__ __forceinline__ void dg_pack_rows(Val val, int q, uint8_t* blob, int r8, int ks, int rg) {
+__device__ __forceinline__ int dg_pack_rows(Val val, int q, uint8_t* blob, int r8, int ks, int rg) {
     const int r = threadIdx.x >> 4, kk = threadIdx.x & 15;
     const uint32_t bytes = kDigits * (uint32_t)r8 * 32;
+    int first = ks;  // this thread's first step with a nonzero value
     for (int s = 0; s < ks; ++s) {
         const double x = val(r, s * 16 + kk);
         const long long v = __double2ll_rn(scalbn(x, q));
+        if (v && first == ks) first = s;
         const unsigned long long u = (unsigned long long)v + 0x0200808080808080ull;
         uint8_t* d = blob + (size_t)s * bytes + rg * 256 + (kk >> 3) * 128 + r * 16 + (kk & 7) * 2;
 #pragma unroll
@@ -1016,14 +1023,18 @@ __device__ __forceinline__ void dg_pack_rows(Val val, int q, uint8_t* blob, int 
             *(__half*)(d + (size_t)a * r8 * 32) =
                 __int2half_rn(a ? (int)((u >> (8 * (6 - a))) & 255) - 128 : (int)(u >> 48) - 512);
     }
+    return first;
 }
+
+// A node's row of the inverse that is below this anywhere (2^-64 of the order's largest values) is zero.
+constexpr double kDgTiny = 5.4e-20;
 
 // Legendre tables of the orders m0 ..: one block per (tile, 8-row group); tiles of kind F2 (rows degrees,
 // weighted) or I1 (rows nodes).
 __global__ void __launch_bounds__(128) k_dg_pack_leg(int B, int fwd, const DgTile* __restrict__ tiles, int m0,
                                                      const double* __restrict__ tmp, const int64_t* __restrict__ off,
                                                      const double* __restrict__ w, double wscale, uint8_t* tab,
-                                                     short* qs) {
+                                                     short* qs, int* first) {
     __shared__ double red[8][17];
     const DgTile tl = tiles[blockIdx.x];
     const int rg = blockIdx.y;
@@ -1042,9 +1053,11 @@ __global__ void __launch_bounds__(128) k_dg_pack_leg(int B, int fwd, const DgTil
     red[r][kk] = mx;
     __syncthreads();
     for (int q = 0; q < 16; ++q) mx = fmax(mx, red[r][q]);
-    const int q = dg_scale(mx, tl.tb);
+    const bool tiny = !fwd && mx < kDgTiny;
+    const int q = tiny ? 0 : dg_scale(mx, tl.tb);
     if (kk == 0 && rg * 8 + r < tl.nrows) qs[tl.qoff + tl.row0 + rg * 8 + r] = (short)q;
-    dg_pack_rows(val, q, tab + tl.off, tl.r8, tl.ks, rg);
+    const int f = dg_pack_rows([&](int a, int k) { return tiny ? 0.0 : val(a, k); }, q, tab + tl.off, tl.r8, tl.ks, rg);
+    atomicMin(first + blockIdx.x, f);
 }
 
 // On-the-fly family: the same tables, a chunk of orders at a time in scratch, from what a plan keeps per
@@ -1098,7 +1111,7 @@ __global__ void __launch_bounds__(32) k_dg_legendre64(int B, int m0, const doubl
 // by sixteen runs of eight K entries.
 __global__ void __launch_bounds__(128) k_dg_pack_fly(int B, int fwd, const DgTile* __restrict__ tiles,
                                                      const double* __restrict__ tmp, const int64_t* __restrict__ off,
-                                                     uint8_t* tab, short* qs) {
+                                                     uint8_t* tab, short* qs, int* first) {
     __shared__ uint32_t red[8][17];
     const DgTile tl = tiles[blockIdx.x];
     const int rg = blockIdx.y;
@@ -1118,14 +1131,23 @@ __global__ void __launch_bounds__(128) k_dg_pack_fly(int B, int fwd, const DgTil
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < 16; ++i) mx = max(mx, red[r][i]);
+    const bool tiny = !fwd && mx < 1022 - 63;  // below 2^-64, as kDgTiny
     const int em = max((int)mx, 1);
+    int zero = tl.ks;  // first: null, or where the tile's first step with a nonzero digit goes
     if (kc == 0 && live) qs[tl.qoff + row] = (short)(tl.tb + 1022 - em);
     const uint32_t bytes = kDigits * (uint32_t)tl.r8 * 32;
     for (int k = kc * 8; k < tl.ks * 16; k += 128) {
         unsigned long long u[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i)
-            u[i] = (unsigned long long)(k + i < n ? dg_fix(src[step * (k + i)], em, tl.tb) : 0) + 0x0200808080808080ull;
+            u[i] = (unsigned long long)(k + i < n && !tiny ? dg_fix(src[step * (k + i)], em, tl.tb) : 0) + 0x0200808080808080ull;
+        if (first && zero == tl.ks) {
+            bool any = false;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) any |= u[i] != 0x0200808080808080ull;
+            if (any) zero = k >> 4;
+        }
+        if (!first && (k >> 4) < tl.k0) continue;
         uint8_t* d = tab + tl.off + (size_t)(k >> 4) * bytes + rg * 256 + ((k >> 3) & 1) * 128 + r * 16;
         const size_t ds = (size_t)tl.r8 * 32;
 #define S2G_DG_PUT(a)                                                                                       \
@@ -1140,6 +1162,7 @@ __global__ void __launch_bounds__(128) k_dg_pack_fly(int B, int fwd, const DgTil
         S2G_DG_PUT(6);
 #undef S2G_DG_PUT
     }
+    if (first) atomicMin(first + blockIdx.x, zero);
 }
 
 // DFT tables: F1 (rows orders, K longitudes) and I2 (rows longitudes, K orders), folds as k_dg_fold.
@@ -1320,11 +1343,49 @@ static int dg_low_orders(int B, double* tmp, const std::vector<int64_t>& off, in
     return S2G_OK;
 }
 
+// The tiles' first steps with nonzero digits: an array for the pack kernels, then into the tiles.
+static int dg_first_alloc(const DgTable& t, void** mem, int** first, cudaStream_t st) {
+    S2G_CUDA(cudaMalloc(mem, sizeof(int) * t.h.size()));
+    S2G_CUDA(cudaMemsetAsync(*mem, 0x7f, sizeof(int) * t.h.size(), st));
+    *first = (int*)*mem;
+    return S2G_OK;
+}
+static int dg_first_read(DgTable& t, const int* first, cudaStream_t st) {
+    std::vector<int> f(t.h.size());
+    S2G_CUDA(cudaMemcpyAsync(f.data(), first, sizeof(int) * f.size(), cudaMemcpyDeviceToHost, st));
+    S2G_CUDA(cudaStreamSynchronize(st));
+    for (size_t i = 0; i < f.size(); ++i) t.h[i].k0 = std::min(f[i], t.h[i].ks - 1);
+    S2G_CUDA(cudaMemcpyAsync(t.tiles, t.h.data(), sizeof(DgTile) * t.h.size(), cudaMemcpyHostToDevice, st));
+    S2G_CUDA(cudaStreamSynchronize(st));
+    return S2G_OK;
+}
+
 // Digits in scratch at a time, on-the-fly family: enough orders to fill the GPU.
 static int64_t dg_fly_budget(int bw) { return (int64_t)(bw <= 256 ? 64 : bw <= 512 ? 128 : 384) << 20; }
 
+// Tables of one chunk of orders in scratch; first: see dg_first_alloc.
+static int dg_fly_tables(const DgTabs* d, int stage, const DgChunk& c, const double* weights, double* tmp, uint8_t* tab,
+                         short* q, int* first, cudaStream_t st) {
+    const int B = d->bw;
+    const DgTable& t = d->t[stage];
+    {
+        ProfScope ps_("dg_fly_legendre", st);
+        k_dg_legendre64<<<dim3(c.m1 - c.m0, (B + 31) / 32), 32, 0, st>>>(
+            B, c.m0, d->nodes, d->nodes + 3 * (size_t)B, d->first, stage == kF2 ? weights : nullptr,
+            sqrt(2.0 * 3.14159265358979323846) / (2 * B), tmp, d->off[stage]);
+    }
+    S2G_CUDA(cudaGetLastError());
+    {
+        ProfScope ps_("dg_fly_pack", st);
+        k_dg_pack_fly<<<dim3((unsigned)(c.t1 - c.t0), 16), 128, 0, st>>>(B, stage == kF2, t.tiles + c.t0, tmp,
+                                                                        d->off[stage], tab, q, first);
+    }
+    S2G_CUDA(cudaGetLastError());
+    return S2G_OK;
+}
+
 // Tiles of F2 and I1 in chunks of orders, their offsets counted from the chunk's start.
-static int dg_fly_chunks(DgTabs* d, cudaStream_t st) {
+static int dg_fly_chunks(DgTabs* d, const double* weights, cudaStream_t st) {
     const int B = d->bw;
     for (int s = kF2; s <= kI1; ++s) {
         DgTable& t = d->t[s];
@@ -1356,7 +1417,22 @@ static int dg_fly_chunks(DgTabs* d, cudaStream_t st) {
         S2G_CUDA(cudaMemcpyAsync(t.tiles, t.h.data(), sizeof(DgTile) * t.h.size(), cudaMemcpyHostToDevice, st));
         S2G_CUDA(cudaMalloc(&d->off[s], sizeof(int64_t) * B));
         S2G_CUDA(cudaMemcpyAsync(d->off[s], off.data(), sizeof(int64_t) * B, cudaMemcpyHostToDevice, st));
-        S2G_CUDA(cudaStreamSynchronize(st));  // off is a local
+        // generated once here, for the tiles' first steps
+        struct Buf {
+            void* p[4] = {nullptr, nullptr, nullptr, nullptr};
+            ~Buf() {
+                for (void* q : p) cudaFree(q);
+            }
+        } b;
+        int* first = nullptr;
+        S2G_TRY(dg_first_alloc(t, &b.p[0], &first, st));
+        S2G_CUDA(cudaMalloc(&b.p[1], d->tmp_bytes[s]));
+        S2G_CUDA(cudaMalloc(&b.p[2], d->tab_bytes[s]));
+        S2G_CUDA(cudaMalloc(&b.p[3], sizeof(short) * t.rows));
+        for (const DgChunk& q : d->chunks[s])
+            S2G_TRY(dg_fly_tables(d, s, q, s == kF2 ? weights : nullptr, (double*)b.p[1], (uint8_t*)b.p[2], (short*)b.p[3],
+                                  first + q.t0, st));
+        S2G_TRY(dg_first_read(t, first, st));
     }
     return S2G_OK;
 }
@@ -1397,10 +1473,10 @@ static int dg_build(DgTabs* d, const double* weights, cudaStream_t st) {
             k_dg_fly_init<<<B, 128, 0, st>>>(B, d->nodes + B, d->nodes + 2 * (size_t)B, d->nodes + h.size(), d->first);
         }
         S2G_CUDA(cudaGetLastError());
-        return dg_fly_chunks(d, st);
+        return dg_fly_chunks(d, weights, st);
     }
     struct Tmp {
-        void* p[3] = {nullptr, nullptr, nullptr};
+        void* p[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
         ~Tmp() {
             for (void* q : p) cudaFree(q);
         }
@@ -1422,6 +1498,8 @@ static int dg_build(DgTabs* d, const double* weights, cudaStream_t st) {
     S2G_CUDA(cudaMalloc(&tmp.p[2], sizeof(int64_t) * B));
     S2G_CUDA(cudaMemcpyAsync(tmp.p[2], off.data(), sizeof(int64_t) * B, cudaMemcpyHostToDevice, st));
     const double2* nodes = (const double2*)tmp.p[0];
+    int* first[4] = {nullptr, nullptr, nullptr, nullptr};
+    for (int s = kF2; s <= kI1; ++s) S2G_TRY(dg_first_alloc(d->t[s], &tmp.p[s + 2], &first[s], st));
     const size_t smem = sizeof(double2) * 2 * (size_t)B;
     S2G_CUDA(cudaFuncSetAttribute((const void*)k_dg_legendre, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     for (int m0 = 0; m0 < B;) {
@@ -1442,12 +1520,12 @@ static int dg_build(DgTabs* d, const double* weights, cudaStream_t st) {
             ProfScope ps_("dg_pack_leg", st);
             k_dg_pack_leg<<<dim3((unsigned)(b - a), 16), 128, 0, st>>>(
                 B, s == kF2, t.tiles + a, m0, (const double*)tmp.p[1], (const int64_t*)tmp.p[2] + m0, weights,
-                sqrt(2.0 * 3.14159265358979323846) / S, t.tab, t.q);
+                sqrt(2.0 * 3.14159265358979323846) / S, t.tab, t.q, first[s] + a);
             S2G_CUDA(cudaGetLastError());
         }
         m0 = m1;
     }
-    S2G_CUDA(cudaStreamSynchronize(st));
+    for (int s = kF2; s <= kI1; ++s) S2G_TRY(dg_first_read(d->t[s], first[s], st));
     return S2G_OK;
 }
 
@@ -1525,23 +1603,11 @@ static int launch_dg(const DgTabs* d, DgArgs p, const double* weights, char* scr
     p.q = t.q;
     p.ntiles = (int)t.h.size();
     if (!d->fly || STAGE == kF1 || STAGE == kI2) return launch_dg_tiles<STAGE>(d, p, st);
-    const int B = d->bw;
     double* tmp = (double*)scratch;
     uint8_t* tab = (uint8_t*)scratch + ((d->tmp_bytes[STAGE] + 255) & ~(size_t)255);
     short* q = (short*)(tab + ((d->tab_bytes[STAGE] + 4096 + 255) & ~(size_t)255));
     for (const DgChunk& c : d->chunks[STAGE]) {
-        {
-            ProfScope ps_("dg_fly_legendre", st);
-            k_dg_legendre64<<<dim3(c.m1 - c.m0, (B + 31) / 32), 32, 0, st>>>(
-                B, c.m0, d->nodes, d->nodes + 3 * (size_t)B, d->first, STAGE == kF2 ? weights : nullptr, sqrt(2.0 * 3.14159265358979323846) / (2 * B), tmp, d->off[STAGE]);
-        }
-        S2G_CUDA(cudaGetLastError());
-        {
-            ProfScope ps_("dg_fly_pack", st);
-            k_dg_pack_fly<<<dim3((unsigned)(c.t1 - c.t0), 16), 128, 0, st>>>(B, STAGE == kF2, t.tiles + c.t0, tmp, d->off[STAGE],
-                                                                            tab, q);
-        }
-        S2G_CUDA(cudaGetLastError());
+        S2G_TRY(dg_fly_tables(d, STAGE, c, weights, tmp, tab, q, nullptr, st));
         p.tiles = t.tiles + c.t0;
         p.ntiles = (int)(c.t1 - c.t0);
         p.tab = tab;
