@@ -217,6 +217,7 @@ static void free_tables(Tables* t) {
     cudaFree(t->tw_D);
     free_split(t);
     dg_put(t->dg);
+    dg_put(t->dg32);
     delete[] t->h_off;
     delete t;
 }
@@ -1209,7 +1210,7 @@ int s2g_fst_complex_f32(s2g_plan p, const float* rgrid, const float* igrid, floa
     S2G_TRY(plan_check(p, batch));
     if (!rgrid || !igrid || !rc || !ic) return fail(S2G_ERR_ARG, "NULL argument");
     S2G_TRY(check_aligned16({rgrid, igrid, rc, ic}));
-    S2G_TRY(p->work.ensure(split_work_bytes(p->bw, batch)));
+    S2G_TRY(p->work.ensure(split_complex_work_bytes(p->bw, batch)));
     S2G_TRY(p->cx.ensure(split_complex_bytes(p->bw, batch)));
     return fst_split_complex(p->t, rgrid, igrid, rc, ic, batch, precision, p->work.ptr, p->cx.ptr,
                              (cudaStream_t)stream);
@@ -1220,7 +1221,7 @@ int s2g_inv_fst_complex_f32(s2g_plan p, const float* rc, const float* ic, float*
     S2G_TRY(plan_check(p, batch));
     if (!rgrid || !igrid || !rc || !ic) return fail(S2G_ERR_ARG, "NULL argument");
     S2G_TRY(check_aligned16({rgrid, igrid, rc, ic}));
-    S2G_TRY(p->work.ensure(split_work_bytes(p->bw, batch)));
+    S2G_TRY(p->work.ensure(split_complex_work_bytes(p->bw, batch)));
     S2G_TRY(p->cx.ensure(split_complex_bytes(p->bw, batch)));
     return inv_fst_split_complex(p->t, rc, ic, rgrid, igrid, batch, precision, p->work.ptr, p->cx.ptr,
                                  (cudaStream_t)stream);

@@ -38,6 +38,7 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <type_traits>
 #include <vector>
 
 #include "s2g_common.cuh"
@@ -46,13 +47,34 @@
 
 namespace s2g {
 
-constexpr int kDigits = 7;
-constexpr int kDgThreads = 896;          // warp 0 tables, 1 MMA, 4-19 epilogue, 20-27 data digits
-constexpr int kDgProdWarps = 8;
-constexpr int kDgStagesA = 4;            // table ring: 16-deep K steps of 7 x 128 x 16 FP16
-constexpr uint32_t kDgABytes = kDigits * 128 * 32;
-constexpr uint32_t kDgBRing = 100352;    // data ring: as many K steps as fit
+constexpr int kDgThreads = 896;          // warp 0 tables, 1 MMA, then from 4 the epilogue's and the data's
+constexpr int kSub = 2;                   // 16-deep K steps of a stage
+constexpr uint32_t kDgBRing = 86016;     // data ring: as many stages as fit
+constexpr uint32_t kDgStash = 32 * 33 * 4;  // FP32 F1: an epilogue warp's results, rows by columns
 constexpr int kDgMaxStagesB = 16;
+
+// Precision of an instance.  64: FP64 transforms, seven digits each.  32: FP32 transforms: table values of
+// 25 bits in three digits, data of 30 bits in four, accumulator groups 0 to 3 (nine of the twelve
+// products; the rest are below 2^-28 of the result's scale).
+template <int P>
+struct Dg;
+template <>
+struct Dg<64> {
+    static constexpr int DA = 7, DB = 7, G = 7, stagesA = 2, epilogue = 16, data = 8;  // warps
+    using Real = double;
+    using Int = long long;
+    using Int2 = longlong2;
+};
+template <>
+struct Dg<32> {
+    static constexpr int DA = 3, DB = 4, G = 4, stagesA = 4, epilogue = 8, data = 16;
+    using Real = float;
+    using Int = int;
+    using Int2 = int2;
+};
+template <int P>
+constexpr uint32_t kDgABytes = kSub * Dg<P>::DA * 128 * 32;  // a stage of a full table tile
+constexpr int kDigits = 7;
 enum { kF1 = 0, kF2 = 1, kI1 = 2, kI2 = 3 };
 // REAL without imaginary arrays / REAL with them / COMPLEX
 enum { kReal = 0, kReal2 = 1, kCplx = 2 };
@@ -81,22 +103,35 @@ struct DgArgs {
     const short* q;            // table value = digits * 2^-q
     int ntiles, ncolblk, col_major;
     int B, S, N, ncols, mode;  // N functions as the caller counts them
-    int BP, RL;                // latitudes of a half row of X (B, made even); values of a column of Z
+    int BP, RL;                // latitudes of a half row of X (B, rounded up to 4); values of a column of Z
     int vbz;                   // bits of Z's samples before folds
     int tbz;                   // F2: bits of F1's table
-    const double* in_r;        // I1: coefficients
-    const double* in_i;
-    double* out_r;             // F2: coefficients
-    double* out_i;
-    void* X;                   // [field, part][m][t][BP]: integers (F1 -> F2) or doubles (I1 -> I2)
-    long long* Z;              // [field][t][j][RL]: folded samples (F1) or parts of samples (I2)
+    const void* in_r;          // I1: coefficients
+    const void* in_i;
+    void* out_r;               // F2: coefficients
+    void* out_i;
+    void* X;                   // [field, part][m][t][BP]: FP64 integers (F1 -> F2), else reals
+    void* Z;                   // [field][t][j][RL]: folded samples (F1) or parts of samples (I2)
     const uint32_t* ein;       // F1: exponents of the latitude pairs; I1: of the orders; I2: of the fields
-    const uint32_t* efield;    // F1, F2: exponents of the fields
-    uint32_t* emax;            // F1 writes, F2 reads: bits of X's rows; I1 writes: exponents of the fields
+    const uint32_t* efield;    // FP64 F1, F2: exponents of the fields
+    const int64_t* cmap;       // function -> coefficient offset (null: f B^2; real fields only)
+    uint32_t* emax;            // F1 writes, F2 reads: X's rows (FP64 bits, FP32 exponents); I1 writes: fields
     int* err;
 };
 
 __device__ __forceinline__ uint32_t dexp(double x) { return ((uint32_t)__double2hiint(x) >> 20) & 0x7ffu; }
+__device__ __forceinline__ uint32_t dexp(float x) { return (__float_as_uint(x) >> 23) & 0xffu; }
+
+// x as an integer of unit 2^(em - 126 - vb) (|x| < 2^(em - 126), vb at most 31), rounded to nearest
+__device__ __forceinline__ int dg_fix(float x, int em, int vb) {
+    const uint32_t b = __float_as_uint(x);
+    int e = (b >> 23) & 0xff;
+    uint32_t m = b & 0x7fffffu;
+    if (e) m |= 0x800000u;
+    else e = 1;
+    const int v = (int)((((m << 8) >> min(em - e + 31 - vb, 31)) + 1) >> 1);
+    return (int)b < 0 ? -v : v;
+}
 
 // x as an integer of unit 2^(em - 1022 - vb) (|x| < 2^(em - 1022), vb at most 56), rounded to nearest
 __device__ __forceinline__ long long dg_fix(double x, int em, int vb) {
@@ -126,19 +161,41 @@ __device__ __forceinline__ uint32_t dg_digit2(unsigned long long u0, unsigned lo
     return *reinterpret_cast<const uint32_t*>(&d);
 }
 
-// Stores the seven digits of the pair (v0, v1) (columns k, k + 1 of row n of every digit's tile).
+// Stores the seven digits of four consecutive K entries of one column, eight bytes a digit.
 template <int NT>
-__device__ __forceinline__ void dg_store2(uint8_t* dst, long long v0, long long v1) {
+__device__ __forceinline__ void dg_store4(uint8_t* dst, const long long* v) {
     constexpr unsigned long long bias = 0x0200808080808080ull;
-    const unsigned long long u0 = (unsigned long long)v0 + bias, u1 = (unsigned long long)v1 + bias;
+    unsigned long long u[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) u[i] = (unsigned long long)v[i] + bias;
     constexpr int step = NT * 32;  // bytes between digits
-    *(uint32_t*)(dst) = dg_digit2<0>(u0, u1);
-    *(uint32_t*)(dst + step) = dg_digit2<1>(u0, u1);
-    *(uint32_t*)(dst + 2 * step) = dg_digit2<2>(u0, u1);
-    *(uint32_t*)(dst + 3 * step) = dg_digit2<3>(u0, u1);
-    *(uint32_t*)(dst + 4 * step) = dg_digit2<4>(u0, u1);
-    *(uint32_t*)(dst + 5 * step) = dg_digit2<5>(u0, u1);
-    *(uint32_t*)(dst + 6 * step) = dg_digit2<6>(u0, u1);
+    *(uint2*)(dst) = make_uint2(dg_digit2<0>(u[0], u[1]), dg_digit2<0>(u[2], u[3]));
+    *(uint2*)(dst + step) = make_uint2(dg_digit2<1>(u[0], u[1]), dg_digit2<1>(u[2], u[3]));
+    *(uint2*)(dst + 2 * step) = make_uint2(dg_digit2<2>(u[0], u[1]), dg_digit2<2>(u[2], u[3]));
+    *(uint2*)(dst + 3 * step) = make_uint2(dg_digit2<3>(u[0], u[1]), dg_digit2<3>(u[2], u[3]));
+    *(uint2*)(dst + 4 * step) = make_uint2(dg_digit2<4>(u[0], u[1]), dg_digit2<4>(u[2], u[3]));
+    *(uint2*)(dst + 5 * step) = make_uint2(dg_digit2<5>(u[0], u[1]), dg_digit2<5>(u[2], u[3]));
+    *(uint2*)(dst + 6 * step) = make_uint2(dg_digit2<6>(u[0], u[1]), dg_digit2<6>(u[2], u[3]));
+}
+
+// Four digits of 32-bit values, all in [-128, 127].
+template <int b>
+__device__ __forceinline__ uint32_t dg_byte2(uint32_t u0, uint32_t u1) {
+    constexpr int i = 3 - b;
+    const uint32_t t = (__byte_perm(u0, u1, i | ((4 + i) << 8)) & 0x00ff00ffu) | 0x64006400u;
+    const __half2 d = __hsub2(*reinterpret_cast<const __half2*>(&t), __half2half2(__ushort_as_half(0x6480)));
+    return *reinterpret_cast<const uint32_t*>(&d);
+}
+template <int NT>
+__device__ __forceinline__ void dg_store4(uint8_t* dst, const int* v) {
+    uint32_t u[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) u[i] = (uint32_t)v[i] + 0x80808080u;
+    constexpr int step = NT * 32;
+    *(uint2*)(dst) = make_uint2(dg_byte2<0>(u[0], u[1]), dg_byte2<0>(u[2], u[3]));
+    *(uint2*)(dst + step) = make_uint2(dg_byte2<1>(u[0], u[1]), dg_byte2<1>(u[2], u[3]));
+    *(uint2*)(dst + 2 * step) = make_uint2(dg_byte2<2>(u[0], u[1]), dg_byte2<2>(u[2], u[3]));
+    *(uint2*)(dst + 3 * step) = make_uint2(dg_byte2<3>(u[0], u[1]), dg_byte2<3>(u[2], u[3]));
 }
 
 // Accumulator groups (exact integers) -> their sum in units of group 5.  Adding 1.5 2^23 leaves an
@@ -219,6 +276,12 @@ __device__ __forceinline__ void tm_wait() { asm volatile("tcgen05.wait::ld.sync.
 // Eight of I2's sums are added: each gives up its last bits.
 constexpr int kDgOutShift = 2;
 
+// FP32: unit of a column whose largest value has exponent field em, times 2^tb of the table's digits
+// (groups in units of the leading one's products, 2^40 of the digits' last places).
+__device__ __forceinline__ float dg_col_scale(uint32_t em, int tb, int vb) {
+    return em == 0xffu ? __int_as_float(0x7fc00000) : ldexpf(1.0f, 40 - tb - vb - 126 + max((int)em, 1));
+}
+
 // Waits for a phase, for about half a second at most; another role's failure ends the wait at once.
 __device__ __forceinline__ bool dg_wait(uint64_t* bar, uint32_t parity, volatile int* failed) {
     if (tc::mbar_try_wait(bar, parity)) return true;
@@ -238,6 +301,18 @@ __device__ __forceinline__ bool dg_wait_warp(uint64_t* bar, uint32_t parity, vol
     return __all_sync(0xffffffffu, dg_wait(bar, parity, failed));
 }
 
+// Both barriers at once: two lanes poll, one each.
+__device__ __forceinline__ bool dg_wait_both(uint64_t* a, uint32_t pa, uint64_t* b, uint32_t pb, volatile int* failed) {
+    const bool second = (threadIdx.x & 31) != 0;
+    uint64_t* bar = second ? b : a;
+    const uint32_t parity = second ? pb : pa;
+    if (!__all_sync(0xffffffffu, (threadIdx.x & 30) || tc::mbar_try_wait(bar, parity)) &&
+        !dg_wait_warp(bar, parity, failed))
+        return false;
+    __syncwarp();  // what either lane acquired, the issuing lane sees
+    return true;
+}
+
 // F2's columns keep the two fields of COMPLEX data together: column -> (field, part).
 __device__ __forceinline__ int dg_f2_field(const DgArgs& p, int col) {
     if (p.mode == kReal) return col;
@@ -246,16 +321,17 @@ __device__ __forceinline__ int dg_f2_field(const DgArgs& p, int col) {
 }
 
 // What one lane of a data warp needs of an item: its two columns (8 apart).
-template <int STAGE>
 struct DgLane {
-    const char* src[2];  // null: no such column
-    int par[2];          // F2: right shift; I1, I2: exponent
+    const void* src[2];  // null: no such column
+    int par[2];          // FP64 F2: right shift; else exponent
     int n;               // K entries there are
     int vb;
 };
 
-template <int STAGE>
-__device__ __forceinline__ void dg_lane(const DgArgs& p, const DgTile& tl, int col0, DgLane<STAGE>& L) {
+template <int STAGE, int P>
+__device__ __forceinline__ void dg_lane(const DgArgs& p, const DgTile& tl, int col0, DgLane& L) {
+    using Real = typename Dg<P>::Real;
+    using Int = typename Dg<P>::Int;
     L.vb = tl.vb;
     const int B = p.B;
     if constexpr (STAGE == kF1) L.n = tl.ks * 16;
@@ -269,74 +345,97 @@ __device__ __forceinline__ void dg_lane(const DgArgs& p, const DgTile& tl, int c
         L.par[c] = 0;
         if (col >= p.ncols) continue;
         if constexpr (STAGE == kF1) {
-            L.src[c] = (const char*)(p.Z + (size_t)col * p.RL + tl.zoff);
+            L.src[c] = (const Int*)p.Z + (size_t)col * p.RL + tl.zoff;
         } else if constexpr (STAGE == kF2) {
             const size_t row = (size_t)dg_f2_field(p, col) * B + tl.m;
-            L.src[c] = (const char*)((const long long*)p.X + row * 2 * p.BP + tl.t * p.BP);
-            L.par[c] = max((int)p.emax[row] - tl.vb, 0);
+            L.src[c] = (const Int*)p.X + row * 2 * p.BP + tl.t * p.BP;  // Int and Real have one size
+            L.par[c] = P == 64 ? max((int)p.emax[row] - tl.vb, 0) : max((int)p.emax[row], 1);
         } else if constexpr (STAGE == kI1) {
-            const double* x = (col & 1) ? p.in_i : p.in_r;
+            const Real* x = (const Real*)((col & 1) ? p.in_i : p.in_r);
             if (tl.m || !(col & 1))  // a real field's Im f(l, 0) is ignored
-                L.src[c] = (const char*)(x + (size_t)(col >> 1) * B * B + index_of_harmonic_coeff(tl.m, tl.m + tl.t, B));
+                L.src[c] = x + (p.cmap ? (size_t)p.cmap[col >> 1] : (size_t)(col >> 1) * B * B) + index_of_harmonic_coeff(tl.m, tl.m + tl.t, B);
             L.par[c] = max((int)p.ein[(size_t)col * B + tl.m], 1);
         } else {
             const int f = col / p.S, rem = col - f * p.S, t = rem >= B, j = rem - t * B;
-            L.src[c] = (const char*)((const double*)p.X + ((size_t)(f * 2 + tl.t) * B + tl.m) * 2 * p.BP + t * p.BP + j);
+            L.src[c] = (const Real*)p.X + ((size_t)(f * 2 + tl.t) * B + tl.m) * 2 * p.BP + t * p.BP + j;
             L.par[c] = max((int)p.ein[f], 1);
         }
     }
 }
 
-// Loads entries k, k + 1 of column c.
-template <int STAGE>
-__device__ __forceinline__ longlong2 dg_load(const DgArgs& p, const DgTile& tl, const DgLane<STAGE>& L, int c, int k) {
-    longlong2 v = make_longlong2(0, 0);
-    if (!L.src[c] || k >= L.n) return v;
-    if constexpr (STAGE == kF1) {
-        v = *((const longlong2*)L.src[c] + (k >> 1));
-    } else if constexpr (STAGE == kF2) {
-        v = *((const longlong2*)L.src[c] + (k >> 1));  // rows have an even length
-        if (k + 1 >= L.n) v.y = 0;
+// Loads entries k .. k + 3 of column c.
+template <int STAGE, int P>
+__device__ __forceinline__ void dg_load(const DgArgs& p, const DgTile& tl, const DgLane& L, int c, int k,
+                                        typename Dg<P>::Int* v) {
+    using Int = typename Dg<P>::Int;
+    using Int2 = typename Dg<P>::Int2;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = 0;
+    if (!L.src[c] || k >= L.n) return;
+    if constexpr (STAGE == kF1 || STAGE == kF2) {
+        const Int2* x = (const Int2*)((const Int*)L.src[c] + k);  // rows start 16-byte aligned
+        if constexpr (P == 32) {
+            const int4 q = *(const int4*)x;
+            v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+        } else {
+            const Int2 a = x[0], b = x[1];
+            v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
+        }
+#pragma unroll
+        for (int i = 1; i < 4; ++i)
+            if (k + i >= L.n) v[i] = 0;
     } else {
         const size_t step = STAGE == kI1 ? 2 : (size_t)(tl.kind < 4 ? 2 : 1) * 2 * p.BP;
-        const long long* x = (const long long*)L.src[c];
-        v.x = __ldg(x + step * k);
-        if (k + 1 < L.n) v.y = __ldg(x + step * (k + 1));
+        const Int* x = (const Int*)L.src[c] + step * k;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (k + i < L.n) v[i] = __ldg(x + step * i);
     }
-    return v;
 }
 
 // Raw entry -> integer of at most vb bits.
 template <int STAGE>
-__device__ __forceinline__ long long dg_conv(const DgLane<STAGE>& L, int c, long long v) {
+__device__ __forceinline__ long long dg_conv(int par, int vb, long long v) {
     if constexpr (STAGE == kF1) return v;
-    if constexpr (STAGE == kF2) return L.par[c] ? ((v >> (L.par[c] - 1)) + 1) >> 1 : v;
-    return dg_fix(__longlong_as_double(v), L.par[c], L.vb);
+    if constexpr (STAGE == kF2) return par ? ((v >> (par - 1)) + 1) >> 1 : v;
+    return dg_fix(__longlong_as_double(v), par, vb);
+}
+template <int STAGE>
+__device__ __forceinline__ int dg_conv(int par, int vb, int v) {
+    if constexpr (STAGE == kF1) return v;
+    return dg_fix(__int_as_float(v), par, vb);
 }
 
-template <int STAGE, int NT>
+template <int STAGE, int NT, int P>
 __global__ void __launch_bounds__(kDgThreads, 1) k_dg(DgArgs p) {
+    using Real = typename Dg<P>::Real;
+    using Int2 = typename Dg<P>::Int2;
+    constexpr int DA = Dg<P>::DA, DB = Dg<P>::DB, G = Dg<P>::G, kDgStagesA = Dg<P>::stagesA;
+    constexpr uint32_t kABytes = kDgABytes<P>;
     extern __shared__ __align__(1024) uint8_t dsm[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)dsm + 1023) & ~(uintptr_t)1023);
     __shared__ uint64_t fullA[kDgStagesA], emptyA[kDgStagesA], fullB[kDgMaxStagesB], emptyB[kDgMaxStagesB];
     __shared__ uint64_t accFull[2], accEmpty[2], drained;
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int failed;
-    constexpr uint32_t accCols = kDigits * NT;        // TMEM columns of one accumulator
-    constexpr int kSlots = NT == 64 ? 1 : 2;          // accumulators
-    constexpr int kEpi = 4 / kSlots, kCols = NT / kEpi;  // epilogue groups of an accumulator, columns of each
-    constexpr uint32_t stageB = kDigits * NT * 32;    // bytes of one K step's data digits
+    constexpr uint32_t accCols = G * NT;              // TMEM columns of one accumulator
+    constexpr int kSlots = 2 * accCols > 512 ? 1 : 2;  // accumulators
+    constexpr int kEW = Dg<P>::epilogue;              // epilogue warps: groups of four cover the rows
+    constexpr int kEpi = kEW / 4 / kSlots, kCols = NT / kEpi;  // groups of an accumulator, columns of each
+    constexpr int kLanes = kCols > 32 ? 32 : kCols, kHalf = kCols / kLanes;
+    constexpr uint32_t stepB = DB * NT * 32, stageB = kSub * stepB;  // bytes of the data digits
     constexpr int nsb = kDgBRing / stageB < kDgMaxStagesB ? kDgBRing / stageB : kDgMaxStagesB;
-    constexpr int W = NT / 16;                        // data warps per K step
-    constexpr int groups = kDgProdWarps / W;
+    constexpr int W = NT / 16;                        // data warps per K step, W kSub per stage
+    constexpr int groups = Dg<P>::data / (W * kSub);
     uint8_t* ringA = smem;
-    uint8_t* ringB = smem + kDgStagesA * kDgABytes;
+    uint8_t* ringB = smem + kDgStagesA * kABytes;
+    [[maybe_unused]] float* stash0 = (float*)(ringB + kDgBRing);
     const uint32_t sdA0 = dg_desc(ringA), sdB0 = dg_desc(ringB);
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         failed = 0;
         for (int i = 0; i < kDgStagesA; ++i) tc::mbar_init(&fullA[i], 1), tc::mbar_init(&emptyA[i], 1);
-        for (int i = 0; i < nsb; ++i) tc::mbar_init(&fullB[i], W), tc::mbar_init(&emptyB[i], 1);
+        for (int i = 0; i < nsb; ++i) tc::mbar_init(&fullB[i], W * kSub), tc::mbar_init(&emptyB[i], 1);
         for (int i = 0; i < 2; ++i) tc::mbar_init(&accFull[i], 1), tc::mbar_init(&accEmpty[i], kEpi * 4);
         tc::mbar_init(&drained, 1);
         tc::fence_mbar_init();
@@ -360,17 +459,17 @@ __global__ void __launch_bounds__(kDgThreads, 1) k_dg(DgArgs p) {
                 int tile, cb;
                 decode(it, tile, cb);
                 const DgTile* tl = p.tiles + tile;
-                const uint32_t bytes = kDigits * (uint32_t)tl->r8 * 32;
+                const uint32_t bytes = DA * (uint32_t)tl->r8 * 32;
                 const uint8_t* src = p.tab + tl->off;
                 const int n = tl->ks;
-                for (int k = tl->k0; k < n; ++k, ++c) {
-                    const uint32_t slot = c % kDgStagesA;
+                for (int k = tl->k0; k < n; k += kSub, ++c) {
+                    const uint32_t slot = c % kDgStagesA, nb = min(kSub, n - k) * bytes;
                     if (!dg_wait(&emptyA[slot], ((c / kDgStagesA) & 1) ^ 1, &failed)) {
                         ok = false;
                         break;
                     }
-                    tc::mbar_arrive_expect_tx(&fullA[slot], bytes);
-                    tc::bulk_g2s(ringA + slot * kDgABytes, src + (size_t)k * bytes, bytes, &fullA[slot]);
+                    tc::mbar_arrive_expect_tx(&fullA[slot], nb);
+                    tc::bulk_g2s(ringA + slot * kABytes, src + (size_t)k * bytes, nb, &fullA[slot]);
                 }
             }
             if (!ok)  // own copies still in flight land before the block ends
@@ -392,22 +491,29 @@ __global__ void __launch_bounds__(kDgThreads, 1) k_dg(DgArgs p) {
             ok = dg_wait_warp(&accEmpty[s0], (use[s0]++ & 1) ^ 1, &failed);
             tc::tc_fence_after();
             const uint32_t d0 = tmem + s0 * accCols;
-            for (int k = 0; k < n && ok; ++k) {
-                ok = dg_wait_warp(&fullA[sa], pa, &failed) && dg_wait_warp(&fullB[sb], pb, &failed);
+            for (int k = 0; k < n && ok; k += kSub) {
+                ok = dg_wait_both(&fullA[sa], pa, &fullB[sb], pb, &failed);
                 if (!ok) break;
                 tc::tc_fence_after();
                 if (leader) {
-                    const uint32_t da = sdA0 + sa * (kDgABytes >> 4), db = sdB0 + sb * (stageB >> 4);
+                    uint32_t da = sdA0 + sa * (kABytes >> 4), db = sdB0 + sb * (stageB >> 4);
+                    const int sub = min(kSub, n - k);
 #pragma unroll
-                    for (int a = 0; a < kDigits; ++a) {
-                        // groups a .. 6; an MMA takes at most 256 columns
-                        constexpr uint32_t one = 1;
-                        const uint32_t acc = a > 0 ? one : (uint32_t)(k > 0);
-                        const int n1 = (kDigits - a) * NT, parts = n1 > 256 ? 2 : 1, np = n1 / parts;
-                        const uint32_t idesc = tc::idesc_f16_f32(128, np);
+                    for (int j = 0; j < kSub; ++j) {
+                        if (j >= sub) break;
 #pragma unroll
-                        for (int h = 0; h < parts; ++h)
-                            dg_mma(d0 + a * NT + h * np, da + a * stepA, db + h * np * 2, idesc, acc);
+                        for (int a = 0; a < DA; ++a) {
+                            // groups a .. G - 1; an MMA takes at most 256 columns
+                            constexpr uint32_t one = 1;
+                            const uint32_t acc = a > 0 || j > 0 ? one : (uint32_t)(k > 0);
+                            const int n1 = (G - a < DB ? G - a : DB) * NT, parts = n1 > 256 ? 2 : 1, np = n1 / parts;
+                            const uint32_t idesc = tc::idesc_f16_f32(128, np);
+#pragma unroll
+                            for (int h = 0; h < parts; ++h)
+                                dg_mma(d0 + a * NT + h * np, da + a * stepA, db + h * np * 2, idesc, acc);
+                        }
+                        da += DA * stepA;
+                        db += stepB >> 4;
                     }
                     tc::mma_commit(&emptyA[sa]);
                     tc::mma_commit(&emptyB[sb]);
@@ -421,47 +527,48 @@ __global__ void __launch_bounds__(kDgThreads, 1) k_dg(DgArgs p) {
             tc::mma_commit(&drained);
             tc::mbar_wait(&drained, 0);
         }
-    } else if (warp >= 20) {  // data digits
-        const int pw = warp - 20, g = pw / W, wi = pw - g * W;
-        // this group's K steps: every groups-th of the block's; the next one's values are loaded
+    } else if (warp >= 4 + kEW) {  // data digits
+        const int pw = warp - 4 - kEW, g = pw / (W * kSub), wi = pw % W, sub = pw / W % kSub;
+        // this group's stages: every groups-th of the block's; this warp's K step of the next one is loaded
         // before the current one is turned into digits
         struct Step {
-            DgLane<STAGE> L;
-            longlong2 v[4];
+            int par[2], vb;
+            typename Dg<P>::Int v[2][4];
         };
         int it = blockIdx.x, ks = 0, tile, cb;
         uint32_t c = 0;
         DgTile tl{};
-        DgLane<STAGE> L{};
+        DgLane L{};
         auto enter = [&]() {  // per-item state
             decode(it, tile, cb);
             tl = p.tiles[tile];
-            dg_lane<STAGE>(p, tl, cb * NT + wi * 16 + (lane >> 2), L);
+            dg_lane<STAGE, P>(p, tl, cb * NT + wi * 16 + (lane & 7), L);
         };
-        auto skip = [&](int n) {  // n K steps on; false past the last item
-            ks += n;
+        auto skip = [&](int n) {  // n stages on; false past the last item
+            ks += n * kSub;
             c += n;
             bool moved = false;
             while (it < nitems && ks >= tl.ks) {
-                const int over = ks - tl.ks;
+                const int over = (ks - tl.ks) / kSub;  // stages into the next item
                 it += gridDim.x;
                 moved = true;
                 if (it < nitems) {
                     int t2, c2;
                     decode(it, t2, c2);
                     tl.ks = p.tiles[t2].ks;
-                    ks = p.tiles[t2].k0 + over;
+                    ks = p.tiles[t2].k0 + over * kSub;
                 }
             }
             if (it >= nitems) return false;
             if (moved) enter();
             return true;
         };
-        auto fetch = [&](Step& st) {
-            st.L = L;
+        auto fetch = [&](Step& x) {
+            x.vb = L.vb;
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-                st.v[q] = dg_load<STAGE>(p, tl, L, q >> 1, ks * 16 + ((q & 1) ^ (lane >> 4)) * 8 + (lane & 3) * 2);
+            for (int h = 0; h < 2; ++h) x.par[h] = L.par[h];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) dg_load<STAGE, P>(p, tl, L, h, (ks + sub) * 16 + (lane >> 3) * 4, x.v[h]);
         };
         bool more = it < nitems;
         if (more) {
@@ -478,12 +585,14 @@ __global__ void __launch_bounds__(kDgThreads, 1) k_dg(DgArgs p) {
             if (more) fetch(nxt);
             const uint32_t slot = cc % nsb;
             if (!dg_wait_warp(&emptyB[slot], ((cc / nsb) & 1) ^ 1, &failed)) break;
-            uint8_t* dst = ringB + slot * stageB;
+            uint8_t* dst = ringB + slot * stageB + sub * stepB;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int r = wi * 16 + (q >> 1) * 8 + (lane >> 2);  // column of the item
-                dg_store2<NT>(dst + (r >> 3) * 256 + ((q & 1) ^ (lane >> 4)) * 128 + (r & 7) * 16 + (lane & 3) * 4,
-                              dg_conv<STAGE>(cur.L, q >> 1, cur.v[q].x), dg_conv<STAGE>(cur.L, q >> 1, cur.v[q].y));
+            for (int h = 0; h < 2; ++h) {
+                typename Dg<P>::Int v[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[i] = dg_conv<STAGE>(cur.par[h], cur.vb, cur.v[h][i]);
+                // eight columns of a core matrix by four runs of K entries: half a warp covers 128 bytes
+                dg_store4<NT>(dst + (wi * 2 + h) * 256 + (lane >> 4) * 128 + (lane & 7) * 16 + ((lane >> 3) & 1) * 8, v);
             }
             tc::fence_proxy_async_smem();
             __syncwarp();
@@ -491,7 +600,7 @@ __global__ void __launch_bounds__(kDgThreads, 1) k_dg(DgArgs p) {
             cur = nxt;
         }
     } else if (warp >= 4) {  // epilogue
-        const int slot = kSlots == 1 ? 0 : (warp - 4) >> 3, grp = ((warp - 4) >> 2) % kEpi, ew = warp & 3;
+        const int slot = kSlots == 1 ? 0 : ((warp - 4) >> 2) / kEpi, grp = ((warp - 4) >> 2) % kEpi, ew = warp & 3;
         const uint32_t lane_off = (uint32_t)(ew * 32) << 16;
         const int B = p.B, S = p.S;
         uint32_t nit = 0, use = 0;
@@ -504,90 +613,131 @@ __global__ void __launch_bounds__(kDgThreads, 1) k_dg(DgArgs p) {
             const bool live = r < tl.nrows;
             const int row = tl.row0 + r;
             const int qrow = live ? p.q[tl.qoff + row] : 0;
-            const int colb = cb * NT + grp * kCols;
-            const int ncol = min(kCols, p.ncols - colb);  // may be negative
-            // lane c holds what the rows need to know of column c: field, place in X, exponent or shift
-            int cfield = 0, cpar = 0;
-            uint32_t coff = 0;
-            if (lane < ncol) {
-                const int col = colb + lane;
-                if constexpr (STAGE == kF1) {
-                    cfield = col / S;
-                    const int rem = col - cfield * S, t = rem >= B, j = rem - t * B;
-                    cpar = min(max((int)p.efield[cfield], 1) - max((int)p.ein[cfield * B + j], 1), 63);
-                    coff = (uint32_t)(cfield * 2 + tl.t) * B * 2 * p.BP + t * p.BP + j;
-                } else if constexpr (STAGE == kF2) {
-                    const int fp = dg_f2_field(p, col);
-                    cpar = dg_eb(p.efield[fp >> 1], 176 - p.tbz - p.vbz + max((int)p.emax[(size_t)fp * B + tl.m] - tl.vb, 0));
-                } else if constexpr (STAGE == kI1) {
-                    cpar = dg_eb(p.ein[(size_t)col * B + tl.m], 120 - tl.vb);
+            const float rscale = P == 32 && live ? ldexpf(1.0f, tl.tb - qrow) : 0.0f;
+            // lane c holds what the rows need to know of column c (of 32): field, place in X, exponent or
+            // shift, and for FP32 the column's unit
+            int cfield_[kHalf], cpar_[kHalf];
+            uint32_t coff_[kHalf];
+            float cscale_[kHalf];
+#pragma unroll
+            for (int h = 0; h < kHalf; ++h) {
+                int cfield = 0, cpar = 0;
+                uint32_t coff = 0;
+                float cscale = 0.0f;
+                const int col = cb * NT + grp * kCols + h * 32 + lane;
+                if (lane < kLanes && col < p.ncols) {
+                    if constexpr (STAGE == kF1) {
+                        cfield = col / S;
+                        const int rem = col - cfield * S, t = rem >= B, j = rem - t * B;
+                        if constexpr (P == 64) cpar = min(max((int)p.efield[cfield], 1) - max((int)p.ein[cfield * B + j], 1), 63);
+                        else cscale = dg_col_scale(p.ein[cfield * B + j], tl.tb, p.vbz);
+                        coff = (uint32_t)(cfield * 2 + tl.t) * B * 2 * p.BP + t * p.BP + j;
+                    } else if constexpr (STAGE == kF2) {
+                        const int fp = dg_f2_field(p, col);
+                        if constexpr (P == 32) cscale = dg_col_scale(p.emax[(size_t)fp * B + tl.m], tl.tb, tl.vb);
+                        else cpar = dg_eb(p.efield[fp >> 1], 176 - p.tbz - p.vbz + max((int)p.emax[(size_t)fp * B + tl.m] - tl.vb, 0));
+                    } else if constexpr (STAGE == kI1) {
+                        if constexpr (P == 32) cscale = dg_col_scale(p.ein[(size_t)col * B + tl.m], tl.tb, tl.vb);
+                        else cpar = dg_eb(p.ein[(size_t)col * B + tl.m], 120 - tl.vb);
+                    } else if constexpr (P == 32) {
+                        cscale = dg_col_scale(p.ein[col / S], tl.tb, tl.vb);
+                    }
                 }
+                cfield_[h] = cfield, cpar_[h] = cpar, coff_[h] = coff, cscale_[h] = cscale;
             }
             if (!dg_wait_warp(&accFull[slot], use & 1, &failed)) break;
             ++use;
             tc::tc_fence_after();
-            const uint32_t tb = tmem + lane_off + slot * accCols + grp * kCols;
             constexpr int CH = 4;  // columns at a time
+#pragma unroll
+            for (int h = 0; h < kHalf; ++h) {
+            const int cfield = cfield_[h], cpar = cpar_[h];
+            const uint32_t coff = coff_[h];
+            [[maybe_unused]] const float cscale = cscale_[h];
+            const int colb = cb * NT + grp * kCols + h * 32;
+            const int ncol = min(kLanes, p.ncols - colb);  // may be negative
+            const uint32_t tb = tmem + lane_off + slot * accCols + grp * kCols + h * 32;
             uint32_t mx = 0;
 #pragma unroll 1
             for (int c0 = 0; c0 < ncol; c0 += CH) {
-                uint32_t a[kDigits * CH];
+                uint32_t a[G * CH];
 #pragma unroll
-                for (int d = 0; d < kDigits; ++d) tm_ld4(tb + d * NT + c0, &a[d * CH]);
+                for (int d = 0; d < G; ++d) tm_ld4(tb + d * NT + c0, &a[d * CH]);
                 tm_wait();
+                Real v[CH];
                 long long T[CH];
-                uint32_t odd = 0;
-#pragma unroll
-                for (int c = 0; c < CH; ++c) T[c] = dg_sum(&a[c], CH, odd);
-                if (odd & 0xff800000u) {
-#pragma unroll
-                    for (int c = 0; c < CH; ++c)
-                        T[c] = dg_sum_big(__uint_as_float(a[c]), __uint_as_float(a[CH + c]), __uint_as_float(a[2 * CH + c]),
-                                          __uint_as_float(a[3 * CH + c]), __uint_as_float(a[4 * CH + c]),
-                                          __uint_as_float(a[5 * CH + c]), __uint_as_float(a[6 * CH + c]));
-                }
-                double v[CH];
-                if constexpr (STAGE == kF2 || STAGE == kI1) {
-                    bool bad = false;
-                    int eb[CH];
+                if constexpr (P == 32) {
 #pragma unroll
                     for (int c = 0; c < CH; ++c) {
-                        eb[c] = __shfl_sync(0xffffffffu, cpar, (c0 + c) & 31) - qrow;
-                        v[c] = dg_fast(T[c], eb[c], bad);
-                    }
-                    if (bad)
+                        float x = __uint_as_float(a[(G - 1) * CH + c]);
 #pragma unroll
-                        for (int c = 0; c < CH; ++c) v[c] = dg_slow(T[c], eb[c]);
+                        for (int d = G - 2; d >= 0; --d) x = fmaf(x, 0.00390625f, __uint_as_float(a[d * CH + c]));
+                        v[c] = x * __shfl_sync(0xffffffffu, cscale, (c0 + c) & 31) * rscale;
+                    }
+                } else {
+                    uint32_t odd = 0;
+#pragma unroll
+                    for (int c = 0; c < CH; ++c) T[c] = dg_sum(&a[c], CH, odd);
+                    if (odd & 0xff800000u) {
+#pragma unroll
+                        for (int c = 0; c < CH; ++c)
+                            T[c] = dg_sum_big(__uint_as_float(a[c]), __uint_as_float(a[CH + c]), __uint_as_float(a[2 * CH + c]),
+                                              __uint_as_float(a[3 * CH + c]), __uint_as_float(a[4 * CH + c]),
+                                              __uint_as_float(a[5 * CH + c]), __uint_as_float(a[6 * CH + c]));
+                    }
+                    if constexpr (STAGE == kF2 || STAGE == kI1) {
+                        bool bad = false;
+                        int eb[CH];
+#pragma unroll
+                        for (int c = 0; c < CH; ++c) {
+                            eb[c] = __shfl_sync(0xffffffffu, cpar, (c0 + c) & 31) - qrow;
+                            v[c] = dg_fast(T[c], eb[c], bad);
+                        }
+                        if (bad)
+#pragma unroll
+                            for (int c = 0; c < CH; ++c) v[c] = dg_slow(T[c], eb[c]);
+                    }
                 }
                 const int col0 = colb + c0, nc = ncol - c0;  // columns of this chunk: min(CH, nc)
                 if constexpr (STAGE == kF1) {
-                    // integers in the scale of the function
-                    const size_t xm = (size_t)((tl.kind < 4 ? 2 : 1) * row + tl.m) * 2 * p.BP;
-                    long long* X = (long long*)p.X + xm;
-#pragma unroll
-                    for (int c = 0; c < CH; ++c) T[c] >>= __shfl_sync(0xffffffffu, cpar, (c0 + c) & 31);
+                    // FP64: integers in the scale of the function
+                    const int m = (tl.kind < 4 ? 2 : 1) * row + tl.m;
+                    const size_t xm = (size_t)m * 2 * p.BP;
                     const int fa = __shfl_sync(0xffffffffu, cfield, c0 & 31);
                     const int fb = __shfl_sync(0xffffffffu, cfield, (c0 + min(CH - 1, nc - 1)) & 31);
-                    if ((B & 1) == 0) {
+                    uint32_t x[CH], o[CH];  // sizes for the row's largest, places
 #pragma unroll
-                        for (int c = 0; c < CH; c += 2) {
-                            const uint32_t o = __shfl_sync(0xffffffffu, coff, (c0 + c) & 31);
-                            if (live && c < nc) *(longlong2*)(X + o) = make_longlong2(T[c], T[c + 1]);
+                    for (int c = 0; c < CH; ++c) {
+                        o[c] = __shfl_sync(0xffffffffu, coff, (c0 + c) & 31);
+                        if constexpr (P == 64) {
+                            T[c] >>= __shfl_sync(0xffffffffu, cpar, (c0 + c) & 31);
+                            x[c] = 64u - (uint32_t)__clzll(T[c] < 0 ? -T[c] : T[c]);
+                        } else {
+                            x[c] = dexp(v[c]);
                         }
-                    } else {
-#pragma unroll
-                        for (int c = 0; c < CH; ++c) {
-                            const uint32_t o = __shfl_sync(0xffffffffu, coff, (c0 + c) & 31);
-                            if (live && c < nc) X[o] = T[c];
-                        }
+                        if (c >= nc) x[c] = 0;
                     }
-                    // bits of the row's largest value, per field
-                    const int m = (tl.kind < 4 ? 2 : 1) * row + tl.m;
-                    if (fa == fb) {
-                        uint32_t x = 0;
+                    if constexpr (P == 64) {
+                        long long* X = (long long*)p.X + xm;
+                        if ((B & 1) == 0) {
 #pragma unroll
-                        for (int c = 0; c < CH; ++c) x = max(x, c < nc ? 64u - (uint32_t)__clzll(T[c] < 0 ? -T[c] : T[c]) : 0u);
-                        mx = max(mx, x);
+                            for (int c = 0; c < CH; c += 2)
+                                if (live && c < nc) *(longlong2*)(X + o[c]) = make_longlong2(T[c], T[c + 1]);
+                        } else {
+#pragma unroll
+                            for (int c = 0; c < CH; ++c)
+                                if (live && c < nc) X[o[c]] = T[c];
+                        }
+                    } else if ((B & 3) == 0) {
+                        if (live) *(float4*)((float*)p.X + xm + o[0]) = make_float4(v[0], v[1], v[2], v[3]);
+                    } else {
+                        float* stash = stash0 + (warp - 4) * (kDgStash / 4) + lane * 33 + c0;
+#pragma unroll
+                        for (int c = 0; c < CH; ++c) stash[c] = v[c];
+                    }
+                    if (fa == fb) {
+#pragma unroll
+                        for (int c = 0; c < CH; ++c) mx = max(mx, x[c]);
                         const int fn = c0 + CH < ncol ? __shfl_sync(0xffffffffu, cfield, (c0 + CH) & 31) : -1;
                         if (fn != fa) {
                             if (live) atomicMax(p.emax + (size_t)(fa * 2 + tl.t) * B + m, mx);
@@ -597,7 +747,7 @@ __global__ void __launch_bounds__(kDgThreads, 1) k_dg(DgArgs p) {
 #pragma unroll
                         for (int c = 0; c < CH; ++c) {
                             const int f = __shfl_sync(0xffffffffu, cfield, (c0 + c) & 31);
-                            mx = max(mx, 64u - (uint32_t)__clzll(T[c] < 0 ? -T[c] : T[c]));
+                            mx = max(mx, x[c]);
                             if (live && c < nc) atomicMax(p.emax + (size_t)(f * 2 + tl.t) * B + m, mx);
                             const int fn = __shfl_sync(0xffffffffu, cfield, (c0 + c + 1) & 31);
                             if (fn != f) mx = 0;
@@ -608,11 +758,13 @@ __global__ void __launch_bounds__(kDgThreads, 1) k_dg(DgArgs p) {
                     const bool modd = (m & 1) != 0;
                     const int i0 = index_of_harmonic_coeff(m, l, B), i1 = index_of_harmonic_coeff(-m, l, B);
                     if (p.mode == kReal) {
-                        double* qr = p.out_r + (size_t)(col0 >> 1) * B * B;
-                        double* qi = p.out_i + (size_t)(col0 >> 1) * B * B;
 #pragma unroll
                         for (int c = 0; c < CH; c += 2) {
+                            const int f = (col0 + c) >> 1;
                             if (live && c < nc) {
+                                const size_t fb = p.cmap ? (size_t)p.cmap[f] : (size_t)f * B * B;
+                                Real* qr = (Real*)p.out_r + fb;
+                                Real* qi = (Real*)p.out_i + fb;
                                 qr[i0] = v[c];
                                 qi[i0] = v[c + 1];
                                 if (m) {
@@ -620,22 +772,20 @@ __global__ void __launch_bounds__(kDgThreads, 1) k_dg(DgArgs p) {
                                     qi[i1] = modd ? v[c + 1] : -v[c + 1];
                                 }
                             }
-                            qr += B * B;
-                            qi += B * B;
                         }
                     } else {
-                        double* qr = p.out_r + (size_t)(col0 >> 2) * B * B;
-                        double* qi = p.out_i + (size_t)(col0 >> 2) * B * B;
+                        Real* qr = (Real*)p.out_r + (size_t)(col0 >> 2) * B * B;
+                        Real* qi = (Real*)p.out_i + (size_t)(col0 >> 2) * B * B;
 #pragma unroll
                         for (int c = 0; c < CH; c += 4) {
-                            const double gr = v[c], gi = v[c + 1], hr = v[c + 2], hi = v[c + 3];
+                            const Real gr = v[c], gi = v[c + 1], hr = v[c + 2], hi = v[c + 3];
                             if (live && c < nc) {
-                                const double vr = gr - hi, vi = gi + hr;
+                                const Real vr = gr - hi, vi = gi + hr;
                                 qr[i0] = vr;
                                 qi[i0] = vi;
                                 if (m) {
-                                    const double nr = p.mode == kCplx ? gr + hi : vr;
-                                    const double ni = p.mode == kCplx ? hr - gi : -vi;
+                                    const Real nr = p.mode == kCplx ? gr + hi : vr;
+                                    const Real ni = p.mode == kCplx ? hr - gi : -vi;
                                     qr[i1] = modd ? -nr : nr;
                                     qi[i1] = modd ? -ni : ni;
                                 }
@@ -645,7 +795,7 @@ __global__ void __launch_bounds__(kDgThreads, 1) k_dg(DgArgs p) {
                         }
                     }
                 } else if constexpr (STAGE == kI1) {
-                    double* X = (double*)p.X + ((size_t)col0 * B + tl.m) * 2 * p.BP + tl.t * p.BP + row;
+                    Real* X = (Real*)p.X + ((size_t)col0 * B + tl.m) * 2 * p.BP + tl.t * p.BP + row;
                     const size_t step = (size_t)B * 2 * p.BP;
                     uint32_t x[CH];
 #pragma unroll
@@ -661,11 +811,27 @@ __global__ void __launch_bounds__(kDgThreads, 1) k_dg(DgArgs p) {
                     }
                     if (lane < CH / 2 && 2 * lane < nc) atomicMax(p.emax + (col0 >> 1) + lane, mx);
                 } else {
-                    long long* Z = p.Z + (size_t)col0 * p.RL + tl.zoff + row;
+                    const size_t z = (size_t)col0 * p.RL + tl.zoff + row;
 #pragma unroll
                     for (int c = 0; c < CH; ++c)
-                        if (live && c < nc) Z[(size_t)c * p.RL] = (T[c] + 2) >> kDgOutShift;
+                        if (live && c < nc) {
+                            if constexpr (P == 32) ((float*)p.Z)[z + (size_t)c * p.RL] = v[c];
+                            else ((long long*)p.Z)[z + (size_t)c * p.RL] = (T[c] + 2) >> kDgOutShift;
+                        }
                 }
+            }
+            if (P == 32 && STAGE == kF1 && (B & 3) != 0) {
+                // rows that no float4 fits: a row's columns are consecutive latitudes, stored as whole lines
+                // (bw 255, 64 functions: 144 us with a thread's scalar stores, 107 so)
+                __syncwarp();
+                const float* stash = stash0 + (warp - 4) * (kDgStash / 4) + lane;
+                const int rows = min(32, tl.nrows - ew * 32), row0 = tl.row0 + ew * 32;
+                float* X = (float*)p.X + coff;
+#pragma unroll 4
+                for (int i = 0; i < rows; ++i)
+                    if (lane < ncol) X[(size_t)((tl.kind < 4 ? 2 : 1) * (row0 + i) + tl.m) * 2 * p.BP] = stash[i * 33];
+                __syncwarp();
+            }
             }
             tc::tc_fence_before();
             __syncwarp();
@@ -687,6 +853,11 @@ __global__ void __launch_bounds__(kDgThreads, 1) k_dg(DgArgs p) {
 struct DgFold {
     int n[6], off[6], len;  // entries, place and total (padded to the K steps)
 };
+// Rows of 2B samples fold twice where B is even and from 128 on: four tables of B/2 orders, a quarter of the DFT
+// matrix.  Below, one tile of 128 rows holds all orders, or all B + 1 longitudes of a fold, and a second fold
+// would halve the rows a tile uses along with its K, at twice the epilogues and a pass more (bw 100, 1024
+// functions, FP32: once F1 179 us, I2 168; twice 263, 228 and k_dg_mid 15).
+static bool dg_twice(int B) { return B % 2 == 0 && B >= 128; }
 static DgFold dg_fold_layout(int B, bool inv) {
     DgFold f{};
     const int h = B / 2;
@@ -695,7 +866,7 @@ static DgFold dg_fold_layout(int B, bool inv) {
         f.off[kd] = f.len;
         f.len += (n + 15) & ~15;
     };
-    if (B % 2 == 0) {
+    if (dg_twice(B)) {
         // inverse: the cosines of even orders at longitude index B/2 come from k_dg_mid
         put(0, inv ? h : h + 1);
         for (int kd = 1; kd < 4; ++kd) put(kd, h);
@@ -708,17 +879,23 @@ static DgFold dg_fold_layout(int B, bool inv) {
 
 // Latitudes j and 2B-1-j of one field -> fixed point (|x| < 2^vb, scale in e[field][j]) -> even and odd
 // latitude parts of the folded rows, Z[field][t][j][..].  One block per (j, field).
-__global__ void __launch_bounds__(128) k_dg_fold(const double* __restrict__ r, const double* __restrict__ im, int B,
-                                                 int N, int vb, DgFold fl, long long* Z, uint32_t* e, uint32_t* ef) {
-    extern __shared__ long long rows[];  // [2][S]
+template <int P>
+__global__ void __launch_bounds__(128) k_dg_fold(const typename Dg<P>::Real* __restrict__ r,
+                                                 const typename Dg<P>::Real* __restrict__ im, int B, int N, int vb,
+                                                 DgFold fl, const int64_t* __restrict__ gmap, typename Dg<P>::Int* Z,
+                                                 uint32_t* e, uint32_t* ef) {
+    using Real = typename Dg<P>::Real;
+    using Int = typename Dg<P>::Int;
+    extern __shared__ __align__(16) uint8_t fold_sm[];  // [2][S]
+    Int* rows = reinterpret_cast<Int*>(fold_sm);
     __shared__ uint32_t red[4];
     const int S = 2 * B, j = blockIdx.x, ff = blockIdx.y;
-    const double* g = ff < N ? r + (size_t)ff * S * S : im + (size_t)(ff - N) * S * S;
-    const double* x[2] = {g + (size_t)j * S, g + (size_t)(S - 1 - j) * S};
+    const Real* g = gmap ? r + gmap[ff] : ff < N ? r + (size_t)ff * S * S : im + (size_t)(ff - N) * S * S;
+    const Real* x[2] = {g + (size_t)j * S, g + (size_t)(S - 1 - j) * S};
     uint32_t mx = 0;
     for (int i = threadIdx.x; i < 2 * S; i += blockDim.x) {
-        const double v = i < S ? x[0][i] : x[1][i - S];
-        rows[i] = __double_as_longlong(v);
+        const Real v = i < S ? x[0][i] : x[1][i - S];
+        reinterpret_cast<Real*>(rows)[i] = v;
         mx = max(mx, dexp(v));
     }
     mx = __reduce_max_sync(0xffffffffu, mx);
@@ -730,26 +907,26 @@ __global__ void __launch_bounds__(128) k_dg_fold(const double* __restrict__ r, c
         atomicMax(ef + ff, mx);
     }
     const int em = max((int)mx, 1);
-    for (int i = threadIdx.x; i < 2 * S; i += blockDim.x) rows[i] = dg_fix(__longlong_as_double(rows[i]), em, vb);
+    for (int i = threadIdx.x; i < 2 * S; i += blockDim.x) rows[i] = dg_fix(reinterpret_cast<const Real*>(rows)[i], em, vb);
     __syncthreads();
-    long long* z0 = Z + ((size_t)ff * S + j) * fl.len;
-    long long* z1 = z0 + (size_t)B * fl.len;
-    const long long* a = rows;
-    const long long* b = rows + S;
-    auto both = [&](int at, long long u, long long w) {
+    Int* z0 = Z + ((size_t)ff * S + j) * fl.len;
+    Int* z1 = z0 + (size_t)B * fl.len;
+    const Int* a = rows;
+    const Int* b = rows + S;
+    auto both = [&](int at, Int u, Int w) {
         z0[at] = u + w;
         z1[at] = u - w;
     };
-    if (B % 2 == 0) {
+    if (fl.n[0]) {
         const int h = B / 2, pad = ((h + 1 + 15) & ~15);
         for (int k = threadIdx.x; k < pad; k += blockDim.x) {
-            long long c[2][4] = {};
+            Int c[2][4] = {};
             if (k <= h) {
                 const int ks = k ? S - k : 0;
-                const long long* row[2] = {a, b};
+                const Int* row[2] = {a, b};
 #pragma unroll
                 for (int q = 0; q < 2; ++q) {
-                    const long long p0 = row[q][k], p1 = row[q][ks], p2 = row[q][B - k], p3 = row[q][B + k];
+                    const Int p0 = row[q][k], p1 = row[q][ks], p2 = row[q][B - k], p3 = row[q][B + k];
                     c[q][0] = (p0 + p1) + (p2 + p3);
                     c[q][1] = (p0 + p1) - (p2 + p3);
                     c[q][2] = (p0 - p1) - (p2 - p3);
@@ -770,7 +947,7 @@ __global__ void __launch_bounds__(128) k_dg_fold(const double* __restrict__ r, c
     } else {
         const int pad = ((B + 1 + 15) & ~15), sp = ((B - 1 + 15) & ~15);
         for (int k = threadIdx.x; k < pad; k += blockDim.x) {
-            long long u0 = 0, u1 = 0, w0 = 0, w1 = 0;
+            Int u0 = 0, u1 = 0, w0 = 0, w1 = 0;
             if (k <= B) {
                 const int ks = k ? S - k : 0;
                 u0 = a[k] + a[ks];
@@ -787,59 +964,68 @@ __global__ void __launch_bounds__(128) k_dg_fold(const double* __restrict__ r, c
 
 // Inverse, even B: sum over the even orders of c_m (-1)^(m/2) Re F_m, the cosine part at longitude index
 // B/2, for every column of I2.
-__global__ void __launch_bounds__(256) k_dg_mid(const double* __restrict__ X, int B, int ncols, double* mid) {
-    __shared__ double part[8][33];
+template <class Real>
+__global__ void __launch_bounds__(256) k_dg_mid(const Real* __restrict__ X, int B, int ncols, Real* mid) {
+    __shared__ Real part[8][33];
     const int col = blockIdx.x * 32 + threadIdx.x, S = 2 * B;  // 32 columns, eight runs of orders
     const int nb = (B + 3) / 4, per = (nb + 7) / 8;
-    double s = 0.0;
+    Real s = 0;
     if (col < ncols) {
         const int f = col / S, rem = col - f * S;
-        const double* x = X + (size_t)(f * 2) * B * S + rem;  // even B: rows of X have 2B values
+        const int BP = (B + 3) & ~3, t = rem >= B;
+        const Real* x = X + (size_t)(f * 2) * B * 2 * BP + t * BP + (rem - t * B);
         const int b1 = min(nb, (int)(threadIdx.y + 1) * per);
 #pragma unroll 4
         for (int b = threadIdx.y * per; b < b1; ++b) {
             const int m = 4 * b;
-            s += x[(size_t)m * S] - (m + 2 < B ? x[(size_t)(m + 2) * S] : 0.0);
+            s += x[(size_t)m * 2 * BP] - (m + 2 < B ? x[(size_t)(m + 2) * 2 * BP] : Real(0));
         }
     }
     part[threadIdx.y][threadIdx.x] = s;
     __syncthreads();
     if (threadIdx.y == 0 && col < ncols) {
         for (int q = 1; q < 8; ++q) s += part[q][threadIdx.x];
-        const int f = col / S;
-        mid[col] = (2.0 * s - X[(size_t)(f * 2) * B * S + (col - f * S)]) * 0.39894228040143267794;
+        const int f = col / S, rem = col - f * S, BP = (B + 3) & ~3, t = rem >= B;
+        mid[col] = (2 * s - X[(size_t)(f * 2) * B * 2 * BP + t * BP + (rem - t * B)]) * Real(0.39894228040143267794);
     }
 }
 
 // Parts of I2 -> samples of latitudes j and 2B-1-j.  One block per (j, field).
-__global__ void __launch_bounds__(128) k_dg_unfold(const long long* __restrict__ Z, const double* __restrict__ mid,
+template <int P>
+__global__ void __launch_bounds__(128) k_dg_unfold(const void* __restrict__ Zv, const typename Dg<P>::Real* __restrict__ mid,
                                                    const uint32_t* __restrict__ ef, int B, int N, int qv, DgFold fl,
-                                                   double* r, double* im) {
+                                                   const int64_t* __restrict__ gmap, typename Dg<P>::Real* r, typename Dg<P>::Real* im) {
+    using Real = typename Dg<P>::Real;
+    using Part = std::conditional_t<P == 64, long long, float>;
+    const Part* Z = (const Part*)Zv;
     const int S = 2 * B, j = blockIdx.x, ff = blockIdx.y;
-    double* g = ff < N ? r + (size_t)ff * S * S : im + (size_t)(ff - N) * S * S;
-    double* out[2] = {g + (size_t)j * S, g + (size_t)(S - 1 - j) * S};
-    const long long* z0 = Z + ((size_t)ff * S + j) * fl.len;
-    const long long* z1 = z0 + (size_t)B * fl.len;
-    const uint32_t em = ef[ff];
-    const int eb = dg_eb(em, 120 + kDgOutShift - qv);  // qv: bits of table and data values
-    auto value = [&](long long T) {
-        bool bad = false;
-        const double v = dg_fast(T, eb, bad);
-        return bad ? dg_slow(T, eb) : v;
+    Real* g = gmap ? r + gmap[ff] : ff < N ? r + (size_t)ff * S * S : im + (size_t)(ff - N) * S * S;
+    Real* out[2] = {g + (size_t)j * S, g + (size_t)(S - 1 - j) * S};
+    const Part* z0 = Z + ((size_t)ff * S + j) * fl.len;
+    const Part* z1 = z0 + (size_t)B * fl.len;
+    [[maybe_unused]] const int eb = P == 64 ? dg_eb(ef[ff], 120 + kDgOutShift - qv) : 0;  // qv: bits of table and data values
+    auto value = [&](Part T) -> Real {
+        if constexpr (P == 32) {
+            return T;
+        } else {
+            bool bad = false;
+            const double v = dg_fast(T, eb, bad);
+            return bad ? dg_slow(T, eb) : v;
+        }
     };
-    auto put = [&](int k, long long u, long long w) {  // even and odd latitude parts
+    auto put = [&](int k, Part u, Part w) {  // even and odd latitude parts
         out[0][k] = value(u + w);
         out[1][k] = value(u - w);
     };
-    if (B % 2 == 0) {
+    if (fl.n[0]) {
         const int h = B / 2;
         for (int k = threadIdx.x; k < h; k += blockDim.x) {
-            long long c[2], d[2], s[2], q[2];
-            const long long* z[2] = {z0, z1};
+            Part c[2], d[2], s[2], q[2];
+            const Part* z[2] = {z0, z1};
 #pragma unroll
             for (int t = 0; t < 2; ++t) {
-                const long long ce = z[t][fl.off[0] + k], co = z[t][fl.off[1] + k];
-                const long long se = k ? z[t][fl.off[2] + k] : 0, so = k ? z[t][fl.off[3] + k - 1] : 0;
+                const Part ce = z[t][fl.off[0] + k], co = z[t][fl.off[1] + k];
+                const Part se = k ? z[t][fl.off[2] + k] : 0, so = k ? z[t][fl.off[3] + k - 1] : 0;
                 c[t] = ce + co;
                 d[t] = ce - co;
                 s[t] = se + so;
@@ -853,18 +1039,18 @@ __global__ void __launch_bounds__(128) k_dg_unfold(const long long* __restrict__
             }
         }
         if (threadIdx.x < 2) {  // k = B/2 and 3B/2
-            const double sg = threadIdx.x ? -1.0 : 1.0;
-            const double m0 = mid[(size_t)ff * S + j], m1 = mid[(size_t)ff * S + B + j];
-            const double s0 = value(z0[fl.off[3] + h - 1]), s1 = value(z1[fl.off[3] + h - 1]);
+            const Real sg = threadIdx.x ? -1 : 1;
+            const Real m0 = mid[(size_t)ff * S + j], m1 = mid[(size_t)ff * S + B + j];
+            const Real s0 = value(z0[fl.off[3] + h - 1]), s1 = value(z1[fl.off[3] + h - 1]);
             const int k = threadIdx.x ? B + h : h;
             out[0][k] = (m0 + m1) + sg * (s0 + s1);
             out[1][k] = (m0 - m1) + sg * (s0 - s1);
         }
     } else {
         for (int k = threadIdx.x; k <= B; k += blockDim.x) {
-            const long long c0 = z0[fl.off[4] + k], c1 = z1[fl.off[4] + k];
+            const Part c0 = z0[fl.off[4] + k], c1 = z1[fl.off[4] + k];
             const bool in = k >= 1 && k < B;
-            const long long s0 = in ? z0[fl.off[5] + k - 1] : 0, s1 = in ? z1[fl.off[5] + k - 1] : 0;
+            const Part s0 = in ? z0[fl.off[5] + k - 1] : 0, s1 = in ? z1[fl.off[5] + k - 1] : 0;
             put(k, c0 + s0, c1 + s1);
             if (in) put(S - k, c0 - s0, c1 - s1);
         }
@@ -875,29 +1061,30 @@ __global__ void __launch_bounds__(128) k_dg_unfold(const long long* __restrict__
 // imaginary output, are first split into two real fields' coefficients (cr, ci, orders m >= 0):
 //   g = (a + s conj b) / 2, h = (a - s conj b) / 2i with a = f(l,m), b = f(l,-m), s = (-1)^m.
 // One warp per (function, order).
-__global__ void k_dg_coefmax(const double* __restrict__ rc, const double* __restrict__ ic, int B, int N, int mode,
-                             double* cr, double* ci, uint32_t* e) {
+template <class Real>
+__global__ void k_dg_coefmax(const Real* __restrict__ rc, const Real* __restrict__ ic, int B, int N, int mode,
+                             const int64_t* __restrict__ cmap, Real* cr, Real* ci, uint32_t* e) {
     const int id = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (id >= N * B) return;
     const int f = id / B, m = id - f * B;
-    const size_t cb = (size_t)f * B * B, hb = (size_t)(N + f) * B * B;
+    const size_t cb = cmap ? (size_t)cmap[f] : (size_t)f * B * B, hb = (size_t)(N + f) * B * B;
     uint32_t mx[4] = {0, 0, 0, 0};
     for (int l = m + lane; l < B; l += 32) {
         const int i = index_of_harmonic_coeff(m, l, B);
-        const double ar = rc[cb + i], ai = ic[cb + i];
+        const Real ar = rc[cb + i], ai = ic[cb + i];
         if (mode == kReal) {
             mx[0] = max(mx[0], dexp(ar));
             if (m) mx[1] = max(mx[1], dexp(ai));
             continue;
         }
-        double v[4] = {ar, m ? ai : 0.0, m ? 0.0 : ai, 0.0};  // Im f(l, 0) is the second field's
+        Real v[4] = {ar, m ? ai : Real(0), m ? Real(0) : ai, 0};  // Im f(l, 0) is the second field's
         if (mode == kCplx && m) {
             const int k = index_of_harmonic_coeff(-m, l, B);
-            const double s = (m & 1) ? -1.0 : 1.0, br = s * rc[cb + k], bi = s * ic[cb + k];
-            v[0] = 0.5 * ar + 0.5 * br;
-            v[1] = 0.5 * ai - 0.5 * bi;
-            v[2] = 0.5 * ai + 0.5 * bi;
-            v[3] = 0.5 * br - 0.5 * ar;
+            const Real s = (m & 1) ? -1 : 1, br = s * rc[cb + k], bi = s * ic[cb + k];
+            v[0] = Real(0.5) * ar + Real(0.5) * br;
+            v[1] = Real(0.5) * ai - Real(0.5) * bi;
+            v[2] = Real(0.5) * ai + Real(0.5) * bi;
+            v[3] = Real(0.5) * br - Real(0.5) * ar;
         }
         cr[cb + i] = v[0];
         ci[cb + i] = v[1];
@@ -1007,21 +1194,22 @@ __device__ __forceinline__ int dg_scale(double mx, int tb) {
 }
 
 // Digits of one 8-row group; 128 threads = 8 rows x 16 K entries per step.  val(row, k): the table value.
-template <class Val>
+template <int P, class Val>
 __device__ __forceinline__ int dg_pack_rows(Val val, int q, uint8_t* blob, int r8, int ks, int rg) {
     const int r = threadIdx.x >> 4, kk = threadIdx.x & 15;
-    const uint32_t bytes = kDigits * (uint32_t)r8 * 32;
+    constexpr int DA = Dg<P>::DA;
+    const uint32_t bytes = DA * (uint32_t)r8 * 32;
     int first = ks;  // this thread's first step with a nonzero value
     for (int s = 0; s < ks; ++s) {
         const double x = val(r, s * 16 + kk);
         const long long v = __double2ll_rn(scalbn(x, q));
         if (v && first == ks) first = s;
-        const unsigned long long u = (unsigned long long)v + 0x0200808080808080ull;
+        const unsigned long long u = (unsigned long long)v + (P == 64 ? 0x0200808080808080ull : 0x02008080ull);
         uint8_t* d = blob + (size_t)s * bytes + rg * 256 + (kk >> 3) * 128 + r * 16 + (kk & 7) * 2;
 #pragma unroll
-        for (int a = 0; a < kDigits; ++a)
+        for (int a = 0; a < DA; ++a)
             *(__half*)(d + (size_t)a * r8 * 32) =
-                __int2half_rn(a ? (int)((u >> (8 * (6 - a))) & 255) - 128 : (int)(u >> 48) - 512);
+                __int2half_rn(a ? (int)((u >> (8 * (DA - 1 - a))) & 255) - 128 : (int)(u >> (8 * DA - 8)) - 512);
     }
     return first;
 }
@@ -1031,6 +1219,7 @@ constexpr double kDgTiny = 5.4e-20;
 
 // Legendre tables of the orders m0 ..: one block per (tile, 8-row group); tiles of kind F2 (rows degrees,
 // weighted) or I1 (rows nodes).
+template <int P>
 __global__ void __launch_bounds__(128) k_dg_pack_leg(int B, int fwd, const DgTile* __restrict__ tiles, int m0,
                                                      const double* __restrict__ tmp, const int64_t* __restrict__ off,
                                                      const double* __restrict__ w, double wscale, uint8_t* tab,
@@ -1039,13 +1228,13 @@ __global__ void __launch_bounds__(128) k_dg_pack_leg(int B, int fwd, const DgTil
     const DgTile tl = tiles[blockIdx.x];
     const int rg = blockIdx.y;
     if (rg * 8 >= tl.r8) return;
-    const double* P = tmp + off[tl.m - m0];
+    const double* leg = tmp + off[tl.m - m0];
     const int nl = (B - tl.m - tl.t + 1) / 2;  // degrees of this parity
     auto val = [&](int r, int k) -> double {
         const int row = tl.row0 + rg * 8 + r;
         if (rg * 8 + r >= tl.nrows) return 0.0;
-        if (fwd) return k < B ? P[(size_t)(tl.t + 2 * row) * B + k] * (w[k] * wscale) : 0.0;
-        return k < nl ? P[(size_t)(tl.t + 2 * k) * B + row] : 0.0;
+        if (fwd) return k < B ? leg[(size_t)(tl.t + 2 * row) * B + k] * (w[k] * wscale) : 0.0;
+        return k < nl ? leg[(size_t)(tl.t + 2 * k) * B + row] : 0.0;
     };
     const int r = threadIdx.x >> 4, kk = threadIdx.x & 15;
     double mx = 0.0;
@@ -1056,7 +1245,7 @@ __global__ void __launch_bounds__(128) k_dg_pack_leg(int B, int fwd, const DgTil
     const bool tiny = !fwd && mx < kDgTiny;
     const int q = tiny ? 0 : dg_scale(mx, tl.tb);
     if (kk == 0 && rg * 8 + r < tl.nrows) qs[tl.qoff + tl.row0 + rg * 8 + r] = (short)q;
-    const int f = dg_pack_rows([&](int a, int k) { return tiny ? 0.0 : val(a, k); }, q, tab + tl.off, tl.r8, tl.ks, rg);
+    const int f = dg_pack_rows<P>([&](int a, int k) { return tiny ? 0.0 : val(a, k); }, q, tab + tl.off, tl.r8, tl.ks, rg);
     atomicMin(first + blockIdx.x, f);
 }
 
@@ -1166,6 +1355,7 @@ __global__ void __launch_bounds__(128) k_dg_pack_fly(int B, int fwd, const DgTil
 }
 
 // DFT tables: F1 (rows orders, K longitudes) and I2 (rows longitudes, K orders), folds as k_dg_fold.
+template <int P>
 __global__ void __launch_bounds__(128) k_dg_pack_dft(int B, int inv, const DgTile* __restrict__ tiles, uint8_t* tab,
                                                      short* qs) {
     const DgTile tl = tiles[blockIdx.x];
@@ -1185,7 +1375,7 @@ __global__ void __launch_bounds__(128) k_dg_pack_dft(int B, int inv, const DgTil
         const double a = 2.0 * (double)((long long)m * lon % S) / (double)S;  // angle / pi
         return tl.t ? -f * sinpi(a) : f * cospi(a);
     };
-    dg_pack_rows(val, tl.tb, tab + tl.off, tl.r8, tl.ks, rg);
+    dg_pack_rows<P>(val, tl.tb, tab + tl.off, tl.r8, tl.ks, rg);
     const int r = threadIdx.x >> 4;
     if ((threadIdx.x & 15) == 0 && rg * 8 + r < tl.nrows) qs[tl.qoff + tl.row0 + rg * 8 + r] = (short)tl.tb;
 }
@@ -1215,7 +1405,7 @@ struct DgChunk {
 };
 
 struct DgTabs {
-    int device = -1, bw = 0, refs = 0;
+    int device = -1, bw = 0, refs = 0, prec = 64;
     bool fly = false;  // no Legendre tables: chunks, nodes and offsets instead
     DgTable t[4];
     int* err = nullptr;
@@ -1227,7 +1417,7 @@ struct DgTabs {
 };
 
 static std::mutex g_dg_mu;
-static std::map<std::tuple<int, int, bool>, DgTabs*> g_dg;
+static std::map<std::tuple<int, int, int, bool>, DgTabs*> g_dg;
 
 static void dg_free(DgTabs* d) {
     for (auto& t : d->t) t.release();
@@ -1243,13 +1433,16 @@ void dg_put(void* h) {
     if (!d) return;
     std::lock_guard<std::mutex> lk(g_dg_mu);
     if (--d->refs == 0) {
-        g_dg.erase(std::make_tuple(d->device, d->bw, d->fly));
+        g_dg.erase(std::make_tuple(d->device, d->bw, d->prec, d->fly));
         dg_free(d);
     }
 }
 
-static int dg_vbz(int bw) {  // bits of a sample: eight (odd bw: four) of them add up to a data value
-    return (bw % 2 ? 52 : 51) + (dg_fold_layout(bw, false).n[bw % 2 ? 4 : 0] <= 272 ? 2 : 0);
+// Bits of a sample: eight (rows folded once: four) of them add up to a data value.
+static int dg_vbz(int bw, int prec) {
+    const bool two = dg_twice(bw);
+    if (prec == 32) return two ? 27 : 28;
+    return (two ? 51 : 52) + (dg_fold_layout(bw, false).n[two ? 0 : 4] <= 272 ? 2 : 0);
 }
 
 // Bits of a table value: the leading group, at most K 2^(vb - 48) 2^(tb - 48), stays near 2^22, so that the
@@ -1261,7 +1454,7 @@ static int dg_table_bits(int K, int vb, bool inv_rows) {
     return 48 + std::min(8, 22 - kb - (vb - 48));
 }
 
-static void dg_tiles(DgTable& t, int stage, int B) {
+static void dg_tiles(DgTable& t, int stage, int B, int prec) {
     auto add = [&](int rows, int k, int m, int par, int kind, int zoff) {
         const int q0 = t.rows;
         for (int r0 = 0; r0 < rows; r0 += 128) {
@@ -1278,17 +1471,22 @@ static void dg_tiles(DgTable& t, int stage, int B) {
             // F1's data have vbz bits and folds; I2's sums of eight parts stay below 2^63
             tl.vb = stage == kI2 ? (k <= 128 ? 55 : k <= 256 ? 54 : 53) : (stage == kI1 ? (k <= 256 ? 55 : 54) : (k <= 256 ? 56 : 54));
             // the panels of F1 share one scale
-            if (stage == kF1) tl.tb = dg_table_bits(B % 2 ? B + 1 : B / 2 + 1, dg_vbz(B) >= 53 ? 56 : 54, false);
+            if (stage == kF1) tl.tb = dg_table_bits(dg_twice(B) ? B / 2 + 1 : B + 1, dg_vbz(B, 64) >= 53 ? 56 : 54, false);
             else tl.tb = dg_table_bits(k, tl.vb, stage == kI2);
+            if (prec == 32) {
+                tl.vb = 30;
+                tl.tb = k <= 257 ? 25 : 24;
+                if (stage == kF1) tl.tb = B <= 512 ? 25 : 24;
+            }
             tl.off = t.bytes;
-            t.bytes += (int64_t)tl.ks * kDigits * tl.r8 * 32;
+            t.bytes += (int64_t)tl.ks * (prec == 32 ? Dg<32>::DA : Dg<64>::DA) * tl.r8 * 32;
             t.h.push_back(tl);
         }
         t.rows += rows;
     };
     if (stage == kF1 || stage == kI2) {
         const DgFold f = dg_fold_layout(B, stage == kI2);
-        for (int kd = B % 2 ? 4 : 0; kd < (B % 2 ? 6 : 4); ++kd) {
+        for (int kd = dg_twice(B) ? 0 : 4; kd < (dg_twice(B) ? 4 : 6); ++kd) {
             const int m0 = kd < 4 ? kd & 1 : 0, part = kd < 4 ? kd >> 1 : kd - 4, nm = kd < 4 ? B / 2 : B;
             if (stage == kF1) add(nm, f.n[kd], m0, part, kd, f.off[kd]);
             else add(f.n[kd], nm, m0, part, kd, f.off[kd]);
@@ -1303,8 +1501,8 @@ static void dg_tiles(DgTable& t, int stage, int B) {
         }
 }
 
-static int dg_upload(DgTable& t, int stage, int B, cudaStream_t st) {
-    dg_tiles(t, stage, B);
+static int dg_upload(DgTable& t, int stage, int B, int prec, cudaStream_t st) {
+    dg_tiles(t, stage, B, prec);
     S2G_CUDA(cudaMalloc(&t.tiles, sizeof(DgTile) * t.h.size()));
     S2G_CUDA(cudaMalloc(&t.tab, (size_t)t.bytes + 4096));
     S2G_CUDA(cudaMalloc(&t.q, sizeof(short) * t.rows));
@@ -1389,7 +1587,7 @@ static int dg_fly_chunks(DgTabs* d, const double* weights, cudaStream_t st) {
     const int B = d->bw;
     for (int s = kF2; s <= kI1; ++s) {
         DgTable& t = d->t[s];
-        dg_tiles(t, s, B);
+        dg_tiles(t, s, B, d->prec);
         std::vector<int64_t> off(B);
         int64_t base = 0, at = 0;
         size_t k = 0;
@@ -1442,11 +1640,13 @@ static int dg_build(DgTabs* d, const double* weights, cudaStream_t st) {
     S2G_CUDA(cudaMalloc(&d->err, sizeof(int)));
     S2G_CUDA(cudaMemsetAsync(d->err, 0, sizeof(int), st));
     for (int s = 0; s < 4; ++s)
-        if (!d->fly || s == kF1 || s == kI2) S2G_TRY(dg_upload(d->t[s], s, B, st));
+        if (!d->fly || s == kF1 || s == kI2) S2G_TRY(dg_upload(d->t[s], s, B, d->prec, st));
     for (int s = kF1; s <= kI2; s += kI2 - kF1) {
         const DgTable& t = d->t[s];
         ProfScope ps_("dg_pack_dft", st);
-        k_dg_pack_dft<<<dim3((unsigned)t.h.size(), 16), 128, 0, st>>>(B, s == kI2, t.tiles, t.tab, t.q);
+        const dim3 grid((unsigned)t.h.size(), 16);
+        if (d->prec == 32) k_dg_pack_dft<32><<<grid, 128, 0, st>>>(B, s == kI2, t.tiles, t.tab, t.q);
+        else k_dg_pack_dft<64><<<grid, 128, 0, st>>>(B, s == kI2, t.tiles, t.tab, t.q);
         S2G_CUDA(cudaGetLastError());
     }
     // nodes, seeds P(m,m) = seed_m sin^m: long double, split in two doubles
@@ -1512,13 +1712,14 @@ static int dg_build(DgTabs* d, const double* weights, cudaStream_t st) {
         }
         S2G_CUDA(cudaGetLastError());
         for (int s = kI1; s >= kF2; --s) {
-            if (s == kF2 && B > kDgNaiveBw && m0 <= 1) S2G_TRY(dg_low_orders(B, (double*)tmp.p[1], off, m1, st));
+            if (s == kF2 && B > kDgNaiveBw && m0 <= 1 && d->prec == 64) S2G_TRY(dg_low_orders(B, (double*)tmp.p[1], off, m1, st));
             const DgTable& t = d->t[s];
             size_t a = 0, b = t.h.size();
             while (a < b && t.h[a].m < m0) ++a;
             while (b > a && t.h[b - 1].m >= m1) --b;
             ProfScope ps_("dg_pack_leg", st);
-            k_dg_pack_leg<<<dim3((unsigned)(b - a), 16), 128, 0, st>>>(
+            const auto pack = d->prec == 32 ? k_dg_pack_leg<32> : k_dg_pack_leg<64>;
+            pack<<<dim3((unsigned)(b - a), 16), 128, 0, st>>>(
                 B, s == kF2, t.tiles + a, m0, (const double*)tmp.p[1], (const int64_t*)tmp.p[2] + m0, weights,
                 sqrt(2.0 * 3.14159265358979323846) / S, t.tab, t.q, first[s] + a);
             S2G_CUDA(cudaGetLastError());
@@ -1530,11 +1731,11 @@ static int dg_build(DgTabs* d, const double* weights, cudaStream_t st) {
 }
 
 // Digit tables of bandwidth bw on the current device, shared by every plan; the caller holds a reference.
-static int dg_get(int bw, bool fly, const double* weights, DgTabs** out) {
+static int dg_get(int bw, int prec, bool fly, const double* weights, DgTabs** out) {
     int dev = 0;
     S2G_CUDA(cudaGetDevice(&dev));
     std::lock_guard<std::mutex> lk(g_dg_mu);
-    auto it = g_dg.find(std::make_tuple(dev, bw, fly));
+    auto it = g_dg.find(std::make_tuple(dev, bw, prec, fly));
     if (it != g_dg.end()) {
         ++it->second->refs;
         *out = it->second;
@@ -1543,6 +1744,7 @@ static int dg_get(int bw, bool fly, const double* weights, DgTabs** out) {
     DgTabs* d = new DgTabs();
     d->device = dev;
     d->bw = bw;
+    d->prec = prec;
     d->fly = fly;
     cudaStream_t st;
     S2G_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
@@ -1553,23 +1755,25 @@ static int dg_get(int bw, bool fly, const double* weights, DgTabs** out) {
         return r;
     }
     d->refs = 1;
-    g_dg[std::make_tuple(dev, bw, fly)] = d;
+    g_dg[std::make_tuple(dev, bw, prec, fly)] = d;
     *out = d;
     return S2G_OK;
 }
 
-template <int STAGE, int NT>
+template <int STAGE, int NT, int P>
 static int launch_dg_nt(const DgArgs& p, cudaStream_t st) {
-    static const char* names[4] = {"dg_rows_fwd", "dg_leg_fwd", "dg_leg_inv", "dg_rows_inv"};
-    const size_t smem = 1024 + kDgStagesA * kDgABytes + kDgBRing;
-    S2G_CUDA(cudaFuncSetAttribute((const void*)k_dg<STAGE, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static const char* names[8] = {"dg_rows_fwd", "dg_leg_fwd", "dg_leg_inv", "dg_rows_inv",
+                                   "dg_rows_fwd_f32", "dg_leg_fwd_f32", "dg_leg_inv_f32", "dg_rows_inv_f32"};
+    const size_t smem = 1024 + Dg<P>::stagesA * kDgABytes<P> + kDgBRing +
+                        (P == 32 && STAGE == kF1 ? Dg<P>::epilogue * kDgStash : 0);
+    S2G_CUDA(cudaFuncSetAttribute((const void*)k_dg<STAGE, NT, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int dev = 0, sms = 0;
     S2G_CUDA(cudaGetDevice(&dev));
     S2G_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const int64_t items = (int64_t)p.ntiles * p.ncolblk;
     {
-        ProfScope ps_(names[STAGE], st);
-        k_dg<STAGE, NT><<<(unsigned)std::min<int64_t>(items, sms), kDgThreads, smem, st>>>(p);
+        ProfScope ps_(names[STAGE + (P == 32 ? 4 : 0)], st);
+        k_dg<STAGE, NT, P><<<(unsigned)std::min<int64_t>(items, sms), kDgThreads, smem, st>>>(p);
     }
     S2G_CUDA(cudaGetLastError());
     return S2G_OK;
@@ -1579,8 +1783,8 @@ static int launch_dg_nt(const DgArgs& p, cudaStream_t st) {
 // fewer columns in all take 32 or 16 (two accumulators, so that the epilogue of one item runs beside the
 // MMAs of the next).  Items of F1 and I2 go column by column (their four tables, 1 MB at bw 256, stay in
 // L2), those of F2 and I1 table by table (117 MB each at bw 256).
-// At bw 256, 64 functions: F1 160 us, F2 130, I1 135, I2 127, k_dg_fold 68, k_dg_unfold 54, k_dg_mid 17;
-// forward and inverse together 0.69 ms against 4.59 ms on the FP64 units (DFMA-bound there).  The tensor
+// At bw 256, 64 functions: F1 164 us, F2 119, I1 133, I2 118, k_dg_fold 67, k_dg_unfold 53, k_dg_mid 17;
+// forward and inverse together 0.68 ms against 4.59 ms on the FP64 units (DFMA-bound there).  The tensor
 // pipe alone would take 47 us for each of the four; MMA issue and the part of the epilogue that the next
 // item's MMAs wait for (dg_sum, the stores) make up the rest.
 template <int STAGE>
@@ -1589,9 +1793,14 @@ static int launch_dg_tiles(const DgTabs* d, DgArgs p, cudaStream_t st) {
     p.err = d->err;
     const int per = p.ncols <= 16 ? 16 : (p.ncols <= 32 ? 32 : 64);
     p.ncolblk = (p.ncols + per - 1) / per;
-    if (per == 16) return launch_dg_nt<STAGE, 16>(p, st);
-    if (per == 32) return launch_dg_nt<STAGE, 32>(p, st);
-    return launch_dg_nt<STAGE, 64>(p, st);
+    if (d->prec == 32) {
+        if (per == 16) return launch_dg_nt<STAGE, 16, 32>(p, st);
+        if (per == 32) return launch_dg_nt<STAGE, 32, 32>(p, st);
+        return launch_dg_nt<STAGE, 64, 32>(p, st);
+    }
+    if (per == 16) return launch_dg_nt<STAGE, 16, 64>(p, st);
+    if (per == 32) return launch_dg_nt<STAGE, 32, 64>(p, st);
+    return launch_dg_nt<STAGE, 64, 64>(p, st);
 }
 
 // A stage over its whole table; on the fly, F2 and I1 generate theirs chunk by chunk in `scratch`.
@@ -1621,20 +1830,19 @@ static int dg_fields(int mode) { return mode == kReal ? 1 : 2; }
 static int dg_mode(const void* imag, int fmt) { return fmt == COMPLEX ? kCplx : (imag ? kReal2 : kReal); }
 
 // Functions transformed at a time.
-static int dg_chunk(int bw, int batch) {
-    const int64_t per = 2 * 8 * 4 * (int64_t)bw * bw;
+static int dg_chunk(int bw, int batch, int es) {
+    const int64_t per = 2 * es * 4 * (int64_t)bw * bw;
     return (int)std::min<int64_t>(batch, std::min<int64_t>(16384, std::max<int64_t>(64, ((int64_t)256 << 20) / per)));
 }
 
 struct DgWork {
-    void* X;
-    long long* Z;
+    void *X, *Z;
     uint32_t *ej, *ef, *ex;
-    double *mid, *cr, *ci;
+    void *mid, *cr, *ci;
     size_t bytes;
 };
-static DgWork dg_work(char* w, int bw, int n, bool two) {
-    const size_t ff = (size_t)n * (two ? 2 : 1), S = 2 * (size_t)bw, BP = bw + (bw & 1);
+static DgWork dg_work(char* w, int bw, int n, bool two, int es) {
+    const size_t ff = (size_t)n * (two ? 2 : 1), S = 2 * (size_t)bw, BP = (bw + 3) & ~3;
     const size_t len = std::max(dg_fold_layout(bw, false).len, dg_fold_layout(bw, true).len);
     size_t at = 0;
     auto take = [&](size_t bytes) {
@@ -1643,14 +1851,14 @@ static DgWork dg_work(char* w, int bw, int n, bool two) {
         return (void*)q;
     };
     DgWork k{};
-    k.X = take(ff * 2 * bw * 2 * BP * 8);
-    k.Z = (long long*)take(ff * S * len * 8);
+    k.X = take(ff * 2 * bw * 2 * BP * es);
+    k.Z = take(ff * S * len * es);
     k.ej = (uint32_t*)take(ff * bw * 4);
     k.ef = (uint32_t*)take(ff * 4);
     k.ex = (uint32_t*)take(ff * 2 * bw * 4);
-    k.mid = (double*)take(ff * S * 8);
-    k.cr = (double*)take(two ? ff * bw * bw * 8 : 0);
-    k.ci = (double*)take(two ? ff * bw * bw * 8 : 0);
+    k.mid = take(ff * S * es);
+    k.cr = take(two ? ff * bw * bw * es : 0);
+    k.ci = take(two ? ff * bw * bw * es : 0);
     k.bytes = at;
     return k;
 }
@@ -1660,10 +1868,15 @@ size_t dg_fly_bytes(const Tables* t, int batch, bool two) {
     size_t need = 0;
     for (int s = kF2; s <= kI1; ++s)
         need = std::max(need, d->tmp_bytes[s] + d->tab_bytes[s] + 2 * (size_t)d->t[s].rows + 4096 + 1024);
-    return dg_work(nullptr, t->bw, dg_chunk(t->bw, batch), two).bytes + need;
+    return dg_work(nullptr, t->bw, dg_chunk(t->bw, batch, 8), two, 8).bytes + need;
 }
 
-size_t dg_work_bytes(int bw, int batch, bool two) { return dg_work(nullptr, bw, dg_chunk(bw, batch), two).bytes; }
+size_t dg_work_bytes(int bw, int batch, bool two) {
+    return dg_work(nullptr, bw, dg_chunk(bw, batch, 8), two, 8).bytes;
+}
+size_t dg32_work_bytes(int bw, int batch, bool two) {
+    return dg_work(nullptr, bw, dg_chunk(bw, batch, 4), two, 4).bytes;
+}
 
 // Bandwidths of the digit path: up to 1024 (its Legendre tables take 14 bw^3 bytes: 15 GB there).  Below 32
 // its five or six launches cost more than the FP64 kernels' two where those have a radix-2 FFT (one
@@ -1671,91 +1884,106 @@ size_t dg_work_bytes(int bw, int batch, bool two) { return dg_work(nullptr, bw, 
 // 34 us against 87 and 87).
 bool dg_takes(int bw) { return bw <= 1024 && (bw >= 32 || (bw > 8 && (bw & (bw - 1)))); }
 
-// Builds (or finds) the digit tables of t's bandwidth.  Where the stream is being captured, or they do
-// not fit in device memory, t stays without them and the FP64 kernels run.
 bool dg_fly_takes(int bw, int fields) { return dg_takes(bw) && bw >= 64 && fields >= (bw > 512 ? 4 : 2); }
 
-int dg_prepare(Tables* t, cudaStream_t st) {
-    if (!dg_takes(t->bw) || __atomic_load_n(&t->dg, __ATOMIC_ACQUIRE) || t->dg_off) return S2G_OK;
+// Builds (or finds) the digit tables of t's bandwidth.  Where the stream is being captured, or they do
+// not fit in device memory, t stays without them and the FP64 kernels run.
+static int prepare(Tables* t, int prec, void** slot, bool* off, cudaStream_t st) {
+    if (__atomic_load_n(slot, __ATOMIC_ACQUIRE) || *off) return S2G_OK;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
         cudaGetLastError();
         return S2G_OK;
     }
     DgTabs* d;
-    const int r = dg_get(t->bw, t->cutoff == 0, t->weights, &d);
+    const int r = dg_get(t->bw, prec, t->cutoff == 0, t->weights, &d);
     if (r == S2G_ERR_NOMEM) {
         cudaGetLastError();
-        t->dg_off = true;
+        *off = true;
         return S2G_OK;
     }
     if (r != S2G_OK) return r;
     void* none = nullptr;
-    if (!__atomic_compare_exchange_n(&t->dg, &none, (void*)d, false, __ATOMIC_ACQ_REL, __ATOMIC_ACQUIRE)) dg_put(d);
+    if (!__atomic_compare_exchange_n(slot, &none, (void*)d, false, __ATOMIC_ACQ_REL, __ATOMIC_ACQUIRE)) dg_put(d);
     return S2G_OK;
 }
+int dg_prepare(Tables* t, cudaStream_t st) { return dg_takes(t->bw) ? prepare(t, 64, &t->dg, &t->dg_off, st) : S2G_OK; }
+// Bandwidths whose FP32 transforms take the digit path: chirp-z ones, where its matrix products beat the two
+// FFTs of each chirp-z stage (forward 1.1 to 1.6 times as fast over bw 65 .. 255 and batches of 1 to 1024,
+// inverse 1.1 to 1.8; bw 255, 256 functions: 798 us against 880 and 703 against 912).  Below 64 they do not for large batches (bw 33, 4096 functions: 498 us against
+// 452), nor where a warp FFT takes the length (bw 256, 64 functions: 187 us against 96).
+bool dg32_takes(int bw) { return bw >= 64 && split_czt(bw); }
+int dg32_prepare(Tables* t, cudaStream_t st) { return prepare(t, 32, &t->dg32, &t->dg32_off, st); }
 
 static int set_dyn_smem(const void* fn, size_t bytes) {
     S2G_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     return S2G_OK;
 }
 
-int fst_f64_dg(const Tables* t, const double* rdata, const double* idata, double* rc, double* ic, int batch, int fmt,
-               void* work, cudaStream_t st) {
-    const DgTabs* d = (const DgTabs*)t->dg;
-    const int B = t->bw, S = 2 * B, mode = dg_mode(idata, fmt), chunk = dg_chunk(B, batch);
+template <int P>
+static int dg_fst(const DgTabs* d, const double* weights, const typename Dg<P>::Real* rdata,
+                  const typename Dg<P>::Real* idata, typename Dg<P>::Real* rc, typename Dg<P>::Real* ic, int batch, int fmt,
+                  void* work, cudaStream_t st, const int64_t* gmap = nullptr, const int64_t* cmap = nullptr) {
+    using Real = typename Dg<P>::Real;
+    const int B = d->bw, S = 2 * B, mode = dg_mode(idata, fmt), chunk = dg_chunk(B, batch, sizeof(Real));
     const DgFold fl = dg_fold_layout(B, false);
-    const DgWork w = dg_work((char*)work, B, chunk, mode != kReal);
+    const DgWork w = dg_work((char*)work, B, chunk, mode != kReal, sizeof(Real));
     char* scratch = (char*)work + w.bytes;  // on the fly: tables
-    S2G_TRY(set_dyn_smem((const void*)k_dg_fold, 2 * (size_t)S * 8));
+    S2G_TRY(set_dyn_smem((const void*)k_dg_fold<P>, 2 * (size_t)S * sizeof(Real)));
     for (int f0 = 0; f0 < batch; f0 += chunk) {
         const int n = std::min(chunk, batch - f0), ff = n * dg_fields(mode);
-        const size_t g0 = (size_t)f0 * S * S, c0 = (size_t)f0 * B * B;
+        const size_t g0 = gmap ? 0 : (size_t)f0 * S * S, c0 = cmap ? 0 : (size_t)f0 * B * B;
+        const int64_t *gm = gmap ? gmap + f0 : nullptr, *cm = cmap ? cmap + f0 : nullptr;
         S2G_CUDA(cudaMemsetAsync(w.ef, 0, (size_t)((char*)(w.ex + (size_t)ff * 2 * B) - (char*)w.ef), st));
         DgArgs p{};
         p.B = B;
         p.S = S;
         p.N = n;
         p.mode = mode;
-        p.BP = B + (B & 1);
+        p.cmap = cm;
+        p.BP = (B + 3) & ~3;
         p.RL = fl.len;
-        p.vbz = dg_vbz(B);
+        p.vbz = dg_vbz(B, P);
         p.tbz = d->t[kF1].h[0].tb;
         p.X = w.X;
         p.Z = w.Z;
         {
-            ProfScope ps_("dg_fold", st);
-            k_dg_fold<<<dim3(B, ff), 128, 2 * (size_t)S * 8, st>>>(rdata + g0, idata ? idata + g0 : nullptr, B, n, p.vbz, fl,
-                                                                 w.Z, w.ej, w.ef);
+            ProfScope ps_(P == 32 ? "dg_fold_f32" : "dg_fold", st);
+            k_dg_fold<P><<<dim3(B, ff), 128, 2 * (size_t)S * sizeof(Real), st>>>(
+                rdata + g0, idata ? idata + g0 : nullptr, B, n, p.vbz, fl, gm, (typename Dg<P>::Int*)w.Z, w.ej, w.ef);
         }
         S2G_CUDA(cudaGetLastError());
         p.ncols = ff * S;
         p.ein = w.ej;
         p.efield = w.ef;
         p.emax = w.ex;
-        S2G_TRY(launch_dg<kF1>(d, p, t->weights, scratch, st));
+        S2G_TRY(launch_dg<kF1>(d, p, weights, scratch, st));
         p.ncols = ff * 2;
         p.out_r = rc + c0;
         p.out_i = ic + c0;
-        S2G_TRY(launch_dg<kF2>(d, p, t->weights, scratch, st));
+        S2G_TRY(launch_dg<kF2>(d, p, weights, scratch, st));
     }
     return S2G_OK;
 }
 
-int inv_fst_f64_dg(const Tables* t, const double* rc, const double* ic, double* rdata, double* idata, int batch,
-                   int fmt, void* work, cudaStream_t st) {
-    const DgTabs* d = (const DgTabs*)t->dg;
-    const int B = t->bw, S = 2 * B, mode = dg_mode(idata, fmt), chunk = dg_chunk(B, batch);
+template <int P>
+static int dg_inv_fst(const DgTabs* d, const double* weights, const typename Dg<P>::Real* rc,
+                      const typename Dg<P>::Real* ic, typename Dg<P>::Real* rdata, typename Dg<P>::Real* idata, int batch,
+                      int fmt, void* work, cudaStream_t st, const int64_t* gmap = nullptr,
+                      const int64_t* cmap = nullptr) {
+    using Real = typename Dg<P>::Real;
+    const int B = d->bw, S = 2 * B, mode = dg_mode(idata, fmt), chunk = dg_chunk(B, batch, sizeof(Real));
     const DgFold fl = dg_fold_layout(B, true);
-    const DgWork w = dg_work((char*)work, B, chunk, mode != kReal);
+    const DgWork w = dg_work((char*)work, B, chunk, mode != kReal, sizeof(Real));
     char* scratch = (char*)work + w.bytes;  // on the fly: tables
     for (int f0 = 0; f0 < batch; f0 += chunk) {
         const int n = std::min(chunk, batch - f0), ff = n * dg_fields(mode);
-        const size_t g0 = (size_t)f0 * S * S, c0 = (size_t)f0 * B * B;
+        const size_t g0 = gmap ? 0 : (size_t)f0 * S * S, c0 = cmap ? 0 : (size_t)f0 * B * B;
+        const int64_t *gm = gmap ? gmap + f0 : nullptr, *cm = cmap ? cmap + f0 : nullptr;
         S2G_CUDA(cudaMemsetAsync(w.ef, 0, (size_t)ff * 4, st));
         {
-            ProfScope ps_("dg_coefmax", st);
-            k_dg_coefmax<<<(n * B + 7) / 8, 256, 0, st>>>(rc + c0, ic + c0, B, n, mode, w.cr, w.ci, w.ex);
+            ProfScope ps_(P == 32 ? "dg_coefmax_f32" : "dg_coefmax", st);
+            k_dg_coefmax<Real><<<(n * B + 7) / 8, 256, 0, st>>>(rc + c0, ic + c0, B, n, mode, cm, (Real*)w.cr, (Real*)w.ci, w.ex);
         }
         S2G_CUDA(cudaGetLastError());
         DgArgs p{};
@@ -1763,42 +1991,64 @@ int inv_fst_f64_dg(const Tables* t, const double* rc, const double* ic, double* 
         p.S = S;
         p.N = n;
         p.mode = mode;
-        p.BP = B + (B & 1);
+        p.cmap = cm;
+        p.BP = (B + 3) & ~3;
         p.RL = fl.len;
         p.X = w.X;
         p.Z = w.Z;
         p.ncols = ff * 2;
-        p.in_r = mode == kReal ? rc + c0 : w.cr;
-        p.in_i = mode == kReal ? ic + c0 : w.ci;
+        p.in_r = mode == kReal ? (const void*)(rc + c0) : w.cr;
+        p.in_i = mode == kReal ? (const void*)(ic + c0) : w.ci;
         p.ein = w.ex;
         p.emax = w.ef;
-        S2G_TRY(launch_dg<kI1>(d, p, t->weights, scratch, st));
+        S2G_TRY(launch_dg<kI1>(d, p, weights, scratch, st));
         p.ncols = ff * S;
         p.ein = w.ef;
-        S2G_TRY(launch_dg<kI2>(d, p, t->weights, scratch, st));
-        if (B % 2 == 0) {
-            ProfScope ps_("dg_mid", st);
-            k_dg_mid<<<(ff * S + 31) / 32, dim3(32, 8), 0, st>>>((const double*)w.X, B, ff * S, w.mid);
+        S2G_TRY(launch_dg<kI2>(d, p, weights, scratch, st));
+        if (fl.n[0]) {
+            ProfScope ps_(P == 32 ? "dg_mid_f32" : "dg_mid", st);
+            k_dg_mid<Real><<<(ff * S + 31) / 32, dim3(32, 8), 0, st>>>((const Real*)w.X, B, ff * S, (Real*)w.mid);
             S2G_CUDA(cudaGetLastError());
         }
         {
-            ProfScope ps_("dg_unfold", st);
-            k_dg_unfold<<<dim3(B, ff), 128, 0, st>>>(w.Z, w.mid, w.ef, B, n, d->t[kI2].h[0].vb + d->t[kI2].h[0].tb, fl,
-                                                    rdata + g0,
-                                                    idata ? idata + g0 : nullptr);
+            ProfScope ps_(P == 32 ? "dg_unfold_f32" : "dg_unfold", st);
+            k_dg_unfold<P><<<dim3(B, ff), 128, 0, st>>>(w.Z, (const Real*)w.mid, w.ef, B, n,
+                                                        d->t[kI2].h[0].vb + d->t[kI2].h[0].tb, fl, gm, rdata + g0,
+                                                        idata ? idata + g0 : nullptr);
         }
         S2G_CUDA(cudaGetLastError());
     }
     return S2G_OK;
 }
 
+int fst_f64_dg(const Tables* t, const double* rdata, const double* idata, double* rc, double* ic, int batch, int fmt,
+               void* work, cudaStream_t st) {
+    return dg_fst<64>((const DgTabs*)t->dg, t->weights, rdata, idata, rc, ic, batch, fmt, work, st);
+}
+int inv_fst_f64_dg(const Tables* t, const double* rc, const double* ic, double* rdata, double* idata, int batch, int fmt,
+                   void* work, cudaStream_t st) {
+    return dg_inv_fst<64>((const DgTabs*)t->dg, t->weights, rc, ic, rdata, idata, batch, fmt, work, st);
+}
+int fst_dg32(const Tables* t, const float* rgrid, const float* igrid, float* rc, float* ic, int batch, void* work,
+             cudaStream_t st, const int64_t* gmap, const int64_t* cmap) {
+    return dg_fst<32>((const DgTabs*)t->dg32, t->weights, rgrid, igrid, rc, ic, batch, igrid ? COMPLEX : REAL, work, st,
+                      gmap, cmap);
+}
+int inv_fst_dg32(const Tables* t, const float* rc, const float* ic, float* rgrid, float* igrid, int batch, void* work,
+                 cudaStream_t st, const int64_t* gmap, const int64_t* cmap) {
+    return dg_inv_fst<32>((const DgTabs*)t->dg32, t->weights, rc, ic, rgrid, igrid, batch, igrid ? COMPLEX : REAL, work, st,
+                          gmap, cmap);
+}
+
 int dg_status(const Tables* t, int clear) {
-    const DgTabs* d = (const DgTabs*)t->dg;
-    if (!d) return S2G_OK;
-    int v = 0;
-    S2G_CUDA(cudaMemcpy(&v, d->err, sizeof(int), cudaMemcpyDeviceToHost));
-    if (clear && v) S2G_CUDA(cudaMemset(d->err, 0, sizeof(int)));
-    if (v) return fail(v, "a bounded wait in the digit-product kernel expired");
+    for (const void* h : {t->dg, t->dg32}) {
+        const DgTabs* d = (const DgTabs*)h;
+        if (!d) continue;
+        int v = 0;
+        S2G_CUDA(cudaMemcpy(&v, d->err, sizeof(int), cudaMemcpyDeviceToHost));
+        if (clear && v) S2G_CUDA(cudaMemset(d->err, 0, sizeof(int)));
+        if (v) return fail(v, "a bounded wait in the digit-product kernel expired");
+    }
     return S2G_OK;
 }
 

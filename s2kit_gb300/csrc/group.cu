@@ -14,8 +14,8 @@
 // (bw <= 64), compiled for the per-length kernels' small register budgets, and the long ones
 // (bw >= 128).  The two tiers run concurrently on two streams, so those classes take at most two
 // launches per stage whatever their number.  A class of another bandwidth (transform length 32 R
-// with R not a power of two, or a chirp-z length) runs each stage as its own launch on the
-// long tier's stream.  The sequence is captured once as a CUDA graph (on an internal stream, the tiers as
+// with R not a power of two, or a chirp-z length below bw 64) runs each stage as its own launch on the
+// long tier's stream; the chirp-z classes from 64 on take the digit path (digit_gemm.cu) instead.  The sequence is captured once as a CUDA graph (on an internal stream, the tiers as
 // parallel branches) and replayed on the caller's stream; the first call with a given set of
 // pointers runs eagerly and captures, later calls replay.
 //
@@ -51,6 +51,7 @@ struct GroupClass {
     int64_t* cmap = nullptr;    // device: member i -> coefficient offset
     float* buf0 = nullptr;      // X (forward) / F (inverse): [2][N][B][SX]  (split_layout)
     float* buf1 = nullptr;      // C (forward) / Fc (inverse): [2][N][B][2 BH]
+    void* digits = nullptr;     // scratch of the digit path (digit_gemm.cu), for the classes that take it
 };
 
 struct GroupGraph {
@@ -112,7 +113,7 @@ static int group_stages(s2g_group g, const int* which, int nstage, In in, Out ou
         // the other classes: one launch each, in stage order on st
         for (int c = 0; c < nc; ++c) {
             GroupClass& k = g->cls[c];
-            if (stage_groupable(k.B)) continue;
+            if (stage_groupable(k.B) || k.digits) continue;
             S2G_TRY(split_stage_one(which[w], k.t, k.N, in(w, c), out(w, c), k.gmap, st));
         }
     }
@@ -125,14 +126,18 @@ static int group_stages(s2g_group g, const int* which, int nstage, In in, Out ou
 
 static int group_fwd_seq(s2g_group g, const float* grid, float* rc, float* ic, cudaStream_t st) {
     const int nc = (int)g->cls.size();
+    for (auto& k : g->cls)
+        if (k.digits) S2G_TRY(fst_dg32(k.t, grid, nullptr, rc, ic, k.N, k.digits, st, k.gmap, k.cmap));
     const int which[2] = {0, 1};  // grid -> X -> C
     S2G_TRY(group_stages(
         g, which, 2, [&](int w, int c) -> const void* { return w == 0 ? (const void*)grid : g->cls[c].buf0; },
         [&](int w, int c) -> void* { return w == 0 ? g->cls[c].buf0 : g->cls[c].buf1; }, st));
     LegSpec spec[kGroupMaxClasses] = {};
+    int ns = 0;
     for (int c = 0; c < nc; ++c) {
         GroupClass& k = g->cls[c];
-        LegSpec& q = spec[c];
+        if (k.digits) continue;
+        LegSpec& q = spec[ns++];
         q.t = k.t;
         q.N = k.N;
         q.NB = k.NB;
@@ -142,15 +147,20 @@ static int group_fwd_seq(s2g_group g, const float* grid, float* rc, float* ic, c
         q.ic = ic;
         q.cmap = k.cmap;
     }
-    return split_leg(true, g->precision, spec, nc, g->counters, g->table_stages, st);
+    return ns ? split_leg(true, g->precision, spec, ns, g->counters, g->table_stages, st) : S2G_OK;
 }
 
 static int group_inv_seq(s2g_group g, const float* rc, const float* ic, float* grid, cudaStream_t st) {
     const int nc = (int)g->cls.size();
     LegSpec spec[kGroupMaxClasses] = {};
+    int ns = 0;
     for (int c = 0; c < nc; ++c) {
         GroupClass& k = g->cls[c];
-        LegSpec& q = spec[c];
+        if (k.digits) {
+            S2G_TRY(inv_fst_dg32(k.t, rc, ic, grid, nullptr, k.N, k.digits, st, k.gmap, k.cmap));
+            continue;
+        }
+        LegSpec& q = spec[ns++];
         q.t = k.t;
         q.N = k.N;
         q.NB = k.NB;
@@ -160,7 +170,7 @@ static int group_inv_seq(s2g_group g, const float* rc, const float* ic, float* g
         q.F = k.buf0;
         q.cmap = k.cmap;
     }
-    S2G_TRY(split_leg(false, g->precision, spec, nc, g->counters + 1, g->table_stages, st));
+    if (ns) S2G_TRY(split_leg(false, g->precision, spec, ns, g->counters + 1, g->table_stages, st));
     const int which[2] = {2, 3};  // Fc -> F -> grid
     return group_stages(
         g, which, 2, [&](int w, int c) -> const void* { return w == 0 ? g->cls[c].buf1 : g->cls[c].buf0; },
@@ -468,7 +478,9 @@ int s2g_group_create(s2g_group* out, int nfunc, const int* bw, int precision) {
     for (auto& c : g->cls) {
         if (r == S2G_OK) r = get_tables(c.B, c.B, &c.t);
         else c.t = nullptr;
+        if (r == S2G_OK && dg32_takes(c.B)) r = dg32_prepare(c.t, 0);
     }
+    auto digits = [](const GroupClass& c) { return dg32_takes(c.B) && c.t && c.t->dg32; };
     // device memory: maps, intermediates (256-byte aligned pieces), two counters
     auto rnd = [](size_t x) { return (x + 255) & ~(size_t)255; };
     size_t total = 256;
@@ -476,7 +488,8 @@ int s2g_group_create(s2g_group* out, int nfunc, const int* bw, int precision) {
     auto c_floats = [](const GroupClass& c) { return 2 * (size_t)c.N * c.B * 2 * split_layout(c.B).BH; };
     for (auto& c : g->cls) {
         total += 2 * rnd(sizeof(int64_t) * c.N);
-        total += rnd(sizeof(float) * x_floats(c)) + rnd(sizeof(float) * c_floats(c));
+        total += digits(c) ? rnd(dg32_work_bytes(c.B, c.N, false))
+                           : rnd(sizeof(float) * x_floats(c)) + rnd(sizeof(float) * c_floats(c));
     }
     if (r == S2G_OK && cudaMalloc(&g->mem, total) != cudaSuccess)
         r = fail(S2G_ERR_NOMEM, "group: cudaMalloc of %zu bytes failed", total);
@@ -490,10 +503,15 @@ int s2g_group_create(s2g_group* out, int nfunc, const int* bw, int precision) {
             p += rnd(sizeof(int64_t) * c.N);
             c.cmap = (int64_t*)p;
             p += rnd(sizeof(int64_t) * c.N);
-            c.buf0 = (float*)p;
-            p += rnd(sizeof(float) * x_floats(c));
-            c.buf1 = (float*)p;
-            p += rnd(sizeof(float) * c_floats(c));
+            if (digits(c)) {
+                c.digits = p;
+                p += rnd(dg32_work_bytes(c.B, c.N, false));
+            } else {
+                c.buf0 = (float*)p;
+                p += rnd(sizeof(float) * x_floats(c));
+                c.buf1 = (float*)p;
+                p += rnd(sizeof(float) * c_floats(c));
+            }
             gm.clear();
             cm.clear();
             for (int f : c.funcs) gm.push_back(g->goff[f]), cm.push_back(g->coff[f]);
@@ -622,8 +640,8 @@ int s2g_group_sync_status(s2g_group g) {
     S2G_CUDA(cudaDeviceSynchronize());
     int r = S2G_OK;
     for (auto& c : g->cls) {
-        const int v = split_device_status(c.t, 1);
-        if (v != S2G_OK && r == S2G_OK) r = v;
+        const int v = split_device_status(c.t, 1), d = dg_status(c.t, 1);
+        if (r == S2G_OK) r = v != S2G_OK ? v : d;
     }
     return r;
 }

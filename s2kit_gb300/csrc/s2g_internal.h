@@ -62,6 +62,8 @@ struct Tables {
     // digit tables of the tensor-core FP64 path (digit_gemm.cu), built on first use
     void* dg = nullptr;
     bool dg_off = false;        // they did not fit in device memory
+    void* dg32 = nullptr;       // the same for FP32 transforms
+    bool dg32_off = false;
     int refs = 0;               // references (cache, plans, groups, calls in flight); under the cache lock
 };
 
@@ -115,6 +117,15 @@ size_t f64_plan_bytes(int bw, int batch, int data_format, bool two);
 // ---- FP64 transforms as exact digit products on the tensor cores (digit_gemm.cu) ----
 bool dg_takes(int bw);
 size_t dg_work_bytes(int bw, int batch, bool two);
+// FP32 samples and coefficients (igrid null: real fields); readied by dg32_prepare into t->dg32.
+// gmap, cmap: per-function grid and coefficient offsets (real fields), null for functions back to back.
+bool dg32_takes(int bw);
+size_t dg32_work_bytes(int bw, int batch, bool two);
+int dg32_prepare(Tables* t, cudaStream_t st);
+int fst_dg32(const Tables* t, const float* rgrid, const float* igrid, float* rc, float* ic, int batch, void* work,
+             cudaStream_t st, const int64_t* gmap = nullptr, const int64_t* cmap = nullptr);
+int inv_fst_dg32(const Tables* t, const float* rc, const float* ic, float* rgrid, float* igrid, int batch, void* work,
+                 cudaStream_t st, const int64_t* gmap = nullptr, const int64_t* cmap = nullptr);
 // On-the-fly family (tables of cutoff 0): real fields for which it pays, and the scratch once prepared.
 bool dg_fly_takes(int bw, int fields);
 size_t dg_fly_bytes(const Tables* t, int batch, bool two);
@@ -197,6 +208,7 @@ int czt_build_tables(int bw, float2** d_h, float2** d_K, float2** d_tw);
 int czt_stage(int which, const CztTabs& g, const void* in, void* out, int N, float scale, const int64_t* gmap,
               cudaStream_t st);
 size_t split_work_bytes(int bw, int batch);
+size_t split_complex_work_bytes(int bw, int batch);
 int fst_split(Tables* t, const float* grid, float* rc, float* ic, int batch, int precision, void* work,
               cudaStream_t st);
 int inv_fst_split(Tables* t, const float* rc, const float* ic, float* grid, int batch, int precision, void* work,

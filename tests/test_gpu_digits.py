@@ -132,3 +132,53 @@ def test_digit_path_under_capture():
     torch.cuda.synchronize()
     plan.sync_status()
     assert (rc == 2 * want[0]).all() and (ic == 2 * want[1]).all()
+
+
+def _run32(bw, nb, rc, ic, gr, gi):
+    """FP32 inverse of (rc, ic) and forward of (gr, gi) at a chirp-z bandwidth (gi None: real fields)."""
+    import torch
+
+    def dev(x):
+        return torch.from_numpy(np.ascontiguousarray(x, dtype=np.float32)).cuda().reshape(-1)
+
+    plan = api.Plan(bw, bw)
+    og = [dev(np.full((nb, 4 * bw * bw), 7.0)) for _ in range(2)]
+    oc = [dev(np.full((nb, bw * bw), 7.0)) for _ in range(2)]
+    if gi is None:
+        plan.inv_fst_real_f32(dev(rc), dev(ic), og[0], nb)
+        plan.fst_real_f32(dev(gr), oc[0], oc[1], nb)
+    else:
+        plan.inv_fst_complex_f32(dev(rc), dev(ic), og[0], og[1], nb)
+        plan.fst_complex_f32(dev(gr), dev(gi), oc[0], oc[1], nb)
+    torch.cuda.synchronize()
+    plan.sync_status()
+    return [x.cpu().numpy().astype(np.float64).reshape(nb, -1) for x in og + oc]
+
+
+# FP32 samples and coefficients: inputs and results round at 2^-24 = 6e-8; the table's 25 and the data's 30 bits
+# of a row's largest value, and one more rounding between the stages, leave a few times that: 5e-7.
+@pytest.mark.parametrize("bw,nb,cplx", [(65, 9, False), (65, 2, True), (66, 33, False), (77, 1, False), (100, 17, True),
+                                        (127, 3, False), (130, 70, False), (250, 2, True), (254, 5, False),
+                                        (255, 1, True), (255, 33, False)])
+def test_fp32_digit_path_matches_oracle(oracle, bw, nb, cplx):
+    rc, ic, gr, gi = (x.astype(np.float32).astype(np.float64) for x in _data(bw, nb, "complex" if cplx else "real"))
+    igr, igi, orc, oic = _run32(bw, nb, rc, ic, gr, gi if cplx else None)
+    fmt = api.COMPLEX if cplx else api.REAL
+    for f in {0, nb // 2, nb - 1}:
+        er, ei = oracle.inv_fst(rc[f], ic[f], bw, fmt, bw)
+        assert rel_err_norm(igr[f], igi[f] if cplx else 0.0, er, ei if cplx else 0.0) <= 5e-7
+        er, ei = oracle.fst(gr[f], gi[f], bw, fmt, 1)
+        assert rel_err_norm(orc[f], oic[f], er, ei) <= 5e-7
+
+
+def test_fp32_digit_path_scales_and_nan_stay_with_their_function():
+    bw, nb = 90, 9
+    rc, ic, gr, gi = _data(bw, nb, "real")
+    want = _run32(bw, nb, rc, ic, gr, None)
+    gr[3] *= 2.0 ** 60  # exact, and so are its results
+    rc[4, 7], gr[5, 11] = np.nan, np.inf
+    got = _run32(bw, nb, rc, ic, gr, None)
+    for w, g, bad in zip(want[:1] + want[2:], got[:1] + got[2:], (4, 5, 5)):
+        assert not np.isfinite(g[bad]).any()
+        for f in set(range(nb)) - {bad}:
+            assert (g[f] == w[f] * (2.0 ** 60 if bad == 5 and f == 3 else 1.0)).all()
