@@ -1761,15 +1761,12 @@ static int dg_get(int bw, int prec, bool fly, const double* weights, DgTabs** ou
 }
 
 template <int STAGE, int NT, int P>
-static int launch_dg_nt(const DgArgs& p, cudaStream_t st) {
+static int launch_dg_nt(const DgArgs& p, int sms, cudaStream_t st) {
     static const char* names[8] = {"dg_rows_fwd", "dg_leg_fwd", "dg_leg_inv", "dg_rows_inv",
                                    "dg_rows_fwd_f32", "dg_leg_fwd_f32", "dg_leg_inv_f32", "dg_rows_inv_f32"};
     const size_t smem = 1024 + Dg<P>::stagesA * kDgABytes<P> + kDgBRing +
                         (P == 32 && STAGE == kF1 ? Dg<P>::epilogue * kDgStash : 0);
     S2G_CUDA(cudaFuncSetAttribute((const void*)k_dg<STAGE, NT, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int dev = 0, sms = 0;
-    S2G_CUDA(cudaGetDevice(&dev));
-    S2G_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const int64_t items = (int64_t)p.ntiles * p.ncolblk;
     {
         ProfScope ps_(names[STAGE + (P == 32 ? 4 : 0)], st);
@@ -1779,28 +1776,47 @@ static int launch_dg_nt(const DgArgs& p, cudaStream_t st) {
     return S2G_OK;
 }
 
-// 64 columns per item: an accumulator of 7 x 64 TMEM columns, each table digit read once per 64 columns;
-// fewer columns in all take 32 or 16 (two accumulators, so that the epilogue of one item runs beside the
-// MMAs of the next).  Items of F1 and I2 go column by column (their four tables, 1 MB at bw 256, stay in
-// L2), those of F2 and I1 table by table (117 MB each at bw 256).
-// At bw 256, 64 functions: F1 164 us, F2 119, I1 133, I2 118, k_dg_fold 67, k_dg_unfold 53, k_dg_mid 17;
-// forward and inverse together 0.68 ms against 4.59 ms on the FP64 units (DFMA-bound there).  The tensor
-// pipe alone would take 47 us for each of the four; MMA issue and the part of the epilogue that the next
-// item's MMAs wait for (dg_sum, the stores) make up the rest.
+// Columns per item.  While one wave of blocks holds them all, more and smaller items are faster (bw 64, one
+// function: F1 16.4 us at 64 columns, 11.2 at 16).  Beyond one wave, FP64: 64 columns take one accumulator (7 x 64 TMEM columns) whose epilogue the next
+// item's MMAs wait for (F1 at bw 256: 44% of the time), 32 take two by turns, but seven dependent MMAs of
+// about 115 cycles for each 16-deep K step where 64 take ten for twice the columns.  So 64 is for the long K
+// ranges: I1 (K = the degrees of a parity) never, F2 (K = bw) above bw 256 (bw 256, 256 functions: 478 us at
+// 64, 463 at 32; bw 512, 64 functions: 519 and 601), F1 above 300 (bw 256, 64 functions: 165 and 156; bw 512:
+// 897 and 998), I2 (whose epilogue is the shortest) above 112 orders (bw 192, 64 functions: 97 and 79; bw 256:
+// 118 and 126).  FP32 (G = 4) has two accumulators at 64 columns.
+// Items of F1 and I2 go column by column (their tables, 1 MB at bw 256, stay in L2), those of F2 and I1 table
+// by table (117 MB each at bw 256).
+// At bw 256, 64 functions: F1 156 us, F2 116, I1 123, I2 118, k_dg_fold 67, k_dg_unfold 53, k_dg_mid 17;
+// forward and inverse together 0.66 ms against 4.59 ms on the FP64 units (DFMA-bound there).  The tensor
+// pipe alone would take 47 us for each of the four; MMA issue and the waits around it make up the rest.
+template <int STAGE>
+static int dg_columns(const DgTabs* d, const DgArgs& p, int sms) {
+    auto items = [&](int n) { return (int64_t)p.ntiles * ((p.ncols + n - 1) / n); };
+    for (int n : {16, 32, 64})
+        if (p.ncols <= n || items(n) <= sms) return n;
+    if (d->prec == 32) return 64;
+    if (STAGE == kI1) return 32;
+    if (STAGE == kF2) return d->bw <= 256 ? 32 : 64;
+    if (STAGE == kF1) return d->bw <= 300 ? 32 : 64;
+    return d->t[kI2].h[0].ks <= 7 ? 32 : 64;
+}
 template <int STAGE>
 static int launch_dg_tiles(const DgTabs* d, DgArgs p, cudaStream_t st) {
     p.col_major = STAGE == kF1 || STAGE == kI2;
     p.err = d->err;
-    const int per = p.ncols <= 16 ? 16 : (p.ncols <= 32 ? 32 : 64);
+    int dev = 0, sms = 0;
+    S2G_CUDA(cudaGetDevice(&dev));
+    S2G_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int per = dg_columns<STAGE>(d, p, sms);
     p.ncolblk = (p.ncols + per - 1) / per;
     if (d->prec == 32) {
-        if (per == 16) return launch_dg_nt<STAGE, 16, 32>(p, st);
-        if (per == 32) return launch_dg_nt<STAGE, 32, 32>(p, st);
-        return launch_dg_nt<STAGE, 64, 32>(p, st);
+        if (per == 16) return launch_dg_nt<STAGE, 16, 32>(p, sms, st);
+        if (per == 32) return launch_dg_nt<STAGE, 32, 32>(p, sms, st);
+        return launch_dg_nt<STAGE, 64, 32>(p, sms, st);
     }
-    if (per == 16) return launch_dg_nt<STAGE, 16, 64>(p, st);
-    if (per == 32) return launch_dg_nt<STAGE, 32, 64>(p, st);
-    return launch_dg_nt<STAGE, 64, 64>(p, st);
+    if (per == 16) return launch_dg_nt<STAGE, 16, 64>(p, sms, st);
+    if (per == 32) return launch_dg_nt<STAGE, 32, 64>(p, sms, st);
+    return launch_dg_nt<STAGE, 64, 64>(p, sms, st);
 }
 
 // A stage over its whole table; on the fly, F2 and I1 generate theirs chunk by chunk in `scratch`.
