@@ -15,7 +15,9 @@
 // (bw >= 128).  The two tiers run concurrently on two streams, so those classes take at most two
 // launches per stage whatever their number.  A class of another bandwidth (transform length 32 R
 // with R not a power of two, or a chirp-z length below bw 64) runs each stage as its own launch on the
-// long tier's stream; the chirp-z classes from 64 on take the digit path (digit_gemm.cu) instead.  The sequence is captured once as a CUDA graph (on an internal stream, the tiers as
+// long tier's stream; the chirp-z classes from 64 on take the digit path (digit_gemm.cu) instead.
+// Classes of bw <= 32 are transformed whole (small32.cuh): 16 and 32 by blocks of the short tier's rows
+// launch (k_stage_small), the others each by a launch of its own.  The sequence is captured once as a CUDA graph (on an internal stream, the tiers as
 // parallel branches) and replayed on the caller's stream; the first call with a given set of
 // pointers runs eagerly and captures, later calls replay.
 //
@@ -51,6 +53,7 @@ struct GroupClass {
     int64_t* cmap = nullptr;    // device: member i -> coefficient offset
     float* buf0 = nullptr;      // X (forward) / F (inverse): [2][N][B][SX]  (split_layout)
     float* buf1 = nullptr;      // C (forward) / Fc (inverse): [2][N][B][2 BH]
+    bool small = false;         // transformed whole in the rows stage (small_takes): no intermediates
     void* digits = nullptr;     // scratch of the digit path (digit_gemm.cu), for the classes that take it
 };
 
@@ -89,35 +92,40 @@ static constexpr int kShortTierMaxBw = 64;
 // FFT stage `which` of every class, from in(c) to out(c): the long tier on st, the short tier on the
 // side stream (forked from and joined back into st).
 template <typename In, typename Out>
-static int group_stages(s2g_group g, const int* which, int nstage, In in, Out out, cudaStream_t st) {
+static int group_stages(s2g_group g, const int* which, int nstage, In in, Out out, float* rc, float* ic,
+                        cudaStream_t st) {
     const int nc = (int)g->cls.size();
     StageSpec lo[kGroupMaxClasses], hi[kGroupMaxClasses];
     int nlo = 0, nhi = 0;
+    bool forked = false;
     for (int w = 0; w < nstage; ++w) {
         nlo = nhi = 0;
         for (int c = 0; c < nc; ++c) {
             GroupClass& k = g->cls[c];
             if (!stage_groupable(k.B)) continue;
             const bool rows = which[w] == 0 || which[w] == 3;
-            const StageSpec q{k.t, k.N, in(w, c), out(w, c), rows ? k.gmap : nullptr};
+            if (k.small && !rows) continue;
+            StageSpec q{k.t, k.N, in(w, c), out(w, c), rows ? k.gmap : nullptr};
+            if (k.small) q.rc = rc, q.ic = ic, q.cmap = k.cmap;
             if (k.B <= kShortTierMaxBw) lo[nlo++] = q;
             else hi[nhi++] = q;
         }
-        if (w == 0 && nlo && nhi) {
+        if (nlo && nhi && !forked) {
+            forked = true;
             S2G_CUDA(cudaEventRecord(g->fork, st));
             S2G_CUDA(cudaStreamWaitEvent(g->side, g->fork, 0));
         }
         const int dc = (which[w] == 1 || which[w] == 2) ? g->dct_ctas : 0;
         if (nhi) S2G_TRY(split_stage_group(which[w], hi, nhi, dc, st));
-        if (nlo) S2G_TRY(split_stage_group(which[w], lo, nlo, dc, nhi ? g->side : st));
+        if (nlo) S2G_TRY(split_stage_group(which[w], lo, nlo, dc, forked ? g->side : st));
         // the other classes: one launch each, in stage order on st
         for (int c = 0; c < nc; ++c) {
             GroupClass& k = g->cls[c];
-            if (stage_groupable(k.B) || k.digits) continue;
+            if (stage_groupable(k.B) || k.digits || k.small) continue;
             S2G_TRY(split_stage_one(which[w], k.t, k.N, in(w, c), out(w, c), k.gmap, st));
         }
     }
-    if (nlo && nhi) {
+    if (forked) {
         S2G_CUDA(cudaEventRecord(g->join, g->side));
         S2G_CUDA(cudaStreamWaitEvent(st, g->join, 0));
     }
@@ -128,15 +136,16 @@ static int group_fwd_seq(s2g_group g, const float* grid, float* rc, float* ic, c
     const int nc = (int)g->cls.size();
     for (auto& k : g->cls)
         if (k.digits) S2G_TRY(fst_dg32(k.t, grid, nullptr, rc, ic, k.N, k.digits, st, k.gmap, k.cmap));
+        else if (k.small && !stage_groupable(k.B)) S2G_TRY(fst_small(k.t, grid, rc, ic, k.N, st, k.gmap, k.cmap));
     const int which[2] = {0, 1};  // grid -> X -> C
     S2G_TRY(group_stages(
         g, which, 2, [&](int w, int c) -> const void* { return w == 0 ? (const void*)grid : g->cls[c].buf0; },
-        [&](int w, int c) -> void* { return w == 0 ? g->cls[c].buf0 : g->cls[c].buf1; }, st));
+        [&](int w, int c) -> void* { return w == 0 ? g->cls[c].buf0 : g->cls[c].buf1; }, rc, ic, st));
     LegSpec spec[kGroupMaxClasses] = {};
     int ns = 0;
     for (int c = 0; c < nc; ++c) {
         GroupClass& k = g->cls[c];
-        if (k.digits) continue;
+        if (k.digits || k.small) continue;
         LegSpec& q = spec[ns++];
         q.t = k.t;
         q.N = k.N;
@@ -160,6 +169,10 @@ static int group_inv_seq(s2g_group g, const float* rc, const float* ic, float* g
             S2G_TRY(inv_fst_dg32(k.t, rc, ic, grid, nullptr, k.N, k.digits, st, k.gmap, k.cmap));
             continue;
         }
+        if (k.small) {
+            if (!stage_groupable(k.B)) S2G_TRY(inv_fst_small(k.t, rc, ic, grid, k.N, st, k.gmap, k.cmap));
+            continue;
+        }
         LegSpec& q = spec[ns++];
         q.t = k.t;
         q.N = k.N;
@@ -174,7 +187,7 @@ static int group_inv_seq(s2g_group g, const float* rc, const float* ic, float* g
     const int which[2] = {2, 3};  // Fc -> F -> grid
     return group_stages(
         g, which, 2, [&](int w, int c) -> const void* { return w == 0 ? g->cls[c].buf1 : g->cls[c].buf0; },
-        [&](int w, int c) -> void* { return w == 0 ? (void*)g->cls[c].buf0 : (void*)grid; }, st);
+        [&](int w, int c) -> void* { return w == 0 ? (void*)g->cls[c].buf0 : (void*)grid; }, (float*)rc, (float*)ic, st);
 }
 
 static int group_seq(s2g_group g, int kind, const void* const* ptr, cudaStream_t st) {
@@ -479,6 +492,7 @@ int s2g_group_create(s2g_group* out, int nfunc, const int* bw, int precision) {
         if (r == S2G_OK) r = get_tables(c.B, c.B, &c.t);
         else c.t = nullptr;
         if (r == S2G_OK && dg32_takes(c.B)) r = dg32_prepare(c.t, 0);
+        c.small = small_takes(c.B);
     }
     auto digits = [](const GroupClass& c) { return dg32_takes(c.B) && c.t && c.t->dg32; };
     // device memory: maps, intermediates (256-byte aligned pieces), two counters

@@ -230,10 +230,19 @@ struct StageSpec {
     const void* in;
     void* out;
     const int64_t* gmap;
+    float *rc = nullptr, *ic = nullptr;  // rows stages, bw <= 32 (small_takes): the whole transform, to or from these
+    const int64_t* cmap = nullptr;       // (their coefficient offsets); out, in are then the grid or unused
 };
 int split_stage_group(int which, const StageSpec* spec, int ncls, int dct_ctas_per_sm, cudaStream_t st);
 // The same stage for one class of any split-path bandwidth, as its own launch.
 int split_stage_one(int which, Tables* t, int N, const void* in, void* out, const int64_t* gmap, cudaStream_t st);
+// Bandwidths transformed whole by one kernel (small32.cuh), and those transforms: real fields, functions back to
+// back or at the offsets gmap (samples) and cmap (coefficients).
+bool small_takes(int bw);
+int fst_small(Tables* t, const float* grid, float* rc, float* ic, int N, cudaStream_t st, const int64_t* gmap = nullptr,
+              const int64_t* cmap = nullptr);
+int inv_fst_small(Tables* t, const float* rc, const float* ic, float* grid, int N, cudaStream_t st,
+                  const int64_t* gmap = nullptr, const int64_t* cmap = nullptr);
 // Reads (and optionally clears) the device error word of the tensor-core kernels.
 int split_device_status(Tables* t, int clear);
 

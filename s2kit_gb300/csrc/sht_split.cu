@@ -35,6 +35,7 @@
 
 #include "s2g_common.cuh"
 #include "s2g_internal.h"
+#include "small32.cuh"
 #include "fft32.cuh"
 #include "tc_sm103.cuh"
 
@@ -66,6 +67,8 @@ struct Split {
     // per (direction, tile N extent NB): the work items of one 64-function tile, in order, as
     // (order m, index j within the order) -- item decoding is one load
     std::vector<std::pair<int, int2*>> itab[2];
+    float* small = nullptr;      // tables of the one-kernel transforms (small_takes)
+    SmallTab sm{};
     int* err = nullptr;          // device error word (S2G_ERR_TIMEOUT on an expired wait)
     size_t fwd_bytes = 0, inv_bytes = 0;
 };
@@ -90,6 +93,7 @@ void free_split(Tables* t) {
     cudaFree(s->czh);
     cudaFree(s->czK);
     cudaFree(s->cztw);
+    cudaFree(s->small);
     for (auto& v : s->itab)
         for (auto& e : v) cudaFree(e.second);
     cudaFree(s->err);
@@ -341,6 +345,30 @@ static bool split_bw_ok(int B) {
     return (B % 16 == 0 && B / 16 <= 15) || split_czt(B);
 }
 
+// Bandwidths transformed whole by one kernel each way (small32.cuh): those whose tables and data fit the
+// caches.  Against the three kernels of the staged path: one function at bw 16 forward and inverse 42.0 -> 12.3 us;
+// bw 16, 65536 functions: 815 -> 365 and 1043 -> 332; bw 20, 16384 functions: 786 -> 173 and 749 -> 139 (chirp-z
+// stages before); bw 32, 16384 functions: 485 -> 305 and 625 -> 351.  bw 48's table takes 226 KB.
+bool small_takes(int bw) { return bw <= 32; }
+
+static int small_build(const Tables* t, Split* s, cudaStream_t st) {
+    const int B = t->bw;
+    std::vector<double> w(2 * (size_t)B);
+    S2G_CUDA(cudaMemcpyAsync(w.data(), t->weights, sizeof(double) * w.size(), cudaMemcpyDeviceToHost, st));
+    S2G_CUDA(cudaStreamSynchronize(st));
+    size_t off[4], tiles;
+    const std::vector<float> v = small_tables(B, w.data(), off, tiles, s->sm.ntiles);
+    S2G_CUDA(cudaMalloc(&s->small, sizeof(float) * v.size()));
+    S2G_CUDA(cudaMemcpyAsync(s->small, v.data(), sizeof(float) * v.size(), cudaMemcpyHostToDevice, st));
+    S2G_CUDA(cudaStreamSynchronize(st));
+    s->sm.ft = s->small + off[0];
+    s->sm.it = s->small + off[1];
+    s->sm.pf = s->small + off[2];
+    s->sm.pi = s->small + off[3];
+    s->sm.tiles = (const int*)(s->small + tiles);
+    return S2G_OK;
+}
+
 static int build_split(Tables* t) {
     std::lock_guard<std::mutex> lk(g_split_mu);
     if (t->split) return S2G_OK;
@@ -395,6 +423,7 @@ static int build_split(Tables* t) {
         r = czt_build_tables(B, &s->czh, &s->czK, &s->cztw);
         if (r == S2G_OK) s->czM = czt_len(B);
     }
+    if (r == S2G_OK && small_takes(B)) r = small_build(t, s, st);
     if (r == S2G_OK) r = pack_blobs(t, s, false, st);
     cudaStreamDestroy(st);
     t->split = s;
@@ -946,6 +975,7 @@ struct StageCls {
 struct StageArgs {
     int ncls;
     StageCls c[kStageMaxClasses];
+    SmallArgs sm[kStageMaxClasses];  // rows stages: classes transformed whole (B 0: not)
 };
 
 template <int WHICH, int R>
@@ -991,6 +1021,20 @@ __global__ void __launch_bounds__(256, StageOcc<WHICH, RMAX>::v) k_stage_group(c
             if constexpr (RMAX >= 32) stage_body<WHICH, 32>(k, vb);
             break;
     }
+}
+
+// Short-tier rows stage with classes that are transformed whole (small32.cuh) next to bw 64's rows: one
+// launch for both, so that small classes add none.
+template <bool FWD>
+__global__ void __launch_bounds__(256, 3) k_stage_small(const __grid_constant__ StageArgs a) {
+    extern __shared__ __align__(16) float stage_sm[];
+    int ci = 0;
+    while (ci + 1 < a.ncls && (int)blockIdx.x >= a.c[ci + 1].blk0) ++ci;
+    const StageCls& k = a.c[ci];
+    const int vb = (int)blockIdx.x - k.blk0;
+    if (!a.sm[ci].B) stage_body<FWD ? 0 : 3, 4>(k, vb);
+    else if constexpr (FWD) small_fwd_body(a.sm[ci], vb, stage_sm);
+    else small_inv_body(a.sm[ci], vb, stage_sm);
 }
 
 // ------------------------------------------------------------------------------------
@@ -2547,6 +2591,7 @@ int split_stage_group(int which, const StageSpec* spec, int ncls, int dct_ctas_p
     int rmax = 1;
     size_t smem = 0;
     double wsum = 0.0;
+    bool small = false;
     for (int c = 0; c < ncls; ++c) {
         const StageSpec& q = spec[c];
         S2G_TRY(build_split(q.t));
@@ -2565,10 +2610,18 @@ int split_stage_group(int which, const StageSpec* spec, int ncls, int dct_ctas_p
         k.twD = sp->twD;
         k.scale = which == 0 ? (float)(sqrt(2.0 * kPi) / S) : which == 2 ? (float)(1.0 / sqrt(2.0 * kPi)) : 1.f;
         rmax = std::max(rmax, R);
+        if (q.rc) {  // transformed whole
+            a.sm[c] = SmallArgs{B, q.N, sp->sm, (const float*)q.in, (float*)q.out, q.rc, q.ic, q.gmap, q.cmap};
+            smem = std::max(smem, small_smem(B, which == 0));
+            small = true;
+            continue;
+        }
         smem = std::max(smem, fft_smem_rt(R, which));
         wsum += (double)q.N * B * R;
     }
-    const void* fn = which == 0 ? stage_kernel<0>(rmax) : which == 1 ? stage_kernel<1>(rmax)
+    if (small && (rmax > 4 || (which != 0 && which != 3))) return fail(S2G_ERR_ARG, "small classes in stage %d", which);
+    const void* fn = small      ? (which == 0 ? (const void*)k_stage_small<true> : (const void*)k_stage_small<false>)
+                   : which == 0 ? stage_kernel<0>(rmax) : which == 1 ? stage_kernel<1>(rmax)
                    : which == 2 ? stage_kernel<2>(rmax) : stage_kernel<3>(rmax);
     S2G_TRY(set_smem(fn, smem));
     int budget = 0;  // DCT stages: blocks shared out by work (rows x length), as many as fit at once
@@ -2584,15 +2637,18 @@ int split_stage_group(int which, const StageSpec* spec, int ncls, int dct_ctas_p
     // the short classes' blocks for the tail of the launch
     int order[kStageMaxClasses];
     for (int c = 0; c < ncls; ++c) order[c] = c;
-    std::sort(order, order + ncls, [&](int x, int y) { return a.c[x].R > a.c[y].R; });
+    auto length = [&](int c) { return a.c[c].R + (a.sm[c].B ? 64 : 0); };  // a whole transform takes longer yet
+    std::sort(order, order + ncls, [&](int x, int y) { return length(x) > length(y); });
     const StageArgs unsorted = a;
-    for (int c = 0; c < ncls; ++c) a.c[c] = unsorted.c[order[c]];
+    for (int c = 0; c < ncls; ++c) a.c[c] = unsorted.c[order[c]], a.sm[c] = unsorted.sm[order[c]];
     int blk = 0;
     for (int c = 0; c < ncls; ++c) {
         StageCls& k = a.c[c];
         const int B = 16 * k.R, S = 2 * B;
         long long nb;
-        if (which == 0 || which == 3) {
+        if (a.sm[c].B) {
+            nb = (k.N + small_nf(B) - 1) / small_nf(B);
+        } else if (which == 0 || which == 3) {
             nb = (long long)k.N * (S / FftShape<1>::LAT);
         } else {
             const long long rows = (long long)k.N * B, most = (rows + FftShape<1>::W - 1) / FftShape<1>::W;
@@ -2614,6 +2670,36 @@ int split_stage_group(int which, const StageSpec* spec, int ncls, int dct_ctas_p
     return S2G_OK;
 }
 
+// One small class on its own launch (small32.cuh).  The forward, with up to four blocks an SM, takes the registers
+// of two (its loads further ahead: bw 32, 256 functions 17.6 -> 14.5 us), beyond that of three (bw 32, 16384
+// functions: 334 -> 305); the inverse gains nothing by two (17.8 and 17.2; 351 and 435).
+static int small_run(bool fwd, const SmallArgs& p, cudaStream_t st) {
+    int dev = 0, sms = 0;
+    S2G_CUDA(cudaGetDevice(&dev));
+    S2G_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int blocks = (p.N + small_nf(p.B) - 1) / small_nf(p.B);
+    const auto fn = !fwd ? k_small<false, 3> : blocks <= 4 * sms ? k_small<true, 2> : k_small<true, 3>;
+    const size_t smem = small_smem(p.B, fwd);
+    S2G_TRY(set_smem((const void*)fn, smem));
+    {
+        ProfScope ps_(fwd ? "small_fwd_f32" : "small_inv_f32", st);
+        fn<<<blocks, kSmallT, smem, st>>>(p);
+    }
+    S2G_CUDA(cudaGetLastError());
+    return S2G_OK;
+}
+int fst_small(Tables* t, const float* grid, float* rc, float* ic, int N, cudaStream_t st, const int64_t* gmap,
+              const int64_t* cmap) {
+    S2G_TRY(build_split(t));
+    return small_run(true, SmallArgs{t->bw, N, ((const Split*)t->split)->sm, grid, nullptr, rc, ic, gmap, cmap}, st);
+}
+int inv_fst_small(Tables* t, const float* rc, const float* ic, float* grid, int N, cudaStream_t st, const int64_t* gmap,
+                  const int64_t* cmap) {
+    S2G_TRY(build_split(t));
+    return small_run(false, SmallArgs{t->bw, N, ((const Split*)t->split)->sm, nullptr, grid, (float*)rc, (float*)ic,
+                                         gmap, cmap}, st);
+}
+
 // Work counter of the contraction kernel: the int after the two intermediate arrays.
 static int* work_counter(void* work, int B, int batch) {
     const SplitLayout L = split_layout(B);
@@ -2629,6 +2715,7 @@ int fst_split(Tables* t, const float* grid, float* rc, float* ic, int batch, int
     S2G_TRY(build_split(t));
     Split* s = (Split*)t->split;
     const int B = t->bw, S = 2 * B;
+    if (small_takes(B)) return fst_small(t, grid, rc, ic, batch, st);
     bool digits;
     S2G_TRY(use_dg32(t, st, &digits));
     if (digits) return fst_dg32(t, grid, nullptr, rc, ic, batch, work, st);
@@ -2655,6 +2742,7 @@ int inv_fst_split(Tables* t, const float* rc, const float* ic, float* grid, int 
     bool f16 = false;
     S2G_TRY(check_prec(precision, &nprod, &f16));
     S2G_TRY(build_split(t));
+    if (small_takes(t->bw)) return inv_fst_small(t, rc, ic, grid, batch, st);
     bool digits;
     S2G_TRY(use_dg32(t, st, &digits));
     if (digits) return inv_fst_dg32(t, rc, ic, grid, nullptr, batch, work, st);
