@@ -241,7 +241,9 @@ int s2g_inv_fst_complex_f32(s2g_plan plan, const float* rcoeffs, const float* ic
  * the output sees, F64(g) - a -- falls to about e^2 as well, but the split synthesis rounds its
  * samples to FP32, and that rounding noise lies outside the band the residual can see, so the
  * pointwise sample error stays at the FP32 level (about 1e-7).  Both cost one FP64 transform
- * (the residual) plus two split transforms.  Layouts as
+ * (the residual) plus two split transforms; so where the plan's FP64 transforms run as digit products
+ * (and at bw 16) these calls are the FP64 transforms themselves, faster and to their precision, whatever
+ * the precision asked for.  Layouts as
  * s2g_fst_real_f32 (the inverse reads the non-negative orders); bandwidths as s2g_fst_real_f32,
  * plan cutoff == bw.  The plan grows its own scratch. */
 int s2g_fst_refined(s2g_plan plan, const double* grid, double* rcoeffs, double* icoeffs, int batch, int precision,

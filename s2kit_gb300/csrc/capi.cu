@@ -1227,13 +1227,24 @@ int s2g_inv_fst_complex_f32(s2g_plan p, const float* rc, const float* ic, float*
                                  (cudaStream_t)stream);
 }
 
+static int refined_scratch(s2g_plan p, int batch, int precision, cudaStream_t st, bool* direct) {
+    S2G_TRY(split_check(p->t, precision));
+    S2G_TRY(dg_prepare(p->t, st));
+    *direct = refine_direct(p->t);
+    if (*direct) return p->work.ensure(f64_plan_bytes(p->bw, batch, REAL, false));
+    S2G_TRY(p->work.ensure(refine_work_bytes(p->bw, batch)));
+    return p->io.ensure(refine_io_bytes(p->bw, batch));
+}
+
 int s2g_fst_refined(s2g_plan p, const double* grid, double* rc, double* ic, int batch, int precision,
                     void* stream) {
     S2G_TRY(plan_check(p, batch));
     if (!grid || !rc || !ic) return fail(S2G_ERR_ARG, "NULL argument");
     S2G_TRY(check_aligned16({grid, rc, ic}));
-    S2G_TRY(p->work.ensure(refine_work_bytes(p->bw, batch)));
-    S2G_TRY(p->io.ensure(refine_io_bytes(p->bw, batch)));
+    bool direct = false;
+    S2G_TRY(refined_scratch(p, batch, precision, (cudaStream_t)stream, &direct));
+    if (direct)
+        return fst_f64(p->t, grid, nullptr, rc, ic, batch, REAL, p->cutoff, p->work.ptr, (cudaStream_t)stream);
     return fst_refined(p->t, grid, rc, ic, batch, precision, p->io.ptr, p->work.ptr, (cudaStream_t)stream);
 }
 
@@ -1242,8 +1253,10 @@ int s2g_inv_fst_refined(s2g_plan p, const double* rc, const double* ic, double* 
     S2G_TRY(plan_check(p, batch));
     if (!grid || !rc || !ic) return fail(S2G_ERR_ARG, "NULL argument");
     S2G_TRY(check_aligned16({grid, rc, ic}));
-    S2G_TRY(p->work.ensure(refine_work_bytes(p->bw, batch)));
-    S2G_TRY(p->io.ensure(refine_io_bytes(p->bw, batch)));
+    bool direct = false;
+    S2G_TRY(refined_scratch(p, batch, precision, (cudaStream_t)stream, &direct));
+    if (direct)
+        return inv_fst_f64(p->t, rc, ic, grid, nullptr, batch, REAL, p->cutoff, p->work.ptr, (cudaStream_t)stream);
     return inv_fst_refined(p->t, rc, ic, grid, batch, precision, p->io.ptr, p->work.ptr, (cudaStream_t)stream);
 }
 

@@ -272,7 +272,12 @@ int split_fwd_head(Tables* t, const float* grid, float* X, float* C, int batch, 
                    cudaStream_t st);
 int split_inv_tail(Tables* t, float* F, float* Fc, float* grid, int batch, const int64_t* gmap, cudaStream_t st);
 
+// What the split path would refuse (bandwidth, cutoff, precision).
+int split_check(const Tables* t, int precision);
+
 // ---- split transforms with one FP64-residual refinement step (refine.cu) ----
+// Whether the refined transforms run as FP64 transforms instead (dg_prepare called before).
+bool refine_direct(const Tables* t);
 size_t refine_io_bytes(int bw, int batch);
 size_t refine_work_bytes(int bw, int batch);
 int fst_refined(Tables* t, const double* grid, double* rc, double* ic, int batch, int precision, void* io,

@@ -345,6 +345,17 @@ static bool split_bw_ok(int B) {
     return (B % 16 == 0 && B / 16 <= 15) || split_czt(B);
 }
 
+// What the split path refuses, without building anything.
+static int split_refuses(const Tables* t) {
+    const int B = t->bw;
+    if (!split_bw_ok(B))
+        return fail(S2G_ERR_UNSUPPORTED,
+                    "split-precision path needs a bw in [16, 256] or a power of two up to 1024 (got %d)",
+                    B);
+    if (t->cutoff != B) return fail(S2G_ERR_UNSUPPORTED, "split-precision path is seminaive at every order (cutoff == bw)");
+    return S2G_OK;
+}
+
 // Bandwidths transformed whole by one kernel each way (small32.cuh): those whose tables and data fit the
 // caches.  Against the three kernels of the staged path: one function at bw 16 forward and inverse 42.0 -> 12.3 us;
 // bw 16, 65536 functions: 815 -> 365 and 1043 -> 332; bw 20, 16384 functions: 786 -> 173 and 749 -> 139 (chirp-z
@@ -373,11 +384,7 @@ static int build_split(Tables* t) {
     std::lock_guard<std::mutex> lk(g_split_mu);
     if (t->split) return S2G_OK;
     const int B = t->bw, S = 2 * B;
-    if (!split_bw_ok(B))
-        return fail(S2G_ERR_UNSUPPORTED,
-                    "split-precision path needs a bw in [16, 256] or a power of two up to 1024 (got %d)",
-                    B);
-    if (t->cutoff != B) return fail(S2G_ERR_UNSUPPORTED, "split-precision path is seminaive at every order (cutoff == bw)");
+    S2G_TRY(split_refuses(t));
     // every work item's N extent (table rows) must be a valid tcgen05 N: a multiple of 16, at most 256
     for (int m = 0; m < B; ++m)
         for (int d = 0; d < 2; ++d) {
@@ -2986,6 +2993,13 @@ int split_inv_tail(Tables* t, float* F, float* Fc, float* grid, int batch, const
     S2G_TRY(fft_kernels(2, B, Fc, F, batch, s, st, scale));
     // DFT with sign +1 over the orders, Hermitian rows                      (FST_semi_memo.c:334-350)
     return fft_kernels(3, B, F, grid, batch, s, st, 1.f, gmap);
+}
+
+int split_check(const Tables* t, int precision) {
+    int nprod = 0;
+    bool f16 = false;
+    S2G_TRY(check_prec(precision, &nprod, &f16));
+    return split_refuses(t);
 }
 
 int split_prepare(Tables* t, int precision) {

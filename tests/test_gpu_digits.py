@@ -182,3 +182,27 @@ def test_fp32_digit_path_scales_and_nan_stay_with_their_function():
         assert not np.isfinite(g[bad]).any()
         for f in set(range(nb)) - {bad}:
             assert (g[f] == w[f] * (2.0 ** 60 if bad == 5 and f == 3 else 1.0)).all()
+
+
+@pytest.mark.parametrize("bw,nb,prec", [(16, 3, api.PREC_BF16X3), (33, 2, api.PREC_BF16X2), (64, 9, api.PREC_FP16X2),
+                                        (101, 2, api.PREC_BF16X3), (512, 1, api.PREC_BF16X3)])
+def test_refined_transforms_have_fp64_precision(oracle, bw, nb, prec):
+    import torch
+
+    from s2kit_gb300 import S2GError
+
+    rc, ic, gr, gi = _data(bw, nb, "real")
+    plan = api.Plan(bw, bw)
+    d = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (rc, ic, gr)]
+    og = torch.full_like(d[2], 7.0)
+    oc = [torch.full_like(d[0], 7.0) for _ in range(2)]
+    plan.inv_fst_refined(d[0], d[1], og, nb, prec)
+    plan.fst_refined(d[2], oc[0], oc[1], nb, prec)
+    torch.cuda.synchronize()
+    for f in {0, nb - 1}:
+        er, _ = oracle.inv_fst(rc[f], ic[f], bw, api.REAL, bw)
+        assert rel_err_norm(og[f].cpu().numpy().ravel(), 0.0, er, 0.0) <= TOL
+        er, ei = oracle.fst(gr[f], gi[f], bw, api.REAL, 1)
+        assert rel_err_norm(oc[0][f].cpu().numpy(), oc[1][f].cpu().numpy(), er, ei) <= TOL
+    with pytest.raises(S2GError):
+        plan.fst_refined(d[2], oc[0], oc[1], nb, api.PREC_FP64)
