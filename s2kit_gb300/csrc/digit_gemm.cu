@@ -878,9 +878,14 @@ static DgFold dg_fold_layout(int B, bool inv) {
 }
 
 // Latitudes j and 2B-1-j of one field -> fixed point (|x| < 2^vb, scale in e[field][j]) -> even and odd
-// latitude parts of the folded rows, Z[field][t][j][..].  One block per (j, field).
+// latitude parts of the folded rows, Z[field][t][j][..].  One block per (j, field), a thread for every kDgFoldV
+// samples: they are all loaded before the first is used and stay in registers until the scale is known (with a
+// loop over shared memory instead, loads waited for one another: bw 256, 64 functions 67 us against 52, bw 1024, 16
+// functions 406 against 204, bw 255, 64 functions in FP32 54 against 39).
+constexpr int kDgFoldV = 8;
+static int dg_fold_threads(int S) { return std::max(64, ((2 * S + kDgFoldV - 1) / kDgFoldV + 31) & ~31); }  // 512 at bw 1024
 template <int P>
-__global__ void __launch_bounds__(128) k_dg_fold(const typename Dg<P>::Real* __restrict__ r,
+__global__ void __launch_bounds__(512) k_dg_fold(const typename Dg<P>::Real* __restrict__ r,
                                                  const typename Dg<P>::Real* __restrict__ im, int B, int N, int vb,
                                                  DgFold fl, const int64_t* __restrict__ gmap, typename Dg<P>::Int* Z,
                                                  uint32_t* e, uint32_t* ef) {
@@ -888,26 +893,34 @@ __global__ void __launch_bounds__(128) k_dg_fold(const typename Dg<P>::Real* __r
     using Int = typename Dg<P>::Int;
     extern __shared__ __align__(16) uint8_t fold_sm[];  // [2][S]
     Int* rows = reinterpret_cast<Int*>(fold_sm);
-    __shared__ uint32_t red[4];
+    __shared__ uint32_t red[16];
     const int S = 2 * B, j = blockIdx.x, ff = blockIdx.y;
     const Real* g = gmap ? r + gmap[ff] : ff < N ? r + (size_t)ff * S * S : im + (size_t)(ff - N) * S * S;
-    const Real* x[2] = {g + (size_t)j * S, g + (size_t)(S - 1 - j) * S};
+    const Real *x0 = g + (size_t)j * S, *x1 = g + (size_t)(S - 1 - j) * S - S;
     uint32_t mx = 0;
-    for (int i = threadIdx.x; i < 2 * S; i += blockDim.x) {
-        const Real v = i < S ? x[0][i] : x[1][i - S];
-        reinterpret_cast<Real*>(rows)[i] = v;
-        mx = max(mx, dexp(v));
+    Real v[kDgFoldV];
+#pragma unroll
+    for (int u = 0; u < kDgFoldV; ++u) {
+        const int i = threadIdx.x + u * blockDim.x;
+        v[u] = i < 2 * S ? (i < S ? x0 : x1)[i] : Real(0);
     }
+#pragma unroll
+    for (int u = 0; u < kDgFoldV; ++u) mx = max(mx, dexp(v[u]));
     mx = __reduce_max_sync(0xffffffffu, mx);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
     __syncthreads();
-    mx = max(max(red[0], red[1]), max(red[2], red[3]));
+    mx = red[0];
+    for (int q = 1; q < (int)blockDim.x >> 5; ++q) mx = max(mx, red[q]);
     if (threadIdx.x == 0) {
         e[ff * B + j] = mx;
         atomicMax(ef + ff, mx);
     }
     const int em = max((int)mx, 1);
-    for (int i = threadIdx.x; i < 2 * S; i += blockDim.x) rows[i] = dg_fix(reinterpret_cast<const Real*>(rows)[i], em, vb);
+#pragma unroll
+    for (int u = 0; u < kDgFoldV; ++u) {
+        const int i = threadIdx.x + u * blockDim.x;
+        if (i < 2 * S) rows[i] = dg_fix(v[u], em, vb);
+    }
     __syncthreads();
     Int* z0 = Z + ((size_t)ff * S + j) * fl.len;
     Int* z1 = z0 + (size_t)B * fl.len;
@@ -992,7 +1005,7 @@ __global__ void __launch_bounds__(256) k_dg_mid(const Real* __restrict__ X, int 
 
 // Parts of I2 -> samples of latitudes j and 2B-1-j.  One block per (j, field).
 template <int P>
-__global__ void __launch_bounds__(128) k_dg_unfold(const void* __restrict__ Zv, const typename Dg<P>::Real* __restrict__ mid,
+__global__ void __launch_bounds__(128, P == 64 ? 10 : 16) k_dg_unfold(const void* __restrict__ Zv, const typename Dg<P>::Real* __restrict__ mid,
                                                    const uint32_t* __restrict__ ef, int B, int N, int qv, DgFold fl,
                                                    const int64_t* __restrict__ gmap, typename Dg<P>::Real* r, typename Dg<P>::Real* im) {
     using Real = typename Dg<P>::Real;
@@ -1786,8 +1799,8 @@ static int launch_dg_nt(const DgArgs& p, int sms, cudaStream_t st) {
 // 118 and 126).  FP32 (G = 4) has two accumulators at 64 columns.
 // Items of F1 and I2 go column by column (their tables, 1 MB at bw 256, stay in L2), those of F2 and I1 table
 // by table (117 MB each at bw 256).
-// At bw 256, 64 functions: F1 156 us, F2 116, I1 123, I2 118, k_dg_fold 67, k_dg_unfold 53, k_dg_mid 17;
-// forward and inverse together 0.66 ms against 4.59 ms on the FP64 units (DFMA-bound there).  The tensor
+// At bw 256, 64 functions: F1 156 us, F2 116, I1 123, I2 118, k_dg_fold 52, k_dg_unfold 53, k_dg_mid 17;
+// forward and inverse together 0.64 ms against 4.59 ms on the FP64 units (DFMA-bound there).  The tensor
 // pipe alone would take 47 us for each of the four; MMA issue and the waits around it make up the rest.
 template <int STAGE>
 static int dg_columns(const DgTabs* d, const DgArgs& p, int sms) {
@@ -1965,7 +1978,7 @@ static int dg_fst(const DgTabs* d, const double* weights, const typename Dg<P>::
         p.Z = w.Z;
         {
             ProfScope ps_(P == 32 ? "dg_fold_f32" : "dg_fold", st);
-            k_dg_fold<P><<<dim3(B, ff), 128, 2 * (size_t)S * sizeof(Real), st>>>(
+            k_dg_fold<P><<<dim3(B, ff), dg_fold_threads(S), 2 * (size_t)S * sizeof(Real), st>>>(
                 rdata + g0, idata ? idata + g0 : nullptr, B, n, p.vbz, fl, gm, (typename Dg<P>::Int*)w.Z, w.ej, w.ef);
         }
         S2G_CUDA(cudaGetLastError());
