@@ -212,7 +212,7 @@ int s2g_conv(s2g_plan plan, const double* rdata, const double* idata, const doub
 /* Real-field batched transforms with FP32 samples/coefficients and a selectable
  * precision for the Legendre contraction (s2g_precision); any bw in [16, 256] and the powers
  * of two up to 1024 (lengths 2bw that no warp FFT takes, odd bw among them, run as chirp-z
- * transforms, from bw 64 on as exact digit products whatever the precision; bw 16 to 32 run in FP32
+ * transforms, from bw 64 on as exact digit products whatever the precision; bw 16 to 31 run in FP32
  * whatever the precision), plan cutoff == bw.
  * grid: batch*(2bw)^2 floats; rcoeffs/icoeffs: batch*bw*bw floats in the reference layout, negative orders filled by
  * f(l,-m) = (-1)^m conj f(l,m) on output and ignored on input. */

@@ -13,7 +13,7 @@
 // j), so one pair of tables serves all four stages.  n^2 is reduced mod 2S in integers before the
 // angle is formed, so the chirp is exact to FP64 rounding at every n.
 //
-// From bw 64 on the digit products of digit_gemm.cu take these bandwidths, up to 32 the kernels of small32.cuh;
+// From bw 64 on the digit products of digit_gemm.cu take these bandwidths, below 32 the kernels of small32.cuh;
 // the stages here serve 33 to 63, and any above where the digit tables are not there (first call under capture, out of memory).
 //
 // The four stage kernels compute what the warp-FFT stage kernels of sht_split.cu compute

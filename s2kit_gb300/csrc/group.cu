@@ -16,8 +16,8 @@
 // launches per stage whatever their number.  A class of another bandwidth (transform length 32 R
 // with R not a power of two, or a chirp-z length below bw 64) runs each stage as its own launch on the
 // long tier's stream; the chirp-z classes from 64 on take the digit path (digit_gemm.cu) instead.
-// Classes of bw <= 32 are transformed whole (small32.cuh): 16 and 32 by blocks of the short tier's rows
-// launch (k_stage_small), the others each by a launch of its own.  The sequence is captured once as a CUDA graph (on an internal stream, the tiers as
+// Classes below bw 32 are transformed whole (small32.cuh): 16 by blocks of a tier's rows launch
+// (k_stage_small), the others each by a launch of its own.  The sequence is captured once as a CUDA graph (on an internal stream, the tiers as
 // parallel branches) and replayed on the caller's stream; the first call with a given set of
 // pointers runs eagerly and captures, later calls replay.
 //
@@ -97,7 +97,19 @@ static int group_stages(s2g_group g, const int* which, int nstage, In in, Out ou
     const int nc = (int)g->cls.size();
     StageSpec lo[kGroupMaxClasses], hi[kGroupMaxClasses];
     int nlo = 0, nhi = 0;
-    bool forked = false;
+    // Classes transformed whole go with the short tier's rows as long as those fill at most three blocks an SM, which
+    // is what their registers allow (33 functions: 106.0 us staged, 108.9 among the long tier's rows), else with the
+    // long tier's (512 functions: 241 us staged, 239 so, 245 with the short tier's).
+    bool forked = false, small_long = false;
+    int sms = 0;
+    S2G_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g->device));
+    long long blocks = 0;
+    for (auto& k : g->cls) {
+        if (!stage_groupable(k.B)) continue;
+        if (k.B > kShortTierMaxBw) small_long = true;
+        else blocks += k.small ? k.N : (long long)k.N * (2 * k.B / 16);
+    }
+    small_long &= blocks > 3LL * sms;
     for (int w = 0; w < nstage; ++w) {
         nlo = nhi = 0;
         for (int c = 0; c < nc; ++c) {
@@ -107,7 +119,7 @@ static int group_stages(s2g_group g, const int* which, int nstage, In in, Out ou
             if (k.small && !rows) continue;
             StageSpec q{k.t, k.N, in(w, c), out(w, c), rows ? k.gmap : nullptr};
             if (k.small) q.rc = rc, q.ic = ic, q.cmap = k.cmap;
-            if (k.B <= kShortTierMaxBw) lo[nlo++] = q;
+            if (k.B <= kShortTierMaxBw && !(k.small && small_long)) lo[nlo++] = q;
             else hi[nhi++] = q;
         }
         if (nlo && nhi && !forked) {

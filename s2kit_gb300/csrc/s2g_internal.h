@@ -230,7 +230,7 @@ struct StageSpec {
     const void* in;
     void* out;
     const int64_t* gmap;
-    float *rc = nullptr, *ic = nullptr;  // rows stages, bw <= 32 (small_takes): the whole transform, to or from these
+    float *rc = nullptr, *ic = nullptr;  // rows stages, bw < 32 (small_takes): the whole transform, to or from these
     const int64_t* cmap = nullptr;       // (their coefficient offsets); out, in are then the grid or unused
 };
 int split_stage_group(int which, const StageSpec* spec, int ncls, int dct_ctas_per_sm, cudaStream_t st);

@@ -359,8 +359,10 @@ static int split_refuses(const Tables* t) {
 // Bandwidths transformed whole by one kernel each way (small32.cuh): those whose tables and data fit the
 // caches.  Against the three kernels of the staged path: one function at bw 16 forward and inverse 42.0 -> 12.3 us;
 // bw 16, 65536 functions: 815 -> 365 and 1043 -> 332; bw 20, 16384 functions: 786 -> 173 and 749 -> 139 (chirp-z
-// stages before); bw 32, 16384 functions: 485 -> 305 and 625 -> 351.  bw 48's table takes 226 KB.
-bool small_takes(int bw) { return bw <= 32; }
+// stages before).  At bw 32 large batches gain (16384 functions: 485 -> 305 and 625 -> 351), but one block takes
+// 11 to 14 us, which a group of a few dozen functions waits for (66 -> 73 us), and a group's results are those of
+// its bandwidths alone.
+bool small_takes(int bw) { return bw < 32; }
 
 static int small_build(const Tables* t, Split* s, cudaStream_t st) {
     const int B = t->bw;
@@ -1030,17 +1032,30 @@ __global__ void __launch_bounds__(256, StageOcc<WHICH, RMAX>::v) k_stage_group(c
     }
 }
 
-// Short-tier rows stage with classes that are transformed whole (small32.cuh) next to bw 64's rows: one
-// launch for both, so that small classes add none.
-template <bool FWD>
-__global__ void __launch_bounds__(256, 3) k_stage_small(const __grid_constant__ StageArgs a) {
+// Rows stage of a tier with classes that are transformed whole (small32.cuh) among its blocks, so that small classes
+// add no launch: the short tier's, or the long one's (see group_stages).  Compiled for three blocks an SM, where the
+// short tier's rows alone take eight.
+template <bool FWD, int RMAX>
+__global__ void __launch_bounds__(256, RMAX <= 16 ? 3 : 2) k_stage_small(const __grid_constant__ StageArgs a) {
     extern __shared__ __align__(16) float stage_sm[];
     int ci = 0;
     while (ci + 1 < a.ncls && (int)blockIdx.x >= a.c[ci + 1].blk0) ++ci;
     const StageCls& k = a.c[ci];
     const int vb = (int)blockIdx.x - k.blk0;
-    if (!a.sm[ci].B) stage_body<FWD ? 0 : 3, 4>(k, vb);
-    else if constexpr (FWD) small_fwd_body(a.sm[ci], vb, stage_sm);
+    constexpr int W = FWD ? 0 : 3;
+    if (!a.sm[ci].B) {
+        if constexpr (RMAX <= 4) {
+            if (k.R == 4) stage_body<W, 4>(k, vb);
+            else stage_body<W, 2>(k, vb);
+        } else if constexpr (RMAX <= 16) {
+            if (k.R == 16) stage_body<W, 16>(k, vb);
+            else stage_body<W, 8>(k, vb);
+        } else {
+            if (k.R == 32) stage_body<W, 32>(k, vb);
+            else if (k.R == 16) stage_body<W, 16>(k, vb);
+            else stage_body<W, 8>(k, vb);
+        }
+    } else if constexpr (FWD) small_fwd_body(a.sm[ci], vb, stage_sm);
     else small_inv_body(a.sm[ci], vb, stage_sm);
 }
 
@@ -2590,6 +2605,12 @@ static const void* stage_kernel(int rmax) {
          : rmax <= 16 ? (const void*)k_stage_group<WHICH, 16> : (const void*)k_stage_group<WHICH, 32>;
 }
 
+template <bool FWD>
+static const void* small_stage_kernel(int rmax) {
+    return rmax <= 4 ? (const void*)k_stage_small<FWD, 4>
+         : rmax <= 16 ? (const void*)k_stage_small<FWD, 16> : (const void*)k_stage_small<FWD, 32>;
+}
+
 int split_stage_group(int which, const StageSpec* spec, int ncls, int dct_ctas_per_sm, cudaStream_t st) {
     if (ncls < 1 || ncls > kStageMaxClasses) return fail(S2G_ERR_ARG, "%d classes in one stage launch", ncls);
     if (which < 0 || which > 3) return fail(S2G_ERR_ARG, "stage %d", which);
@@ -2599,6 +2620,9 @@ int split_stage_group(int which, const StageSpec* spec, int ncls, int dct_ctas_p
     size_t smem = 0;
     double wsum = 0.0;
     bool small = false;
+    int dev = 0, nsm = 0;
+    S2G_CUDA(cudaGetDevice(&dev));
+    S2G_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     for (int c = 0; c < ncls; ++c) {
         const StageSpec& q = spec[c];
         S2G_TRY(build_split(q.t));
@@ -2618,25 +2642,25 @@ int split_stage_group(int which, const StageSpec* spec, int ncls, int dct_ctas_p
         k.scale = which == 0 ? (float)(sqrt(2.0 * kPi) / S) : which == 2 ? (float)(1.0 / sqrt(2.0 * kPi)) : 1.f;
         rmax = std::max(rmax, R);
         if (q.rc) {  // transformed whole
-            a.sm[c] = SmallArgs{B, q.N, sp->sm, (const float*)q.in, (float*)q.out, q.rc, q.ic, q.gmap, q.cmap};
-            smem = std::max(smem, small_smem(B, which == 0));
+            const int nf = small_nf(B, q.N, nsm);
+            a.sm[c] = SmallArgs{B, q.N, nf, sp->sm, (const float*)q.in, (float*)q.out, q.rc, q.ic, q.gmap, q.cmap};
+            smem = std::max(smem, small_smem(B, nf, which == 0));
             small = true;
             continue;
         }
         smem = std::max(smem, fft_smem_rt(R, which));
         wsum += (double)q.N * B * R;
     }
-    if (small && (rmax > 4 || (which != 0 && which != 3))) return fail(S2G_ERR_ARG, "small classes in stage %d", which);
-    const void* fn = small      ? (which == 0 ? (const void*)k_stage_small<true> : (const void*)k_stage_small<false>)
+    if (small && which != 0 && which != 3) return fail(S2G_ERR_ARG, "small classes in stage %d", which);
+    const void* fn = small && which == 0 ? small_stage_kernel<true>(rmax)
+                   : small               ? small_stage_kernel<false>(rmax)
                    : which == 0 ? stage_kernel<0>(rmax) : which == 1 ? stage_kernel<1>(rmax)
                    : which == 2 ? stage_kernel<2>(rmax) : stage_kernel<3>(rmax);
     S2G_TRY(set_smem(fn, smem));
     int budget = 0;  // DCT stages: blocks shared out by work (rows x length), as many as fit at once
     if (which == 1 || which == 2) {
-        int occ = 0, dev = 0, nsm = 0;
+        int occ = 0;
         S2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, 256, smem));
-        S2G_CUDA(cudaGetDevice(&dev));
-        S2G_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
         if (dct_ctas_per_sm > 0) occ = std::min(std::max(occ, 1), dct_ctas_per_sm);
         budget = std::max(1, occ) * nsm;
     }
@@ -2644,7 +2668,7 @@ int split_stage_group(int which, const StageSpec* spec, int ncls, int dct_ctas_p
     // the short classes' blocks for the tail of the launch
     int order[kStageMaxClasses];
     for (int c = 0; c < ncls; ++c) order[c] = c;
-    auto length = [&](int c) { return a.c[c].R + (a.sm[c].B ? 64 : 0); };  // a whole transform takes longer yet
+    auto length = [&](int c) { return a.c[c].R + (a.sm[c].B ? 7 : 0); };  // a whole transform: between bw 64 and 128
     std::sort(order, order + ncls, [&](int x, int y) { return length(x) > length(y); });
     const StageArgs unsorted = a;
     for (int c = 0; c < ncls; ++c) a.c[c] = unsorted.c[order[c]], a.sm[c] = unsorted.sm[order[c]];
@@ -2654,7 +2678,7 @@ int split_stage_group(int which, const StageSpec* spec, int ncls, int dct_ctas_p
         const int B = 16 * k.R, S = 2 * B;
         long long nb;
         if (a.sm[c].B) {
-            nb = (k.N + small_nf(B) - 1) / small_nf(B);
+            nb = (k.N + a.sm[c].nf - 1) / a.sm[c].nf;
         } else if (which == 0 || which == 3) {
             nb = (long long)k.N * (S / FftShape<1>::LAT);
         } else {
@@ -2678,15 +2702,16 @@ int split_stage_group(int which, const StageSpec* spec, int ncls, int dct_ctas_p
 }
 
 // One small class on its own launch (small32.cuh).  The forward, with up to four blocks an SM, takes the registers
-// of two (its loads further ahead: bw 32, 256 functions 17.6 -> 14.5 us), beyond that of three (bw 32, 16384
-// functions: 334 -> 305); the inverse gains nothing by two (17.8 and 17.2; 351 and 435).
-static int small_run(bool fwd, const SmallArgs& p, cudaStream_t st) {
+// of two (its loads further ahead: bw 29, 1024 functions 39.8 -> 34.2 us), beyond that of three (bw 29, 16384
+// functions: 455 -> 390); the inverse gains little by two (31.2 and 29.9; 301 and 366).
+static int small_run(bool fwd, SmallArgs p, cudaStream_t st) {
     int dev = 0, sms = 0;
     S2G_CUDA(cudaGetDevice(&dev));
     S2G_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const int blocks = (p.N + small_nf(p.B) - 1) / small_nf(p.B);
+    p.nf = small_nf(p.B, p.N, sms);
+    const int blocks = (p.N + p.nf - 1) / p.nf;
     const auto fn = !fwd ? k_small<false, 3> : blocks <= 4 * sms ? k_small<true, 2> : k_small<true, 3>;
-    const size_t smem = small_smem(p.B, fwd);
+    const size_t smem = small_smem(p.B, p.nf, fwd);
     S2G_TRY(set_smem((const void*)fn, smem));
     {
         ProfScope ps_(fwd ? "small_fwd_f32" : "small_inv_f32", st);
@@ -2698,12 +2723,12 @@ static int small_run(bool fwd, const SmallArgs& p, cudaStream_t st) {
 int fst_small(Tables* t, const float* grid, float* rc, float* ic, int N, cudaStream_t st, const int64_t* gmap,
               const int64_t* cmap) {
     S2G_TRY(build_split(t));
-    return small_run(true, SmallArgs{t->bw, N, ((const Split*)t->split)->sm, grid, nullptr, rc, ic, gmap, cmap}, st);
+    return small_run(true, SmallArgs{t->bw, N, 0, ((const Split*)t->split)->sm, grid, nullptr, rc, ic, gmap, cmap}, st);
 }
 int inv_fst_small(Tables* t, const float* rc, const float* ic, float* grid, int N, cudaStream_t st, const int64_t* gmap,
                   const int64_t* cmap) {
     S2G_TRY(build_split(t));
-    return small_run(false, SmallArgs{t->bw, N, ((const Split*)t->split)->sm, nullptr, grid, (float*)rc, (float*)ic,
+    return small_run(false, SmallArgs{t->bw, N, 0, ((const Split*)t->split)->sm, nullptr, grid, (float*)rc, (float*)ic,
                                          gmap, cmap}, st);
 }
 

@@ -1,6 +1,6 @@
 // small32.cuh -- FP32 real-field transforms of small bandwidths, one kernel each way.
 //
-// A function of bandwidth 16 to 32 is 4 to 16 KB: a block holds a few whole functions in shared memory
+// A function of bandwidth 16 to 31 is 4 to 15 KB: a block holds a few whole functions in shared memory
 // and takes them from samples to coefficients (or back) by direct sums on the FP32 units, where the staged
 // path writes and reads the intermediates twice and gives the contraction tiles that are mostly padding.
 // Per function and direction (B = bw, S = 2B, everything folded about the equator, so that a latitude j < B
@@ -26,11 +26,16 @@ namespace s2g {
 
 constexpr int kSmallT = 256;
 
-// Functions of a block: enough rows for its threads.
-__host__ __device__ constexpr int small_nf(int B) { return B <= 16 ? 4 : 2; }
+// Functions of a block, N in all: enough rows for its threads (bw 16: four, above: two), fewer as long as every
+// block has its SM (bw 20, four functions: 12.8 and 11.1 us with two a block, 9.9 and 8.8 with one).
+inline int small_nf(int B, int N, int sms) {
+    int nf = B <= 16 ? 4 : 2;
+    while (nf > 1 && (N + nf / 2 - 1) / (nf / 2) <= sms) nf /= 2;
+    return nf;
+}
 __host__ __device__ constexpr int small_pad(int n) { return (n + 3) & ~3; }
 // Row of Z, Y, O: 2B entries for each function, an odd number of 16-byte units.
-__host__ __device__ constexpr int small_pitch(int B) { return 4 * ((small_nf(B) * 2 * B + 3) / 4 | 1); }
+__host__ __device__ constexpr int small_pitch(int B, int nf) { return 4 * ((nf * 2 * B + 3) / 4 | 1); }
 
 // The row DFT's parts (odd B: cosines, sines; even B: each for even and odd orders): rows of Z and O, orders.
 struct SmallKind {
@@ -59,7 +64,7 @@ struct SmallTab {  // device, per bandwidth
 };
 
 struct SmallArgs {
-    int B, N;           // B 0: not a small class
+    int B, N, nf;       // B 0: not a small class; nf: functions of a block (small_nf)
     SmallTab t;
     const float* in;    // grid (forward)
     float* out;         // grid (inverse)
@@ -67,9 +72,9 @@ struct SmallArgs {
     const int64_t *gmap, *cmap;  // function -> offset of its samples, coefficients (null: back to back)
 };
 
-inline size_t small_smem(int B, bool fwd) {
-    const size_t z = (size_t)2 * B * small_pitch(B);
-    return sizeof(float) * (fwd ? z + (size_t)2 * B * (2 * small_nf(B) * small_pad(B) + 4) : 2 * z);
+inline size_t small_smem(int B, int nf, bool fwd) {
+    const size_t z = (size_t)2 * B * small_pitch(B, nf);
+    return sizeof(float) * (fwd ? z + (size_t)2 * B * (2 * nf * small_pad(B) + 4) : 2 * z);
 }
 
 __device__ __forceinline__ void small_fma(float (&a)[4][4], const float4& x, const float4& y) {
@@ -80,8 +85,8 @@ __device__ __forceinline__ void small_fma(float (&a)[4][4], const float4& x, con
         for (int j = 0; j < 4; ++j) a[i][j] = fmaf(u[i], v[j], a[i][j]);
 }
 
-// acc = sum over i < n of x(i) y(i), the even and the odd terms apart: half the roundings of one chain (bw 32,
-// inverse: 1.12e-7 against 1.37e-7)
+// acc = sum over i < n of x(i) y(i), the even and the odd terms apart: half the roundings of one chain (error
+// of the inverse at bw 16: 0.93e-7 against 1.03e-7)
 template <class X, class Y>
 __device__ __forceinline__ void small_sum(float (&acc)[4][4], int n, X x, Y y) {
     float odd[4][4] = {};
@@ -106,11 +111,11 @@ __device__ __forceinline__ void small_prefetch(const float* p, int n) {
 }
 
 __device__ __forceinline__ void small_fwd_body(const SmallArgs& p, int blk, float* sm) {
-    const int B = p.B, S = 2 * B, NF = small_nf(B), RP = small_pitch(B), BP = small_pad(B), GS = 2 * NF * BP + 4;
+    const int B = p.B, S = 2 * B, NF = p.nf, RP = small_pitch(B, NF), BP = small_pad(B), GS = 2 * NF * BP + 4;
     const int f0 = blk * NF, nf = min(NF, p.N - f0), R = nf * S;
     float *Z = sm, *G = sm + S * RP;
     small_prefetch(p.t.ft, S * small_pad(small_orders(B)));
-    if (B <= 20) small_prefetch(p.t.pf, p.t.ntiles * 4 * BP);
+    if (B <= 20 || NF == 1) small_prefetch(p.t.pf, p.t.ntiles * 4 * BP);
     // fold: eight longitudes by four latitudes a warp (whole sectors in, no bank conflicts out)
     {
         const int lane = threadIdx.x & 31, nj = (B + 3) / 4, KX = small_longs(B), nk = (KX + 7) / 8, h = B / 2;
@@ -227,13 +232,14 @@ __device__ __forceinline__ void small_fwd_body(const SmallArgs& p, int blk, floa
 }
 
 __device__ __forceinline__ void small_inv_body(const SmallArgs& p, int blk, float* sm) {
-    const int B = p.B, S = 2 * B, NF = small_nf(B), RP = small_pitch(B), BP = small_pad(B), KP = small_pad(small_longs(B));
-    const int f0 = blk * NF, nf = min(NF, p.N - f0), R = nf * S, NC = 2 * NF, np = B * (B + 1) / 2;
+    const int B = p.B, S = 2 * B, NF = p.nf, RP = small_pitch(B, NF), BP = small_pad(B), KP = small_pad(small_longs(B));
+    const int f0 = blk * NF, nf = min(NF, p.N - f0), R = nf * S, NC = (2 * NF + 3) & ~3, np = B * (B + 1) / 2;
     float *Y = sm, *O = sm + S * RP, *C = O;  // the coefficients' place is the sums' later
-    small_prefetch(p.t.pi, min(np * BP, 8192));
+    small_prefetch(p.t.pi, NF == 1 ? np * BP : min(np * BP, 8192));
     small_prefetch(p.t.it, small_kinds(B) * small_orders(B) * KP);
     for (int f = 0; f < nf; ++f) {
         const int64_t o = p.cmap ? p.cmap[f0 + f] : (int64_t)(f0 + f) * B * B;
+#pragma unroll 2
         for (int i = threadIdx.x; i < np; i += kSmallT) {
             C[i * NC + 2 * f] = p.rc[o + i];
             C[i * NC + 2 * f + 1] = p.ic[o + i];

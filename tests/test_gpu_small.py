@@ -1,4 +1,4 @@
-"""FP32 transforms of bandwidths 16 to 32 (one kernel each way, csrc/small32.cuh) against the oracle, at the sizes
+"""FP32 transforms of bandwidths 16 to 31 (one kernel each way, csrc/small32.cuh) and 32 against the oracle, at the sizes
 where folds, 4 x 4 tiles and a block's functions have remainders.
 
 Tolerance: tables, samples and results are rounded at 2^-24 = 6e-8, the sums are two chains of at most 16
