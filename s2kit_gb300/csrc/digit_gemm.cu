@@ -1790,9 +1790,10 @@ static int launch_dg_nt(const DgArgs& p, int sms, cudaStream_t st) {
 }
 
 // Columns per item.  While one wave of blocks holds them all, more and smaller items are faster (bw 64, one
-// function: F1 16.4 us at 64 columns, 11.2 at 16).  Beyond one wave, FP64: 64 columns take one accumulator (7 x 64 TMEM columns) whose epilogue the next
-// item's MMAs wait for (F1 at bw 256: 44% of the time), 32 take two by turns, but seven dependent MMAs of
-// about 115 cycles for each 16-deep K step where 64 take ten for twice the columns.  So 64 is for the long K
+// function: F1 16.4 us at 64 columns, 11.2 at 16).  Beyond one wave, FP64: 64 columns take one accumulator (7 x 64
+// TMEM columns) whose epilogue the next item's MMAs wait for (F1 at bw 256: 44% of the time), 32 take two by
+// turns, but seven dependent MMAs of about 115 cycles for each 16-deep K step where 64 take ten for twice the
+// columns.  So 64 is for the long K
 // ranges: I1 (K = the degrees of a parity) never, F2 (K = bw) above bw 256 (bw 256, 256 functions: 478 us at
 // 64, 463 at 32; bw 512, 64 functions: 519 and 601), F1 above 300 (bw 256, 64 functions: 165 and 156; bw 512:
 // 897 and 998), I2 (whose epilogue is the shortest) above 112 orders (bw 192, 64 functions: 97 and 79; bw 256:
