@@ -25,9 +25,9 @@
 //   F2  Legendre fwd    row = degree l       K = latitude            column = (field, re / im)
 //   I1  Legendre inv    row = latitude j     K = degree              column = (field, re / im)
 //   I2  rows inverse    row = longitude      K = order               column = (field, latitude part)
-// F2 and I1 are the naive transform (naive.c:34-96) in every order: on the tensor cores its extra
-// multiply-adds cost less than the DCTs of the seminaive form would, and it is the better
-// conditioned of the two.  k_dg_fold turns samples into fixed point and takes the even and odd
+// F2 and I1 are the naive transform (naive.c:34-96) in every order, F2 but for up to three odd ones above
+// bw 512 (dg_semi_orders): on the tensor cores its extra multiply-adds cost less than the DCTs of the
+// seminaive form would, and it is the better conditioned of the two.  k_dg_fold turns samples into fixed point and takes the even and odd
 // parts in latitude (P(m,l) has one parity) and, for even B, twice in longitude (cos and sin, m even
 // and odd), so that each of F1's four tables is a quarter of the DFT matrix; k_dg_unfold undoes the
 // same after I2.  Between the stages the forward keeps integers (one scale per function).  COMPLEX
@@ -1420,6 +1420,7 @@ struct DgChunk {
 struct DgTabs {
     int device = -1, bw = 0, refs = 0, prec = 64;
     bool fly = false;  // no Legendre tables: chunks, nodes and offsets instead
+    int semi = 0;      // orders of F2 in seminaive form (dg_semi_orders)
     DgTable t[4];
     int* err = nullptr;
     std::vector<DgChunk> chunks[4];
@@ -1430,7 +1431,7 @@ struct DgTabs {
 };
 
 static std::mutex g_dg_mu;
-static std::map<std::tuple<int, int, int, bool>, DgTabs*> g_dg;
+static std::map<std::tuple<int, int, int, bool, int>, DgTabs*> g_dg;  // device, bw, prec, fly, semi
 
 static void dg_free(DgTabs* d) {
     for (auto& t : d->t) t.release();
@@ -1446,7 +1447,7 @@ void dg_put(void* h) {
     if (!d) return;
     std::lock_guard<std::mutex> lk(g_dg_mu);
     if (--d->refs == 0) {
-        g_dg.erase(std::make_tuple(d->device, d->bw, d->prec, d->fly));
+        g_dg.erase(std::make_tuple(d->device, d->bw, d->prec, d->fly, d->semi));
         dg_free(d);
     }
 }
@@ -1523,13 +1524,20 @@ static int dg_upload(DgTable& t, int stage, int B, int prec, cudaStream_t st) {
     return S2G_OK;
 }
 
-// Above this bandwidth the forward's orders 1, 3 and 5 take their rows from the cosine series.  The
-// series of G = P / sin have large coefficients there, and their FP64 rounding is part of the reference's
-// results: on samples that are not band-limited, at bw 1024, the exact transform is 3.2e-11 away from
-// them at order 1 (8e-12 at order 3), more than the 1e-11 that the FP64 path keeps to the reference.
+// Above this bandwidth the forward's orders 1, 3 and 5 take their rows from the cosine series, where they are
+// seminaive (below the cutoff).  The series of G = P / sin have large coefficients there, and their FP64
+// rounding is part of the reference's results: on samples that are not band-limited (noise), at bw 1024, the
+// exact transform is 4.1e-11 of the order's largest coefficient away from them at order 1, 6e-12 at order 3 and
+// 4.5e-12 at order 5, while the FP64 path keeps to the reference within 1e-11.  From the cutoff on the reference
+// is naive, and within 1e-13 of the exact transform.
 constexpr int kDgNaiveBw = 512;
-static int dg_low_orders(int B, double* tmp, const std::vector<int64_t>& off, int m1, cudaStream_t st) {
+// How many of these orders a table has: tables are shared by all cutoffs but for this.
+static int dg_semi_orders(int B, int cutoff, int prec, bool fly) {
+    return B > kDgNaiveBw && prec == 64 && !fly ? std::min(cutoff, 6) / 2 : 0;
+}
+static int dg_low_orders(int B, int semi, double* tmp, const std::vector<int64_t>& off, int m1, cudaStream_t st) {
     const int S = 2 * B;
+    m1 = std::min(m1, 2 * semi);
     struct Buf {
         void* p[3] = {nullptr, nullptr, nullptr};
         ~Buf() {
@@ -1537,14 +1545,14 @@ static int dg_low_orders(int B, double* tmp, const std::vector<int64_t>& off, in
         }
     } b;
     int64_t most = 0;
-    for (int m = 1; m <= 5 && m < m1; m += 2) most = std::max(most, table_size(m, B));
+    for (int m = 1; m < m1; m += 2) most = std::max(most, table_size(m, B));
     const std::vector<int64_t> zero(8, 0);  // each order's table alone, at the buffer's start
     S2G_CUDA(cudaMalloc(&b.p[0], sizeof(double) * (size_t)most));
     S2G_CUDA(cudaMalloc(&b.p[1], sizeof(double2) * 4 * S));
     S2G_CUDA(cudaMalloc(&b.p[2], sizeof(int64_t) * zero.size()));
     S2G_CUDA(cudaMemcpyAsync(b.p[2], zero.data(), sizeof(int64_t) * zero.size(), cudaMemcpyHostToDevice, st));
     S2G_TRY(twiddles_device(4 * S, (double2*)b.p[1], nullptr, st));
-    for (int m = 1; m <= 5 && m < m1; m += 2) {
+    for (int m = 1; m < m1; m += 2) {
         S2G_TRY(generate_cos_pml_device(B, m, m + 1, (double*)b.p[0], (const int64_t*)b.p[2], st));
         ProfScope ps_("dg_seminaive", st);
         k_dg_seminaive<<<B - m, 256, 0, st>>>(B, m, (const double*)b.p[0], (const double2*)b.p[1], tmp + off[m]);
@@ -1725,7 +1733,7 @@ static int dg_build(DgTabs* d, const double* weights, cudaStream_t st) {
         }
         S2G_CUDA(cudaGetLastError());
         for (int s = kI1; s >= kF2; --s) {
-            if (s == kF2 && B > kDgNaiveBw && m0 <= 1 && d->prec == 64) S2G_TRY(dg_low_orders(B, (double*)tmp.p[1], off, m1, st));
+            if (s == kF2 && d->semi && m0 <= 1) S2G_TRY(dg_low_orders(B, d->semi, (double*)tmp.p[1], off, m1, st));
             const DgTable& t = d->t[s];
             size_t a = 0, b = t.h.size();
             while (a < b && t.h[a].m < m0) ++a;
@@ -1744,11 +1752,12 @@ static int dg_build(DgTabs* d, const double* weights, cudaStream_t st) {
 }
 
 // Digit tables of bandwidth bw on the current device, shared by every plan; the caller holds a reference.
-static int dg_get(int bw, int prec, bool fly, const double* weights, DgTabs** out) {
+static int dg_get(int bw, int prec, bool fly, int semi, const double* weights, DgTabs** out) {
     int dev = 0;
     S2G_CUDA(cudaGetDevice(&dev));
     std::lock_guard<std::mutex> lk(g_dg_mu);
-    auto it = g_dg.find(std::make_tuple(dev, bw, prec, fly));
+    const auto key = std::make_tuple(dev, bw, prec, fly, semi);
+    auto it = g_dg.find(key);
     if (it != g_dg.end()) {
         ++it->second->refs;
         *out = it->second;
@@ -1759,6 +1768,7 @@ static int dg_get(int bw, int prec, bool fly, const double* weights, DgTabs** ou
     d->bw = bw;
     d->prec = prec;
     d->fly = fly;
+    d->semi = semi;
     cudaStream_t st;
     S2G_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     const int r = dg_build(d, weights, st);
@@ -1768,7 +1778,7 @@ static int dg_get(int bw, int prec, bool fly, const double* weights, DgTabs** ou
         return r;
     }
     d->refs = 1;
-    g_dg[std::make_tuple(dev, bw, prec, fly)] = d;
+    g_dg[key] = d;
     *out = d;
     return S2G_OK;
 }
@@ -1926,7 +1936,8 @@ static int prepare(Tables* t, int prec, void** slot, bool* off, cudaStream_t st)
         return S2G_OK;
     }
     DgTabs* d;
-    const int r = dg_get(t->bw, prec, t->cutoff == 0, t->weights, &d);
+    const bool fly = t->cutoff == 0;
+    const int r = dg_get(t->bw, prec, fly, dg_semi_orders(t->bw, t->cutoff, prec, fly), t->weights, &d);
     if (r == S2G_ERR_NOMEM) {
         cudaGetLastError();
         *off = true;
