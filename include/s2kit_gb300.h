@@ -290,7 +290,9 @@ int s2g_inv_fst_real_f32_host_async(s2g_plan plan, const float* rcoeffs, const f
 int s2g_plan_wait(s2g_plan plan);
 
 /* Waits for the plan's device work and reports a failure recorded on the device by the
- * tensor-core kernels (S2G_ERR_TIMEOUT when a bounded wait expired); clears the record. */
+ * tensor-core kernels (S2G_ERR_TIMEOUT when a bounded wait expired); clears the record.  Every transform
+ * that runs on them can end so: the FP32 and refined ones, s2g_fst, s2g_inv_fst and s2g_conv.  The digit products
+ * (FP64, chirp-z bandwidths) record it for the plan, the split contraction for all plans of its bandwidth. */
 int s2g_plan_sync_status(s2g_plan plan);
 
 /* Grouped transforms of many real functions of uneven bandwidth (no counterpart in the
@@ -355,6 +357,10 @@ int s2g_set_contraction_kernel(int which);
  * device word, frees its tensor memory and returns.  No fault, trap or hang is involved, and the
  * context stays usable: s2g_plan_sync_status reports the timeout and clears it. */
 int s2g_test_stall_contraction(int on);
+/* The same for the digit-product kernels (the FP64 transforms of plans, convolutions, and the FP32 transforms at
+ * chirp-z bandwidths): with on != 0 no table is copied, so that every wait runs out, and the kernels report it in the
+ * word of the plan, group or drop-in call that launched them. */
+int s2g_test_stall_digits(int on);
 
 /* Kernel timing: while enabled, every kernel the library launches is bracketed by CUDA
  * events on the stream it is launched on.  s2g_prof_enable() also discards earlier records.

@@ -348,7 +348,6 @@ static int do_fst(double* rdata, double* idata, double* rcoeffs, double* icoeffs
     TabRef tref_{base};
     Tables view = *base;
     view.split = nullptr;
-    view.dg = nullptr;  // the caller's own tables
     if (table) S2G_TRY(upload_table(base, table, 0, &view.fwd));  // null: the device's own table (on the fly)
     const size_t S = 2 * (size_t)bw, ng = S * S, nc = (size_t)bw * bw;
     const size_t need = 2 * rnd(ng) + 2 * rnd(nc) + rnd(4 * (size_t)bw) + f64_work_bytes(bw, 1, fmt) + 256;
@@ -393,7 +392,6 @@ static int do_inv_fst(double* rcoeffs, double* icoeffs, double* rdata, double* i
     TabRef tref_{base};
     Tables view = *base;
     view.split = nullptr;
-    view.dg = nullptr;  // the caller's own tables
     if (ttable) S2G_TRY(upload_table(base, ttable, 1, &view.inv));  // null: the device's own table
     const size_t S = 2 * (size_t)bw, ng = S * S, nc = (size_t)bw * bw;
     const size_t need = 2 * rnd(ng) + 2 * rnd(nc) + f64_work_bytes(bw, 1, fmt) + 256;
@@ -434,7 +432,6 @@ static int do_fzt(double* rdata, double* idata, double* rres, double* ires, int 
     TabRef tref_{base};
     Tables view = *base;
     view.split = nullptr;
-    view.dg = nullptr;  // the caller's own tables
     const size_t S = 2 * (size_t)bw, ng = S * S, nt = (size_t)table_size(0, bw);
     const size_t need = 2 * rnd(ng) + 2 * rnd(S) + rnd(nt) + rnd(4 * (size_t)bw) + f64_work_bytes(bw, 1, REAL) + 256;
     S2G_TRY(g_dscratch.s.ensure(need));
@@ -467,7 +464,7 @@ static int do_fzt(double* rdata, double* idata, double* rres, double* ires, int 
 
 // t without Legendre tables (cutoff 0): the on-the-fly kernels.
 static int conv_device(Tables* t, const double* dr, const double* di, const double* fr, const double* fi,
-                       double* rr, double* ri, int batch, Scratch& scr, cudaStream_t st) {
+                       double* rr, double* ri, int batch, Scratch& scr, cudaStream_t st, int* err) {
     const bool fly = (t->cutoff == 0);
     const int bw = t->bw;
     const size_t nc = (size_t)bw * bw;
@@ -483,14 +480,14 @@ static int conv_device(Tables* t, const double* dr, const double* di, const doub
         S2G_TRY(fst_f64_fly(t, dr, di, cr, ci, batch, REAL, w, st));
         S2G_TRY(fzt_f64_fly(t, fr, fi, hr, hi, batch, REAL, w, st));
     } else {
-        S2G_TRY(fst_f64(t, dr, di, cr, ci, batch, REAL, bw, w, st));
+        S2G_TRY(fst_f64(t, dr, di, cr, ci, batch, REAL, bw, w, st, err));
         S2G_TRY(fzt_f64(t, fr, fi, hr, hi, batch, REAL, w, st));
     }
     S2G_TRY(transmult_f64(cr, ci, hr, hi, tr, ti, bw, batch, st));
     if (fly)
         S2G_TRY(inv_fst_f64_fly(t, tr, ti, rr, ri, batch, REAL, w, st));
     else
-        S2G_TRY(inv_fst_f64(t, tr, ti, rr, ri, batch, REAL, bw, w, st));
+        S2G_TRY(inv_fst_f64(t, tr, ti, rr, ri, batch, REAL, bw, w, st, err));
     return S2G_OK;
 }
 
@@ -504,23 +501,27 @@ static int do_conv(double* rdata, double* idata, double* rfilter, double* ifilte
     TabRef tref_{t};
     const size_t S = 2 * (size_t)bw, ng = S * S;
     static thread_local DropinScratch io;
-    S2G_TRY(io.s.ensure(6 * rnd(ng) + 256));
+    S2G_TRY(io.s.ensure(6 * rnd(ng) + rnd(1) + 256));
     Carve c{(char*)io.s.ptr};
     double *dr = c.take(ng), *di = c.take(ng), *fr = c.take(ng), *fi = c.take(ng), *orr = c.take(ng),
            *oi = c.take(ng);
     if (host_direct()) {
-        S2G_TRY(conv_device(t, rdata, idata, rfilter, ifilter, rres, ires, 1, g_dscratch.s, 0));
+        static thread_local volatile int expired;  // the kernels' error word, in host memory
+        expired = 0;
+        S2G_TRY(conv_device(t, rdata, idata, rfilter, ifilter, rres, ires, 1, g_dscratch.s, 0, (int*)&expired));
         S2G_CUDA(cudaStreamSynchronize(0));
-        return S2G_OK;
+        return expired ? dg_expired(expired) : S2G_OK;
     }
+    int* err = (int*)c.take(1);
+    S2G_CUDA(cudaMemsetAsync(err, 0, sizeof(int), 0));
     S2G_CUDA(cudaMemcpy(dr, rdata, ng * 8, cudaMemcpyHostToDevice));
     S2G_CUDA(cudaMemcpy(di, idata, ng * 8, cudaMemcpyHostToDevice));
     S2G_CUDA(cudaMemcpy(fr, rfilter, ng * 8, cudaMemcpyHostToDevice));
     S2G_CUDA(cudaMemcpy(fi, ifilter, ng * 8, cudaMemcpyHostToDevice));
-    S2G_TRY(conv_device(t, dr, di, fr, fi, orr, oi, 1, g_dscratch.s, 0));
+    S2G_TRY(conv_device(t, dr, di, fr, fi, orr, oi, 1, g_dscratch.s, 0, err));
     S2G_CUDA(cudaMemcpy(rres, orr, ng * 8, cudaMemcpyDeviceToHost));
     S2G_CUDA(cudaMemcpy(ires, oi, ng * 8, cudaMemcpyDeviceToHost));
-    return S2G_OK;
+    return dg_status(err);
 }
 
 // 1-D Legendre transforms with the caller's tables.
@@ -982,6 +983,7 @@ struct s2g_plan_s {
     int bw, cutoff, device;
     bool fly = false;  // s2g_plan_create_fly: no Legendre table, on-the-fly kernels
     Tables* t;
+    int* err = nullptr;  // device word, see dg_status
     Scratch work;
     Scratch io;
     Scratch cx;  // the two real fields' coefficients of COMPLEX split transforms
@@ -1062,6 +1064,8 @@ int s2g_plan_create(s2g_plan* plan, int bw, int cutoff) {
     p->t = t;
     for (auto& s : p->streams) S2G_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
     for (auto& e : p->events) S2G_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    S2G_CUDA(cudaMalloc(&p->err, sizeof(int)));
+    S2G_CUDA(cudaMemset(p->err, 0, sizeof(int)));
     tref_.t = nullptr;  // the plan keeps the reference
     *plan = p;
     return S2G_OK;
@@ -1084,6 +1088,8 @@ int s2g_plan_create_fly(s2g_plan* plan, int bw) {
     p->t = t;
     for (auto& s : p->streams) S2G_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
     for (auto& e : p->events) S2G_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    S2G_CUDA(cudaMalloc(&p->err, sizeof(int)));
+    S2G_CUDA(cudaMemset(p->err, 0, sizeof(int)));
     tref_.t = nullptr;
     *plan = p;
     return S2G_OK;
@@ -1102,6 +1108,7 @@ int s2g_plan_destroy(s2g_plan p) {
     p->work.release();
     p->io.release();
     p->cx.release();
+    cudaFree(p->err);
     put_tables(p->t);
     delete p;
     return S2G_OK;
@@ -1150,7 +1157,7 @@ int s2g_fst(s2g_plan p, const double* rdata, const double* idata, double* rcoeff
     S2G_TRY(f64_scratch(p, batch, fmt, idata != nullptr, (cudaStream_t)stream, &digits));
     if (p->fly && !digits)
         return fst_f64_fly(p->t, rdata, idata, rcoeffs, icoeffs, batch, fmt, p->work.ptr, (cudaStream_t)stream);
-    return fst_f64(p->t, rdata, idata, rcoeffs, icoeffs, batch, fmt, p->cutoff, p->work.ptr, (cudaStream_t)stream);
+    return fst_f64(p->t, rdata, idata, rcoeffs, icoeffs, batch, fmt, p->cutoff, p->work.ptr, (cudaStream_t)stream, p->err);
 }
 
 int s2g_inv_fst(s2g_plan p, const double* rcoeffs, const double* icoeffs, double* rdata, double* idata, int batch,
@@ -1162,7 +1169,7 @@ int s2g_inv_fst(s2g_plan p, const double* rcoeffs, const double* icoeffs, double
     if (p->fly && !digits)
         return inv_fst_f64_fly(p->t, rcoeffs, icoeffs, rdata, idata, batch, fmt, p->work.ptr, (cudaStream_t)stream);
     return inv_fst_f64(p->t, rcoeffs, icoeffs, rdata, idata, batch, fmt, p->cutoff, p->work.ptr,
-                       (cudaStream_t)stream);
+                       (cudaStream_t)stream, p->err);
 }
 
 int s2g_fzt(s2g_plan p, const double* rdata, const double* idata, double* rres, double* ires, int batch,
@@ -1185,7 +1192,7 @@ int s2g_conv(s2g_plan p, const double* rdata, const double* idata, const double*
     S2G_TRY(plan_check(p, batch, false, true));
     if (p->cutoff != p->bw) return fail(S2G_ERR_ARG, "s2g_conv needs a plan with cutoff == bw");
     if (!rdata || !rfilter || !rres || !ires) return fail(S2G_ERR_ARG, "NULL argument");
-    return conv_device(p->t, rdata, idata, rfilter, ifilter, rres, ires, batch, p->work, (cudaStream_t)stream);
+    return conv_device(p->t, rdata, idata, rfilter, ifilter, rres, ires, batch, p->work, (cudaStream_t)stream, p->err);
 }
 
 int s2g_fst_real_f32(s2g_plan p, const float* grid, float* rc, float* ic, int batch, int precision, void* stream) {
@@ -1193,7 +1200,7 @@ int s2g_fst_real_f32(s2g_plan p, const float* grid, float* rc, float* ic, int ba
     if (!grid || !rc || !ic) return fail(S2G_ERR_ARG, "NULL argument");
     S2G_TRY(check_aligned16({grid, rc, ic}));
     S2G_TRY(p->work.ensure(split_work_bytes(p->bw, batch)));
-    return fst_split(p->t, grid, rc, ic, batch, precision, p->work.ptr, (cudaStream_t)stream);
+    return fst_split(p->t, grid, rc, ic, batch, precision, p->work.ptr, (cudaStream_t)stream, p->err);
 }
 
 int s2g_inv_fst_real_f32(s2g_plan p, const float* rc, const float* ic, float* grid, int batch, int precision,
@@ -1202,7 +1209,7 @@ int s2g_inv_fst_real_f32(s2g_plan p, const float* rc, const float* ic, float* gr
     if (!grid || !rc || !ic) return fail(S2G_ERR_ARG, "NULL argument");
     S2G_TRY(check_aligned16({grid, rc, ic}));
     S2G_TRY(p->work.ensure(split_work_bytes(p->bw, batch)));
-    return inv_fst_split(p->t, rc, ic, grid, batch, precision, p->work.ptr, (cudaStream_t)stream);
+    return inv_fst_split(p->t, rc, ic, grid, batch, precision, p->work.ptr, (cudaStream_t)stream, p->err);
 }
 
 int s2g_fst_complex_f32(s2g_plan p, const float* rgrid, const float* igrid, float* rc, float* ic, int batch,
@@ -1213,7 +1220,7 @@ int s2g_fst_complex_f32(s2g_plan p, const float* rgrid, const float* igrid, floa
     S2G_TRY(p->work.ensure(split_complex_work_bytes(p->bw, batch)));
     S2G_TRY(p->cx.ensure(split_complex_bytes(p->bw, batch)));
     return fst_split_complex(p->t, rgrid, igrid, rc, ic, batch, precision, p->work.ptr, p->cx.ptr,
-                             (cudaStream_t)stream);
+                             (cudaStream_t)stream, p->err);
 }
 
 int s2g_inv_fst_complex_f32(s2g_plan p, const float* rc, const float* ic, float* rgrid, float* igrid, int batch,
@@ -1224,7 +1231,7 @@ int s2g_inv_fst_complex_f32(s2g_plan p, const float* rc, const float* ic, float*
     S2G_TRY(p->work.ensure(split_complex_work_bytes(p->bw, batch)));
     S2G_TRY(p->cx.ensure(split_complex_bytes(p->bw, batch)));
     return inv_fst_split_complex(p->t, rc, ic, rgrid, igrid, batch, precision, p->work.ptr, p->cx.ptr,
-                                 (cudaStream_t)stream);
+                                 (cudaStream_t)stream, p->err);
 }
 
 static int refined_scratch(s2g_plan p, int batch, int precision, cudaStream_t st, bool* direct) {
@@ -1244,8 +1251,8 @@ int s2g_fst_refined(s2g_plan p, const double* grid, double* rc, double* ic, int 
     bool direct = false;
     S2G_TRY(refined_scratch(p, batch, precision, (cudaStream_t)stream, &direct));
     if (direct)
-        return fst_f64(p->t, grid, nullptr, rc, ic, batch, REAL, p->cutoff, p->work.ptr, (cudaStream_t)stream);
-    return fst_refined(p->t, grid, rc, ic, batch, precision, p->io.ptr, p->work.ptr, (cudaStream_t)stream);
+        return fst_f64(p->t, grid, nullptr, rc, ic, batch, REAL, p->cutoff, p->work.ptr, (cudaStream_t)stream, p->err);
+    return fst_refined(p->t, grid, rc, ic, batch, precision, p->io.ptr, p->work.ptr, (cudaStream_t)stream, p->err);
 }
 
 int s2g_inv_fst_refined(s2g_plan p, const double* rc, const double* ic, double* grid, int batch, int precision,
@@ -1256,8 +1263,8 @@ int s2g_inv_fst_refined(s2g_plan p, const double* rc, const double* ic, double* 
     bool direct = false;
     S2G_TRY(refined_scratch(p, batch, precision, (cudaStream_t)stream, &direct));
     if (direct)
-        return inv_fst_f64(p->t, rc, ic, grid, nullptr, batch, REAL, p->cutoff, p->work.ptr, (cudaStream_t)stream);
-    return inv_fst_refined(p->t, rc, ic, grid, batch, precision, p->io.ptr, p->work.ptr, (cudaStream_t)stream);
+        return inv_fst_f64(p->t, rc, ic, grid, nullptr, batch, REAL, p->cutoff, p->work.ptr, (cudaStream_t)stream, p->err);
+    return inv_fst_refined(p->t, rc, ic, grid, batch, precision, p->io.ptr, p->work.ptr, (cudaStream_t)stream, p->err);
 }
 
 int s2g_plan_sync_status(s2g_plan p) {
@@ -1265,7 +1272,7 @@ int s2g_plan_sync_status(s2g_plan p) {
     S2G_CUDA(cudaSetDevice(p->device));
     S2G_TRY(drain_host(p));
     S2G_CUDA(cudaDeviceSynchronize());
-    const int r = split_device_status(p->t, 1), d = dg_status(p->t, 1);
+    const int r = split_device_status(p->t, 1), d = dg_status(p->err);
     return r != S2G_OK ? r : d;
 }
 
@@ -1329,9 +1336,9 @@ static int host_pipeline(s2g_plan p, int fwd, const float* in0, const float* in1
         S2G_CUDA(cudaStreamWaitEvent(comp, in_ready[b], 0));
         S2G_CUDA(cudaStreamWaitEvent(comp, out_free[b], 0));  // the download that last read dout[b]
         if (fwd)
-            S2G_TRY(fst_split(p->t, din[b], dout[b], dout[b] + (size_t)n * nc, n, precision, p->work.ptr, comp));
+            S2G_TRY(fst_split(p->t, din[b], dout[b], dout[b] + (size_t)n * nc, n, precision, p->work.ptr, comp, p->err));
         else
-            S2G_TRY(inv_fst_split(p->t, din[b], din[b] + (size_t)n * nc, dout[b], n, precision, p->work.ptr, comp));
+            S2G_TRY(inv_fst_split(p->t, din[b], din[b] + (size_t)n * nc, dout[b], n, precision, p->work.ptr, comp, p->err));
         S2G_CUDA(cudaEventRecord(done[b], comp));
         S2G_CUDA(cudaStreamWaitEvent(d2h, done[b], 0));
         if (fwd) {

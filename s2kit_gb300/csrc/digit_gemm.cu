@@ -35,6 +35,7 @@
 //
 #include <math.h>
 
+#include <atomic>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -116,7 +117,8 @@ struct DgArgs {
     const uint32_t* efield;    // FP64 F1, F2: exponents of the fields
     const int64_t* cmap;       // function -> coefficient offset (null: f B^2; real fields only)
     uint32_t* emax;            // F1 writes, F2 reads: X's rows (FP64 bits, FP32 exponents); I1 writes: fields
-    int* err;
+    int* err;                  // gets S2G_ERR_TIMEOUT where a bounded wait expired; device memory, or the host's
+    int stall;                 // test hook: the table warp copies nothing, so that the waits run out
 };
 
 __device__ __forceinline__ uint32_t dexp(double x) { return ((uint32_t)__double2hiint(x) >> 20) & 0x7ffu; }
@@ -455,7 +457,7 @@ __global__ void __launch_bounds__(kDgThreads, 1) k_dg(DgArgs p) {
         if (lane == 0) {  // table digits
             uint32_t c = 0;
             bool ok = true;
-            for (int it = blockIdx.x; it < nitems && ok; it += gridDim.x) {
+            for (int it = blockIdx.x; it < nitems && ok && !p.stall; it += gridDim.x) {
                 int tile, cb;
                 decode(it, tile, cb);
                 const DgTile* tl = p.tiles + tile;
@@ -844,7 +846,7 @@ __global__ void __launch_bounds__(kDgThreads, 1) k_dg(DgArgs p) {
     if (warp == 0) {
         tc::tc_fence_after();
         tc::tmem_dealloc(tmem, 512);
-        if (lane == 0 && failed) atomicExch(p.err, S2G_ERR_TIMEOUT);
+        if (lane == 0 && failed) *(volatile int*)p.err = S2G_ERR_TIMEOUT;
     }
 }
 
@@ -1422,7 +1424,6 @@ struct DgTabs {
     bool fly = false;  // no Legendre tables: chunks, nodes and offsets instead
     int semi = 0;      // orders of F2 in seminaive form (dg_semi_orders)
     DgTable t[4];
-    int* err = nullptr;
     std::vector<DgChunk> chunks[4];
     size_t tmp_bytes[4] = {0, 0, 0, 0}, tab_bytes[4] = {0, 0, 0, 0};
     double2* nodes = nullptr;          // cos, sin, seeds: B each; recurrence coefficients: B x B
@@ -1431,6 +1432,7 @@ struct DgTabs {
 };
 
 static std::mutex g_dg_mu;
+static std::atomic<int> g_dg_stall{0};  // see s2g_test_stall_digits
 static std::map<std::tuple<int, int, int, bool, int>, DgTabs*> g_dg;  // device, bw, prec, fly, semi
 
 static void dg_free(DgTabs* d) {
@@ -1438,7 +1440,6 @@ static void dg_free(DgTabs* d) {
     for (auto* o : d->off) cudaFree(o);
     cudaFree(d->nodes);
     cudaFree(d->first);
-    cudaFree(d->err);
     delete d;
 }
 
@@ -1658,8 +1659,6 @@ static int dg_fly_chunks(DgTabs* d, const double* weights, cudaStream_t st) {
 
 static int dg_build(DgTabs* d, const double* weights, cudaStream_t st) {
     const int B = d->bw, S = 2 * B;
-    S2G_CUDA(cudaMalloc(&d->err, sizeof(int)));
-    S2G_CUDA(cudaMemsetAsync(d->err, 0, sizeof(int), st));
     for (int s = 0; s < 4; ++s)
         if (!d->fly || s == kF1 || s == kI2) S2G_TRY(dg_upload(d->t[s], s, B, d->prec, st));
     for (int s = kF1; s <= kI2; s += kI2 - kF1) {
@@ -1827,7 +1826,7 @@ static int dg_columns(const DgTabs* d, const DgArgs& p, int sms) {
 template <int STAGE>
 static int launch_dg_tiles(const DgTabs* d, DgArgs p, cudaStream_t st) {
     p.col_major = STAGE == kF1 || STAGE == kI2;
-    p.err = d->err;
+    p.stall = g_dg_stall.load(std::memory_order_relaxed);
     int dev = 0, sms = 0;
     S2G_CUDA(cudaGetDevice(&dev));
     S2G_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -1964,7 +1963,7 @@ static int set_dyn_smem(const void* fn, size_t bytes) {
 template <int P>
 static int dg_fst(const DgTabs* d, const double* weights, const typename Dg<P>::Real* rdata,
                   const typename Dg<P>::Real* idata, typename Dg<P>::Real* rc, typename Dg<P>::Real* ic, int batch, int fmt,
-                  void* work, cudaStream_t st, const int64_t* gmap = nullptr, const int64_t* cmap = nullptr) {
+                  void* work, cudaStream_t st, int* err, const int64_t* gmap = nullptr, const int64_t* cmap = nullptr) {
     using Real = typename Dg<P>::Real;
     const int B = d->bw, S = 2 * B, mode = dg_mode(idata, fmt), chunk = dg_chunk(B, batch, sizeof(Real));
     const DgFold fl = dg_fold_layout(B, false);
@@ -1982,6 +1981,7 @@ static int dg_fst(const DgTabs* d, const double* weights, const typename Dg<P>::
         p.N = n;
         p.mode = mode;
         p.cmap = cm;
+        p.err = err;
         p.BP = (B + 3) & ~3;
         p.RL = fl.len;
         p.vbz = dg_vbz(B, P);
@@ -2010,7 +2010,7 @@ static int dg_fst(const DgTabs* d, const double* weights, const typename Dg<P>::
 template <int P>
 static int dg_inv_fst(const DgTabs* d, const double* weights, const typename Dg<P>::Real* rc,
                       const typename Dg<P>::Real* ic, typename Dg<P>::Real* rdata, typename Dg<P>::Real* idata, int batch,
-                      int fmt, void* work, cudaStream_t st, const int64_t* gmap = nullptr,
+                      int fmt, void* work, cudaStream_t st, int* err, const int64_t* gmap = nullptr,
                       const int64_t* cmap = nullptr) {
     using Real = typename Dg<P>::Real;
     const int B = d->bw, S = 2 * B, mode = dg_mode(idata, fmt), chunk = dg_chunk(B, batch, sizeof(Real));
@@ -2033,6 +2033,7 @@ static int dg_inv_fst(const DgTabs* d, const double* weights, const typename Dg<
         p.N = n;
         p.mode = mode;
         p.cmap = cm;
+        p.err = err;
         p.BP = (B + 3) & ~3;
         p.RL = fl.len;
         p.X = w.X;
@@ -2063,34 +2064,35 @@ static int dg_inv_fst(const DgTabs* d, const double* weights, const typename Dg<
 }
 
 int fst_f64_dg(const Tables* t, const double* rdata, const double* idata, double* rc, double* ic, int batch, int fmt,
-               void* work, cudaStream_t st) {
-    return dg_fst<64>((const DgTabs*)t->dg, t->weights, rdata, idata, rc, ic, batch, fmt, work, st);
+               void* work, cudaStream_t st, int* err) {
+    return dg_fst<64>((const DgTabs*)t->dg, t->weights, rdata, idata, rc, ic, batch, fmt, work, st, err);
 }
 int inv_fst_f64_dg(const Tables* t, const double* rc, const double* ic, double* rdata, double* idata, int batch, int fmt,
-                   void* work, cudaStream_t st) {
-    return dg_inv_fst<64>((const DgTabs*)t->dg, t->weights, rc, ic, rdata, idata, batch, fmt, work, st);
+                   void* work, cudaStream_t st, int* err) {
+    return dg_inv_fst<64>((const DgTabs*)t->dg, t->weights, rc, ic, rdata, idata, batch, fmt, work, st, err);
 }
 int fst_dg32(const Tables* t, const float* rgrid, const float* igrid, float* rc, float* ic, int batch, void* work,
-             cudaStream_t st, const int64_t* gmap, const int64_t* cmap) {
+             cudaStream_t st, int* err, const int64_t* gmap, const int64_t* cmap) {
     return dg_fst<32>((const DgTabs*)t->dg32, t->weights, rgrid, igrid, rc, ic, batch, igrid ? COMPLEX : REAL, work, st,
-                      gmap, cmap);
+                      err, gmap, cmap);
 }
 int inv_fst_dg32(const Tables* t, const float* rc, const float* ic, float* rgrid, float* igrid, int batch, void* work,
-                 cudaStream_t st, const int64_t* gmap, const int64_t* cmap) {
+                 cudaStream_t st, int* err, const int64_t* gmap, const int64_t* cmap) {
     return dg_inv_fst<32>((const DgTabs*)t->dg32, t->weights, rc, ic, rgrid, igrid, batch, igrid ? COMPLEX : REAL, work, st,
-                          gmap, cmap);
+                          err, gmap, cmap);
 }
 
-int dg_status(const Tables* t, int clear) {
-    for (const void* h : {t->dg, t->dg32}) {
-        const DgTabs* d = (const DgTabs*)h;
-        if (!d) continue;
-        int v = 0;
-        S2G_CUDA(cudaMemcpy(&v, d->err, sizeof(int), cudaMemcpyDeviceToHost));
-        if (clear && v) S2G_CUDA(cudaMemset(d->err, 0, sizeof(int)));
-        if (v) return fail(v, "a bounded wait in the digit-product kernel expired");
-    }
-    return S2G_OK;
+int dg_status(int* err) {
+    int v = 0;
+    S2G_CUDA(cudaMemcpy(&v, err, sizeof(int), cudaMemcpyDeviceToHost));
+    if (v) S2G_CUDA(cudaMemset(err, 0, sizeof(int)));
+    return v ? dg_expired(v) : S2G_OK;
 }
+int dg_expired(int code) { return fail(code, "a bounded wait in the digit-product kernel expired"); }
 
 }  // namespace s2g
+
+extern "C" int s2g_test_stall_digits(int on) {
+    s2g::g_dg_stall = on ? 1 : 0;
+    return S2G_OK;
+}

@@ -73,6 +73,7 @@ struct s2g_group_s {
     std::vector<s2g::GroupClass> cls;
     void* mem = nullptr;        // one device allocation: maps, intermediates, counters
     int* counters = nullptr;    // [0] forward, [1] inverse contraction work counters
+    int* err = nullptr;         // error word of the digit path (dg_status)
     int table_stages = 0;       // contraction: table-copy ring depth, 0 = as many as fit
     int dct_ctas = 0;           // DCT stages: resident blocks per SM they are sized for, 0 = as many as fit
     cudaStream_t cap = nullptr;
@@ -147,7 +148,7 @@ static int group_stages(s2g_group g, const int* which, int nstage, In in, Out ou
 static int group_fwd_seq(s2g_group g, const float* grid, float* rc, float* ic, cudaStream_t st) {
     const int nc = (int)g->cls.size();
     for (auto& k : g->cls)
-        if (k.digits) S2G_TRY(fst_dg32(k.t, grid, nullptr, rc, ic, k.N, k.digits, st, k.gmap, k.cmap));
+        if (k.digits) S2G_TRY(fst_dg32(k.t, grid, nullptr, rc, ic, k.N, k.digits, st, g->err, k.gmap, k.cmap));
         else if (k.small && !stage_groupable(k.B)) S2G_TRY(fst_small(k.t, grid, rc, ic, k.N, st, k.gmap, k.cmap));
     const int which[2] = {0, 1};  // grid -> X -> C
     S2G_TRY(group_stages(
@@ -178,7 +179,7 @@ static int group_inv_seq(s2g_group g, const float* rc, const float* ic, float* g
     for (int c = 0; c < nc; ++c) {
         GroupClass& k = g->cls[c];
         if (k.digits) {
-            S2G_TRY(inv_fst_dg32(k.t, rc, ic, grid, nullptr, k.N, k.digits, st, k.gmap, k.cmap));
+            S2G_TRY(inv_fst_dg32(k.t, rc, ic, grid, nullptr, k.N, k.digits, st, g->err, k.gmap, k.cmap));
             continue;
         }
         if (k.small) {
@@ -507,7 +508,7 @@ int s2g_group_create(s2g_group* out, int nfunc, const int* bw, int precision) {
         c.small = small_takes(c.B);
     }
     auto digits = [](const GroupClass& c) { return dg32_takes(c.B) && c.t && c.t->dg32; };
-    // device memory: maps, intermediates (256-byte aligned pieces), two counters
+    // device memory: maps, intermediates (256-byte aligned pieces), two counters and the error word
     auto rnd = [](size_t x) { return (x + 255) & ~(size_t)255; };
     size_t total = 256;
     auto x_floats = [](const GroupClass& c) { return 2 * (size_t)c.N * c.B * split_layout(c.B).SX; };
@@ -522,7 +523,9 @@ int s2g_group_create(s2g_group* out, int nfunc, const int* bw, int precision) {
     if (r == S2G_OK) {
         char* p = (char*)g->mem;
         g->counters = (int*)p;
+        g->err = g->counters + 2;
         p += 256;
+        if (cudaMemset(g->err, 0, sizeof(int)) != cudaSuccess) r = cuda_fail(cudaGetLastError(), "group error word");
         std::vector<int64_t> gm, cm;
         for (auto& c : g->cls) {
             c.gmap = (int64_t*)p;
@@ -666,10 +669,11 @@ int s2g_group_sync_status(s2g_group g) {
     S2G_CUDA(cudaDeviceSynchronize());
     int r = S2G_OK;
     for (auto& c : g->cls) {
-        const int v = split_device_status(c.t, 1), d = dg_status(c.t, 1);
-        if (r == S2G_OK) r = v != S2G_OK ? v : d;
+        const int v = split_device_status(c.t, 1);
+        if (r == S2G_OK) r = v;
     }
-    return r;
+    const int d = dg_status(g->err);
+    return r != S2G_OK ? r : d;
 }
 
 }  // extern "C"

@@ -71,7 +71,7 @@ size_t refine_work_bytes(int bw, int batch) {
 }
 
 int fst_refined(Tables* t, const double* grid, double* rc, double* ic, int batch, int precision, void* io,
-                void* work, cudaStream_t st) {
+                void* work, cudaStream_t st, int* dg) {
     const int B = t->bw;
     const size_t ng = 4 * (size_t)B * B * batch, nc = (size_t)B * B * batch;
     S2G_TRY(dg_prepare(t, st));
@@ -85,21 +85,21 @@ int fst_refined(Tables* t, const double* grid, double* rc, double* ic, int batch
     double* g64 = (double*)p;
     // a1 = F_split(f)
     S2G_EW("refine_d2f", k_d2f, ng, st, grid, g32);
-    S2G_TRY(fst_split(t, g32, c32r, c32i, batch, precision, work, st));
+    S2G_TRY(fst_split(t, g32, c32r, c32i, batch, precision, work, st, dg));
     S2G_EW("refine_f2d", k_f2d, nc, st, c32r, rc);
     S2G_EW("refine_f2d", k_f2d, nc, st, c32i, ic);
     // r = f - I_fp64(a1)
-    S2G_TRY(inv_fst_f64(t, rc, ic, g64, nullptr, batch, REAL, t->cutoff, work, st));
+    S2G_TRY(inv_fst_f64(t, rc, ic, g64, nullptr, batch, REAL, t->cutoff, work, st, dg));
     S2G_EW("refine_resid", k_resid, ng, st, grid, g64, g32);
     // a = a1 + F_split(r)
-    S2G_TRY(fst_split(t, g32, c32r, c32i, batch, precision, work, st));
+    S2G_TRY(fst_split(t, g32, c32r, c32i, batch, precision, work, st, dg));
     S2G_EW("refine_accum", k_accum, nc, st, rc, c32r);
     S2G_EW("refine_accum", k_accum, nc, st, ic, c32i);
     return S2G_OK;
 }
 
 int inv_fst_refined(Tables* t, const double* rc, const double* ic, double* grid, int batch, int precision, void* io,
-                    void* work, cudaStream_t st) {
+                    void* work, cudaStream_t st, int* dg) {
     const int B = t->bw;
     const size_t ng = 4 * (size_t)B * B * batch, nc = (size_t)B * B * batch;
     S2G_TRY(dg_prepare(t, st));
@@ -115,14 +115,14 @@ int inv_fst_refined(Tables* t, const double* rc, const double* ic, double* grid,
     // g1 = I_split(a)
     S2G_EW("refine_d2f", k_d2f, nc, st, rc, c32r);
     S2G_EW("refine_d2f", k_d2f, nc, st, ic, c32i);
-    S2G_TRY(inv_fst_split(t, c32r, c32i, g32, batch, precision, work, st));
+    S2G_TRY(inv_fst_split(t, c32r, c32i, g32, batch, precision, work, st, dg));
     S2G_EW("refine_f2d", k_f2d, ng, st, g32, grid);
     // r = a - F_fp64(g1)
-    S2G_TRY(fst_f64(t, grid, nullptr, a64r, a64i, batch, REAL, t->cutoff, work, st));
+    S2G_TRY(fst_f64(t, grid, nullptr, a64r, a64i, batch, REAL, t->cutoff, work, st, dg));
     S2G_EW("refine_resid", k_resid, nc, st, rc, a64r, c32r);
     S2G_EW("refine_resid", k_resid, nc, st, ic, a64i, c32i);
     // g = g1 + I_split(r)
-    S2G_TRY(inv_fst_split(t, c32r, c32i, g32, batch, precision, work, st));
+    S2G_TRY(inv_fst_split(t, c32r, c32i, g32, batch, precision, work, st, dg));
     S2G_EW("refine_accum", k_accum, ng, st, grid, g32);
     return S2G_OK;
 }

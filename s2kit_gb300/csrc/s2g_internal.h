@@ -115,6 +115,9 @@ size_t f64_work_bytes(int bw, int batch, int data_format);
 // The same for calls that may take the digit path (dg_prepare); two: the data have imaginary parts.
 size_t f64_plan_bytes(int bw, int batch, int data_format, bool two);
 // ---- FP64 transforms as exact digit products on the tensor cores (digit_gemm.cu) ----
+// Their kernels' waits are bounded; `err` is the word of the plan, group or call that gets S2G_ERR_TIMEOUT
+// where one expired (device memory, or the host's where host_direct).  The functions further down that may take
+// this path take the word as `dg`: null keeps them off it.
 bool dg_takes(int bw);
 size_t dg_work_bytes(int bw, int batch, bool two);
 // FP32 samples and coefficients (igrid null: real fields); readied by dg32_prepare into t->dg32.
@@ -123,21 +126,22 @@ bool dg32_takes(int bw);
 size_t dg32_work_bytes(int bw, int batch, bool two);
 int dg32_prepare(Tables* t, cudaStream_t st);
 int fst_dg32(const Tables* t, const float* rgrid, const float* igrid, float* rc, float* ic, int batch, void* work,
-             cudaStream_t st, const int64_t* gmap = nullptr, const int64_t* cmap = nullptr);
+             cudaStream_t st, int* err, const int64_t* gmap = nullptr, const int64_t* cmap = nullptr);
 int inv_fst_dg32(const Tables* t, const float* rc, const float* ic, float* rgrid, float* igrid, int batch, void* work,
-                 cudaStream_t st, const int64_t* gmap = nullptr, const int64_t* cmap = nullptr);
+                 cudaStream_t st, int* err, const int64_t* gmap = nullptr, const int64_t* cmap = nullptr);
 // On-the-fly family (tables of cutoff 0): real fields for which it pays, and the scratch once prepared.
 bool dg_fly_takes(int bw, int fields);
 size_t dg_fly_bytes(const Tables* t, int batch, bool two);
 int dg_prepare(Tables* t, cudaStream_t st);
 void dg_put(void* dg);
-int dg_status(const Tables* t, int clear);
+int dg_status(int* err);    // reads the (device) word and clears it
+int dg_expired(int code);  // records the failure
 int fst_f64_dg(const Tables* t, const double* rdata, const double* idata, double* rc, double* ic, int batch,
-               int data_format, void* work, cudaStream_t st);
+               int data_format, void* work, cudaStream_t st, int* err);
 int inv_fst_f64_dg(const Tables* t, const double* rc, const double* ic, double* rdata, double* idata, int batch,
-                   int data_format, void* work, cudaStream_t st);
+                   int data_format, void* work, cudaStream_t st, int* err);
 int fst_f64(const Tables* t, const double* rdata, const double* idata, double* rc, double* ic, int batch,
-            int data_format, int cutoff, void* work, cudaStream_t st);
+            int data_format, int cutoff, void* work, cudaStream_t st, int* dg = nullptr);
 // fst_f64 with the DFT geometry of length 2bw (Bluestein tables included when 2bw is not a
 // power of two) supplied by the caller instead of looked up in the per-device length cache,
 // which builds missing tables with cudaMalloc.  Null `len_S` behaves like fst_f64.
@@ -145,7 +149,7 @@ struct Len;
 int fst_f64_len(const Tables* t, const Len* len_S, const double* rdata, const double* idata, double* rc,
                 double* ic, int batch, int data_format, int cutoff, void* work, cudaStream_t st);
 int inv_fst_f64(const Tables* t, const double* rc, const double* ic, double* rdata, double* idata, int batch,
-                int data_format, int cutoff, void* work, cudaStream_t st);
+                int data_format, int cutoff, void* work, cudaStream_t st, int* dg = nullptr);
 // On-the-fly family (FST_semi_fly.c): the Legendre functions are generated inside the
 // contraction kernels, so `t` needs only its weights and twiddles (tables of cutoff 0, see
 // get_tables); work as f64_work_bytes.
@@ -210,15 +214,15 @@ int czt_stage(int which, const CztTabs& g, const void* in, void* out, int N, flo
 size_t split_work_bytes(int bw, int batch);
 size_t split_complex_work_bytes(int bw, int batch);
 int fst_split(Tables* t, const float* grid, float* rc, float* ic, int batch, int precision, void* work,
-              cudaStream_t st);
+              cudaStream_t st, int* dg);
 int inv_fst_split(Tables* t, const float* rc, const float* ic, float* grid, int batch, int precision, void* work,
-                  cudaStream_t st);
+                  cudaStream_t st, int* dg);
 // COMPLEX data as two real fields (cwork: split_complex_bytes of scratch besides work).
 size_t split_complex_bytes(int bw, int batch);
 int fst_split_complex(Tables* t, const float* rgrid, const float* igrid, float* rc, float* ic, int batch,
-                      int precision, void* work, void* cwork, cudaStream_t st);
+                      int precision, void* work, void* cwork, cudaStream_t st, int* dg);
 int inv_fst_split_complex(Tables* t, const float* rc, const float* ic, float* rgrid, float* igrid, int batch,
-                          int precision, void* work, void* cwork, cudaStream_t st);
+                          int precision, void* work, void* cwork, cudaStream_t st, int* dg);
 // One FFT stage of several bandwidth classes (split path, power-of-two bw <= 512) in ONE launch:
 // which 0 rows forward (grid -> X), 1 weighted DCT-II (X -> C), 2 DCT-III (Fc -> F), 3 rows
 // inverse (F -> grid); in/out as the per-class kernels, gmap per-function grid offsets for the
@@ -281,8 +285,8 @@ bool refine_direct(const Tables* t);
 size_t refine_io_bytes(int bw, int batch);
 size_t refine_work_bytes(int bw, int batch);
 int fst_refined(Tables* t, const double* grid, double* rc, double* ic, int batch, int precision, void* io,
-                void* work, cudaStream_t st);
+                void* work, cudaStream_t st, int* dg);
 int inv_fst_refined(Tables* t, const double* rc, const double* ic, double* grid, int batch, int precision, void* io,
-                    void* work, cudaStream_t st);
+                    void* work, cudaStream_t st, int* dg);
 
 }  // namespace s2g

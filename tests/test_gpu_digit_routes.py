@@ -41,3 +41,60 @@ def test_low_orders_are_seminaive_below_the_cutoff_only(oracle, cutoff):
         at = harmonic_index(m, np.arange(m, bw), bw)
         e = np.hypot(rc[at] - er, ic[at] - ei).max() / np.hypot(er, ei).max()
         assert e <= (1e-11 if m < cutoff else 1e-12), (m, e)
+
+
+def _cuda(*shape, dtype="float64"):
+    import torch
+    return torch.randn(*shape, dtype=getattr(torch, dtype), device="cuda", generator=torch.Generator("cuda").manual_seed(7))
+
+
+def _expire(lib, call):
+    """call() with the digit kernels' table copies left out: every wait runs out (half a second), nothing hangs."""
+    import torch
+    assert lib.s2g_test_stall_digits(1) == 0
+    try:
+        call()
+        torch.cuda.synchronize()
+    finally:
+        lib.s2g_test_stall_digits(0)
+
+
+def test_expired_wait_is_reported_to_its_own_plan():
+    import s2kit_gb300 as s2
+    lib, bw, nb = s2.load(), 48, 4
+    grid, oc = _cuda(nb, 4 * bw * bw), [_cuda(nb, bw * bw) for _ in range(2)]
+    plan, other = api.Plan(bw, bw), api.Plan(bw, bw)
+    plan.fst(grid, None, oc[0], oc[1], nb, api.REAL)
+    want = oc[0].clone()
+    _expire(lib, lambda: plan.fst(grid, None, oc[0], oc[1], nb, api.REAL))
+    assert lib.s2g_plan_sync_status(other.h) == 0
+    assert lib.s2g_plan_sync_status(plan.h) == 5  # S2G_ERR_TIMEOUT, read and cleared
+    assert lib.s2g_plan_sync_status(plan.h) == 0
+    plan.fst(grid, None, oc[0], oc[1], nb, api.REAL)
+    plan.sync_status()
+    assert (oc[0] == want).all()
+
+
+def test_expired_wait_is_reported_to_its_own_group():
+    import s2kit_gb300 as s2
+    lib, bws = s2.load(), [77, 77, 32]
+    group, other = api.Group(bws), api.Group(bws)
+    grid = _cuda(group.grid_total, dtype="float32")
+    oc = [_cuda(group.coeff_total, dtype="float32") for _ in range(2)]
+    _expire(lib, lambda: group.fst(grid, oc[0], oc[1]))
+    assert lib.s2g_group_sync_status(other.h) == 0
+    assert lib.s2g_group_sync_status(group.h) == 5
+    assert lib.s2g_group_sync_status(group.h) == 0
+
+
+def test_expired_wait_is_reported_by_the_convolution_drop_in(capfd):
+    import s2kit_gb300 as s2
+    lib, bw = s2.load(), 48
+    a = np.random.default_rng(3).standard_normal((6, 4 * bw * bw))
+    api.ConvOn2SphereSemiMemo(*a, bw)
+    want = a[4].copy()
+    assert capfd.readouterr().err == ""
+    _expire(lib, lambda: api.ConvOn2SphereSemiMemo(*a, bw))
+    assert "ConvOn2SphereSemiMemo failed (5)" in capfd.readouterr().err
+    api.ConvOn2SphereSemiMemo(*a, bw)
+    assert capfd.readouterr().err == "" and (a[4] == want).all()
