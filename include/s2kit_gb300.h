@@ -357,10 +357,11 @@ int s2g_set_contraction_kernel(int which);
  * device word, frees its tensor memory and returns.  No fault, trap or hang is involved, and the
  * context stays usable: s2g_plan_sync_status reports the timeout and clears it. */
 int s2g_test_stall_contraction(int on);
-/* The same for the digit-product kernels (the FP64 transforms of plans, convolutions, and the FP32 transforms at
- * chirp-z bandwidths): with on != 0 no table is copied, so that every wait runs out, and the kernels report it in the
- * word of the plan, group or drop-in call that launched them. */
-int s2g_test_stall_digits(int on);
+/* Test hook for the digit-product kernels (the FP64 transforms of plans, convolutions, and the FP32 transforms at
+ * chirp-z bandwidths), process-wide, 0 = off.  1: no table is copied, so that every wait runs out as above; the kernels
+ * report it in the word of the plan, group or drop-in call that launched them.  2: as if their tables, 3: as if their
+ * scratch did not fit in device memory, so that the kernels which then run can be tested. */
+int s2g_test_digits(int what);
 
 /* Kernel timing: while enabled, every kernel the library launches is bracketed by CUDA
  * events on the stream it is launched on.  s2g_prof_enable() also discards earlier records.

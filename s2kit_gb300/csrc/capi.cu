@@ -468,10 +468,17 @@ static int conv_device(Tables* t, const double* dr, const double* di, const doub
     const bool fly = (t->cutoff == 0);
     const int bw = t->bw;
     const size_t nc = (size_t)bw * bw;
-    const size_t work = fly ? f64_work_bytes(bw, batch, REAL) : f64_plan_bytes(bw, batch, REAL, di || ri);
-    if (!fly) S2G_TRY(dg_prepare(t, st));
-    const size_t need = 4 * rnd(nc * batch) + 2 * rnd(2 * (size_t)bw * batch) + work + 256;
-    S2G_TRY(scr.ensure(need));
+    const size_t coeffs = 4 * rnd(nc * batch) + 2 * rnd(2 * (size_t)bw * batch) + 256;
+    size_t work = f64_work_bytes(bw, batch, REAL);  // the filter's analysis
+    bool digits = false;
+    if (!fly) S2G_TRY(dg_prepare(t, st, &digits));
+    if (digits) {
+        const size_t most = std::max(work, dg_work_bytes(bw, batch, di || ri));
+        S2G_TRY(dg_scratch(scr, coeffs + most, st, &digits));
+        if (digits) work = most;
+    }
+    if (!digits) S2G_TRY(scr.ensure(coeffs + work));
+    int* dg = digits ? err : nullptr;
     Carve c{(char*)scr.ptr};
     double *cr = c.take(nc * batch), *ci = c.take(nc * batch), *tr = c.take(nc * batch), *ti = c.take(nc * batch);
     double *hr = c.take(2 * (size_t)bw * batch), *hi = c.take(2 * (size_t)bw * batch);
@@ -480,14 +487,14 @@ static int conv_device(Tables* t, const double* dr, const double* di, const doub
         S2G_TRY(fst_f64_fly(t, dr, di, cr, ci, batch, REAL, w, st));
         S2G_TRY(fzt_f64_fly(t, fr, fi, hr, hi, batch, REAL, w, st));
     } else {
-        S2G_TRY(fst_f64(t, dr, di, cr, ci, batch, REAL, bw, w, st, err));
+        S2G_TRY(fst_f64(t, dr, di, cr, ci, batch, REAL, bw, w, st, dg));
         S2G_TRY(fzt_f64(t, fr, fi, hr, hi, batch, REAL, w, st));
     }
     S2G_TRY(transmult_f64(cr, ci, hr, hi, tr, ti, bw, batch, st));
     if (fly)
         S2G_TRY(inv_fst_f64_fly(t, tr, ti, rr, ri, batch, REAL, w, st));
     else
-        S2G_TRY(inv_fst_f64(t, tr, ti, rr, ri, batch, REAL, bw, w, st, err));
+        S2G_TRY(inv_fst_f64(t, tr, ti, rr, ri, batch, REAL, bw, w, st, dg));
     return S2G_OK;
 }
 
@@ -1116,8 +1123,9 @@ int s2g_plan_destroy(s2g_plan p) {
 
 size_t s2g_plan_workspace_size(s2g_plan p, int batch, int precision) {
     if (!p || batch < 1) return 0;
-    if (precision == S2G_PREC_FP64) return f64_plan_bytes(p->bw, batch, COMPLEX, true) + 256;
-    return split_work_bytes(p->bw, batch);
+    if (precision == S2G_PREC_FP64)
+        return std::max(f64_work_bytes(p->bw, batch, COMPLEX), dg_takes(p->bw) ? dg_work_bytes(p->bw, batch, true) : 0) + 256;
+    return std::max(split_work_bytes(p->bw, batch), dg32_takes(p->bw) ? dg32_work_bytes(p->bw, batch, false) : 0);
 }
 
 // Device-buffer calls share the plan's scratch with the host-buffer pipeline, so they first wait
@@ -1136,40 +1144,51 @@ static int plan_check(s2g_plan p, int batch, bool host = false, bool fly_ok = fa
     return S2G_OK;
 }
 
-// Scratch of an FP64 transform, and whether it takes the digit path (whose tables it readies).
-static int f64_scratch(s2g_plan p, int batch, DataFormat fmt, bool imag, cudaStream_t st, bool* digits) {
+// Scratch of an FP64 transform, and whether it takes the digit path (whose tables it readies): *dg is the plan's
+// error word there, else null.
+static int f64_scratch(s2g_plan p, int batch, DataFormat fmt, bool imag, cudaStream_t st, int** dg) {
     const bool two = imag || fmt == COMPLEX;
-    if (!p->fly) {
-        S2G_TRY(dg_prepare(p->t, st));
-        *digits = p->t->dg != nullptr;
-        return p->work.ensure(f64_plan_bytes(p->bw, batch, fmt, two));
-    }
-    if (dg_fly_takes(p->bw, two ? 2 * batch : batch)) S2G_TRY(dg_prepare(p->t, st));
-    *digits = p->t->dg && dg_fly_takes(p->bw, two ? 2 * batch : batch);
-    return p->work.ensure(*digits ? dg_fly_bytes(p->t, batch, two) : f64_work_bytes(p->bw, batch, fmt));
+    bool yes = false;
+    *dg = nullptr;
+    if (!p->fly || dg_fly_takes(p->bw, two ? 2 * batch : batch)) S2G_TRY(dg_prepare(p->t, st, &yes));
+    if (yes) S2G_TRY(dg_scratch(p->work, p->fly ? dg_fly_bytes(p->t, batch, two) : dg_work_bytes(p->bw, batch, two), st, &yes));
+    if (yes) return *dg = p->err, S2G_OK;
+    return p->work.ensure(f64_work_bytes(p->bw, batch, fmt));
+}
+
+// The same for FP32 transforms, COMPLEX ones with the second field's scratch.
+static int split_scratch(s2g_plan p, int batch, int precision, bool complex, cudaStream_t st, int** dg) {
+    bool yes = false;
+    *dg = nullptr;
+    S2G_TRY(split_check(p->t, precision));
+    S2G_TRY(dg32_prepare(p->t, st, &yes));
+    if (yes) S2G_TRY(dg_scratch(p->work, dg32_work_bytes(p->bw, batch, complex), st, &yes));
+    if (yes) return *dg = p->err, S2G_OK;
+    S2G_TRY(p->work.ensure(split_work_bytes(p->bw, batch)));
+    return complex ? p->cx.ensure(split_complex_bytes(p->bw, batch)) : S2G_OK;
 }
 
 int s2g_fst(s2g_plan p, const double* rdata, const double* idata, double* rcoeffs, double* icoeffs, int batch,
             DataFormat fmt, void* stream) {
     S2G_TRY(plan_check(p, batch, false, true));
     if (!rdata || !rcoeffs || !icoeffs || (fmt == COMPLEX && !idata)) return fail(S2G_ERR_ARG, "NULL argument");
-    bool digits = false;
-    S2G_TRY(f64_scratch(p, batch, fmt, idata != nullptr, (cudaStream_t)stream, &digits));
-    if (p->fly && !digits)
+    int* dg;
+    S2G_TRY(f64_scratch(p, batch, fmt, idata != nullptr, (cudaStream_t)stream, &dg));
+    if (p->fly && !dg)
         return fst_f64_fly(p->t, rdata, idata, rcoeffs, icoeffs, batch, fmt, p->work.ptr, (cudaStream_t)stream);
-    return fst_f64(p->t, rdata, idata, rcoeffs, icoeffs, batch, fmt, p->cutoff, p->work.ptr, (cudaStream_t)stream, p->err);
+    return fst_f64(p->t, rdata, idata, rcoeffs, icoeffs, batch, fmt, p->cutoff, p->work.ptr, (cudaStream_t)stream, dg);
 }
 
 int s2g_inv_fst(s2g_plan p, const double* rcoeffs, const double* icoeffs, double* rdata, double* idata, int batch,
                 DataFormat fmt, void* stream) {
     S2G_TRY(plan_check(p, batch, false, true));
     if (!rdata || !rcoeffs || !icoeffs || (fmt == COMPLEX && !idata)) return fail(S2G_ERR_ARG, "NULL argument");
-    bool digits = false;
-    S2G_TRY(f64_scratch(p, batch, fmt, idata != nullptr, (cudaStream_t)stream, &digits));
-    if (p->fly && !digits)
+    int* dg;
+    S2G_TRY(f64_scratch(p, batch, fmt, idata != nullptr, (cudaStream_t)stream, &dg));
+    if (p->fly && !dg)
         return inv_fst_f64_fly(p->t, rcoeffs, icoeffs, rdata, idata, batch, fmt, p->work.ptr, (cudaStream_t)stream);
     return inv_fst_f64(p->t, rcoeffs, icoeffs, rdata, idata, batch, fmt, p->cutoff, p->work.ptr,
-                       (cudaStream_t)stream, p->err);
+                       (cudaStream_t)stream, dg);
 }
 
 int s2g_fzt(s2g_plan p, const double* rdata, const double* idata, double* rres, double* ires, int batch,
@@ -1199,8 +1218,9 @@ int s2g_fst_real_f32(s2g_plan p, const float* grid, float* rc, float* ic, int ba
     S2G_TRY(plan_check(p, batch));
     if (!grid || !rc || !ic) return fail(S2G_ERR_ARG, "NULL argument");
     S2G_TRY(check_aligned16({grid, rc, ic}));
-    S2G_TRY(p->work.ensure(split_work_bytes(p->bw, batch)));
-    return fst_split(p->t, grid, rc, ic, batch, precision, p->work.ptr, (cudaStream_t)stream, p->err);
+    int* dg;
+    S2G_TRY(split_scratch(p, batch, precision, false, (cudaStream_t)stream, &dg));
+    return fst_split(p->t, grid, rc, ic, batch, precision, p->work.ptr, (cudaStream_t)stream, dg);
 }
 
 int s2g_inv_fst_real_f32(s2g_plan p, const float* rc, const float* ic, float* grid, int batch, int precision,
@@ -1208,8 +1228,9 @@ int s2g_inv_fst_real_f32(s2g_plan p, const float* rc, const float* ic, float* gr
     S2G_TRY(plan_check(p, batch));
     if (!grid || !rc || !ic) return fail(S2G_ERR_ARG, "NULL argument");
     S2G_TRY(check_aligned16({grid, rc, ic}));
-    S2G_TRY(p->work.ensure(split_work_bytes(p->bw, batch)));
-    return inv_fst_split(p->t, rc, ic, grid, batch, precision, p->work.ptr, (cudaStream_t)stream, p->err);
+    int* dg;
+    S2G_TRY(split_scratch(p, batch, precision, false, (cudaStream_t)stream, &dg));
+    return inv_fst_split(p->t, rc, ic, grid, batch, precision, p->work.ptr, (cudaStream_t)stream, dg);
 }
 
 int s2g_fst_complex_f32(s2g_plan p, const float* rgrid, const float* igrid, float* rc, float* ic, int batch,
@@ -1217,10 +1238,10 @@ int s2g_fst_complex_f32(s2g_plan p, const float* rgrid, const float* igrid, floa
     S2G_TRY(plan_check(p, batch));
     if (!rgrid || !igrid || !rc || !ic) return fail(S2G_ERR_ARG, "NULL argument");
     S2G_TRY(check_aligned16({rgrid, igrid, rc, ic}));
-    S2G_TRY(p->work.ensure(split_complex_work_bytes(p->bw, batch)));
-    S2G_TRY(p->cx.ensure(split_complex_bytes(p->bw, batch)));
+    int* dg;
+    S2G_TRY(split_scratch(p, batch, precision, true, (cudaStream_t)stream, &dg));
     return fst_split_complex(p->t, rgrid, igrid, rc, ic, batch, precision, p->work.ptr, p->cx.ptr,
-                             (cudaStream_t)stream, p->err);
+                             (cudaStream_t)stream, dg);
 }
 
 int s2g_inv_fst_complex_f32(s2g_plan p, const float* rc, const float* ic, float* rgrid, float* igrid, int batch,
@@ -1228,17 +1249,22 @@ int s2g_inv_fst_complex_f32(s2g_plan p, const float* rc, const float* ic, float*
     S2G_TRY(plan_check(p, batch));
     if (!rgrid || !igrid || !rc || !ic) return fail(S2G_ERR_ARG, "NULL argument");
     S2G_TRY(check_aligned16({rgrid, igrid, rc, ic}));
-    S2G_TRY(p->work.ensure(split_complex_work_bytes(p->bw, batch)));
-    S2G_TRY(p->cx.ensure(split_complex_bytes(p->bw, batch)));
+    int* dg;
+    S2G_TRY(split_scratch(p, batch, precision, true, (cudaStream_t)stream, &dg));
     return inv_fst_split_complex(p->t, rc, ic, rgrid, igrid, batch, precision, p->work.ptr, p->cx.ptr,
-                                 (cudaStream_t)stream, p->err);
+                                 (cudaStream_t)stream, dg);
 }
 
-static int refined_scratch(s2g_plan p, int batch, int precision, cudaStream_t st, bool* direct) {
+// *direct: the refined transforms run as FP64 transforms (on the digit path with *dg, else on the FP64 kernels, at
+// the bandwidths that never take it).
+static int refined_scratch(s2g_plan p, int batch, int precision, cudaStream_t st, int** dg, bool* direct) {
     S2G_TRY(split_check(p->t, precision));
-    S2G_TRY(dg_prepare(p->t, st));
-    *direct = refine_direct(p->t);
-    if (*direct) return p->work.ensure(f64_plan_bytes(p->bw, batch, REAL, false));
+    *dg = nullptr;
+    *direct = !dg_takes(p->bw);
+    if (*direct) return p->work.ensure(f64_work_bytes(p->bw, batch, REAL));
+    S2G_TRY(dg_prepare(p->t, st, direct));
+    if (*direct) S2G_TRY(dg_scratch(p->work, dg_work_bytes(p->bw, batch, false), st, direct));
+    if (*direct) return *dg = p->err, S2G_OK;
     S2G_TRY(p->work.ensure(refine_work_bytes(p->bw, batch)));
     return p->io.ensure(refine_io_bytes(p->bw, batch));
 }
@@ -1248,11 +1274,12 @@ int s2g_fst_refined(s2g_plan p, const double* grid, double* rc, double* ic, int 
     S2G_TRY(plan_check(p, batch));
     if (!grid || !rc || !ic) return fail(S2G_ERR_ARG, "NULL argument");
     S2G_TRY(check_aligned16({grid, rc, ic}));
-    bool direct = false;
-    S2G_TRY(refined_scratch(p, batch, precision, (cudaStream_t)stream, &direct));
+    int* dg;
+    bool direct;
+    S2G_TRY(refined_scratch(p, batch, precision, (cudaStream_t)stream, &dg, &direct));
     if (direct)
-        return fst_f64(p->t, grid, nullptr, rc, ic, batch, REAL, p->cutoff, p->work.ptr, (cudaStream_t)stream, p->err);
-    return fst_refined(p->t, grid, rc, ic, batch, precision, p->io.ptr, p->work.ptr, (cudaStream_t)stream, p->err);
+        return fst_f64(p->t, grid, nullptr, rc, ic, batch, REAL, p->cutoff, p->work.ptr, (cudaStream_t)stream, dg);
+    return fst_refined(p->t, grid, rc, ic, batch, precision, p->io.ptr, p->work.ptr, (cudaStream_t)stream);
 }
 
 int s2g_inv_fst_refined(s2g_plan p, const double* rc, const double* ic, double* grid, int batch, int precision,
@@ -1260,11 +1287,12 @@ int s2g_inv_fst_refined(s2g_plan p, const double* rc, const double* ic, double* 
     S2G_TRY(plan_check(p, batch));
     if (!grid || !rc || !ic) return fail(S2G_ERR_ARG, "NULL argument");
     S2G_TRY(check_aligned16({grid, rc, ic}));
-    bool direct = false;
-    S2G_TRY(refined_scratch(p, batch, precision, (cudaStream_t)stream, &direct));
+    int* dg;
+    bool direct;
+    S2G_TRY(refined_scratch(p, batch, precision, (cudaStream_t)stream, &dg, &direct));
     if (direct)
-        return inv_fst_f64(p->t, rc, ic, grid, nullptr, batch, REAL, p->cutoff, p->work.ptr, (cudaStream_t)stream, p->err);
-    return inv_fst_refined(p->t, rc, ic, grid, batch, precision, p->io.ptr, p->work.ptr, (cudaStream_t)stream, p->err);
+        return inv_fst_f64(p->t, rc, ic, grid, nullptr, batch, REAL, p->cutoff, p->work.ptr, (cudaStream_t)stream, dg);
+    return inv_fst_refined(p->t, rc, ic, grid, batch, precision, p->io.ptr, p->work.ptr, (cudaStream_t)stream);
 }
 
 int s2g_plan_sync_status(s2g_plan p) {
@@ -1294,12 +1322,14 @@ static int host_pipeline(s2g_plan p, int fwd, const float* in0, const float* in1
     while (chunk > 1 && (size_t)chunk * (in_per + out_per) * 4 * 2 > ((size_t)4 << 30)) chunk /= 2;
     // one staging layout for both directions, so queued chunks of an earlier call keep their buffers
     const size_t stage = (size_t)chunk * std::max(ng, 2 * nc) * 4;
-    if (stage != p->stage || p->io.bytes < 4 * stage + 1024 || p->work.bytes < split_work_bytes(p->bw, chunk)) {
+    const size_t most = std::max(split_work_bytes(p->bw, chunk), dg32_takes(p->bw) ? dg32_work_bytes(p->bw, chunk, false) : 0);
+    if (stage != p->stage || p->io.bytes < 4 * stage + 1024 || p->work.bytes < most) {
         S2G_TRY(drain_host(p));  // a new layout or a larger buffer: nothing queued may still use the old one
         S2G_TRY(p->io.ensure(4 * stage + 1024));
-        S2G_TRY(p->work.ensure(split_work_bytes(p->bw, chunk)));
         p->stage = stage;
     }
+    int* dg;
+    S2G_TRY(split_scratch(p, chunk, precision, false, p->streams[1], &dg));
     prune_deps(p);
     if (p->deps.size() > 4096) S2G_TRY(drain_host(p));
     char* base = (char*)p->io.ptr;
@@ -1336,9 +1366,9 @@ static int host_pipeline(s2g_plan p, int fwd, const float* in0, const float* in1
         S2G_CUDA(cudaStreamWaitEvent(comp, in_ready[b], 0));
         S2G_CUDA(cudaStreamWaitEvent(comp, out_free[b], 0));  // the download that last read dout[b]
         if (fwd)
-            S2G_TRY(fst_split(p->t, din[b], dout[b], dout[b] + (size_t)n * nc, n, precision, p->work.ptr, comp, p->err));
+            S2G_TRY(fst_split(p->t, din[b], dout[b], dout[b] + (size_t)n * nc, n, precision, p->work.ptr, comp, dg));
         else
-            S2G_TRY(inv_fst_split(p->t, din[b], din[b] + (size_t)n * nc, dout[b], n, precision, p->work.ptr, comp, p->err));
+            S2G_TRY(inv_fst_split(p->t, din[b], din[b] + (size_t)n * nc, dout[b], n, precision, p->work.ptr, comp, dg));
         S2G_CUDA(cudaEventRecord(done[b], comp));
         S2G_CUDA(cudaStreamWaitEvent(d2h, done[b], 0));
         if (fwd) {

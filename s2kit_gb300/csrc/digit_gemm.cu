@@ -1432,7 +1432,10 @@ struct DgTabs {
 };
 
 static std::mutex g_dg_mu;
-static std::atomic<int> g_dg_stall{0};  // see s2g_test_stall_digits
+static std::atomic<int> g_dg_test{0};  // see s2g_test_digits
+enum { kDgStall = 1, kDgNoTables = 2, kDgNoScratch = 3 };
+static int dg_test() { return g_dg_test.load(std::memory_order_relaxed); }
+constexpr int kDgSkip = 63;  // calls that do not try again what did not fit
 static std::map<std::tuple<int, int, int, bool, int>, DgTabs*> g_dg;  // device, bw, prec, fly, semi
 
 static void dg_free(DgTabs* d) {
@@ -1826,7 +1829,7 @@ static int dg_columns(const DgTabs* d, const DgArgs& p, int sms) {
 template <int STAGE>
 static int launch_dg_tiles(const DgTabs* d, DgArgs p, cudaStream_t st) {
     p.col_major = STAGE == kF1 || STAGE == kI2;
-    p.stall = g_dg_stall.load(std::memory_order_relaxed);
+    p.stall = dg_test() == kDgStall;
     int dev = 0, sms = 0;
     S2G_CUDA(cudaGetDevice(&dev));
     S2G_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -1925,35 +1928,73 @@ bool dg_takes(int bw) { return bw <= 1024 && (bw >= 32 || (bw > 8 && (bw & (bw -
 
 bool dg_fly_takes(int bw, int fields) { return dg_takes(bw) && bw >= 64 && fields >= (bw > 512 ? 4 : 2); }
 
-// Builds (or finds) the digit tables of t's bandwidth.  Where the stream is being captured, or they do
-// not fit in device memory, t stays without them and the FP64 kernels run.
-static int prepare(Tables* t, int prec, void** slot, bool* off, cudaStream_t st) {
-    if (__atomic_load_n(slot, __ATOMIC_ACQUIRE) || *off) return S2G_OK;
+static bool capturing(cudaStream_t st) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
-        cudaGetLastError();
-        return S2G_OK;
+    if (cudaStreamIsCapturing(st, &cs) == cudaSuccess) return cs != cudaStreamCaptureStatusNone;
+    cudaGetLastError();  // the legacy stream, while another is captured
+    return true;
+}
+
+// Builds (or finds) the digit tables of t's bandwidth; *yes where they are there.  Where the stream is being
+// captured, or they do not fit in device memory, t stays without them and the other kernels run; what did not
+// fit is tried again by every 64th call that asks (an attempt costs the allocations before the one that fails).
+static int prepare(Tables* t, int prec, void** slot, int* skip, cudaStream_t st, bool* yes) {
+    *yes = false;
+    if (dg_test() == kDgNoTables) return S2G_OK;
+    if (!__atomic_load_n(slot, __ATOMIC_ACQUIRE)) {
+        if (__atomic_load_n(skip, __ATOMIC_RELAXED) > 0) {
+            __atomic_fetch_sub(skip, 1, __ATOMIC_RELAXED);
+            return S2G_OK;
+        }
+        if (capturing(st)) return S2G_OK;
+        DgTabs* d;
+        const bool fly = t->cutoff == 0;
+        const int r = dg_get(t->bw, prec, fly, dg_semi_orders(t->bw, t->cutoff, prec, fly), t->weights, &d);
+        if (r == S2G_ERR_NOMEM) {
+            cudaGetLastError();
+            __atomic_store_n(skip, kDgSkip, __ATOMIC_RELAXED);
+            return S2G_OK;
+        }
+        if (r != S2G_OK) return r;
+        void* none = nullptr;
+        if (!__atomic_compare_exchange_n(slot, &none, (void*)d, false, __ATOMIC_ACQ_REL, __ATOMIC_ACQUIRE)) dg_put(d);
     }
-    DgTabs* d;
-    const bool fly = t->cutoff == 0;
-    const int r = dg_get(t->bw, prec, fly, dg_semi_orders(t->bw, t->cutoff, prec, fly), t->weights, &d);
-    if (r == S2G_ERR_NOMEM) {
-        cudaGetLastError();
-        *off = true;
-        return S2G_OK;
-    }
-    if (r != S2G_OK) return r;
-    void* none = nullptr;
-    if (!__atomic_compare_exchange_n(slot, &none, (void*)d, false, __ATOMIC_ACQ_REL, __ATOMIC_ACQUIRE)) dg_put(d);
+    *yes = true;
     return S2G_OK;
 }
-int dg_prepare(Tables* t, cudaStream_t st) { return dg_takes(t->bw) ? prepare(t, 64, &t->dg, &t->dg_off, st) : S2G_OK; }
+int dg_prepare(Tables* t, cudaStream_t st, bool* yes) {
+    *yes = false;
+    return dg_takes(t->bw) ? prepare(t, 64, &t->dg, &t->dg_skip, st, yes) : S2G_OK;
+}
 // Bandwidths whose FP32 transforms take the digit path: chirp-z ones, where its matrix products beat the two
 // FFTs of each chirp-z stage (forward 1.1 to 1.6 times as fast over bw 65 .. 255 and batches of 1 to 1024,
 // inverse 1.1 to 1.8; bw 255, 256 functions: 798 us against 880 and 703 against 912).  Below 64 they do not for large batches (bw 33, 4096 functions: 498 us against
 // 452), nor where a warp FFT takes the length (bw 256, 64 functions: 187 us against 96).
 bool dg32_takes(int bw) { return bw >= 64 && split_czt(bw); }
-int dg32_prepare(Tables* t, cudaStream_t st) { return prepare(t, 32, &t->dg32, &t->dg32_off, st); }
+int dg32_prepare(Tables* t, cudaStream_t st, bool* yes) {
+    *yes = false;
+    return dg32_takes(t->bw) ? prepare(t, 32, &t->dg32, &t->dg32_skip, st, yes) : S2G_OK;
+}
+
+bool dg_no_scratch() { return dg_test() == kDgNoScratch; }
+int dg_scratch(Scratch& s, size_t need, cudaStream_t st, bool* yes) {
+    *yes = need <= s.bytes && !dg_no_scratch();
+    if (*yes || dg_no_scratch()) return S2G_OK;
+    if (need >= s.nofit && s.skip > 0) {
+        --s.skip;
+        return S2G_OK;
+    }
+    if (capturing(st)) return S2G_OK;
+    const int r = s.ensure(need);
+    if (r == S2G_ERR_NOMEM) {
+        cudaGetLastError();
+        s.nofit = need;
+        s.skip = kDgSkip;
+        return S2G_OK;
+    }
+    *yes = r == S2G_OK;
+    return r;
+}
 
 static int set_dyn_smem(const void* fn, size_t bytes) {
     S2G_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
@@ -2092,7 +2133,8 @@ int dg_expired(int code) { return fail(code, "a bounded wait in the digit-produc
 
 }  // namespace s2g
 
-extern "C" int s2g_test_stall_digits(int on) {
-    s2g::g_dg_stall = on ? 1 : 0;
+extern "C" int s2g_test_digits(int what) {
+    if (what < 0 || what > s2g::kDgNoScratch) return s2g::fail(S2G_ERR_ARG, "s2g_test_digits(%d)", what);
+    s2g::g_dg_test = what;
     return S2G_OK;
 }

@@ -54,7 +54,8 @@ struct GroupClass {
     float* buf0 = nullptr;      // X (forward) / F (inverse): [2][N][B][SX]  (split_layout)
     float* buf1 = nullptr;      // C (forward) / Fc (inverse): [2][N][B][2 BH]
     bool small = false;         // transformed whole in the rows stage (small_takes): no intermediates
-    void* digits = nullptr;     // scratch of the digit path (digit_gemm.cu), for the classes that take it
+    bool dg = false;            // takes the digit path (digit_gemm.cu)
+    void* digits = nullptr;     // its scratch
 };
 
 struct GroupGraph {
@@ -504,22 +505,29 @@ int s2g_group_create(s2g_group* out, int nfunc, const int* bw, int precision) {
     for (auto& c : g->cls) {
         if (r == S2G_OK) r = get_tables(c.B, c.B, &c.t);
         else c.t = nullptr;
-        if (r == S2G_OK && dg32_takes(c.B)) r = dg32_prepare(c.t, 0);
+        if (r == S2G_OK) r = dg32_prepare(c.t, 0, &c.dg);
         c.small = small_takes(c.B);
     }
-    auto digits = [](const GroupClass& c) { return dg32_takes(c.B) && c.t && c.t->dg32; };
     // device memory: maps, intermediates (256-byte aligned pieces), two counters and the error word
     auto rnd = [](size_t x) { return (x + 255) & ~(size_t)255; };
-    size_t total = 256;
+    size_t total = 0;
     auto x_floats = [](const GroupClass& c) { return 2 * (size_t)c.N * c.B * split_layout(c.B).SX; };
     auto c_floats = [](const GroupClass& c) { return 2 * (size_t)c.N * c.B * 2 * split_layout(c.B).BH; };
-    for (auto& c : g->cls) {
-        total += 2 * rnd(sizeof(int64_t) * c.N);
-        total += digits(c) ? rnd(dg32_work_bytes(c.B, c.N, false))
-                           : rnd(sizeof(float) * x_floats(c)) + rnd(sizeof(float) * c_floats(c));
+    while (r == S2G_OK && !g->mem) {
+        bool any = false;
+        total = 256;
+        for (auto& c : g->cls) {
+            any |= c.dg;
+            total += 2 * rnd(sizeof(int64_t) * c.N);
+            total += c.dg ? rnd(dg32_work_bytes(c.B, c.N, false))
+                          : rnd(sizeof(float) * x_floats(c)) + rnd(sizeof(float) * c_floats(c));
+        }
+        if (!(any && dg_no_scratch()) && cudaMalloc(&g->mem, total) == cudaSuccess) break;
+        g->mem = nullptr;
+        cudaGetLastError();
+        if (!any) r = fail(S2G_ERR_NOMEM, "group: cudaMalloc of %zu bytes failed", total);
+        for (auto& c : g->cls) c.dg = false;  // once more without the digit path's scratch
     }
-    if (r == S2G_OK && cudaMalloc(&g->mem, total) != cudaSuccess)
-        r = fail(S2G_ERR_NOMEM, "group: cudaMalloc of %zu bytes failed", total);
     if (r == S2G_OK) {
         char* p = (char*)g->mem;
         g->counters = (int*)p;
@@ -532,7 +540,7 @@ int s2g_group_create(s2g_group* out, int nfunc, const int* bw, int precision) {
             p += rnd(sizeof(int64_t) * c.N);
             c.cmap = (int64_t*)p;
             p += rnd(sizeof(int64_t) * c.N);
-            if (digits(c)) {
+            if (c.dg) {
                 c.digits = p;
                 p += rnd(dg32_work_bytes(c.B, c.N, false));
             } else {

@@ -3,10 +3,10 @@
 // The step was made when an FP64 transform cost many times a split one.  With the digit products it costs
 // less than the residual's FP64 transform and the two split ones together, and it is the more precise, so where
 // the digit tables are there (and at the bandwidths that never take them) the refined transforms are FP64
-// transforms (refine_direct): forward at bw 1024, 16 functions, 4.74 -> 2.97 ms with the coefficients'
+// transforms (refined_scratch, capi.cu): forward at bw 1024, 16 functions, 4.74 -> 2.97 ms with the coefficients'
 // error against 64 bits 8.0e-14 -> 5.2e-14, inverse 5.43 -> 2.65 ms and 1.5e-7 -> 5.1e-15; one function at bw
-// 16, on the FP64 kernels, 48 -> 18 us.  The step below serves the rest: a first call under capture, or tables
-// that did not fit (FP64 kernels, one function at bw 1024: forward 7.1 ms, refined 3.8).
+// 16, on the FP64 kernels, 48 -> 18 us.  The step below serves the rest: a first call under capture, or tables or
+// scratch that did not fit (FP64 kernels, one function at bw 1024: forward 7.1 ms, refined 3.8).
 //
 // Forward:  a1 = F_split(f);  r = f - I_fp64(a1);  a = a1 + F_split(r)
 // Inverse:  g1 = I_split(a);  r = a - F_fp64(g1);  g = g1 + I_split(r)
@@ -47,8 +47,6 @@ __global__ void k_accum(double* __restrict__ x, const float* __restrict__ d, siz
         x[i] += (double)d[i];
 }
 
-bool refine_direct(const Tables* t) { return t->dg || !dg_takes(t->bw); }
-
 static int ew_grid(size_t n) { return (int)std::min<size_t>((n + 255) / 256, 152 * 16); }
 
 #define S2G_EW(name, kern, n, st, ...)                                   \
@@ -67,14 +65,13 @@ size_t refine_io_bytes(int bw, int batch) {
 }
 
 size_t refine_work_bytes(int bw, int batch) {
-    return std::max(split_work_bytes(bw, batch), f64_plan_bytes(bw, batch, REAL, false) + 256);
+    return std::max(split_work_bytes(bw, batch), f64_work_bytes(bw, batch, REAL) + 256);
 }
 
 int fst_refined(Tables* t, const double* grid, double* rc, double* ic, int batch, int precision, void* io,
-                void* work, cudaStream_t st, int* dg) {
+                void* work, cudaStream_t st) {
     const int B = t->bw;
     const size_t ng = 4 * (size_t)B * B * batch, nc = (size_t)B * B * batch;
-    S2G_TRY(dg_prepare(t, st));
     char* p = (char*)io;
     float* g32 = (float*)p;
     p += rnd(4 * ng);
@@ -85,24 +82,23 @@ int fst_refined(Tables* t, const double* grid, double* rc, double* ic, int batch
     double* g64 = (double*)p;
     // a1 = F_split(f)
     S2G_EW("refine_d2f", k_d2f, ng, st, grid, g32);
-    S2G_TRY(fst_split(t, g32, c32r, c32i, batch, precision, work, st, dg));
+    S2G_TRY(fst_split(t, g32, c32r, c32i, batch, precision, work, st, nullptr));
     S2G_EW("refine_f2d", k_f2d, nc, st, c32r, rc);
     S2G_EW("refine_f2d", k_f2d, nc, st, c32i, ic);
     // r = f - I_fp64(a1)
-    S2G_TRY(inv_fst_f64(t, rc, ic, g64, nullptr, batch, REAL, t->cutoff, work, st, dg));
+    S2G_TRY(inv_fst_f64(t, rc, ic, g64, nullptr, batch, REAL, t->cutoff, work, st));
     S2G_EW("refine_resid", k_resid, ng, st, grid, g64, g32);
     // a = a1 + F_split(r)
-    S2G_TRY(fst_split(t, g32, c32r, c32i, batch, precision, work, st, dg));
+    S2G_TRY(fst_split(t, g32, c32r, c32i, batch, precision, work, st, nullptr));
     S2G_EW("refine_accum", k_accum, nc, st, rc, c32r);
     S2G_EW("refine_accum", k_accum, nc, st, ic, c32i);
     return S2G_OK;
 }
 
 int inv_fst_refined(Tables* t, const double* rc, const double* ic, double* grid, int batch, int precision, void* io,
-                    void* work, cudaStream_t st, int* dg) {
+                    void* work, cudaStream_t st) {
     const int B = t->bw;
     const size_t ng = 4 * (size_t)B * B * batch, nc = (size_t)B * B * batch;
-    S2G_TRY(dg_prepare(t, st));
     char* p = (char*)io;
     float* g32 = (float*)p;
     p += rnd(4 * ng);
@@ -115,14 +111,14 @@ int inv_fst_refined(Tables* t, const double* rc, const double* ic, double* grid,
     // g1 = I_split(a)
     S2G_EW("refine_d2f", k_d2f, nc, st, rc, c32r);
     S2G_EW("refine_d2f", k_d2f, nc, st, ic, c32i);
-    S2G_TRY(inv_fst_split(t, c32r, c32i, g32, batch, precision, work, st, dg));
+    S2G_TRY(inv_fst_split(t, c32r, c32i, g32, batch, precision, work, st, nullptr));
     S2G_EW("refine_f2d", k_f2d, ng, st, g32, grid);
     // r = a - F_fp64(g1)
-    S2G_TRY(fst_f64(t, grid, nullptr, a64r, a64i, batch, REAL, t->cutoff, work, st, dg));
+    S2G_TRY(fst_f64(t, grid, nullptr, a64r, a64i, batch, REAL, t->cutoff, work, st));
     S2G_EW("refine_resid", k_resid, nc, st, rc, a64r, c32r);
     S2G_EW("refine_resid", k_resid, nc, st, ic, a64i, c32i);
     // g = g1 + I_split(r)
-    S2G_TRY(inv_fst_split(t, c32r, c32i, g32, batch, precision, work, st, dg));
+    S2G_TRY(inv_fst_split(t, c32r, c32i, g32, batch, precision, work, st, nullptr));
     S2G_EW("refine_accum", k_accum, ng, st, grid, g32);
     return S2G_OK;
 }

@@ -61,9 +61,9 @@ struct Tables {
     void* split = nullptr;
     // digit tables of the tensor-core FP64 path (digit_gemm.cu), built on first use
     void* dg = nullptr;
-    bool dg_off = false;        // they did not fit in device memory
+    int dg_skip = 0;            // they did not fit in device memory: calls left before the next attempt
     void* dg32 = nullptr;       // the same for FP32 transforms
-    bool dg32_off = false;
+    int dg32_skip = 0;
     int refs = 0;               // references (cache, plans, groups, calls in flight); under the cache lock
 };
 
@@ -71,6 +71,8 @@ struct Tables {
 struct Scratch {
     void* ptr = nullptr;
     size_t bytes = 0;
+    size_t nofit = 0;  // dg_scratch: what did not fit, and the calls left before the next attempt
+    int skip = 0;
     int ensure(size_t need);
     void release();
 };
@@ -112,19 +114,22 @@ struct F64Work {
     int rows;    // rows per function in X (bw for REAL, 2bw for COMPLEX)
 };
 size_t f64_work_bytes(int bw, int batch, int data_format);
-// The same for calls that may take the digit path (dg_prepare); two: the data have imaginary parts.
-size_t f64_plan_bytes(int bw, int batch, int data_format, bool two);
 // ---- FP64 transforms as exact digit products on the tensor cores (digit_gemm.cu) ----
 // Their kernels' waits are bounded; `err` is the word of the plan, group or call that gets S2G_ERR_TIMEOUT
 // where one expired (device memory, or the host's where host_direct).  The functions further down that may take
-// this path take the word as `dg`: null keeps them off it.
+// this path take the word as `dg`: with it they run there, on tables and scratch that the caller has readied
+// (dg_prepare, dg_scratch); null keeps them off it.
 bool dg_takes(int bw);
-size_t dg_work_bytes(int bw, int batch, bool two);
+size_t dg_work_bytes(int bw, int batch, bool two);  // two: the data have imaginary parts
+// Grows s to `need` bytes for the digit path; *yes false where that does not fit, or cannot be done under capture (as
+// dg_prepare for the tables), and the caller takes the other kernels, whose scratch may fit or be there.
+int dg_scratch(Scratch& s, size_t need, cudaStream_t st, bool* yes);
+bool dg_no_scratch();  // the test hook's
 // FP32 samples and coefficients (igrid null: real fields); readied by dg32_prepare into t->dg32.
 // gmap, cmap: per-function grid and coefficient offsets (real fields), null for functions back to back.
 bool dg32_takes(int bw);
 size_t dg32_work_bytes(int bw, int batch, bool two);
-int dg32_prepare(Tables* t, cudaStream_t st);
+int dg32_prepare(Tables* t, cudaStream_t st, bool* yes);
 int fst_dg32(const Tables* t, const float* rgrid, const float* igrid, float* rc, float* ic, int batch, void* work,
              cudaStream_t st, int* err, const int64_t* gmap = nullptr, const int64_t* cmap = nullptr);
 int inv_fst_dg32(const Tables* t, const float* rc, const float* ic, float* rgrid, float* igrid, int batch, void* work,
@@ -132,7 +137,7 @@ int inv_fst_dg32(const Tables* t, const float* rc, const float* ic, float* rgrid
 // On-the-fly family (tables of cutoff 0): real fields for which it pays, and the scratch once prepared.
 bool dg_fly_takes(int bw, int fields);
 size_t dg_fly_bytes(const Tables* t, int batch, bool two);
-int dg_prepare(Tables* t, cudaStream_t st);
+int dg_prepare(Tables* t, cudaStream_t st, bool* yes);
 void dg_put(void* dg);
 int dg_status(int* err);    // reads the (device) word and clears it
 int dg_expired(int code);  // records the failure
@@ -211,13 +216,12 @@ int czt_build_tables(int bw, float2** d_h, float2** d_K, float2** d_tw);
 // functions at a chirp-z bandwidth; in/out, scale and gmap as the warp-FFT stages.
 int czt_stage(int which, const CztTabs& g, const void* in, void* out, int N, float scale, const int64_t* gmap,
               cudaStream_t st);
-size_t split_work_bytes(int bw, int batch);
-size_t split_complex_work_bytes(int bw, int batch);
+size_t split_work_bytes(int bw, int batch);  // off the digit path
 int fst_split(Tables* t, const float* grid, float* rc, float* ic, int batch, int precision, void* work,
               cudaStream_t st, int* dg);
 int inv_fst_split(Tables* t, const float* rc, const float* ic, float* grid, int batch, int precision, void* work,
                   cudaStream_t st, int* dg);
-// COMPLEX data as two real fields (cwork: split_complex_bytes of scratch besides work).
+// COMPLEX data as two real fields (cwork: split_complex_bytes of scratch besides work, off the digit path).
 size_t split_complex_bytes(int bw, int batch);
 int fst_split_complex(Tables* t, const float* rgrid, const float* igrid, float* rc, float* ic, int batch,
                       int precision, void* work, void* cwork, cudaStream_t st, int* dg);
@@ -280,13 +284,11 @@ int split_inv_tail(Tables* t, float* F, float* Fc, float* grid, int batch, const
 int split_check(const Tables* t, int precision);
 
 // ---- split transforms with one FP64-residual refinement step (refine.cu) ----
-// Whether the refined transforms run as FP64 transforms instead (dg_prepare called before).
-bool refine_direct(const Tables* t);
 size_t refine_io_bytes(int bw, int batch);
 size_t refine_work_bytes(int bw, int batch);
 int fst_refined(Tables* t, const double* grid, double* rc, double* ic, int batch, int precision, void* io,
-                void* work, cudaStream_t st, int* dg);
+                void* work, cudaStream_t st);
 int inv_fst_refined(Tables* t, const double* rc, const double* ic, double* grid, int batch, int precision, void* io,
-                    void* work, cudaStream_t st, int* dg);
+                    void* work, cudaStream_t st);
 
 }  // namespace s2g

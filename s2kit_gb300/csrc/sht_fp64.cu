@@ -712,14 +712,9 @@ size_t f64_work_bytes(int bw, int batch, int data_format) {
     return 2 * (size_t)batch * rows * S * sizeof(double);
 }
 
-size_t f64_plan_bytes(int bw, int batch, int data_format, bool two) {
-    const size_t plain = f64_work_bytes(bw, batch, data_format);
-    return dg_takes(bw) ? std::max(plain, dg_work_bytes(bw, batch, two || data_format == COMPLEX)) : plain;
-}
-
 int fst_f64(const Tables* t, const double* rdata, const double* idata, double* rc, double* ic, int batch,
             int data_format, int cutoff, void* work, cudaStream_t st, int* dg) {
-    if (dg && t->dg) return fst_f64_dg(t, rdata, idata, rc, ic, batch, data_format, work, st, dg);
+    if (dg) return fst_f64_dg(t, rdata, idata, rc, ic, batch, data_format, work, st, dg);
     return fst_f64_len(t, nullptr, rdata, idata, rc, ic, batch, data_format, cutoff, work, st);
 }
 
@@ -754,7 +749,7 @@ int fst_f64_len(const Tables* t, const Len* len_S, const double* rdata, const do
 
 int inv_fst_f64(const Tables* t, const double* rc, const double* ic, double* rdata, double* idata, int batch,
                 int data_format, int cutoff, void* work, cudaStream_t st, int* dg) {
-    if (dg && t->dg) return inv_fst_f64_dg(t, rc, ic, rdata, idata, batch, data_format, work, st, dg);
+    if (dg) return inv_fst_f64_dg(t, rc, ic, rdata, idata, batch, data_format, work, st, dg);
     const int B = t->bw, S = 2 * B;
     const int rows = (data_format == COMPLEX) ? S : B;
     double* Fr = (double*)work;

@@ -2237,23 +2237,7 @@ __global__ void __launch_bounds__(kWsThreads, 1)
 // ------------------------------------------------------------------------------------
 size_t split_work_bytes(int bw, int batch) {
     const SplitLayout L = split_layout(bw);
-    const size_t n = 2 * (size_t)batch * bw * ((size_t)L.SX + 2 * (size_t)L.BH) * sizeof(float) + 1024;
-    return dg32_takes(bw) ? std::max(n, dg32_work_bytes(bw, batch, false)) : n;
-}
-
-size_t split_complex_work_bytes(int bw, int batch) {
-    return dg32_takes(bw) ? std::max(split_work_bytes(bw, batch), dg32_work_bytes(bw, batch, true))
-                          : split_work_bytes(bw, batch);
-}
-
-// Readies the digit path where the bandwidth takes it: *yes when its tables are there (they may not be
-// under capture or out of memory; the FFT stages and the split contraction then run).
-static int use_dg32(Tables* t, cudaStream_t st, bool* yes) {
-    *yes = false;
-    if (!dg32_takes(t->bw)) return S2G_OK;
-    S2G_TRY(dg32_prepare(t, st));
-    *yes = t->dg32 != nullptr;
-    return S2G_OK;
+    return 2 * (size_t)batch * bw * ((size_t)L.SX + 2 * (size_t)L.BH) * sizeof(float) + 1024;
 }
 
 static int set_smem(const void* fn, size_t bytes) {
@@ -2744,13 +2728,11 @@ int fst_split(Tables* t, const float* grid, float* rc, float* ic, int batch, int
     int nprod = 0;
     bool f16 = false;
     S2G_TRY(check_prec(precision, &nprod, &f16));
+    if (dg) return fst_dg32(t, grid, nullptr, rc, ic, batch, work, st, dg);
     S2G_TRY(build_split(t));
     Split* s = (Split*)t->split;
     const int B = t->bw, S = 2 * B;
     if (small_takes(B)) return fst_small(t, grid, rc, ic, batch, st);
-    bool digits = false;
-    if (dg) S2G_TRY(use_dg32(t, st, &digits));
-    if (digits) return fst_dg32(t, grid, nullptr, rc, ic, batch, work, st, dg);
     float* X = (float*)work;
     float* Cb = X + 2 * (size_t)batch * B * split_layout(B).SX;
     // 1. DFT along phi (two real latitudes per warp), scaled by sqrt(2 pi)/S   (FST_semi_memo.c:81-90)
@@ -2773,11 +2755,9 @@ int inv_fst_split(Tables* t, const float* rc, const float* ic, float* grid, int 
     int nprod = 0;
     bool f16 = false;
     S2G_TRY(check_prec(precision, &nprod, &f16));
+    if (dg) return inv_fst_dg32(t, rc, ic, grid, nullptr, batch, work, st, dg);
     S2G_TRY(build_split(t));
     if (small_takes(t->bw)) return inv_fst_small(t, rc, ic, grid, batch, st);
-    bool digits = false;
-    if (dg) S2G_TRY(use_dg32(t, st, &digits));
-    if (digits) return inv_fst_dg32(t, rc, ic, grid, nullptr, batch, work, st, dg);
     const int B = t->bw;
     float* F = (float*)work;
     float* Fc = F + 2 * (size_t)batch * B * split_layout(B).SX;
@@ -2951,17 +2931,15 @@ static int launch_grid_stride(long long n, int* grid) {
 int fst_split_complex(Tables* t, const float* rgrid, const float* igrid, float* rc, float* ic, int batch,
                       int precision, void* work, void* cwork, cudaStream_t st, int* dg) {
     int nprod = 0;
-    bool f16 = false, digits = false;
+    bool f16 = false;
     S2G_TRY(check_prec(precision, &nprod, &f16));
-    S2G_TRY(build_split(t));
-    if (dg) S2G_TRY(use_dg32(t, st, &digits));
-    if (digits) return fst_dg32(t, rgrid, igrid, rc, ic, batch, work, st, dg);
+    if (dg) return fst_dg32(t, rgrid, igrid, rc, ic, batch, work, st, dg);
     const int B = t->bw;
     const size_t n = (size_t)batch * B * B;
     float* g = (float*)cwork;
     float* h = g + 2 * n;
-    S2G_TRY(fst_split(t, rgrid, g, g + n, batch, precision, work, st, dg));
-    S2G_TRY(fst_split(t, igrid, h, h + n, batch, precision, work, st, dg));
+    S2G_TRY(fst_split(t, rgrid, g, g + n, batch, precision, work, st, nullptr));
+    S2G_TRY(fst_split(t, igrid, h, h + n, batch, precision, work, st, nullptr));
     const long long nq = (long long)batch * ((B * B + 3) / 4);  // quads per function, see k_cplx_combine
     int grid;
     S2G_TRY(launch_grid_stride(nq, &grid));
@@ -2974,11 +2952,9 @@ int fst_split_complex(Tables* t, const float* rgrid, const float* igrid, float* 
 int inv_fst_split_complex(Tables* t, const float* rc, const float* ic, float* rgrid, float* igrid, int batch,
                           int precision, void* work, void* cwork, cudaStream_t st, int* dg) {
     int nprod = 0;
-    bool f16 = false, digits = false;
+    bool f16 = false;
     S2G_TRY(check_prec(precision, &nprod, &f16));
-    S2G_TRY(build_split(t));
-    if (dg) S2G_TRY(use_dg32(t, st, &digits));
-    if (digits) return inv_fst_dg32(t, rc, ic, rgrid, igrid, batch, work, st, dg);
+    if (dg) return inv_fst_dg32(t, rc, ic, rgrid, igrid, batch, work, st, dg);
     const int B = t->bw;
     const size_t n = (size_t)batch * B * B;
     float* g = (float*)cwork;
@@ -2991,8 +2967,8 @@ int inv_fst_split_complex(Tables* t, const float* rc, const float* ic, float* rg
         k_cplx_split<<<grid, 256, 0, st>>>(rc, ic, g, g + n, h, h + n, B, nq);
         S2G_CUDA(cudaGetLastError());
     }
-    S2G_TRY(inv_fst_split(t, g, g + n, rgrid, batch, precision, work, st, dg));
-    return inv_fst_split(t, h, h + n, igrid, batch, precision, work, st, dg);
+    S2G_TRY(inv_fst_split(t, g, g + n, rgrid, batch, precision, work, st, nullptr));
+    return inv_fst_split(t, h, h + n, igrid, batch, precision, work, st, nullptr);
 }
 
 // One FFT stage of one bandwidth class on its own launch (the per-length warp-FFT or chirp-z

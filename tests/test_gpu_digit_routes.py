@@ -4,6 +4,9 @@ where they are not there.
 Tolerances as tests/test_gpu_digits.py: 1e-12 for FP64 transforms against the oracle's naive form or against
 band-limited data, 1e-11 where the oracle's seminaive form on noise is meant, 5e-7 for FP32.
 """
+import ctypes
+import json
+
 import numpy as np
 import pytest
 
@@ -51,12 +54,12 @@ def _cuda(*shape, dtype="float64"):
 def _expire(lib, call):
     """call() with the digit kernels' table copies left out: every wait runs out (half a second), nothing hangs."""
     import torch
-    assert lib.s2g_test_stall_digits(1) == 0
+    assert lib.s2g_test_digits(1) == 0
     try:
         call()
         torch.cuda.synchronize()
     finally:
-        lib.s2g_test_stall_digits(0)
+        lib.s2g_test_digits(0)
 
 
 def test_expired_wait_is_reported_to_its_own_plan():
@@ -98,3 +101,99 @@ def test_expired_wait_is_reported_by_the_convolution_drop_in(capfd):
     assert "ConvOn2SphereSemiMemo failed (5)" in capfd.readouterr().err
     api.ConvOn2SphereSemiMemo(*a, bw)
     assert capfd.readouterr().err == "" and (a[4] == want).all()
+
+
+# ---- the kernels that run where the digit tables, or the scratch they need, are not there --------------------------
+# The tests of those kernels, with their own tolerances, which by default meet the digit products.
+@pytest.fixture(params=[2, 3], ids=["no-tables", "no-scratch"])
+def withheld(request):
+    import s2kit_gb300 as s2
+    lib = s2.load()
+    assert lib.s2g_test_digits(request.param) == 0
+    lib.s2g_prof_enable(1)
+    try:
+        yield
+        buf = ctypes.create_string_buffer(1 << 16)
+        assert lib.s2g_prof_report(buf, len(buf)) == 0
+        kernels = json.loads(buf.value)
+        assert kernels and not [k for k in kernels if k.startswith(("dg_rows", "dg_leg_"))], kernels
+    finally:
+        lib.s2g_prof_enable(0)
+        lib.s2g_test_digits(0)
+
+
+def test_without_digits_fp64_plans(withheld, oracle):
+    from tests import test_gpu_fp64 as t
+    for bw, cutoff in ((64, 64), (32, 10), (256, 256)):
+        t.test_batched_real_fast_path(oracle, bw, cutoff)
+    t.test_batched_complex_and_conv(oracle)
+    t.test_single_function_bw256_fwd_inv_conv(oracle)
+    for bw, fmt in ((31, api.REAL), (48, api.COMPLEX), (127, api.REAL)):
+        t.test_fp64_non_power_of_two_bandwidths_vs_oracle(oracle, bw, fmt)
+
+
+def test_without_digits_fly_plans(withheld, oracle):
+    from tests import test_gpu_fly as t
+    for bw, fmt, nb in ((100, api.COMPLEX, 2), (256, api.COMPLEX, 8), (64, api.REAL, 9)):
+        t.test_fly_plan_vs_oracle(oracle, bw, fmt, nb)
+
+
+@pytest.mark.parametrize("bw,nb", [(255, 8), (64, 9), (1024, 16)])
+def test_without_digits_refinement(withheld, bw, nb):
+    from tests import test_gpu_configs as t
+    t.test_split_with_fp64_residual_refinement(bw, nb, api.PREC_BF16X3)
+
+
+@pytest.mark.parametrize("prec", [api.PREC_BF16X3, api.PREC_FP16X2])
+def test_without_digits_chirp_z_stages(withheld, oracle, prec):
+    from tests import test_gpu_complex, test_gpu_split as t
+    for bw, nb in ((65, 3), (100, 70), (127, 2), (130, 5), (255, 33)):
+        t.test_split_forward_inverse_vs_fp64(bw, nb, prec)
+    if prec == api.PREC_BF16X3:
+        for bw in (101, 255):
+            t.test_split_non_power_of_two_vs_oracle(oracle, bw)
+        for bw, nb in ((101, 3), (100, 2)):
+            test_gpu_complex.test_split_complex_vs_fp64_path(bw, nb)
+
+
+def test_without_digits_groups(withheld):
+    from tests import test_gpu_group as t
+    t.test_group_equals_uniform_path_bitwise(api.PREC_FP16X2, [77, 64, 100, 16, 77, 255, 256, 17, 101, 33])
+
+
+def test_without_digits_host_buffers(withheld):
+    import torch
+    bw, nb = 77, 150  # several chunks
+    plan = api.Plan(bw, bw)
+    g = _cuda(nb, 4 * bw * bw, dtype="float32")
+    oc = [torch.empty(nb, bw * bw, dtype=torch.float32, device="cuda") for _ in range(2)]
+    plan.fst_real_f32(g, oc[0], oc[1], nb, api.PREC_BF16X3)
+    hc = [np.zeros((nb, bw * bw), np.float32) for _ in range(2)]
+    plan.fst_real_f32_host(g.cpu().numpy(), hc[0], hc[1], nb, api.PREC_BF16X3)
+    for a, b in zip(oc, hc):
+        assert (a.cpu().numpy() == b).all()
+
+
+@pytest.mark.parametrize("warm", [False, True], ids=["tables-not-there", "tables-there"])
+def test_capture_before_the_first_digit_call(warm):
+    """Nothing can be allocated under capture: the call takes the FP64 kernels, whose scratch a zonal transform has
+    sized, whether or not another plan of the bandwidth has built the digit tables."""
+    import torch
+    bw, nb = 45 if warm else 46, 4
+    grid, oc = _cuda(nb, 4 * bw * bw), [_cuda(nb, bw * bw) for _ in range(2)]
+    if warm:
+        other = api.Plan(bw, bw)
+        other.fst(grid, None, oc[0], oc[1], nb, api.REAL)
+    plan = api.Plan(bw, bw)
+    plan.fzt(grid, None, oc[0], oc[1], nb, api.REAL)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        plan.fst(grid, None, oc[0], oc[1], nb, api.REAL, stream=torch.cuda.current_stream())
+    grid.mul_(2.0)
+    graph.replay()
+    torch.cuda.synchronize()
+    got = [c.clone() for c in oc]
+    plan.fst(grid, None, oc[0], oc[1], nb, api.REAL)
+    plan.sync_status()
+    scale = torch.hypot(oc[0], oc[1]).max()
+    assert (torch.hypot(got[0] - oc[0], got[1] - oc[1]).max() / scale).item() <= 1e-11
