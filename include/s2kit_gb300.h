@@ -184,8 +184,9 @@ int s2g_plan_destroy(s2g_plan plan);
  * plan's scratch (64 to 384 MiB by bandwidth); the split-precision entry points reject it
  * (S2G_ERR_ARG). */
 int s2g_plan_create_fly(s2g_plan* plan, int bw);
-/* Device bytes of scratch a call with this batch needs (the plan grows its own scratch
- * on demand when the caller passes none). */
+/* Device bytes of scratch that a transform or a convolution of this batch on device buffers takes at most, COMPLEX data
+ * included (precision S2G_PREC_FP64: s2g_fst, s2g_inv_fst, s2g_conv; else the FP32 ones).  The plan grows its own scratch
+ * on demand, by an eighth more than the call needs; what does not fit runs on other kernels with less, where there are some. */
 size_t s2g_plan_workspace_size(s2g_plan plan, int batch, int precision);
 
 /* Batched FP64 transforms on device pointers.  Function f of the batch uses

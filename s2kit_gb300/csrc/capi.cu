@@ -462,13 +462,17 @@ static int do_fzt(double* rdata, double* idata, double* rres, double* ires, int 
     return S2G_OK;
 }
 
+static size_t conv_coeff_bytes(int bw, int batch) {
+    return 4 * rnd((size_t)bw * bw * batch) + 2 * rnd(2 * (size_t)bw * batch) + 256;
+}
+
 // t without Legendre tables (cutoff 0): the on-the-fly kernels.
 static int conv_device(Tables* t, const double* dr, const double* di, const double* fr, const double* fi,
                        double* rr, double* ri, int batch, Scratch& scr, cudaStream_t st, int* err) {
     const bool fly = (t->cutoff == 0);
     const int bw = t->bw;
     const size_t nc = (size_t)bw * bw;
-    const size_t coeffs = 4 * rnd(nc * batch) + 2 * rnd(2 * (size_t)bw * batch) + 256;
+    const size_t coeffs = conv_coeff_bytes(bw, batch);
     size_t work = f64_work_bytes(bw, batch, REAL);  // the filter's analysis
     bool digits = false;
     if (!fly) S2G_TRY(dg_prepare(t, st, &digits));
@@ -1123,9 +1127,18 @@ int s2g_plan_destroy(s2g_plan p) {
 
 size_t s2g_plan_workspace_size(s2g_plan p, int batch, int precision) {
     if (!p || batch < 1) return 0;
-    if (precision == S2G_PREC_FP64)
-        return std::max(f64_work_bytes(p->bw, batch, COMPLEX), dg_takes(p->bw) ? dg_work_bytes(p->bw, batch, true) : 0) + 256;
-    return std::max(split_work_bytes(p->bw, batch), dg32_takes(p->bw) ? dg32_work_bytes(p->bw, batch, false) : 0);
+    const int bw = p->bw;
+    if (precision == S2G_PREC_FP64) {
+        const size_t digits = dg_takes(bw) ? dg_work_bytes(bw, batch, true) : 0;
+        size_t most = std::max(f64_work_bytes(bw, batch, COMPLEX), p->fly ? 0 : digits);
+        if (p->fly && dg_fly_takes(bw, 2 * batch)) most = std::max(most, dg_fly_bytes(bw, batch, true));
+        if (p->cutoff == bw)
+            most = std::max(most, conv_coeff_bytes(bw, batch) + std::max(f64_work_bytes(bw, batch, REAL), p->fly ? 0 : digits));
+        return most + 256;
+    }
+    // off the digit path COMPLEX calls take the second field's scratch besides
+    return dg32_takes(bw) ? std::max(dg32_work_bytes(bw, batch, true), split_work_bytes(bw, batch) + split_complex_bytes(bw, batch))
+                          : split_work_bytes(bw, batch) + split_complex_bytes(bw, batch);
 }
 
 // Device-buffer calls share the plan's scratch with the host-buffer pipeline, so they first wait

@@ -1607,35 +1607,42 @@ static int dg_fly_tables(const DgTabs* d, int stage, const DgChunk& c, const dou
     return S2G_OK;
 }
 
-// Tiles of F2 and I1 in chunks of orders, their offsets counted from the chunk's start.
+// Tiles of F2 or I1 in chunks of orders, their offsets counted from the chunk's start; off[m]: doubles of the recurrence
+// before order m in its chunk; the chunks' largest sizes.  Host only.
+static void dg_fly_layout(int s, int B, DgTable& t, std::vector<DgChunk>& chunks, std::vector<int64_t>& off,
+                          size_t& tmp_bytes, size_t& tab_bytes) {
+    dg_tiles(t, s, B, 64);
+    off.resize(B);
+    int64_t base = 0, at = 0;
+    size_t k = 0;
+    DgChunk c{0, 0, 0, 0};
+    for (int m = 0; m < B; ++m) {
+        size_t e = k;
+        while (e < t.h.size() && t.h[e].m == m) ++e;
+        const int64_t end = e < t.h.size() ? t.h[e].off : t.bytes;
+        if (m > c.m0 && end - base > dg_fly_budget(B)) {
+            chunks.push_back(c);
+            c = DgChunk{m, m, k, k};
+            base = t.h[k].off;
+            at = 0;
+        }
+        for (; k < e; ++k) t.h[k].off -= base;
+        c.m1 = m + 1;
+        c.t1 = e;
+        off[m] = at;
+        at += (int64_t)(B - m) * B;
+        tab_bytes = std::max(tab_bytes, (size_t)(end - base));
+        tmp_bytes = std::max(tmp_bytes, (size_t)at * sizeof(double));
+    }
+    chunks.push_back(c);
+}
+
 static int dg_fly_chunks(DgTabs* d, const double* weights, cudaStream_t st) {
     const int B = d->bw;
     for (int s = kF2; s <= kI1; ++s) {
         DgTable& t = d->t[s];
-        dg_tiles(t, s, B, d->prec);
-        std::vector<int64_t> off(B);
-        int64_t base = 0, at = 0;
-        size_t k = 0;
-        DgChunk c{0, 0, 0, 0};
-        for (int m = 0; m < B; ++m) {
-            size_t e = k;
-            while (e < t.h.size() && t.h[e].m == m) ++e;
-            const int64_t end = e < t.h.size() ? t.h[e].off : t.bytes;
-            if (m > c.m0 && end - base > dg_fly_budget(B)) {
-                d->chunks[s].push_back(c);
-                c = DgChunk{m, m, k, k};
-                base = t.h[k].off;
-                at = 0;
-            }
-            for (; k < e; ++k) t.h[k].off -= base;
-            c.m1 = m + 1;
-            c.t1 = e;
-            off[m] = at;
-            at += (int64_t)(B - m) * B;
-            d->tab_bytes[s] = std::max(d->tab_bytes[s], (size_t)(end - base));
-            d->tmp_bytes[s] = std::max(d->tmp_bytes[s], (size_t)at * sizeof(double));
-        }
-        d->chunks[s].push_back(c);
+        std::vector<int64_t> off;
+        dg_fly_layout(s, B, t, d->chunks[s], off, d->tmp_bytes[s], d->tab_bytes[s]);
         S2G_CUDA(cudaMalloc(&t.tiles, sizeof(DgTile) * t.h.size()));
         S2G_CUDA(cudaMemcpyAsync(t.tiles, t.h.data(), sizeof(DgTile) * t.h.size(), cudaMemcpyHostToDevice, st));
         S2G_CUDA(cudaMalloc(&d->off[s], sizeof(int64_t) * B));
@@ -1905,12 +1912,27 @@ static DgWork dg_work(char* w, int bw, int n, bool two, int es) {
     return k;
 }
 
+// Scratch of a stage's generated tables: recurrence, digits, scales (launch_dg).
+static size_t dg_fly_stage(size_t tmp_bytes, size_t tab_bytes, int rows) {
+    return tmp_bytes + tab_bytes + 2 * (size_t)rows + 4096 + 1024;
+}
 size_t dg_fly_bytes(const Tables* t, int batch, bool two) {
     const DgTabs* d = (const DgTabs*)t->dg;
     size_t need = 0;
-    for (int s = kF2; s <= kI1; ++s)
-        need = std::max(need, d->tmp_bytes[s] + d->tab_bytes[s] + 2 * (size_t)d->t[s].rows + 4096 + 1024);
-    return dg_work(nullptr, t->bw, dg_chunk(t->bw, batch, 8), two, 8).bytes + need;
+    for (int s = kF2; s <= kI1; ++s) need = std::max(need, dg_fly_stage(d->tmp_bytes[s], d->tab_bytes[s], d->t[s].rows));
+    return dg_work_bytes(t->bw, batch, two) + need;
+}
+size_t dg_fly_bytes(int bw, int batch, bool two) {
+    size_t need = 0;
+    for (int s = kF2; s <= kI1; ++s) {
+        DgTable t;
+        std::vector<DgChunk> chunks;
+        std::vector<int64_t> off;
+        size_t tmp = 0, tab = 0;
+        dg_fly_layout(s, bw, t, chunks, off, tmp, tab);
+        need = std::max(need, dg_fly_stage(tmp, tab, t.rows));
+    }
+    return dg_work_bytes(bw, batch, two) + need;
 }
 
 size_t dg_work_bytes(int bw, int batch, bool two) {

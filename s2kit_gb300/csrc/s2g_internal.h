@@ -134,9 +134,10 @@ int fst_dg32(const Tables* t, const float* rgrid, const float* igrid, float* rc,
              cudaStream_t st, int* err, const int64_t* gmap = nullptr, const int64_t* cmap = nullptr);
 int inv_fst_dg32(const Tables* t, const float* rc, const float* ic, float* rgrid, float* igrid, int batch, void* work,
                  cudaStream_t st, int* err, const int64_t* gmap = nullptr, const int64_t* cmap = nullptr);
-// On-the-fly family (tables of cutoff 0): real fields for which it pays, and the scratch once prepared.
+// On-the-fly family (tables of cutoff 0): real fields for which it pays, and the scratch, once prepared or at any time.
 bool dg_fly_takes(int bw, int fields);
 size_t dg_fly_bytes(const Tables* t, int batch, bool two);
+size_t dg_fly_bytes(int bw, int batch, bool two);
 int dg_prepare(Tables* t, cudaStream_t st, bool* yes);
 void dg_put(void* dg);
 int dg_status(int* err);    // reads the (device) word and clears it

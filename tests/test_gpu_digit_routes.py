@@ -197,3 +197,32 @@ def test_capture_before_the_first_digit_call(warm):
     plan.sync_status()
     scale = torch.hypot(oc[0], oc[1]).max()
     assert (torch.hypot(got[0] - oc[0], got[1] - oc[1]).max() / scale).item() <= 1e-11
+
+
+@pytest.mark.parametrize("kind,bw,nb", [("fly", 256, 2), ("fly", 64, 9), ("fly", 512, 1), ("f64", 100, 5), ("f64", 16, 3),
+                                        ("conv", 64, 9), ("complex32", 255, 64), ("complex32", 128, 40), ("real32", 101, 64)])
+def test_workspace_size_covers_the_scratch_a_call_takes(kind, bw, nb):
+    import torch
+    f32 = kind.endswith("32")
+    dt, prec = ("float32", api.PREC_BF16X3) if f32 else ("float64", api.PREC_FP64)
+    grid, out = ([_cuda(nb, 4 * bw * bw, dtype=dt) for _ in range(2)] for _ in range(2))
+    oc = [_cuda(nb, bw * bw, dtype=dt) for _ in range(2)]
+
+    def call(plan):
+        if kind == "complex32":
+            plan.fst_complex_f32(*grid, *oc, nb, prec)
+        elif kind == "real32":
+            plan.fst_real_f32(grid[0], *oc, nb, prec)
+        elif kind == "conv":
+            plan.conv(*grid, *grid, *out, nb)
+        else:
+            plan.fst(*grid, *oc, nb, api.COMPLEX)
+        plan.sync_status()
+
+    plans = [api.Plan(bw, bw, fly=kind == "fly") for _ in range(2)]
+    call(plans[0])  # builds the shared tables, loads the kernels
+    free = torch.cuda.mem_get_info()[0]
+    call(plans[1])
+    took = free - torch.cuda.mem_get_info()[0]
+    # scratch grows by an eighth more than it needs, in pages of 2 MiB
+    assert took <= 1.125 * plans[1].workspace_size(nb, prec) + 3 * 2 ** 21
