@@ -104,12 +104,25 @@ void prof_end(cudaStream_t st) {
     if (i < g_prof_recs.size()) cudaEventRecord(g_prof_recs[i].b, st);
 }
 
-int Scratch::ensure(size_t need) {
-    if (need <= bytes) return S2G_OK;
-    if (ptr) cudaFree(ptr);
+bool capturing(cudaStream_t st) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cs) == cudaSuccess) return cs != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
+
+int Scratch::ensure(size_t need, cudaStream_t st) {
+    const bool cap = st && (need > bytes || !held) && capturing(st);  // the legacy stream cannot be captured
+    if (need <= bytes) {
+        held |= cap;
+        return S2G_OK;
+    }
+    if (ptr && (held || cap)) kept.push_back(ptr);
+    else if (ptr) cudaFree(ptr);
     ptr = nullptr;
     bytes = 0;
-    size_t want = need + need / 8;
+    held = cap;
+    const size_t want = need + need / 8;
     cudaError_t e = cudaMalloc(&ptr, want);
     if (e != cudaSuccess) {
         ptr = nullptr;
@@ -120,6 +133,8 @@ int Scratch::ensure(size_t need) {
 }
 
 void Scratch::release() {
+    for (void* p : kept) cudaFree(p);
+    kept.clear();
     if (ptr) cudaFree(ptr);
     ptr = nullptr;
     bytes = 0;
@@ -351,7 +366,7 @@ static int do_fst(double* rdata, double* idata, double* rcoeffs, double* icoeffs
     if (table) S2G_TRY(upload_table(base, table, 0, &view.fwd));  // null: the device's own table (on the fly)
     const size_t S = 2 * (size_t)bw, ng = S * S, nc = (size_t)bw * bw;
     const size_t need = 2 * rnd(ng) + 2 * rnd(nc) + rnd(4 * (size_t)bw) + f64_work_bytes(bw, 1, fmt) + 256;
-    S2G_TRY(g_dscratch.s.ensure(need));
+    S2G_TRY(g_dscratch.s.ensure(need, 0));
     Carve c{(char*)g_dscratch.s.ptr};
     double *dr = c.take(ng), *di = c.take(ng), *cr = c.take(nc), *ci = c.take(nc), *dw = c.take(4 * bw);
     void* work = c.take(f64_work_bytes(bw, 1, fmt) / sizeof(double));
@@ -395,7 +410,7 @@ static int do_inv_fst(double* rcoeffs, double* icoeffs, double* rdata, double* i
     if (ttable) S2G_TRY(upload_table(base, ttable, 1, &view.inv));  // null: the device's own table
     const size_t S = 2 * (size_t)bw, ng = S * S, nc = (size_t)bw * bw;
     const size_t need = 2 * rnd(ng) + 2 * rnd(nc) + f64_work_bytes(bw, 1, fmt) + 256;
-    S2G_TRY(g_dscratch.s.ensure(need));
+    S2G_TRY(g_dscratch.s.ensure(need, 0));
     Carve c{(char*)g_dscratch.s.ptr};
     double *dr = c.take(ng), *di = c.take(ng), *cr = c.take(nc), *ci = c.take(nc);
     void* work = c.take(f64_work_bytes(bw, 1, fmt) / sizeof(double));
@@ -434,7 +449,7 @@ static int do_fzt(double* rdata, double* idata, double* rres, double* ires, int 
     view.split = nullptr;
     const size_t S = 2 * (size_t)bw, ng = S * S, nt = (size_t)table_size(0, bw);
     const size_t need = 2 * rnd(ng) + 2 * rnd(S) + rnd(nt) + rnd(4 * (size_t)bw) + f64_work_bytes(bw, 1, REAL) + 256;
-    S2G_TRY(g_dscratch.s.ensure(need));
+    S2G_TRY(g_dscratch.s.ensure(need, 0));
     Carve c{(char*)g_dscratch.s.ptr};
     double *dr = c.take(ng), *di = c.take(ng), *rr = c.take(S), *ri = c.take(S), *tab = c.take(nt),
            *dw = c.take(4 * bw);
@@ -481,7 +496,7 @@ static int conv_device(Tables* t, const double* dr, const double* di, const doub
         S2G_TRY(dg_scratch(scr, coeffs + most, st, &digits));
         if (digits) work = most;
     }
-    if (!digits) S2G_TRY(scr.ensure(coeffs + work));
+    if (!digits) S2G_TRY(scr.ensure(coeffs + work, st));
     int* dg = digits ? err : nullptr;
     Carve c{(char*)scr.ptr};
     double *cr = c.take(nc * batch), *ci = c.take(nc * batch), *tr = c.take(nc * batch), *ti = c.take(nc * batch);
@@ -512,7 +527,7 @@ static int do_conv(double* rdata, double* idata, double* rfilter, double* ifilte
     TabRef tref_{t};
     const size_t S = 2 * (size_t)bw, ng = S * S;
     static thread_local DropinScratch io;
-    S2G_TRY(io.s.ensure(6 * rnd(ng) + rnd(1) + 256));
+    S2G_TRY(io.s.ensure(6 * rnd(ng) + rnd(1) + 256, 0));
     Carve c{(char*)io.s.ptr};
     double *dr = c.take(ng), *di = c.take(ng), *fr = c.take(ng), *fi = c.take(ng), *orr = c.take(ng),
            *oi = c.take(ng);
@@ -549,7 +564,7 @@ static int do_dlt(int kind, const double* in, int bw, int m, double* out, const 
     const size_t nin = (kind == 0 || kind == 2) ? S : (size_t)(bw - m);
     const size_t nout = (kind == 0 || kind == 2) ? (size_t)(bw - m) : S;
     const size_t naux = (kind == 1) ? S : 4 * (size_t)bw;
-    S2G_TRY(g_dscratch.s.ensure(rnd(nt) + rnd(nin) + rnd(nout) + rnd(naux) + 256));
+    S2G_TRY(g_dscratch.s.ensure(rnd(nt) + rnd(nin) + rnd(nout) + rnd(naux) + 256, 0));
     Carve c{(char*)g_dscratch.s.ptr};
     double *dt = c.take(nt), *di = c.take(nin), *dout = c.take(nout), *da = c.take(naux);
     if (nt) S2G_CUDA(cudaMemcpy(dt, table, nt * 8, cudaMemcpyHostToDevice));
@@ -626,7 +641,7 @@ static int do_order(int kind, int bw, int m, const double* in, double* out) {
     S2G_TRY(dropin_device());
     const size_t n = (kind == 2) ? 2 * (size_t)bw * (bw - m) : (size_t)table_size(m, bw);
     std::vector<int64_t> zero(bw, 0);
-    S2G_TRY(g_dscratch.s.ensure(2 * rnd(n) + rnd(bw) + 256));
+    S2G_TRY(g_dscratch.s.ensure(2 * rnd(n) + rnd(bw) + 256, 0));
     Carve c{(char*)g_dscratch.s.ptr};
     double *a = c.take(n), *b = c.take(n);
     int64_t* doff = (int64_t*)c.take(bw);
@@ -649,7 +664,7 @@ static int do_vec(int kind, int n, int m, const double* in, double* out) {
     if (n < 1 || !out) return fail(S2G_ERR_ARG, "bad vector request");
     S2G_TRY(dropin_device());
     const size_t len = (kind == 3) ? 4 * (size_t)n : (size_t)n;
-    S2G_TRY(g_dscratch.s.ensure(2 * rnd(len) + 256));
+    S2G_TRY(g_dscratch.s.ensure(2 * rnd(len) + 256, 0));
     Carve c{(char*)g_dscratch.s.ptr};
     double *a = c.take(len), *b = c.take(len);
     if (kind == 2) {
@@ -670,7 +685,7 @@ static int do_transmult(const double* rd, const double* id, const double* rf, co
     if (bw < 1 || !rd || !id || !rf || !iff || !rr || !ir) return fail(S2G_ERR_ARG, "bad TransMult arguments");
     S2G_TRY(dropin_device());
     const size_t nc = (size_t)bw * bw;
-    S2G_TRY(g_dscratch.s.ensure(4 * rnd(nc) + 2 * rnd(bw) + 256));
+    S2G_TRY(g_dscratch.s.ensure(4 * rnd(nc) + 2 * rnd(bw) + 256, 0));
     Carve c{(char*)g_dscratch.s.ptr};
     double *a = c.take(nc), *b = c.take(nc), *o1 = c.take(nc), *o2 = c.take(nc), *f1 = c.take(bw), *f2 = c.take(bw);
     S2G_CUDA(cudaMemcpy(a, rd, nc * 8, cudaMemcpyHostToDevice));
@@ -1166,7 +1181,7 @@ static int f64_scratch(s2g_plan p, int batch, DataFormat fmt, bool imag, cudaStr
     if (!p->fly || dg_fly_takes(p->bw, two ? 2 * batch : batch)) S2G_TRY(dg_prepare(p->t, st, &yes));
     if (yes) S2G_TRY(dg_scratch(p->work, p->fly ? dg_fly_bytes(p->t, batch, two) : dg_work_bytes(p->bw, batch, two), st, &yes));
     if (yes) return *dg = p->err, S2G_OK;
-    return p->work.ensure(f64_work_bytes(p->bw, batch, fmt));
+    return p->work.ensure(f64_work_bytes(p->bw, batch, fmt), st);
 }
 
 // The same for FP32 transforms, COMPLEX ones with the second field's scratch.
@@ -1177,8 +1192,8 @@ static int split_scratch(s2g_plan p, int batch, int precision, bool complex, cud
     S2G_TRY(dg32_prepare(p->t, st, &yes));
     if (yes) S2G_TRY(dg_scratch(p->work, dg32_work_bytes(p->bw, batch, complex), st, &yes));
     if (yes) return *dg = p->err, S2G_OK;
-    S2G_TRY(p->work.ensure(split_work_bytes(p->bw, batch)));
-    return complex ? p->cx.ensure(split_complex_bytes(p->bw, batch)) : S2G_OK;
+    S2G_TRY(p->work.ensure(split_work_bytes(p->bw, batch), st));
+    return complex ? p->cx.ensure(split_complex_bytes(p->bw, batch), st) : S2G_OK;
 }
 
 int s2g_fst(s2g_plan p, const double* rdata, const double* idata, double* rcoeffs, double* icoeffs, int batch,
@@ -1208,7 +1223,7 @@ int s2g_fzt(s2g_plan p, const double* rdata, const double* idata, double* rres, 
             DataFormat fmt, void* stream) {
     S2G_TRY(plan_check(p, batch, false, true));
     if (!rdata || !rres || !ires || (fmt == COMPLEX && !idata)) return fail(S2G_ERR_ARG, "NULL argument");
-    S2G_TRY(p->work.ensure(f64_work_bytes(p->bw, batch, REAL)));
+    S2G_TRY(p->work.ensure(f64_work_bytes(p->bw, batch, REAL), (cudaStream_t)stream));
     if (p->fly) return fzt_f64_fly(p->t, rdata, idata, rres, ires, batch, fmt, p->work.ptr, (cudaStream_t)stream);
     return fzt_f64(p->t, rdata, idata, rres, ires, batch, fmt, p->work.ptr, (cudaStream_t)stream);
 }
@@ -1274,12 +1289,12 @@ static int refined_scratch(s2g_plan p, int batch, int precision, cudaStream_t st
     S2G_TRY(split_check(p->t, precision));
     *dg = nullptr;
     *direct = !dg_takes(p->bw);
-    if (*direct) return p->work.ensure(f64_work_bytes(p->bw, batch, REAL));
+    if (*direct) return p->work.ensure(f64_work_bytes(p->bw, batch, REAL), st);
     S2G_TRY(dg_prepare(p->t, st, direct));
     if (*direct) S2G_TRY(dg_scratch(p->work, dg_work_bytes(p->bw, batch, false), st, direct));
     if (*direct) return *dg = p->err, S2G_OK;
-    S2G_TRY(p->work.ensure(refine_work_bytes(p->bw, batch)));
-    return p->io.ensure(refine_io_bytes(p->bw, batch));
+    S2G_TRY(p->work.ensure(refine_work_bytes(p->bw, batch), st));
+    return p->io.ensure(refine_io_bytes(p->bw, batch), st);
 }
 
 int s2g_fst_refined(s2g_plan p, const double* grid, double* rc, double* ic, int batch, int precision,
@@ -1338,7 +1353,7 @@ static int host_pipeline(s2g_plan p, int fwd, const float* in0, const float* in1
     const size_t most = std::max(split_work_bytes(p->bw, chunk), dg32_takes(p->bw) ? dg32_work_bytes(p->bw, chunk, false) : 0);
     if (stage != p->stage || p->io.bytes < 4 * stage + 1024 || p->work.bytes < most) {
         S2G_TRY(drain_host(p));  // a new layout or a larger buffer: nothing queued may still use the old one
-        S2G_TRY(p->io.ensure(4 * stage + 1024));
+        S2G_TRY(p->io.ensure(4 * stage + 1024, p->streams[1]));
         p->stage = stage;
     }
     int* dg;

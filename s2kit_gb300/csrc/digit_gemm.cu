@@ -1950,13 +1950,6 @@ bool dg_takes(int bw) { return bw <= 1024 && (bw >= 32 || (bw > 8 && (bw & (bw -
 
 bool dg_fly_takes(int bw, int fields) { return dg_takes(bw) && bw >= 64 && fields >= (bw > 512 ? 4 : 2); }
 
-static bool capturing(cudaStream_t st) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cs) == cudaSuccess) return cs != cudaStreamCaptureStatusNone;
-    cudaGetLastError();  // the legacy stream, while another is captured
-    return true;
-}
-
 // Builds (or finds) the digit tables of t's bandwidth; *yes where they are there.  Where the stream is being
 // captured, or they do not fit in device memory, t stays without them and the other kernels run; what did not
 // fit is tried again by every 64th call that asks (an attempt costs the allocations before the one that fails).
@@ -2000,14 +1993,16 @@ int dg32_prepare(Tables* t, cudaStream_t st, bool* yes) {
 
 bool dg_no_scratch() { return dg_test() == kDgNoScratch; }
 int dg_scratch(Scratch& s, size_t need, cudaStream_t st, bool* yes) {
-    *yes = need <= s.bytes && !dg_no_scratch();
-    if (*yes || dg_no_scratch()) return S2G_OK;
-    if (need >= s.nofit && s.skip > 0) {
-        --s.skip;
-        return S2G_OK;
+    *yes = false;
+    if (dg_no_scratch()) return S2G_OK;
+    if (need > s.bytes) {
+        if (need >= s.nofit && s.skip > 0) {
+            --s.skip;
+            return S2G_OK;
+        }
+        if (capturing(st)) return S2G_OK;
     }
-    if (capturing(st)) return S2G_OK;
-    const int r = s.ensure(need);
+    const int r = s.ensure(need, st);
     if (r == S2G_ERR_NOMEM) {
         cudaGetLastError();
         s.nofit = need;

@@ -7,6 +7,7 @@
 #include <initializer_list>
 #include <mutex>
 #include <string>
+#include <vector>
 
 #include "../../include/s2kit_gb300.h"
 
@@ -67,13 +68,19 @@ struct Tables {
     int refs = 0;               // references (cache, plans, groups, calls in flight); under the cache lock
 };
 
-// Device scratch owned by a plan; grown on demand.
+// Whether st is being captured (or, for the legacy stream, another one).
+bool capturing(cudaStream_t st);
+
+// Device scratch owned by a plan; grown on demand.  A buffer handed to a captured call lives as long as the plan:
+// the graph has its address, and calls of other kinds at the same batch may need more of it.
 struct Scratch {
     void* ptr = nullptr;
     size_t bytes = 0;
-    size_t nofit = 0;  // dg_scratch: what did not fit, and the calls left before the next attempt
+    size_t nofit = 0;          // dg_scratch: what did not fit, and the calls left before the next attempt
     int skip = 0;
-    int ensure(size_t need);
+    bool held = false;         // a captured call has it
+    std::vector<void*> kept;   // outgrown buffers that captured calls have
+    int ensure(size_t need, cudaStream_t st);  // st: the stream of the call that it is for
     void release();
 };
 

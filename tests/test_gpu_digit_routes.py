@@ -226,3 +226,45 @@ def test_workspace_size_covers_the_scratch_a_call_takes(kind, bw, nb):
     took = free - torch.cuda.mem_get_info()[0]
     # scratch grows by an eighth more than it needs, in pages of 2 MiB
     assert took <= 1.125 * plans[1].workspace_size(nb, prec) + 3 * 2 ** 21
+
+
+@pytest.mark.parametrize("first,then", [("real32", "f64"), ("real32", "complex32"), ("f64", "imag64"), ("fly", "imagfly")])
+def test_captured_call_keeps_its_scratch_when_another_needs_more(first, then):
+    """A captured call has the scratch's address; a larger need of another call of the same batch leaves that buffer."""
+    import torch
+    bw, nb = (64, 3) if then in ("f64", "imagfly") else (101, 3)
+    f32 = first.endswith("32")
+    grid = _cuda(nb, 4 * bw * bw, dtype="float32" if f32 else "float64")
+    oc = [_cuda(nb, bw * bw, dtype="float32" if f32 else "float64") for _ in range(2)]
+    g2 = _cuda(nb, 4 * bw * bw, dtype="float32" if then == "complex32" else "float64")
+    o2 = [torch.empty(nb, bw * bw, dtype=g2.dtype, device="cuda") for _ in range(2)]
+    plan = api.Plan(bw, bw, fly=first == "fly")
+
+    def call(**kw):
+        if f32:
+            plan.fst_real_f32(grid, *oc, nb, api.PREC_BF16X3, **kw)
+        elif first == "fly":
+            plan.fst(grid, None, *oc, 1, api.REAL, **kw)
+        else:
+            plan.fst(grid, None, *oc, nb, api.REAL, **kw)
+
+    call()
+    torch.cuda.synchronize()
+    want = [c.clone() for c in oc]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call(stream=torch.cuda.current_stream())
+    if then == "complex32":
+        plan.fst_complex_f32(g2, g2, *o2, nb, api.PREC_BF16X3)
+    else:
+        plan.fst(g2, g2 if then.startswith("imag") else None, *o2, nb, api.REAL)
+    torch.cuda.synchronize()
+    junk = [torch.full((2 ** k,), float("nan"), device="cuda") for k in range(16, 25)]  # takes what was freed
+    for c in oc:
+        c.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    plan.sync_status()
+    assert all(torch.isnan(j).all() for j in junk)
+    n = 1 if first == "fly" else nb
+    assert (oc[0][:n] == want[0][:n]).all() and (oc[1][:n] == want[1][:n]).all()
