@@ -216,7 +216,7 @@ __device__ __forceinline__ long long dg_sum(const uint32_t* a, int stride, uint3
     odd |= x;
     const long long lo = (long long)i[2] * (1 << 24) + (long long)i[3] * 65536 + (long long)i[4] * 256 + (long long)i[5] + i[6];
     constexpr unsigned long long bias = ((unsigned long long)(b * 257) << 32) + (unsigned long long)(b * ((1 << 24) + 65536 + 256 + 2));
-    const unsigned long long hi = (unsigned long long)(uint32_t)(i[0] * 256 + i[1]) << 32;
+    const unsigned long long hi = (unsigned long long)(((uint32_t)i[0] << 8) + (uint32_t)i[1]) << 32;  // modulo 2^32
     return (long long)(hi + (unsigned long long)lo - bias);
 }
 // The same for groups of any size; dg_sum sets bits 23.. of `odd` where one is outside its range.
@@ -225,7 +225,7 @@ __device__ __noinline__ long long dg_sum_big(float a0, float a1, float a2, float
     long long i[kDigits];
 #pragma unroll
     for (int g = 0; g < kDigits; ++g) i[g] = __float2int_rn(a[g]);
-    return ((i[0] * 256 + i[1]) << 32) + i[2] * (1 << 24) + i[3] * 65536 + i[4] * 256 + i[5] + (i[6] >> 8);
+    return (i[0] * 256 + i[1]) * (1ll << 32) + i[2] * (1 << 24) + i[3] * 65536 + i[4] * 256 + i[5] + (i[6] >> 8);
 }
 
 // T 2^(eb - 1086) as a double, rounded to nearest; kDgNan in eb stands for a column that held an
@@ -238,7 +238,7 @@ __device__ __forceinline__ double dg_fast(long long T, int eb, bool& bad) {
     const int lz = __clz((int)mw) + (mh ? 0 : 32), e = eb - lz;
     const unsigned long long m = m0 << (lz & 63);
     bad |= (m0 != 0 && (uint32_t)(e - 1) >= 2046u) || eb >= kDgNan / 2;
-    unsigned long long bits = ((unsigned long long)(uint32_t)((e - 1) << 20) << 32) + (m >> 11) + ((m >> 10) & 1);
+    unsigned long long bits = ((unsigned long long)((uint32_t)(e - 1) << 20) << 32) + (m >> 11) + ((m >> 10) & 1);
     bits = m0 ? bits : 0;
     return __longlong_as_double((long long)(bits | ((unsigned long long)T & 0x8000000000000000ull)));
 }
