@@ -104,6 +104,20 @@ void prof_end(cudaStream_t st) {
     if (i < g_prof_recs.size()) cudaEventRecord(g_prof_recs[i].b, st);
 }
 
+int set_smem(const void* fn, size_t bytes) {
+    static std::mutex mu;
+    static std::map<std::pair<int, const void*>, size_t> allowed;
+    int dev = 0;
+    S2G_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(mu);
+    size_t& most = allowed[{dev, fn}];
+    if (bytes <= most) return S2G_OK;
+    // set also below 48 KiB: that default covers static plus dynamic shared memory
+    S2G_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    most = bytes;
+    return S2G_OK;
+}
+
 bool capturing(cudaStream_t st) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cs) == cudaSuccess) return cs != cudaStreamCaptureStatusNone;

@@ -492,7 +492,7 @@ int czt_launch(int which, const CztTabs& g, const void* in, void* out, int N, fl
     const void* fn = which == 0 ? (const void*)k_czt_rows_fwd<RM>
                    : which == 1 ? (const void*)k_czt_dct_fwd<RM>
                    : which == 2 ? (const void*)k_czt_dct_inv<RM> : (const void*)k_czt_rows_inv<RM>;
-    S2G_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    S2G_TRY(set_smem(fn, smem));
     const long long tiles = (long long)N * (L.SX / kLat);
     if (which == 0) {
         ProfScope ps_("rows_fwd_czt", st);

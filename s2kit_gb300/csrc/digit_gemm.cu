@@ -1731,7 +1731,7 @@ static int dg_build(DgTabs* d, const double* weights, cudaStream_t st) {
     int* first[4] = {nullptr, nullptr, nullptr, nullptr};
     for (int s = kF2; s <= kI1; ++s) S2G_TRY(dg_first_alloc(d->t[s], &tmp.p[s + 2], &first[s], st));
     const size_t smem = sizeof(double2) * 2 * (size_t)B;
-    S2G_CUDA(cudaFuncSetAttribute((const void*)k_dg_legendre, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    S2G_TRY(set_smem((const void*)k_dg_legendre, smem));
     for (int m0 = 0; m0 < B;) {
         int m1 = m0 + 1;
         while (m1 < B && off[m1] != 0) ++m1;
@@ -1798,7 +1798,7 @@ static int launch_dg_nt(const DgArgs& p, int sms, cudaStream_t st) {
                                    "dg_rows_fwd_f32", "dg_leg_fwd_f32", "dg_leg_inv_f32", "dg_rows_inv_f32"};
     const size_t smem = 1024 + Dg<P>::stagesA * kDgABytes<P> + kDgBRing +
                         (P == 32 && STAGE == kF1 ? Dg<P>::epilogue * kDgStash : 0);
-    S2G_CUDA(cudaFuncSetAttribute((const void*)k_dg<STAGE, NT, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    S2G_TRY(set_smem((const void*)k_dg<STAGE, NT, P>, smem));
     const int64_t items = (int64_t)p.ntiles * p.ncolblk;
     {
         ProfScope ps_(names[STAGE + (P == 32 ? 4 : 0)], st);
@@ -2013,11 +2013,6 @@ int dg_scratch(Scratch& s, size_t need, cudaStream_t st, bool* yes) {
     return r;
 }
 
-static int set_dyn_smem(const void* fn, size_t bytes) {
-    S2G_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    return S2G_OK;
-}
-
 template <int P>
 static int dg_fst(const DgTabs* d, const double* weights, const typename Dg<P>::Real* rdata,
                   const typename Dg<P>::Real* idata, typename Dg<P>::Real* rc, typename Dg<P>::Real* ic, int batch, int fmt,
@@ -2027,7 +2022,7 @@ static int dg_fst(const DgTabs* d, const double* weights, const typename Dg<P>::
     const DgFold fl = dg_fold_layout(B, false);
     const DgWork w = dg_work((char*)work, B, chunk, mode != kReal, sizeof(Real));
     char* scratch = (char*)work + w.bytes;  // on the fly: tables
-    S2G_TRY(set_dyn_smem((const void*)k_dg_fold<P>, 2 * (size_t)S * sizeof(Real)));
+    S2G_TRY(set_smem((const void*)k_dg_fold<P>, 2 * (size_t)S * sizeof(Real)));
     for (int f0 = 0; f0 < batch; f0 += chunk) {
         const int n = std::min(chunk, batch - f0), ff = n * dg_fields(mode);
         const size_t g0 = gmap ? 0 : (size_t)f0 * S * S, c0 = cmap ? 0 : (size_t)f0 * B * B;

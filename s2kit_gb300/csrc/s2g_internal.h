@@ -46,6 +46,10 @@ struct ProfScope {
     ~ProfScope() { prof_end(st); }
 };
 
+// Allows kernel fn `bytes` of dynamic shared memory on the current device.  The allowance is the function's, shared by
+// all threads, and a launch that asks for more than it fails: it only ever grows.
+int set_smem(const void* fn, size_t bytes);
+
 // Device tables and constants for one (bandwidth, cutoff) on one device.
 struct Tables {
     int bw = 0, cutoff = 0, device = -1;

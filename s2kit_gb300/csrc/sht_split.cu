@@ -2240,12 +2240,6 @@ size_t split_work_bytes(int bw, int batch) {
     return 2 * (size_t)batch * bw * ((size_t)L.SX + 2 * (size_t)L.BH) * sizeof(float) + 1024;
 }
 
-static int set_smem(const void* fn, size_t bytes) {
-    // always set: the 48 KiB default covers static plus dynamic shared memory
-    S2G_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    return S2G_OK;
-}
-
 static int check_prec(int precision, int* nprod, bool* f16) {
     *f16 = false;
     if (precision == S2G_PREC_BF16X3) *nprod = 6;

@@ -253,7 +253,7 @@ int generate_cos_pml_device(int bw, int m_begin, int m_end, double* d_fwd, const
     GenCos p{bw, m_begin, d_fwd, d_off, tw.twB, tw.twQ, tw.tw4, L.logn};
     const size_t smem = (size_t)(7 * bw + 2 * bw) * sizeof(double);
     if (smem > 0)  // the 48 KiB default covers static plus dynamic shared memory
-        S2G_CUDA(cudaFuncSetAttribute((const void*)k_gen_cos, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        S2G_TRY(set_smem((const void*)k_gen_cos, smem));
     {
         ProfScope ps_("gen_cos_pml", st);
         k_gen_cos<<<m_end - m_begin, 256, smem, st>>>(p);
@@ -279,7 +279,7 @@ int generate_pml_device(int bw, int m_begin, int m_end, double* d_fwd, const int
     if (m_end <= m_begin) return S2G_OK;
     const size_t smem = (size_t)3 * 2 * bw * sizeof(double);
     if (smem > 0)  // the 48 KiB default covers static plus dynamic shared memory
-        S2G_CUDA(cudaFuncSetAttribute((const void*)k_gen_pml, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        S2G_TRY(set_smem((const void*)k_gen_pml, smem));
     {
         ProfScope ps_("gen_pml", st);
         k_gen_pml<<<m_end - m_begin, 256, smem, st>>>(bw, m_begin, d_fwd, d_off);

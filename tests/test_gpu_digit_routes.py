@@ -268,3 +268,62 @@ def test_captured_call_keeps_its_scratch_when_another_needs_more(first, then):
     assert all(torch.isnan(j).all() for j in junk)
     n = 1 if first == "fly" else nb
     assert (oc[0][:n] == want[0][:n]).all() and (oc[1][:n] == want[1][:n]).all()
+
+
+def test_plans_of_several_threads_do_not_disturb_each_other():
+    """One plan and stream a thread, the same kernels at different sizes: every call is accepted, every result the one a
+    thread alone gets."""
+    import threading
+
+    import torch
+    errors = []
+
+    def worker(make, stream, want):
+        try:
+            with torch.cuda.stream(stream):
+                run, out = make(stream)
+                for _ in range(300):
+                    run()
+                stream.synchronize()
+                if want is not None:
+                    assert all((a == b).all() for a, b in zip(out, want))
+            return [o.clone() for o in out]
+        except Exception as e:  # noqa: BLE001
+            errors.append(repr(e))
+
+    def f32(bw):
+        g = _cuda(3, 4 * bw * bw, dtype="float32")
+
+        def make(stream):
+            plan, out = api.Plan(bw, bw), [torch.zeros(3, bw * bw, dtype=torch.float32, device="cuda") for _ in range(2)]
+            back = torch.zeros_like(g)
+
+            def run():
+                plan.fst_real_f32(g, *out, 3, api.PREC_BF16X3, stream=stream)
+                plan.inv_fst_real_f32(*out, back, 3, api.PREC_BF16X3, stream=stream)
+            return run, [*out, back]
+        return make
+
+    def f64(bw, fly):
+        g = _cuda(1, 4 * bw * bw)
+
+        def make(stream):
+            plan, out = api.Plan(bw, bw, fly=fly), [torch.zeros(1, bw * bw, dtype=torch.float64, device="cuda") for _ in range(2)]
+            back = torch.zeros_like(g)
+
+            def run():
+                plan.fst(g, None, *out, 1, api.REAL, stream=stream)
+                plan.inv_fst(*out, back, None, 1, api.REAL, stream=stream)
+            return run, [*out, back]
+        return make
+
+    makes = [f32(17), f32(31), f32(33), f32(47), f64(16, False), f64(128, True), f64(32, True), f64(48, False)]
+    streams = [torch.cuda.Stream() for _ in makes]
+    torch.cuda.synchronize()
+    alone = [worker(m, s, None) for m, s in zip(makes, streams)]
+    threads = [threading.Thread(target=worker, args=a) for a in zip(makes, streams, alone)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
