@@ -193,7 +193,8 @@ size_t s2g_plan_workspace_size(s2g_plan plan, int batch, int precision);
  * rdata + f*(2bw)^2 and rcoeffs + f*bw*bw (likewise for the imaginary arrays).
  * REAL with idata == NULL (forward) or idata == NULL (inverse output) selects the
  * real-field fast path (imaginary samples taken as zero / not written).  `stream` is a
- * cudaStream_t (NULL = legacy default stream).  Asynchronous with respect to the host. */
+ * cudaStream_t (NULL = legacy default stream).  Asynchronous with respect to the host.  Results may overlap
+ * the samples or coefficients that they are made from (here, in the FP32 transforms below and in groups). */
 int s2g_fst(s2g_plan plan, const double* rdata, const double* idata, double* rcoeffs, double* icoeffs, int batch,
             DataFormat data_format, void* stream);
 int s2g_inv_fst(s2g_plan plan, const double* rcoeffs, const double* icoeffs, double* rdata, double* idata,

@@ -1026,7 +1026,7 @@ struct s2g_plan_s {
     int* err = nullptr;  // device word, see dg_status
     Scratch work;
     Scratch io;
-    Scratch cx;  // the two real fields' coefficients of COMPLEX split transforms
+    Scratch cx;  // the two real fields' coefficients of COMPLEX split transforms, or inputs (read_apart)
     cudaStream_t streams[3];
     cudaEvent_t events[6];
     // host-buffer pipeline state, kept across asynchronous calls
@@ -1210,12 +1210,41 @@ static int split_scratch(s2g_plan p, int batch, int precision, bool complex, cud
     return complex ? p->cx.ensure(split_complex_bytes(p->bw, batch), st) : S2G_OK;
 }
 
+// Outputs may overlap inputs (samples transformed in place).  Kernels that write results before all input is read --
+// the digit path with more functions than it takes at a time, one kernel for the whole transform -- then read a copy.
+// a, b: inputs of n values each (*b may be null), o0, o1: outputs of no values.
+extern "C++" {
+template <class T>
+static int read_apart(s2g_plan p, bool early, const T** a, const T** b, size_t n, const T* o0, const T* o1, size_t no,
+                      cudaStream_t st) {
+    const size_t by = n * sizeof(T), bo = no * sizeof(T);
+    auto hit = [&](const T* x) { return x && (overlap(x, by, o0, bo) || (o1 && overlap(x, by, o1, bo))); };
+    if (!early || !(hit(*a) || hit(*b))) return S2G_OK;
+    S2G_TRY(p->cx.ensure(2 * by, st));
+    T* to = (T*)p->cx.ptr;
+    S2G_CUDA(cudaMemcpyAsync(to, *a, by, cudaMemcpyDeviceToDevice, st));
+    *a = to;
+    if (!*b) return S2G_OK;
+    S2G_CUDA(cudaMemcpyAsync(to + n, *b, by, cudaMemcpyDeviceToDevice, st));
+    *b = to + n;
+    return S2G_OK;
+}
+}
+static bool f64_early(s2g_plan p, int batch, const int* dg) { return dg && batch > dg_chunk(p->bw, batch, 8); }
+static bool f32_early(s2g_plan p, int batch, const int* dg) {
+    return dg ? batch > dg_chunk(p->bw, batch, 4) : small_takes(p->bw) && batch > 1;
+}
+static size_t grid_values(s2g_plan p, int batch) { return 4 * (size_t)p->bw * p->bw * batch; }
+static size_t coeff_values(s2g_plan p, int batch) { return (size_t)p->bw * p->bw * batch; }
+
 int s2g_fst(s2g_plan p, const double* rdata, const double* idata, double* rcoeffs, double* icoeffs, int batch,
             DataFormat fmt, void* stream) {
     S2G_TRY(plan_check(p, batch, false, true));
     if (!rdata || !rcoeffs || !icoeffs || (fmt == COMPLEX && !idata)) return fail(S2G_ERR_ARG, "NULL argument");
     int* dg;
     S2G_TRY(f64_scratch(p, batch, fmt, idata != nullptr, (cudaStream_t)stream, &dg));
+    S2G_TRY(read_apart<double>(p, f64_early(p, batch, dg), &rdata, &idata, grid_values(p, batch), rcoeffs, icoeffs,
+                               coeff_values(p, batch), (cudaStream_t)stream));
     if (p->fly && !dg)
         return fst_f64_fly(p->t, rdata, idata, rcoeffs, icoeffs, batch, fmt, p->work.ptr, (cudaStream_t)stream);
     return fst_f64(p->t, rdata, idata, rcoeffs, icoeffs, batch, fmt, p->cutoff, p->work.ptr, (cudaStream_t)stream, dg);
@@ -1227,6 +1256,8 @@ int s2g_inv_fst(s2g_plan p, const double* rcoeffs, const double* icoeffs, double
     if (!rdata || !rcoeffs || !icoeffs || (fmt == COMPLEX && !idata)) return fail(S2G_ERR_ARG, "NULL argument");
     int* dg;
     S2G_TRY(f64_scratch(p, batch, fmt, idata != nullptr, (cudaStream_t)stream, &dg));
+    S2G_TRY(read_apart<double>(p, f64_early(p, batch, dg), &rcoeffs, &icoeffs, coeff_values(p, batch), rdata, idata,
+                               grid_values(p, batch), (cudaStream_t)stream));
     if (p->fly && !dg)
         return inv_fst_f64_fly(p->t, rcoeffs, icoeffs, rdata, idata, batch, fmt, p->work.ptr, (cudaStream_t)stream);
     return inv_fst_f64(p->t, rcoeffs, icoeffs, rdata, idata, batch, fmt, p->cutoff, p->work.ptr,
@@ -1262,6 +1293,9 @@ int s2g_fst_real_f32(s2g_plan p, const float* grid, float* rc, float* ic, int ba
     S2G_TRY(check_aligned16({grid, rc, ic}));
     int* dg;
     S2G_TRY(split_scratch(p, batch, precision, false, (cudaStream_t)stream, &dg));
+    const float* none = nullptr;
+    S2G_TRY(read_apart<float>(p, f32_early(p, batch, dg), &grid, &none, grid_values(p, batch), rc, ic, coeff_values(p, batch),
+                              (cudaStream_t)stream));
     return fst_split(p->t, grid, rc, ic, batch, precision, p->work.ptr, (cudaStream_t)stream, dg);
 }
 
@@ -1272,6 +1306,8 @@ int s2g_inv_fst_real_f32(s2g_plan p, const float* rc, const float* ic, float* gr
     S2G_TRY(check_aligned16({grid, rc, ic}));
     int* dg;
     S2G_TRY(split_scratch(p, batch, precision, false, (cudaStream_t)stream, &dg));
+    S2G_TRY(read_apart<float>(p, f32_early(p, batch, dg), &rc, &ic, coeff_values(p, batch), grid, nullptr,
+                              grid_values(p, batch), (cudaStream_t)stream));
     return inv_fst_split(p->t, rc, ic, grid, batch, precision, p->work.ptr, (cudaStream_t)stream, dg);
 }
 
@@ -1282,6 +1318,8 @@ int s2g_fst_complex_f32(s2g_plan p, const float* rgrid, const float* igrid, floa
     S2G_TRY(check_aligned16({rgrid, igrid, rc, ic}));
     int* dg;
     S2G_TRY(split_scratch(p, batch, precision, true, (cudaStream_t)stream, &dg));
+    S2G_TRY(read_apart<float>(p, dg && f32_early(p, batch, dg), &rgrid, &igrid, grid_values(p, batch), rc, ic,
+                              coeff_values(p, batch), (cudaStream_t)stream));
     return fst_split_complex(p->t, rgrid, igrid, rc, ic, batch, precision, p->work.ptr, p->cx.ptr,
                              (cudaStream_t)stream, dg);
 }
@@ -1293,6 +1331,8 @@ int s2g_inv_fst_complex_f32(s2g_plan p, const float* rc, const float* ic, float*
     S2G_TRY(check_aligned16({rgrid, igrid, rc, ic}));
     int* dg;
     S2G_TRY(split_scratch(p, batch, precision, true, (cudaStream_t)stream, &dg));
+    S2G_TRY(read_apart<float>(p, dg && f32_early(p, batch, dg), &rc, &ic, coeff_values(p, batch), rgrid, igrid,
+                              grid_values(p, batch), (cudaStream_t)stream));
     return inv_fst_split_complex(p->t, rc, ic, rgrid, igrid, batch, precision, p->work.ptr, p->cx.ptr,
                                  (cudaStream_t)stream, dg);
 }

@@ -1878,8 +1878,8 @@ static int launch_dg(const DgTabs* d, DgArgs p, const double* weights, char* scr
 static int dg_fields(int mode) { return mode == kReal ? 1 : 2; }
 static int dg_mode(const void* imag, int fmt) { return fmt == COMPLEX ? kCplx : (imag ? kReal2 : kReal); }
 
-// Functions transformed at a time.
-static int dg_chunk(int bw, int batch, int es) {
+// Functions transformed at a time (es: bytes of a value).
+int dg_chunk(int bw, int batch, int es) {
     const int64_t per = 2 * es * 4 * (int64_t)bw * bw;
     return (int)std::min<int64_t>(batch, std::min<int64_t>(16384, std::max<int64_t>(64, ((int64_t)256 << 20) / per)));
 }

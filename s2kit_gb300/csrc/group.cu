@@ -75,6 +75,7 @@ struct s2g_group_s {
     void* mem = nullptr;        // one device allocation: maps, intermediates, counters
     int* counters = nullptr;    // [0] forward, [1] inverse contraction work counters
     int* err = nullptr;         // error word of the digit path (dg_status)
+    s2g::Scratch apart;         // inputs that a call's outputs overlap (group_apart)
     int table_stages = 0;       // contraction: table-copy ring depth, 0 = as many as fit
     int dct_ctas = 0;           // DCT stages: resident blocks per SM they are sized for, 0 = as many as fit
     cudaStream_t cap = nullptr;
@@ -146,8 +147,24 @@ static int group_stages(s2g_group g, const int* which, int nstage, In in, Out ou
     return S2G_OK;
 }
 
+// Classes on the digit path, or transformed whole, write results before the other classes have read their input, so
+// a call whose outputs overlap its inputs reads a copy (the caller of the sequence has made room for it).
+static bool group_apart(s2g_group g, const float* grid, const float* rc, const float* ic) {
+    const size_t bg = sizeof(float) * g->grid_total, bc = sizeof(float) * g->coef_total;
+    bool early = false;
+    for (auto& k : g->cls) early |= k.dg || k.small;
+    return early && (overlap(grid, bg, rc, bc) || overlap(grid, bg, ic, bc));
+}
+static int group_apart_ensure(s2g_group g, cudaStream_t st) {
+    return g->apart.ensure(sizeof(float) * (size_t)std::max(g->grid_total, 2 * g->coef_total), st);
+}
+
 static int group_fwd_seq(s2g_group g, const float* grid, float* rc, float* ic, cudaStream_t st) {
     const int nc = (int)g->cls.size();
+    if (group_apart(g, grid, rc, ic)) {
+        S2G_CUDA(cudaMemcpyAsync(g->apart.ptr, grid, sizeof(float) * g->grid_total, cudaMemcpyDeviceToDevice, st));
+        grid = (const float*)g->apart.ptr;
+    }
     for (auto& k : g->cls)
         if (k.digits) S2G_TRY(fst_dg32(k.t, grid, nullptr, rc, ic, k.N, k.digits, st, g->err, k.gmap, k.cmap));
         else if (k.small && !stage_groupable(k.B)) S2G_TRY(fst_small(k.t, grid, rc, ic, k.N, st, k.gmap, k.cmap));
@@ -175,6 +192,13 @@ static int group_fwd_seq(s2g_group g, const float* grid, float* rc, float* ic, c
 
 static int group_inv_seq(s2g_group g, const float* rc, const float* ic, float* grid, cudaStream_t st) {
     const int nc = (int)g->cls.size();
+    if (group_apart(g, grid, rc, ic)) {
+        float* to = (float*)g->apart.ptr;
+        S2G_CUDA(cudaMemcpyAsync(to, rc, sizeof(float) * g->coef_total, cudaMemcpyDeviceToDevice, st));
+        S2G_CUDA(cudaMemcpyAsync(to + g->coef_total, ic, sizeof(float) * g->coef_total, cudaMemcpyDeviceToDevice, st));
+        rc = to;
+        ic = to + g->coef_total;
+    }
     LegSpec spec[kGroupMaxClasses] = {};
     int ns = 0;
     for (int c = 0; c < nc; ++c) {
@@ -228,6 +252,10 @@ static int group_run(s2g_group g, int kind, const void* const* ptr, int nptr, cu
         return S2G_OK;
     }
     drop_graph(gr);
+    const float* const* q = (const float* const*)ptr;
+    if (kind == 1 ? group_apart(g, q[2], q[0], q[1])
+                  : group_apart(g, q[0], q[1], q[2]) || (kind == 2 && group_apart(g, q[3], q[1], q[2])))
+        S2G_TRY(group_apart_ensure(g, st));
     S2G_TRY(group_seq(g, kind, ptr, st));
     // capture for the next call with these pointers (the capture runs nothing)
     cudaGraph_t graph = nullptr;
@@ -449,6 +477,7 @@ static void group_free(s2g_group g) {
     if (g->fork) cudaEventDestroy(g->fork);
     if (g->join) cudaEventDestroy(g->join);
     cudaFree(g->mem);
+    g->apart.release();
     for (auto& c : g->cls) put_tables(c.t);
     delete g;
 }

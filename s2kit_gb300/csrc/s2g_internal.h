@@ -96,6 +96,10 @@ inline int check_aligned16(std::initializer_list<const void*> ps) {
     return S2G_OK;
 }
 
+inline bool overlap(const void* a, size_t na, const void* b, size_t nb) {
+    return (uintptr_t)a < (uintptr_t)b + nb && (uintptr_t)b < (uintptr_t)a + na;
+}
+
 // Build / fetch device tables (cached per device, bw, cutoff); the caller gets a reference and
 // returns it with put_tables.  cutoff 0 gives the weights, nodes and twiddles of bw without any
 // Legendre table (fwd, inv and off null), for the on-the-fly family.
@@ -131,6 +135,7 @@ size_t f64_work_bytes(int bw, int batch, int data_format);
 // this path take the word as `dg`: with it they run there, on tables and scratch that the caller has readied
 // (dg_prepare, dg_scratch); null keeps them off it.
 bool dg_takes(int bw);
+int dg_chunk(int bw, int batch, int es);  // functions transformed at a time, es: 8 for FP64, 4
 size_t dg_work_bytes(int bw, int batch, bool two);  // two: the data have imaginary parts
 // Grows s to `need` bytes for the digit path; *yes false where that does not fit, or cannot be done under capture (as
 // dg_prepare for the tables), and the caller takes the other kernels, whose scratch may fit or be there.

@@ -327,3 +327,62 @@ def test_plans_of_several_threads_do_not_disturb_each_other():
     for t in threads:
         t.join()
     assert not errors, errors
+
+
+@pytest.mark.parametrize("kind,bw,nb", [("f64", 256, 70), ("real32", 20, 3000), ("real32", 16, 9), ("real32", 255, 140),
+                                        ("complex32", 255, 140), ("real32", 64, 9), ("f64", 40, 9), ("f64", 16, 9)])
+def test_results_may_overlap_what_they_are_made_from(kind, bw, nb):
+    """The coefficients in the first half of the samples' buffer, there and back: the same bits as apart."""
+    import torch
+    n, c, two = 4 * bw * bw, bw * bw, kind == "complex32"
+    dt = "float64" if kind == "f64" else "float32"
+    plan = api.Plan(bw, bw)
+
+    def fwd(g, h, rc, ic):
+        if kind == "f64":
+            plan.fst(g, None, rc, ic, nb, api.REAL)
+        elif two:
+            plan.fst_complex_f32(g, h, rc, ic, nb, api.PREC_BF16X3)
+        else:
+            plan.fst_real_f32(g, rc, ic, nb, api.PREC_BF16X3)
+
+    def inv(rc, ic, g, h):
+        if kind == "f64":
+            plan.inv_fst(rc, ic, g, None, nb, api.REAL)
+        elif two:
+            plan.inv_fst_complex_f32(rc, ic, g, h, nb, api.PREC_BF16X3)
+        else:
+            plan.inv_fst_real_f32(rc, ic, g, nb, api.PREC_BF16X3)
+
+    g, h = _cuda(nb, n, dtype=dt), _cuda(nb, n, dtype=dt)
+    rc, ic = (torch.empty(nb, c, dtype=g.dtype, device="cuda") for _ in range(2))
+    gi, hi = g.clone(), h.clone()
+    ri, ii = (gi.view(-1)[k * nb * c:(k + 1) * nb * c] for k in range(2))
+    fwd(g, h, rc, ic)
+    fwd(gi, hi, ri, ii)
+    torch.cuda.synchronize()
+    assert (ri == rc.view(-1)).all() and (ii == ic.view(-1)).all()
+    inv(rc, ic, g, h)
+    inv(ri, ii, gi, hi)
+    plan.sync_status()
+    assert (gi == g).all() and (not two or (hi == h).all())
+
+
+def test_group_results_may_overlap_what_they_are_made_from():
+    import torch
+    group = api.Group([16, 77, 20, 64, 16, 255, 20, 128, 17, 77, 16] * 4)
+    gt, ct = group.grid_total, group.coeff_total
+    g = _cuda(gt, dtype="float32")
+    rc, ic, back = (torch.empty(k, dtype=torch.float32, device="cuda") for k in (ct, ct, gt))
+    start = g.clone()
+    group.fst_inv(g, rc, ic, back)
+    buf = torch.empty(gt, dtype=torch.float32, device="cuda")
+    for _ in range(2):  # at once, then as the captured graph
+        buf.copy_(start)
+        ri, ii = buf[:ct], buf[(ct + 3) // 4 * 4:][:ct]
+        group.fst(buf, ri, ii)
+        torch.cuda.synchronize()
+        assert (ri == rc).all() and (ii == ic).all()
+        group.inv_fst(ri, ii, buf)
+        group.sync_status()
+        assert (buf == back).all()
