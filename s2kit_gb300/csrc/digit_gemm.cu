@@ -1,19 +1,24 @@
 // digit_gemm.cu -- FP64 transforms on the tensor cores.
 //
 // GB300 gives FP64 about 1.2 TFLOP/s and its FP16 tensor cores about 1900, so the FP64 path's two
-// contractions per direction (the row DFT and the Legendre transform) run as exact integer products:
+// contractions per direction (the row DFT and the Legendre transform) run as integer products:
 // every operand is a 55-bit fixed-point number relative to its row's (table) or column's (data)
 // largest value, written as seven balanced base-256 digits d in [-128, 127]; digits are exact in
-// FP16, their products and the FP32 sums of up to 2^24 / 2^14 of them are exact, and the digit
-// products of equal weight share one accumulator:
+// FP16, so are their products and FP32 sums up to 2^24, and the digit products of equal weight share one
+// accumulator:
 //     sum_k T_k x_k = sum_g 256^-g sum_{a+b=g} sum_k d_a(T_k) d_b(x_k),   g <= 6
 // (products of weight 256^-7 and below are under 2^-54 of the operands' scale and are left out; the
 // scheme is Ozaki, Ogita, Oishi and Rump's error-free matrix product, Numer. Algorithms 59 (2012)).
 // Leading digits may take up to 256 (FP16 holds them): a data value, folds included, has 56 bits up to
-// K = 256 and 54 beyond, a table value 54 to 56, as many as keep the leading group's bound K d_0 d'_0 at
-// 2^22 (dg_table_bits).  A group's sum is exact while at most 2^24: by these bounds group 0 and 1 always
-// are; the others pass 2^24 only where the low digits of table and data agree in sign over almost the
-// whole K range.
+// K = 256 and 54 beyond, a table value 54 to 56, as many as keep the leading group's bound K d_0 d'_0 near
+// 2^22 (at most 1.5 2^22, dg_table_bits).
+// Which sums stay below 2^24, and are exact, follows from the tables (the sum over a row's entries of |digit of the
+// table| times the data digits' bound, its largest over all rows), for any data whatever: up to bw 256 all groups (I2
+// at odd bandwidths above 200: 0 to 4), at bw 512 groups 0 to 3, at bw 511 and 1024 groups 0 and 1 and, but for I2
+// (1.1 2^24), group 2.  A group passes 2^24 where the digits of data and table agree in sign over most of K, and
+// then loses about two of its units for every 16 entries; in data not made for it, digits behind the first agree
+// by chance only, and the sums stay tens of times smaller.  Data made for a row of the forward Legendre table of m = 0
+// lose up to 1.0e-15 of sum |T x| at bw 512 (group 4) and 1.3e-12 at bw 1024 (group 3), where the FP64 kernels round at 1e-16.
 //
 // One MMA covers all data digits of a table digit: the data digits b = 0..6-a lie one after another
 // along N, so A = table digit a times B = [x_0 | ... | x_(6-a)] adds to the accumulator groups
@@ -1463,7 +1468,7 @@ static int dg_vbz(int bw, int prec) {
     return (two ? 51 : 52) + (dg_fold_layout(bw, false).n[two ? 0 : 4] <= 272 ? 2 : 0);
 }
 
-// Bits of a table value: the leading group, at most K 2^(vb - 48) 2^(tb - 48), stays near 2^22, so that the
+// Bits of a table value: the leading group, at most K 2^(vb - 48) 2^(tb - 48), stays below 1.5 2^22, so that the
 // sum in units of 2^8 of the last group's has 63 bits.  I2 (values up to 2/sqrt(2 pi), eight sums of
 // which each gives up kDgOutShift bits) keeps strictly below 2^22.
 static int dg_table_bits(int K, int vb, bool inv_rows) {

@@ -386,3 +386,42 @@ def test_group_results_may_overlap_what_they_are_made_from():
         group.inv_fst(ri, ii, buf)
         group.sync_status()
         assert (buf == back).all()
+
+
+@pytest.mark.parametrize("bw,group", [(256, 4), (256, 6), (512, 2), (512, 3), (1024, 1), (1024, 2)])
+def test_digits_that_agree_in_sign(bw, group):
+    """The digit products' accumulators are FP32: a group of digit products is exact up to 2^24, which these groups stay
+    below for any data.  Data made for one row of the forward Legendre table (l = 4, m = 0; rows of samples constant),
+    the digits of the latitudes chosen so that all products of the group agree in sign.  Allowed: the table's own
+    rounding, two units in the last place of each value."""
+    import torch
+    S, ld, l = 2 * bw, np.longdouble, 4
+    w = np.zeros(4 * bw)
+    api.GenerateWeightsForDLT(bw, w)
+    th = (np.arange(bw).astype(ld) * 2 + 1) * np.arctan(ld(1)) * 2 / S
+    x, prev, cur = np.cos(th), np.zeros(bw, ld), np.full(bw, np.sqrt(ld(0.5)))
+    for k in range(l):
+        d = ld(k + 1) ** 2
+        nxt = np.sqrt((2 * k + 3) * ld(2 * k + 1) / d) * x * cur
+        if k:
+            nxt -= np.sqrt((2 * k + 3) * ld(k) ** 2 / ((2 * k - 1) * d)) * prev
+        prev, cur = cur, nxt
+    row = cur * w[:bw] * np.sqrt(8 * np.arctan(ld(1))) / S
+    tb, vb = {256: (54, 56), 512: (55, 54), 1024: (54, 54)}[bw]  # bits of table and data values
+    u = np.ldexp(row.astype(float), tb - np.frexp(float(np.abs(row).max()))[1])
+    u = np.rint(u).astype(np.int64) + 0x0000808080808080
+    T = [u >> 48] + [((u >> (8 * (6 - b))) & 255) - 128 for b in range(1, 7)]
+    v, s = np.zeros(bw, np.int64), 0
+    for b in range(group + 1):
+        digit = np.where(T[group - b] >= 0, 1, -1) * (2 ** (vb - 48) - 1 if b == 0 else 127)
+        v += digit << (8 * (6 - b))
+        s += int((digit * T[group - b]).sum())
+    assert 2 ** 22 < s < 2 ** 24  # the group's sum
+    samples = np.repeat(np.concatenate([v, v[::-1]]).astype(float)[:, None], S, 1) * 2.0 ** -vb
+    plan = api.Plan(bw, bw)
+    rc, ic = (torch.empty(1, bw * bw, dtype=torch.float64, device="cuda") for _ in range(2))
+    plan.fst(torch.from_numpy(samples).cuda(), None, rc, ic, 1, api.REAL)
+    plan.sync_status()
+    X = v.astype(ld) * ld(2.0) ** -vb * (2 * S)
+    e = abs(ld(rc[0, int(harmonic_index(0, l, bw))].item()) - (row * X).sum())
+    assert e <= 2.0 ** -51 * float((np.abs(row) * np.abs(X)).sum())
