@@ -548,8 +548,8 @@ int s2g_group_create(s2g_group* out, int nfunc, const int* bw, int precision) {
         for (auto& c : g->cls) {
             any |= c.dg;
             total += 2 * rnd(sizeof(int64_t) * c.N);
-            total += c.dg ? rnd(dg32_work_bytes(c.B, c.N, false))
-                          : rnd(sizeof(float) * x_floats(c)) + rnd(sizeof(float) * c_floats(c));
+            if (c.dg) total += rnd(dg32_work_bytes(c.B, c.N, false));
+            else if (!c.small) total += rnd(sizeof(float) * x_floats(c)) + rnd(sizeof(float) * c_floats(c));
         }
         if (!(any && dg_no_scratch()) && cudaMalloc(&g->mem, total) == cudaSuccess) break;
         g->mem = nullptr;
@@ -572,7 +572,7 @@ int s2g_group_create(s2g_group* out, int nfunc, const int* bw, int precision) {
             if (c.dg) {
                 c.digits = p;
                 p += rnd(dg32_work_bytes(c.B, c.N, false));
-            } else {
+            } else if (!c.small) {
                 c.buf0 = (float*)p;
                 p += rnd(sizeof(float) * x_floats(c));
                 c.buf1 = (float*)p;
@@ -599,7 +599,7 @@ int s2g_group_create(s2g_group* out, int nfunc, const int* bw, int precision) {
     }
     // operands packed now, so that no later call allocates (a graph capture cannot)
     for (auto& c : g->cls)
-        if (r == S2G_OK) r = split_prepare(c.t, precision);
+        if (r == S2G_OK && !c.dg) r = split_prepare(c.t, precision);
     if (r != S2G_OK) {
         group_free(g);
         return r;

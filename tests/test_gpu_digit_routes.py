@@ -425,3 +425,13 @@ def test_digits_that_agree_in_sign(bw, group):
     X = v.astype(ld) * ld(2.0) ** -vb * (2 * S)
     e = abs(ld(rc[0, int(harmonic_index(0, l, bw))].item()) - (row * X).sum())
     assert e <= 2.0 ** -51 * float((np.abs(row) * np.abs(X)).sum())
+
+
+def test_groups_of_classes_transformed_whole_hold_no_intermediates():
+    import torch
+    api.Group([16, 20])  # tables
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    group = api.Group([16] * 8192 + [20] * 4096)  # samples: 58 MB
+    assert free - torch.cuda.mem_get_info()[0] <= 4 * 2 ** 21
+    del group
