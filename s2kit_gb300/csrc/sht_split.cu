@@ -1017,7 +1017,6 @@ __global__ void __launch_bounds__(256, StageOcc<WHICH, RMAX>::v) k_stage_group(c
     const StageCls& k = a.c[ci];
     const int vb = (int)blockIdx.x - k.blk0;
     switch (k.R) {
-        case 1: stage_body<WHICH, 1>(k, vb); break;
         case 2: stage_body<WHICH, 2>(k, vb); break;
         case 4: stage_body<WHICH, 4>(k, vb); break;
         case 8:
@@ -2543,7 +2542,6 @@ static int fft_kernels(int which, int B, const void* in, void* out, int N, const
     }
     if ((2 * B) % 32) return fail(S2G_ERR_UNSUPPORTED, "no warp FFT for bandwidth %d", B);
     switch (2 * B / 32) {
-        case 1: return launch_fft_kernels<1>(which, in, out, N, s, st, scale, gmap);
         case 3: return launch_fft_kernels<3>(which, in, out, N, s, st, scale, gmap);
         case 5: return launch_fft_kernels<5>(which, in, out, N, s, st, scale, gmap);
         case 6: return launch_fft_kernels<6>(which, in, out, N, s, st, scale, gmap);
@@ -2567,7 +2565,6 @@ static int fft_kernels(int which, int B, const void* in, void* out, int N, const
 
 static size_t fft_smem_rt(int R, int which) {
     switch (R) {
-        case 1: return fft_smem<1>(which);
         case 2: return fft_smem<2>(which);
         case 4: return fft_smem<4>(which);
         case 8: return fft_smem<8>(which);
