@@ -528,7 +528,7 @@ bool split_czt(int bw) {
 }
 
 int czt_len(int bw) {
-    int M = 128;
+    int M = 256;
     while (M < 4 * bw - 1) M <<= 1;
     return M;
 }
@@ -597,7 +597,6 @@ int czt_stage(int which, const CztTabs& g, const void* in, void* out, int N, flo
               cudaStream_t st) {
     if (which < 0 || which > 3) return fail(S2G_ERR_ARG, "stage %d", which);
     switch (g.M) {
-        case 128: return czt_launch<4>(which, g, in, out, N, scale, gmap, st);
         case 256: return czt_launch<8>(which, g, in, out, N, scale, gmap, st);
         case 512: return czt_launch<16>(which, g, in, out, N, scale, gmap, st);
         case 1024: return czt_launch<32>(which, g, in, out, N, scale, gmap, st);

@@ -215,7 +215,7 @@ SplitLayout split_layout(int bw);
 // True where the split path's length-2bw DFTs run as chirp-z transforms (czt_split.cu): bw in
 // [17, 256] and 2bw not a warp-FFT length.
 bool split_czt(int bw);
-// Length M of the chirp-z convolution at bandwidth bw: the power of two >= 4 bw - 1 (at least 128).
+// Length M of the chirp-z convolution at bandwidth bw, from 33 on (below, small_takes): the power of two >= 4 bw - 1.
 int czt_len(int bw);
 // Device tables of one chirp-z bandwidth (the first three from czt_build_tables, the rest the
 // split path's FP32 weights, sin(theta) and DCT twiddles).

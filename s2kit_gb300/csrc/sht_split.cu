@@ -428,7 +428,7 @@ static int build_split(Tables* t) {
         }
         ck(cudaGetLastError(), "conversion kernels");
     }
-    if (r == S2G_OK && split_czt(B)) {
+    if (r == S2G_OK && split_czt(B) && !small_takes(B)) {
         r = czt_build_tables(B, &s->czh, &s->czK, &s->cztw);
         if (r == S2G_OK) s->czM = czt_len(B);
     }
