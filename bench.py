@@ -658,9 +658,10 @@ def large_bw1024_bench(api, torch, stream, seed):
             "fp64_fwd_inv_per_s": N / (ms64 / 1e3), "refined_fwd_per_s": N / (msr / 1e3),
             "split_fwd_err_vs_fp64": e_split, "refined_fwd_err_vs_fp64": e_ref,
             "fly_fp64_fwd_inv_per_s": N / (msf / 1e3), "fly_device_mib": fly_mib, "fly_err_vs_memo_fp64": e_fly,
-            "fly_note": "on-the-fly plan: Legendre recurrence inside the contraction kernels, no table "
-                        "(the memo tables of bw 1024 take 2 x 1.37 GiB); its device memory is the row-DFT "
-                        "workspace of the 16 functions (2 x 1024 x 2048 doubles each)"}
+            "refined_note": "the refined calls are the FP64 transforms themselves where the digit tables are there",
+            "fly_note": "on-the-fly plan: keeps no Legendre table (the memo tables of bw 1024 take 2 x 1.37 GiB, "
+                        "their digits 14.4 GiB); its device memory is DFT tables, recurrence values and scratch, in "
+                        "which batches generate digit tables a few orders at a time"}
 
 
 def group_bench(api, torch, stream, steps, warmup, seed):

@@ -174,19 +174,26 @@ typedef struct s2g_plan_s* s2g_plan;
  * seminaive/naive cutoff (1 <= cutoff <= bw).  Tables are generated on the current device
  * (FP64 recurrence and DCT, cospml.c:161-242) and shared by every plan with the same
  * (device, bw, cutoff).  A plan owns scratch buffers and streams: use it from one host thread at
- * a time (one plan per thread for concurrent callers; the tables stay shared). */
+ * a time (one plan per thread for concurrent callers; the tables stay shared).
+ * The first FP64 or refined transform or convolution of bw 9 to 1024 (not 16) builds digit tables of 14 bw^3 bytes
+ * beside them, generated from bw alone, also where the plan's tables came from a file (bw 256: 0.25 GiB and 2 ms, bw
+ * 512: 1.9 GiB and 10 ms, bw 1024: 14.4 GiB and 160 ms); the first FP32 transform at a chirp-z bandwidth from 64 on, 6
+ * bw^3 bytes.  They stay as long as the tables (s2g_cache_clear).  Where they, or the scratch of a call on them, do
+ * not fit in device memory, the call runs, slower, on the kernels that need neither. */
 int s2g_plan_create(s2g_plan* plan, int bw, int cutoff);
 int s2g_plan_destroy(s2g_plan plan);
 /* A plan for the on-the-fly family (src/FST_semi_fly.c, as the Fly drop-ins above): it holds no
- * Legendre table, only weights, twiddles, DFT tables and per (order, node) values.  s2g_fst,
- * s2g_inv_fst, s2g_fzt and s2g_conv on it run without one: single functions through kernels that
- * run the recurrence themselves, batches through tables generated a few orders at a time in the
- * plan's scratch (64 to 384 MiB by bandwidth); the split-precision entry points reject it
- * (S2G_ERR_ARG). */
+ * Legendre table, only weights, twiddles and, for batches, DFT tables and 24 bw^2 bytes of recurrence values.
+ * s2g_fst, s2g_inv_fst, s2g_fzt and s2g_conv run on it: single functions, s2g_fzt and s2g_conv through kernels
+ * that run the recurrence themselves; s2g_fst and s2g_inv_fst of bw 64 to 1024 with two real fields or more (above bw
+ * 512 four; COMPLEX data are two) through tables generated a few orders at a time in the plan's scratch (64 to 384 MiB
+ * of digits by bandwidth and 0.6 times that for the recurrence, see s2g_plan_workspace_size), or as single functions
+ * where that does not fit.  The split-precision entry points reject it (S2G_ERR_ARG). */
 int s2g_plan_create_fly(s2g_plan* plan, int bw);
 /* Device bytes of scratch that a transform or a convolution of this batch on device buffers takes at most, COMPLEX data
  * included (precision S2G_PREC_FP64: s2g_fst, s2g_inv_fst, s2g_conv; else the FP32 ones).  The plan grows its own scratch
- * on demand, by an eighth more than the call needs; what does not fit runs on other kernels with less, where there are some. */
+ * on demand, by an eighth more than the call needs; what does not fit runs on other kernels with less, where there are some.  Refined calls that
+ * fall back to the refinement, and copies of inputs that results overlap, come on top. */
 size_t s2g_plan_workspace_size(s2g_plan plan, int batch, int precision);
 
 /* Batched FP64 transforms on device pointers.  Function f of the batch uses

@@ -14,7 +14,8 @@
 // angle is formed, so the chirp is exact to FP64 rounding at every n.
 //
 // From bw 64 on the digit products of digit_gemm.cu take these bandwidths, below 32 the kernels of small32.cuh;
-// the stages here serve 33 to 63, and any above where the digit tables are not there (first call under capture, out of memory).
+// the stages here serve 33 to 63, and any above where
+// the digit tables or their scratch are not there (out of memory, or nothing may be allocated under capture).
 //
 // The four stage kernels compute what the warp-FFT stage kernels of sht_split.cu compute
 // (FST_semi_memo.c:81-90 and 334-350 for the longitude DFTs, seminaive.c:161-176 and 105-114 for

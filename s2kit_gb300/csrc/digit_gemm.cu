@@ -1814,7 +1814,10 @@ static int launch_dg_nt(const DgArgs& p, int sms, cudaStream_t st) {
 }
 
 // Columns per item.  While one wave of blocks holds them all, more and smaller items are faster (bw 64, one
-// function: F1 16.4 us at 64 columns, 11.2 at 16).  Beyond one wave, FP64: 64 columns take one accumulator (7 x 64
+// function: F1 16.4 us at 64 columns, 11.2 at 16); and up to 64 columns in all are one item a tile even beyond one
+// wave.  (For 33 to 64 columns of F2 and I1 that is the better choice for the fewest, 17 fields at bw 512: I1 280 us,
+// 307 at 32; not for the most: 32 fields at bw 101, F2 30.6 and 24.5, at bw 256 75.7 and 69.6, I1 75.7 and 71.6.)
+// More than 64 columns beyond one wave, FP64: 64 columns take one accumulator (7 x 64
 // TMEM columns) whose epilogue the next item's MMAs wait for (F1 at bw 256: 44% of the time), 32 take two by
 // turns, but seven dependent MMAs of about 115 cycles for each 16-deep K step where 64 take ten for twice the
 // columns.  So 64 is for the long K

@@ -1,12 +1,14 @@
 // refine.cu -- split-precision transforms with one FP64-residual refinement step.
 //
 // The step was made when an FP64 transform cost many times a split one.  With the digit products it costs
-// less than the residual's FP64 transform and the two split ones together, and it is the more precise, so where
-// the digit tables are there (and at the bandwidths that never take them) the refined transforms are FP64
-// transforms (refined_scratch, capi.cu): forward at bw 1024, 16 functions, 4.74 -> 2.97 ms with the coefficients'
-// error against 64 bits 8.0e-14 -> 5.2e-14, inverse 5.43 -> 2.65 ms and 1.5e-7 -> 5.1e-15; one function at bw
-// 16, on the FP64 kernels, 48 -> 18 us.  The step below serves the rest: a first call under capture, or tables or
-// scratch that did not fit (FP64 kernels, one function at bw 1024: forward 7.1 ms, refined 3.8).
+// less than the residual's FP64 transform and the two split ones together, so where the digit tables and their
+// scratch are there (and at the bandwidths that never take them) the refined transforms are FP64 transforms
+// (refined_scratch, capi.cu): forward at bw 1024, 16 functions, 2.76 ms, where the step took 4.7 with its residual on
+// the digit products and takes 27.8 without them; inverse 2.66 and 23.1 ms.  Errors there, max |error| over the
+// function's largest value, worst function, smooth fields, against 64 bits: coefficients 2.3e-13 (rms 9.6e-14; the
+// step 2.0e-13, rms 1.4e-13: both are the seminaive rounding of the orders 1, 3 and 5), samples 9.6e-14 (the step
+// 5.9e-7); at bw 256 3.7e-16 and 6.1e-15 (7.0e-14 and 4.4e-7).  One function at bw 16, on the FP64 kernels, 48 -> 18
+// us.  The step serves the rest: tables or scratch that do not fit, or cannot be made under capture.
 //
 // Forward:  a1 = F_split(f);  r = f - I_fp64(a1);  a = a1 + F_split(r)
 // Inverse:  g1 = I_split(a);  r = a - F_fp64(g1);  g = g1 + I_split(r)
