@@ -1777,6 +1777,7 @@ static int dg_get(int bw, int prec, bool fly, int semi, const double* weights, D
         *out = it->second;
         return S2G_OK;
     }
+    const RelaxCapture relax;  // the first call that takes this path may not be the plan's first
     DgTabs* d = new DgTabs();
     d->device = dev;
     d->bw = bw;
@@ -2010,6 +2011,7 @@ int dg_scratch(Scratch& s, size_t need, cudaStream_t st, bool* yes) {
         }
         if (capturing(st)) return S2G_OK;
     }
+    const RelaxCapture relax;
     const int r = s.ensure(need, st);
     if (r == S2G_ERR_NOMEM) {
         cudaGetLastError();

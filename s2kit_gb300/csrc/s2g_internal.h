@@ -75,6 +75,14 @@ struct Tables {
 // Whether st is being captured (or, for the legacy stream, another one).
 bool capturing(cudaStream_t st);
 
+// While it lives, this thread may allocate although another captures a graph in the global mode, whose capture the
+// allocation would otherwise end (and the call fail).  Not for a stream that is itself captured.
+struct RelaxCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // Device scratch owned by a plan; grown on demand.  A buffer handed to a captured call lives as long as the plan:
 // the graph has its address, and calls of other kinds at the same batch may need more of it.
 struct Scratch {

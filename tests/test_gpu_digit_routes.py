@@ -435,3 +435,39 @@ def test_groups_of_classes_transformed_whole_hold_no_intermediates():
     group = api.Group([16] * 8192 + [20] * 4096)  # samples: 58 MB
     assert free - torch.cuda.mem_get_info()[0] <= 4 * 2 ** 21
     del group
+
+
+def test_first_digit_call_while_another_thread_captures():
+    """A plan whose scratch is there allocates nothing in its FP64 calls but for the digit tables and their scratch: that
+    neither fails nor ends a capture of another thread."""
+    import threading
+
+    import torch
+    bw, nb = 53, 4
+    grid, oc = _cuda(nb, 4 * bw * bw), [_cuda(nb, bw * bw) for _ in range(2)]
+    plan = api.Plan(bw, bw)
+    plan.fzt(grid, None, *oc, nb, api.REAL)
+    torch.cuda.synchronize()
+    x, s, errors = torch.ones(1000, device="cuda"), torch.cuda.Stream(), []
+
+    def worker():
+        try:
+            plan.fst(grid, None, *oc, nb, api.REAL, stream=s)
+        except Exception as e:  # noqa: BLE001
+            errors.append(repr(e))
+
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, capture_error_mode="global"):
+        x.mul_(2.0)
+        t = threading.Thread(target=worker)
+        t.start()
+        t.join()
+    assert not errors, errors
+    graph.replay()
+    torch.cuda.synchronize()
+    plan.sync_status()
+    assert (x == 2.0).all()
+    first = [c.clone() for c in oc]
+    plan.fst(grid, None, *oc, nb, api.REAL)
+    plan.sync_status()
+    assert (oc[0] == first[0]).all() and (oc[1] == first[1]).all()
